@@ -28,7 +28,8 @@ ORACLE_BIN = os.path.join(ORACLE, "_bin")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
                      "-I" + os.path.join(ROOT, "include")]
-CUDA_SOURCES = ["gp_api.cu", "gp_geno.cu", "gp_gram_f64.cu", "gp_geno_gemm_f64.cu",
+CUDA_SOURCES = ["gp_api.cu", "gp_geno.cu", "gp_gram_f64.cu", "gp_gram_exact.cu",
+                "gp_geno_gemm_f64.cu",
                 "gp_gram_bf16.cu", "gp_fast.cu",
                 "gp_noalloc.cu", "gp_geno_tc.cu", "gp_eig.cu", "gp_serve.cu", "gp_convert.cu",
                 "gp_fst.cu", "gp_popfill.cu"]

@@ -331,17 +331,30 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
 
   GP_CUDA(ctx, cudaEventRecord(ctx->ev_g0, ctx->stream));
   ctx->gram_launches = 0;
-  if (opts->precision == GP_PREC_FP64)
-    rc = gp_gram_fp64(ctx);
-  else
+  /* FP64: exact integer sums on the tensor cores.  usepopsformissing's filled values are no
+   * linear function of the genotype and keep the FP64-pipe kernel, which also takes over when
+   * the device has no room for the digits of one block of SNPs. */
+  bool symmetric = false;
+  if (opts->precision != GP_PREC_FP64) {
     rc = gp_gram_split(ctx, opts->precision);
+  } else {
+    rc = GP_ERR_NOMEM;
+    if (ctx->npop == 0 && ctx->nkept > 0) {
+      rc = gp_gram_exact(ctx);
+      symmetric = rc == GP_OK;
+    }
+    if (rc == GP_ERR_NOMEM) {
+      cudaGetLastError();
+      rc = gp_gram_fp64(ctx);
+    }
+  }
   if (rc) return rc;
   GP_CUDA(ctx, cudaEventRecord(ctx->ev_g1, ctx->stream));
 
   double *d_tr;
   rc = gp_scratch(ctx, sizeof(double), (void **)&d_tr);
   if (rc) return rc;
-  rc = gp_launch_symmetrize_trace(ctx, d_tr);
+  rc = gp_launch_symmetrize_trace(ctx, d_tr, symmetric);
   if (rc) return rc;
   double tr = 0.0;
   GP_CUDA(ctx, gp_memcpy(ctx, &tr, d_tr, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

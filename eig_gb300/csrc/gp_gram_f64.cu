@@ -1,13 +1,14 @@
 /*
- * Plain FP64 Gram (the drop-in precision): XTX[i][j] = sum over kept SNPs of v_i v_j for the
+ * Plain FP64 Gram on the FP64 pipe: XTX[i][j] = sum over kept SNPs of v_i v_j for the
  * lower-triangle 64x64 tiles, replacing domult_increment_lookup / block_increment_binary
  * (src/eigensrc/smartpca.c:3361-3495) and domult_increment_normal (:3498-3561).
  *
  * The normalised values are never materialised: each k-step decodes a 64-row x 16-SNP tile
  * straight from the packed 2-bit records through the per-SNP value table (the 3-entry
  * tblock of the reference + 0 for missing).  The FP64 FMA pipe bounds this kernel (GB300's
- * FP64 rate is low by design); it is the parity baseline the split-BF16 path is measured
- * against.  When the triangle has fewer tiles than the GPU has SMs the SNP range is split
+ * FP64 rate is low by design), so it runs only where the exact tensor-core sums of
+ * gp_gram_exact.cu do not apply: with usepopsformissing, or without device memory for them
+ * (2,003 samples x 120,011 SNPs: 485 ms here).  When the triangle has fewer tiles than the GPU has SMs the SNP range is split
  * and the partial triangles are summed in a fixed order (deterministic).
  * With usepopsformissing (fill != NULL) a missing genotype of row i takes the value
  * fill[c*npop + rowpop[i]] of its population (0 for a row without one), the getcolxz values
@@ -153,8 +154,8 @@ __global__ void k_reduce_splits(double *out, const double *part, int32_t nsplit,
   }
 }
 
-/* copy the lower triangle to the upper one and sum the diagonal */
-__global__ void k_symmetrize(double *x, int32_t n, double *trace_out)
+/* copy the lower triangle to the upper one */
+__global__ void k_mirror_lower(double *x, int32_t n)
 {
   int64_t total = (int64_t)n * n;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
@@ -162,18 +163,21 @@ __global__ void k_symmetrize(double *x, int32_t n, double *trace_out)
     int64_t i = idx / n, j = idx - i * n;
     if (j > i) x[i * n + j] = x[j * n + i];
   }
-  if (trace_out && blockIdx.x == 0) {
-    __shared__ double red[256];
-    double s = 0.0;
-    for (int32_t i = threadIdx.x; i < n; i += blockDim.x) s += x[(int64_t)i * n + i];
-    red[threadIdx.x] = s;
+}
+
+/* the sum of the diagonal, one CTA of 256, fixed order */
+__global__ void k_trace(const double *x, int32_t n, double *trace_out)
+{
+  __shared__ double red[256];
+  double s = 0.0;
+  for (int32_t i = threadIdx.x; i < n; i += blockDim.x) s += x[(int64_t)i * n + i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = blockDim.x / 2; o; o >>= 1) {
+    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
-    for (int o = blockDim.x / 2; o; o >>= 1) {
-      if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) *trace_out = red[0];
   }
+  if (threadIdx.x == 0) *trace_out = red[0];
 }
 
 int gp_gram_fp64(gp_ctx *ctx)
@@ -228,13 +232,17 @@ int gp_gram_fp64(gp_ctx *ctx)
   return GP_OK;
 }
 
-int gp_launch_symmetrize_trace(gp_ctx *ctx, double *d_trace)
+int gp_launch_symmetrize_trace(gp_ctx *ctx, double *d_trace, bool symmetric)
 {
-  int64_t total = (int64_t)ctx->nrows * ctx->nrows;
-  int blocks = (int)((total + 255) / 256);
-  if (blocks > ctx->num_sms * 16) blocks = ctx->num_sms * 16;
-  if (blocks < 1) blocks = 1;
-  k_symmetrize<<<blocks, 256, 0, ctx->stream>>>(ctx->d_xtx, ctx->nrows, d_trace);
-  GP_LAUNCH_CHECK(ctx, "k_symmetrize");
+  if (!symmetric) {
+    int64_t total = (int64_t)ctx->nrows * ctx->nrows;
+    int blocks = (int)((total + 255) / 256);
+    if (blocks > ctx->num_sms * 16) blocks = ctx->num_sms * 16;
+    if (blocks < 1) blocks = 1;
+    k_mirror_lower<<<blocks, 256, 0, ctx->stream>>>(ctx->d_xtx, ctx->nrows);
+    GP_LAUNCH_CHECK(ctx, "k_mirror_lower");
+  }
+  k_trace<<<1, 256, 0, ctx->stream>>>(ctx->d_xtx, ctx->nrows, d_trace);
+  GP_LAUNCH_CHECK(ctx, "k_trace");
   return GP_OK;
 }

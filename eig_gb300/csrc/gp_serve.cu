@@ -770,7 +770,12 @@ extern "C" int64_t gp_smartpca_footprint(int32_t nind, int64_t nsnp, int32_t pre
                       8 * (nt * (nt + 1) / 2 * 64 * 64 + 27 * nt * 64 + 3 * nt) + 5 * nt * nt;
   int64_t work;
   if (precision == GP_PREC_FP64) {
-    work = 8 * m * (k * (k + 1) / 2 + 1) + 8 * n * 256;
+    /* lsqproject's panel of pair products, or the exact Gram: its right operand (20 bytes per
+     * genotype, at most 2 GiB at a time), integer sums and sample-major codes */
+    int64_t slices = 20 * (n + 48) * (m + 64);
+    if (slices > (int64_t)2 << 30) slices = (int64_t)2 << 30;
+    work = 8 * m * (k * (k + 1) / 2 + 1) + 8 * n * 256 + slices + 8 * (n + 256) * (n + 304) +
+           npad * (m / 4 + 16);
   } else {
     int64_t split = 4 * npad * m;
     if (split > (int64_t)24 << 30) split = (int64_t)24 << 30;
