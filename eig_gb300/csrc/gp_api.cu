@@ -780,6 +780,61 @@ static size_t kept_tables_bytes(int32_t nk)
   return (b + 255) / 256 * 256;
 }
 
+/* Whether the products of weights and lsqproject run on the tensor cores: always at the split
+ * precisions; at FP64 with 12-bit slices, except after a pass with population fill (its SNP
+ * weights take the observed genotypes' table, which is not g fancy - xmean) and for records
+ * longer than the SNP-major code builder stages in shared memory. */
+static int tc_products(const gp_ctx *ctx, int32_t nk)
+{
+  if (nk < 1) return 0;
+  if (ctx->precision != GP_PREC_FP64) return 1;
+  return ctx->npop == 0 && ctx->rlen_dev <= 200 * 1024;
+}
+static int tc_digits(const gp_ctx *ctx) { return ctx->precision == GP_PREC_FP64 ? 5 : 4; }
+
+static int grid16(const gp_ctx *ctx, int64_t work)
+{
+  const int64_t b = (work + 255) / 256;
+  return (int)(b < ctx->num_sms * 16 ? b : ctx->num_sms * 16);
+}
+
+/* ffvT [nk][K] = fancy (G^T W) - xmean (O^T W) */
+static int weights_tc(gp_ctx *ctx, const kept_tables *kt, const double *d_W, int32_t K, double *d_ffvT)
+{
+  const int32_t n = ctx->nrows, nk = ctx->nkept;
+  double *d_yg;
+  int rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&d_yg);
+  if (rc) return rc;
+  double *d_yo = d_yg + (size_t)nk * K;
+  gp_tc_codes A;
+  rc = gp_tc_codes_for(ctx, 0, ctx->d_rows, n, kt->snprec, nk, &A);
+  if (rc) return rc;
+  gp_tc_panel pw = {d_W, K, 1.0, 1};
+  rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pw, K, tc_digits(ctx), d_yg, K);
+  if (rc) return rc;
+  pw.count = 0;
+  rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pw, K, tc_digits(ctx), d_yo, K);
+  if (rc) return rc;
+  k_combine_gx<<<grid16(ctx, (int64_t)nk * K), 256, 0, ctx->stream>>>(
+      d_ffvT, d_yg, d_yo, ctx->d_kept, ctx->d_xfancy, ctx->d_xmean, nk, K);
+  GP_LAUNCH_CHECK(ctx, "k_combine_gx");
+  return GP_OK;
+}
+
+/* Y [rows][K] = G (fancy w) - O (xmean w) for a panel w [nk][K]: the fixxrow products */
+static int scores_tc(gp_ctx *ctx, const gp_tc_codes *A, const double *d_w, int32_t K, double *d_Y)
+{
+  const int32_t nk = ctx->nkept;
+  double *tmp;
+  int rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&tmp);
+  if (rc) return rc;
+  k_scale_rows2<<<grid16(ctx, (int64_t)nk * K), 256, 0, ctx->stream>>>(
+      tmp, tmp + (size_t)nk * K, d_w, ctx->d_kept, ctx->d_xfancy, ctx->d_xmean, nk, K);
+  GP_LAUNCH_CHECK(ctx, "k_scale_rows2");
+  gp_tc_panel pr[2] = {{tmp, K, 1.0, 1}, {tmp + (size_t)nk * K, K, -1.0, 0}};
+  return gp_geno_panel_tc_codes(ctx, A, 2, pr, K, tc_digits(ctx), d_Y, K);
+}
+
 extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, double *fxvecs,
                               double *fxscal)
 {
@@ -808,28 +863,19 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   if (blocks > ctx->num_sms * 16) blocks = ctx->num_sms * 16;
   k_fvecs_T<<<blocks, 256, 0, ctx->stream>>>(d_B, ctx->d_evecs, n, K);
   GP_LAUNCH_CHECK(ctx, "k_fvecs_T");
-  if (ctx->precision != GP_PREC_FP64 && nk > 0) {
+  int tc = tc_products(ctx, nk);
+  if (tc) {
     /* tensor-core exact products: X = G fancy - O xmean, so
      * ffvecs^T = fancy (G^T W) - xmean (O^T W) with W = 10 evecs^T over the rows */
-    double *tmp;
-    rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&tmp);
-    if (rc) return rc;
-    double *d_yg = tmp, *d_yo = tmp + (size_t)nk * K;
-    gp_tc_codes A;
-    rc = gp_tc_codes_for(ctx, 0, ctx->d_rows, n, kt.snprec, nk, &A);
-    if (rc) return rc;
-    gp_tc_panel pw = {d_B, K, 1.0, 1};
-    rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pw, K, d_yg, K);
-    if (rc) return rc;
-    pw.count = 0;
-    rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pw, K, d_yo, K);
-    if (rc) return rc;
-    int b3 = (int)(((int64_t)nk * K + 255) / 256);
-    if (b3 > ctx->num_sms * 16) b3 = ctx->num_sms * 16;
-    k_combine_gx<<<b3, 256, 0, ctx->stream>>>(d_ffvT, d_yg, d_yo, ctx->d_kept, ctx->d_xfancy,
-                                             ctx->d_xmean, nk, K);
-    GP_LAUNCH_CHECK(ctx, "k_combine_gx");
-  } else {
+    rc = weights_tc(ctx, &kt, d_B, K, d_ffvT);
+    if (rc == GP_ERR_NOMEM && ctx->precision == GP_PREC_FP64) {
+      cudaGetLastError();
+      tc = 0;
+    } else if (rc) {
+      return rc;
+    }
+  }
+  if (!tc) {
     /* ffvecs^T[k][j] = sum_r v(r,k) * 10 evec_j[r] */
     rc = gp_geno_gemm_f64(ctx, 0, ctx->d_rows, n, kt.snprec, kt.vt, nk, d_B, K, K, d_ffvT, K);
     if (rc) return rc;
@@ -842,19 +888,18 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
     GP_LAUNCH_CHECK(ctx, "k_scatter_ffvecs");
   }
   /* fxvecs^T[i][j] = xrow_i . ffvecs_j  (fixxrow values g fancy - xmean) */
-  if (ctx->precision != GP_PREC_FP64 && nk > 0) {
-    double *tmp;
-    rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&tmp);
-    if (rc) return rc;
-    int b3 = (int)(((int64_t)nk * K + 255) / 256);
-    if (b3 > ctx->num_sms * 16) b3 = ctx->num_sms * 16;
-    k_scale_rows2<<<b3, 256, 0, ctx->stream>>>(tmp, tmp + (size_t)nk * K, d_ffvT, ctx->d_kept,
-                                              ctx->d_xfancy, ctx->d_xmean, nk, K);
-    GP_LAUNCH_CHECK(ctx, "k_scale_rows2");
-    gp_tc_panel pr[2] = {{tmp, K, 1.0, 1}, {tmp + (size_t)nk * K, K, -1.0, 0}};
-    rc = gp_geno_panel_tc(ctx, 1, ctx->d_rows, n, kt.snprec, nk, 2, pr, K, d_fxT, K);
-    if (rc) return rc;
-  } else {
+  if (tc) {
+    gp_tc_codes A;
+    rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, kt.snprec, nk, &A);
+    if (!rc) rc = scores_tc(ctx, &A, d_ffvT, K, d_fxT);
+    if (rc == GP_ERR_NOMEM && ctx->precision == GP_PREC_FP64) {
+      cudaGetLastError();
+      tc = 0;
+    } else if (rc) {
+      return rc;
+    }
+  }
+  if (!tc) {
     rc = gp_geno_gemm_f64(ctx, 1, ctx->d_rows, n, kt.snprec, kt.rt, nk, d_ffvT, K, K, d_fxT, K);
     if (rc) return rc;
   }
@@ -1054,7 +1099,8 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
     GP_LAUNCH_CHECK(ctx, "k_build_EP");
   }
   /* masked normal equations: co = O P (pair sums + observed count), rr = R E */
-  if (ctx->precision != GP_PREC_FP64 && nk > 0) {
+  int tc = d_raw ? 0 : tc_products(ctx, nk);
+  if (tc) {
     gp_tc_codes A;
     /* projecting exactly the analysis rows: the product can reuse their codes */
     const int32_t *d_list = d_samp;
@@ -1062,22 +1108,17 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
         memcmp(samples, ctx->h_rows, sizeof(int32_t) * (size_t)nproj) == 0)
       d_list = ctx->d_rows;
     rc = gp_tc_codes_for(ctx, 1, d_list, nproj, kt.snprec, nk, &A);
-    if (rc) return rc;
     gp_tc_panel pc = {d_P, ldp, 1.0, 0};
-    rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pc, ldp, d_co, ldp);
-    if (rc) return rc;
-    double *tmp;
-    rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&tmp);
-    if (rc) return rc;
-    int b3 = (int)(((int64_t)nk * K + 255) / 256);
-    if (b3 > ctx->num_sms * 16) b3 = ctx->num_sms * 16;
-    k_scale_rows2<<<b3, 256, 0, ctx->stream>>>(tmp, tmp + (size_t)nk * K, d_E, ctx->d_kept,
-                                              ctx->d_xfancy, ctx->d_xmean, nk, K);
-    GP_LAUNCH_CHECK(ctx, "k_scale_rows2");
-    gp_tc_panel pr[2] = {{tmp, K, 1.0, 1}, {tmp + (size_t)nk * K, K, -1.0, 0}};
-    rc = gp_geno_panel_tc_codes(ctx, &A, 2, pr, K, d_rr, K);
-    if (rc) return rc;
-  } else if (d_raw) {
+    if (!rc) rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pc, ldp, tc_digits(ctx), d_co, ldp);
+    if (!rc) rc = scores_tc(ctx, &A, d_E, K, d_rr);
+    if (rc == GP_ERR_NOMEM && ctx->precision == GP_PREC_FP64) {
+      cudaGetLastError();
+      tc = 0;
+    } else if (rc) {
+      return rc;
+    }
+  }
+  if (d_raw) {
     /* usepopsformissing: a filled genotype counts as observed with its fixxrow value */
     rc = gp_geno_gemm_f64_fill(ctx, d_samp, d_spop, nproj, kt.snprec, kt.ot, d_of, npop, nk,
                                d_P, ldp, ldp, d_co, ldp);
@@ -1085,7 +1126,7 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
     rc = gp_geno_gemm_f64_fill(ctx, d_samp, d_spop, nproj, kt.snprec, kt.rt, d_rf, npop, nk,
                                d_E, K, K, d_rr, K);
     if (rc) return rc;
-  } else {
+  } else if (!tc) {
     rc = gp_geno_gemm_f64(ctx, 1, d_samp, nproj, kt.snprec, kt.ot, nk, d_P, ldp, ldp, d_co, ldp);
     if (rc) return rc;
     rc = gp_geno_gemm_f64(ctx, 1, d_samp, nproj, kt.snprec, kt.rt, nk, d_E, K, K, d_rr, K);

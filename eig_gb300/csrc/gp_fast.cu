@@ -515,10 +515,10 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
   for (int32_t it = 0; it <= I; ++it) {
     if (use_tc) {
       gp_tc_panel pg = {d_G, L, 1.0, 1};
-      rc = gp_geno_panel_tc_codes(ctx, &A_snp, 1, &pg, L, d_Y1, L);
+      rc = gp_geno_panel_tc_codes(ctx, &A_snp, 1, &pg, L, 4, d_Y1, L);
       if (rc) return rc;
       pg.count = 0;
-      rc = gp_geno_panel_tc_codes(ctx, &A_snp, 1, &pg, L, d_Y2, L);
+      rc = gp_geno_panel_tc_codes(ctx, &A_snp, 1, &pg, L, 4, d_Y2, L);
       if (rc) return rc;
       k_fast_combine_xg<<<grid_for_fast(ctx, (int64_t)nQ), 256, 0, ctx->stream>>>(
           d_Q, d_Y1, d_Y2, ctx->d_kept, ctx->d_xfancy, ctx->d_xmean, nk, L, INV_SQRT2);
@@ -558,7 +558,7 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
           d_Y1, d_Y2, d_Q, ctx->d_kept, ctx->d_xfancy, ctx->d_xmean, nk, L);
       GP_LAUNCH_CHECK(ctx, "k_fast_panels");
       gp_tc_panel pp[2] = {{d_Y1, L, 1.0, 1}, {d_Y2, L, -1.0, 0}};
-      rc = gp_geno_panel_tc_codes(ctx, &A_samp, 2, pp, L, d_Hp + ca, c4);
+      rc = gp_geno_panel_tc_codes(ctx, &A_samp, 2, pp, L, 4, d_Hp + ca, c4);
       if (rc) return rc;
     } else {
       rc = gp_geno_gemm_f64(ctx, 1, ctx->d_rows, n, d_snprec, d_vt, nk, d_Q, L, L, d_Hp + ca,

@@ -11,7 +11,12 @@
  * k values sums to an integer below 2^24, which FP32 holds exactly, so the FP32 accumulation
  * of the MMA loses nothing; chunk sums are added in int32 registers and flushed with FP64
  * atomics of exact integers (order-independent, hence deterministic).  The only error left
- * is the slicing, about 2^-41 of the column maximum.
+ * is the slicing, about 2^-41 of the column maximum: the split precisions' products.
+ *
+ * The FP64 precision's products take 5 slices of 12 bits (x = sum_t q_t 2^-(11 + 12 t),
+ * |q_t| <= 2048, at most 4,096 k values per chunk): an error of 2^-60 of the column maximum,
+ * below what FP64 additions in sequence leave, for 5/4 of the MMAs.  They replace the FP64
+ * pipe's products (1,501 x 80,003, K = 10, weights and lsqproject: 59.4 ms there, 2.5 here).
  *
  * This is how the masked per-sample normal equations of lsqproject (regressit
  * src/regsubs.c:19-26, lsqproj src/eigensrc/smartpca.c:4690-4712), the sample scores fxvecs
@@ -53,7 +58,6 @@
 #define X_THREADS 576       /* 18 warps */
 #define X_DEC_WARPS 8       /* decoder warps: two threads per row of the A tile */
 #define X_SMEM (XSTAGES * XSTAGE_BYTES + 1024 + 256)
-#define X_CHUNK_KB 128      /* 8,192 k per exact FP32 chunk */
 #define XPF 8               /* k-blocks of codes a decoder thread loads ahead */
 
 #define XERR_FULL 11
@@ -66,6 +70,12 @@
 #define H1 0x3C00ull
 #define H2 0x4000ull
 static const uint64_t LUT_MASK = H1 | (H1 << 16) | (H1 << 32);      /* {1,1,1,0} */
+/* k-blocks per exact FP32 chunk: 8,192 k with 10-bit slices, 4,096 with 12-bit ones; and the
+ * largest k range of a work item whose int32 sums cannot overflow */
+#define X_CHUNK_KB(digits) ((digits) == 5 ? 64 : 128)
+#define X_MAX_K(digits) ((digits) == 5 ? 1 << 18 : 1 << 19)
+/* columns of a panel cut and multiplied at a time with 5 slices */
+#define X_GROUP5 256
 static const uint64_t LUT_COUNT = H0 | (H1 << 16) | (H2 << 32);     /* {0,1,2,0} */
 
 __device__ __forceinline__ void fence_proxy_async_smem()
@@ -85,7 +95,7 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
                 int64_t ldc, const int32_t *__restrict__ row_map, int32_t nrows, int32_t ncols4,
                 int32_t nkb, int32_t kb_period,
                 int32_t kb_switch, uint64_t lut_lo, uint64_t lut_hi, int32_t ksplit,
-                double *zout, int64_t ldz, int *err, const gp_tc_batch *db)
+                int32_t chunk_kb, double *zout, int64_t ldz, int *err, const gp_tc_batch *db)
 {
   if (db) {
     /* a device-resident loop's batch: rows and their count are read at run time, and the
@@ -167,8 +177,8 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
       for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
         int32_t ks = (w / nrt) % ksplit;
         int32_t kb0 = ks * kb_per, kb1 = kb0 + kb_per < nkb ? kb0 + kb_per : nkb;
-        for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += X_CHUNK_KB, ++chunk) {
-          int32_t c1 = c0 + X_CHUNK_KB < kb1 ? c0 + X_CHUNK_KB : kb1;
+        for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += chunk_kb, ++chunk) {
+          int32_t c1 = c0 + chunk_kb < kb1 ? c0 + chunk_kb : kb1;
           uint32_t buf = chunk & 1u, use = chunk >> 1;
           if (!mbar_wait(&acce[buf], (use & 1u) ^ 1u, abort_flag, err, XERR_ACCE)) {
             ok = false;
@@ -277,7 +287,7 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
       int32_t acc[64];
 #pragma unroll
       for (int u = 0; u < 64; ++u) acc[u] = 0;
-      for (int32_t c0 = kb0; c0 < kb1; c0 += X_CHUNK_KB, ++chunk) {
+      for (int32_t c0 = kb0; c0 < kb1; c0 += chunk_kb, ++chunk) {
         uint32_t buf = chunk & 1u, use = chunk >> 1;
         bool got = mbar_wait(&accf[buf], use & 1u, abort_flag, err, XERR_ACCF);
         if (!__all_sync(0xffffffffu, got)) {
@@ -474,63 +484,73 @@ __global__ void k_panel_absmax(const double *__restrict__ P, int64_t ldp, int32_
     if (smx[c]) atomicMax(mx + c, smx[c]);
 }
 
-/* exponent e_c with max|P| < 2^e_c (frexp), 0 for an all-zero column */
-__global__ void k_panel_expo(const unsigned long long *mx, int32_t ncols, int32_t *expo)
+/* exponent e_c with max|P| < 2^e_c (frexp), 0 for an all-zero column, X_NONFINITE for one with
+ * an infinity or NaN (5 slices: its products are NaN, as FP64 products of 0 and it are) */
+#define X_NONFINITE (-(1 << 30))
+__global__ void k_panel_expo(const unsigned long long *mx, int32_t ncols, int32_t *expo, int mark)
 {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols; c += gridDim.x * blockDim.x) {
     const double v = __longlong_as_double((long long)mx[c]);
     int e = 0;
     if (v > 0.0) frexp(v, &e); /* v = f 2^e, f in [0.5, 1) -> v < 2^e */
+    if (mark && mx[c] >= 0x7FF0000000000000ull) e = X_NONFINITE;
     expo[c] = e;
   }
 }
 
 /*
- * The four slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
- * narrow): N = rint(x 2^40) from the double's mantissa and exponent (round half to even),
- * then balanced base-1024 digits from the bottom, d_3, d_2, d_1 in [-512, 511] and
- * d_0 = the rest (|d_0| <= 1024 since |N| <= 2^40), so that x = sum_t d_t 1024^-(t+1) + O(2^-41).
+ * The slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
+ * narrow): N = rint(x 2^F) from the double's mantissa and exponent (round half to even), F = 40
+ * with S = 4 slices of 10 bits, 59 with 5 of 12, then balanced digits from the bottom: all but
+ * the first in [-2^(b-1), 2^(b-1) - 1], d_0 = the rest (at most 1024 = 2^(40-30) or
+ * 2048 = 2^(59-48) since |N| <= 2^F), so that x = sum_t d_t 2^(b(S-1-t) - F) + O(2^-F-1).
  */
-__device__ __forceinline__ void slice4(double v, int e, bool neg, int d[4])
+template <int S>
+__device__ __forceinline__ void slice(double v, int e, bool neg, int d[S])
 {
+  constexpr int b = S == 5 ? 12 : 10, F = S == 5 ? 59 : 40;
   const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
   const int E = (int)((bits >> 52) & 0x7FF);
   unsigned long long M = bits & 0xFFFFFFFFFFFFFull;
-  /* |v| = M 2^(E' - 1075) with E' = max(E, 1); x 2^40 = M / 2^sh, sh >= 13 when |v| < 2^e */
+  /* |v| = M 2^(E' - 1075) with E' = max(E, 1); x 2^F = M / 2^sh, sh >= 53 - F when |v| < 2^e */
   if (E) M |= 1ull << 52;
-  const int sh = 1035 + e - (E ? E : 1);
+  const int sh = 1075 - F + e - (E ? E : 1);
   long long N = 0;
   if (M != 0 && sh < 64) {
-    const int s = sh < 1 ? 1 : sh;
-    unsigned long long q = M >> s;
-    const unsigned long long rem = M & ((1ull << s) - 1), half = 1ull << (s - 1);
-    if (rem > half || (rem == half && (q & 1ull))) ++q;
-    N = (long long)q;
+    if (sh < 1) {
+      N = (long long)(M << -sh);
+    } else {
+      unsigned long long q = M >> sh;
+      const unsigned long long rem = M & ((1ull << sh) - 1), half = 1ull << (sh - 1);
+      if (rem > half || (rem == half && (q & 1ull))) ++q;
+      N = (long long)q;
+    }
   }
   if (neg != (bool)(bits >> 63)) N = -N;
 #pragma unroll
-  for (int t = 3; t >= 1; --t) {
-    int r = (int)(N & 1023);
-    if (r >= 512) r -= 1024;
+  for (int t = S - 1; t >= 1; --t) {
+    int r = (int)(N & ((1 << b) - 1));
+    if (r >= 1 << (b - 1)) r -= 1 << b;
     d[t] = r;
-    N = (N - r) >> 10; /* exact: N - r is a multiple of 1024 */
+    N = (N - r) >> b; /* exact: N - r is a multiple of 2^b */
   }
   d[0] = (int)N;
 }
 
 /*
- * B[(4c+t)][koff + k] (fp16, row stride ldb elements) = slice t of sign P[k][c] / 2^e_c for
+ * B[(Sc+t)][koff + k] (fp16, row stride ldb elements) = slice t of sign P[k][c] / 2^e_c for
  * k < nk (pad k and pad rows are zero from a memset before).  A tile of 64 k x 32 columns is
  * read row-wise (coalesced) into shared memory and written as 128-byte rows of B.
  */
 #define SL_K 64
 #define SL_C 32
+template <int S>
 __global__ void __launch_bounds__(256)
 k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t ncols,
                const int32_t *__restrict__ expo, double sign, int64_t koff, __half *B, int64_t ldb)
 {
   __shared__ double sp[SL_K][SL_C + 1];
-  __shared__ __align__(16) __half ss[SL_C * 4][SL_K + 8];
+  __shared__ __align__(16) __half ss[SL_C * S][SL_K + 8];
   __shared__ int sexp[SL_C];
   const int tid = threadIdx.x;
   const int32_t kt0 = blockIdx.x * SL_K, ct0 = blockIdx.y * SL_C;
@@ -547,25 +567,27 @@ k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t nc
   __syncthreads();
   for (int i = tid; i < SL_K * SL_C; i += blockDim.x) {
     const int cc = i / SL_K, kk = i - cc * SL_K;
-    int d[4];
-    slice4(sp[kk][cc], sexp[cc], neg, d);
+    int d[S];
+    const bool bad = S == 5 && sexp[cc] == X_NONFINITE;
+    slice<S>(bad ? 0.0 : sp[kk][cc], bad ? 0 : sexp[cc], neg, d);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) ss[4 * cc + t][kk] = __int2half_rn(d[t]);
+    for (int t = 0; t < S; ++t) ss[S * cc + t][kk] = __int2half_rn(d[t]);
   }
   __syncthreads();
-  /* 128 output rows x 64 halves: 8 threads write one row's 128 bytes */
-  for (int i = tid; i < SL_C * 4 * 8; i += blockDim.x) {
+  /* 32 S output rows x 64 halves: 8 threads write one row's 128 bytes */
+  for (int i = tid; i < SL_C * S * 8; i += blockDim.x) {
     const int o = i >> 3, seg = i & 7;
-    const int32_t c = ct0 + (o >> 2);
+    const int32_t c = ct0 + o / S;
     if (c >= ncols) continue;
     const int32_t k = kt0 + seg * 8;
     if (k >= nk) continue;
-    __half *dst = B + (int64_t)(4 * ct0 + o) * ldb + koff + k;
+    __half *dst = B + (int64_t)(S * ct0 + o) * ldb + koff + k;
     *(uint4 *)dst = *(const uint4 *)&ss[o][seg * 8];
   }
 }
 
-/* Y[r][c] = 2^e_c sum_t Z[r][4c+t] 1024^-(t+1) */
+/* Y[r][c] = 2^e_c sum_t Z[r][Sc+t] 2^(b(S-1-t) - F) */
+template <int S>
 __global__ void k_panel_combine(const double *Z, int64_t ldz, int32_t nrows, int32_t ncols,
                                 const int32_t *expo, double *Y, int64_t ldy,
                                 const gp_tc_batch *db)
@@ -576,9 +598,16 @@ __global__ void k_panel_combine(const double *Z, int64_t ldz, int32_t nrows, int
        idx += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = idx / ncols;
     int32_t c = (int32_t)(idx - r * ncols);
-    const double *z = Z + r * ldz + 4 * c;
-    double s = ((z[0] * 0x1p-10 + z[1] * 0x1p-20) + z[2] * 0x1p-30) + z[3] * 0x1p-40;
-    Y[r * ldy + c] = ldexp(s, expo[c]);
+    const double *z = Z + r * ldz + S * c;
+    if (S == 4) {
+      double s = ((z[0] * 0x1p-10 + z[1] * 0x1p-20) + z[2] * 0x1p-30) + z[3] * 0x1p-40;
+      Y[r * ldy + c] = ldexp(s, expo[c]);
+    } else {
+      double s = z[S - 1];
+#pragma unroll
+      for (int t = S - 2; t >= 0; --t) s = fma(s, 0x1p-12, z[t]);
+      Y[r * ldy + c] = expo[c] == X_NONFINITE ? nan("") : ldexp(s, expo[c] - 11);
+    }
   }
 }
 
@@ -658,20 +687,20 @@ int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int
   return GP_OK;
 }
 
-size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0)
+size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits)
 {
   const int32_t kpad0 = (k0 + XK - 1) / XK * XK;
-  const int32_t ncols4_pad = (4 * ncols + XT - 1) / XT * XT;
+  const int32_t ncols4_pad = (digits * ncols + XT - 1) / XT * XT;
   return align256((size_t)ncols4_pad * kpad0 * npanels * 2) + align256((size_t)ncols * 16) + 256;
 }
 
 int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols, int32_t k0,
-                  void *storage, gp_tc_prepared *out)
+                  int digits, void *storage, gp_tc_prepared *out)
 {
-  if (npanels < 1 || npanels > 2 || ncols < 1 || ncols > 1024 || k0 < 1)
+  if ((digits != 4 && digits != 5) || npanels < 1 || npanels > 2 || ncols < 1 || ncols > 1024 || k0 < 1)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_prepare: bad panel shape");
   const int32_t kb0 = (k0 + XK - 1) / XK, kpad0 = kb0 * XK;
-  const int32_t ncols4 = 4 * ncols, ncols4_pad = (ncols4 + XT - 1) / XT * XT;
+  const int32_t ncols4 = digits * ncols, ncols4_pad = (ncols4 + XT - 1) / XT * XT;
   const int64_t ldb = (int64_t)kpad0 * npanels;
   uint8_t *base = (uint8_t *)storage;
   __half *B = (__half *)base;
@@ -686,13 +715,13 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
     k_panel_absmax<<<blocks, 256, 0, ctx->stream>>>(pp[p].P, pp[p].ldp, k0, ncols, mx);
     GP_LAUNCH_CHECK(ctx, "k_panel_absmax");
   }
-  k_panel_expo<<<(ncols + 255) / 256, 256, 0, ctx->stream>>>(mx, ncols, expo);
+  k_panel_expo<<<(ncols + 255) / 256, 256, 0, ctx->stream>>>(mx, ncols, expo, digits == 5);
   GP_LAUNCH_CHECK(ctx, "k_panel_expo");
   GP_CUDA(ctx, cudaMemsetAsync(B, 0, (size_t)ncols4_pad * ldb * 2, ctx->stream));
   for (int p = 0; p < npanels; ++p) {
     dim3 sgrid((unsigned)((k0 + SL_K - 1) / SL_K), (unsigned)((ncols + SL_C - 1) / SL_C));
-    k_panel_slices<<<sgrid, 256, 0, ctx->stream>>>(pp[p].P, pp[p].ldp, k0, ncols, expo,
-                                                   pp[p].sign, (int64_t)p * kpad0, B, ldb);
+    (digits == 5 ? k_panel_slices<5> : k_panel_slices<4>)<<<sgrid, 256, 0, ctx->stream>>>(
+        pp[p].P, pp[p].ldp, k0, ncols, expo, pp[p].sign, (int64_t)p * kpad0, B, ldb);
     GP_LAUNCH_CHECK(ctx, "k_panel_slices");
   }
   PFN_cuTensorMapEncodeTiled_v12000 enc = tc_encode(ctx);
@@ -713,6 +742,7 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   out->ncols4 = ncols4;
   out->ncols4_pad = ncols4_pad;
   out->npanels = npanels;
+  out->digits = digits;
   out->kb0 = kb0;
   out->k0 = k0;
   out->ldb = ldb;
@@ -742,19 +772,20 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   int32_t tiles = nrt * nct;
   int32_t ksplit = 1;
   while (tiles * ksplit < 2 * ctx->num_sms && ksplit * 4 <= nkb) ksplit *= 2;
-  /* keep each work item's k range below 2^19 so that int32 sums stay exact */
-  while ((int64_t)((nkb + ksplit - 1) / ksplit) * XK > (1 << 19)) ksplit *= 2;
+  while ((int64_t)((nkb + ksplit - 1) / ksplit) * XK > X_MAX_K(P->digits)) ksplit *= 2;
   int32_t nitems = tiles * ksplit;
   int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
   k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(P->tmb, A->codes, A->ldc, A->row_map,
                                                            nrows, P->ncols4, nkb, P->kb0, P->kb0,
-                                                           P->lut_lo, P->lut_hi, ksplit, Z, ldz,
-                                                           d_err, NULL);
+                                                           P->lut_lo, P->lut_hi, ksplit,
+                                                           X_CHUNK_KB(P->digits), Z, ldz, d_err,
+                                                           NULL);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   {
     int64_t work = (int64_t)nrows * P->ncols;
-    k_panel_combine<<<grid_cap(ctx, work, 256, 32), 256, 0, ctx->stream>>>(Z, ldz, nrows, P->ncols,
-                                                                            P->expo, d_Y, ldy, NULL);
+    (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
+        <<<grid_cap(ctx, work, 256, 32), 256, 0, ctx->stream>>>(Z, ldz, nrows, P->ncols, P->expo,
+                                                                d_Y, ldy, NULL);
     GP_LAUNCH_CHECK(ctx, "k_panel_combine");
   }
   if (!sync) return GP_OK;
@@ -778,7 +809,7 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
                     const gp_tc_prepared *P, double *Z, double *d_Y, int64_t ldy)
 {
   if (max_rows < 1) return GP_OK;
-  if (ldc < (int64_t)P->kb0 * XK / 4)
+  if (P->digits != 4 || ldc < (int64_t)P->kb0 * XK / 4)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_apply_dev: code rows shorter than the panel");
   const int64_t ldz = P->ncols4_pad;
   k_zero_batch_rows<<<grid_cap(ctx, (int64_t)max_rows * ldz, 256, 8), 256, 0, ctx->stream>>>(
@@ -789,26 +820,37 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
   const int32_t nkb = P->kb0 * P->npanels;
   /* every SM: the kernel takes the batch's row count, and with it its work items, from db */
   k_geno_panel_tc<<<ctx->num_sms, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, NULL, ldc, NULL, 0, P->ncols4, nkb, P->kb0, P->kb0, P->lut_lo, P->lut_hi, 1, Z, ldz,
-      ctx->d_err, db);
+      P->tmb, NULL, ldc, NULL, 0, P->ncols4, nkb, P->kb0, P->kb0, P->lut_lo, P->lut_hi, 1,
+      X_CHUNK_KB(4), Z, ldz, ctx->d_err, db);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
-  k_panel_combine<<<grid_cap(ctx, (int64_t)max_rows * P->ncols, 256, 32), 256, 0, ctx->stream>>>(
+  k_panel_combine<4><<<grid_cap(ctx, (int64_t)max_rows * P->ncols, 256, 32), 256, 0, ctx->stream>>>(
       Z, ldz, 0, P->ncols, P->expo, d_Y, ldy, db);
   GP_LAUNCH_CHECK(ctx, "k_panel_combine");
   return GP_OK;
 }
 
 int gp_geno_panel_tc_codes(gp_ctx *ctx, const gp_tc_codes *A, int npanels, const gp_tc_panel *pp,
-                           int32_t ncols, double *d_Y, int64_t ldy)
+                           int32_t ncols, int digits, double *d_Y, int64_t ldy)
 {
   if (A->nrows < 1 || A->k0 < 1) return GP_OK;
-  uint8_t *storage;
-  int rc = gp_scratch2(ctx, gp_tc_prepared_bytes(npanels, ncols, A->k0), (void **)&storage);
-  if (rc) return rc;
-  gp_tc_prepared P;
-  rc = gp_tc_prepare(ctx, npanels, pp, ncols, A->k0, storage, &P);
-  if (rc) return rc;
-  return gp_tc_apply(ctx, A, &P, d_Y, ldy, 1);
+  /* 5 slices: any number of columns, a group at a time, which bounds the slices and sums */
+  const int32_t step = digits == 5 && ncols > X_GROUP5 ? X_GROUP5 : ncols;
+  for (int32_t c0 = 0; c0 < ncols; c0 += step) {
+    const int32_t nc = ncols - c0 < step ? ncols - c0 : step;
+    gp_tc_panel pg[2];
+    for (int p = 0; p < npanels && p < 2; ++p) {
+      pg[p] = pp[p];
+      pg[p].P += c0;
+    }
+    uint8_t *storage;
+    int rc = gp_scratch2(ctx, gp_tc_prepared_bytes(npanels, nc, A->k0, digits), (void **)&storage);
+    if (rc) return rc;
+    gp_tc_prepared P;
+    rc = gp_tc_prepare(ctx, npanels, pg, nc, A->k0, digits, storage, &P);
+    if (!rc) rc = gp_tc_apply(ctx, A, &P, d_Y + c0, ldy, 1);
+    if (rc) return rc;
+  }
+  return GP_OK;
 }
 
 int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
@@ -850,11 +892,11 @@ int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32
 
 int gp_geno_panel_tc(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
                      const int32_t *d_snprec, int32_t nk, int npanels, const gp_tc_panel *pp,
-                     int32_t ncols, double *d_Y, int64_t ldy)
+                     int32_t ncols, int digits, double *d_Y, int64_t ldy)
 {
   if ((sum_over_snps ? nsamp : nk) < 1 || (sum_over_snps ? nk : nsamp) < 1) return GP_OK;
   gp_tc_codes A;
   int rc = gp_tc_codes_for(ctx, sum_over_snps, d_samp, nsamp, d_snprec, nk, &A);
   if (rc) return rc;
-  return gp_geno_panel_tc_codes(ctx, &A, npanels, pp, ncols, d_Y, ldy);
+  return gp_geno_panel_tc_codes(ctx, &A, npanels, pp, ncols, digits, d_Y, ldy);
 }

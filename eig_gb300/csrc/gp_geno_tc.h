@@ -30,19 +30,20 @@ struct gp_tc_codes {
 int gp_tc_code_bytes(int sum_over_snps, int32_t nsamp, int32_t nk, int64_t *ldc, int32_t *rows_pad);
 int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
                       const int32_t *d_snprec, int32_t nk, uint8_t *codes, gp_tc_codes *out);
-/* a panel cut into fp16 slices once (B operand + column exponents + its tensor map) */
+/* a panel cut into fp16 slices once (B operand + column exponents + its tensor map): `digits`
+ * slices, 4 of 10 bits (the split precisions) or 5 of 12 bits (FP64) */
 struct gp_tc_prepared {
   __half *B;
   int32_t *expo;
-  int32_t ncols, ncols4, ncols4_pad, npanels, kb0, k0;
+  int32_t ncols, ncols4, ncols4_pad, npanels, digits, kb0, k0; /* ncols4: slice columns */
   int64_t ldb;
   uint64_t lut_lo, lut_hi;
   CUtensorMap tmb;
 };
-size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0);
+size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits);
 /* slice the panels into caller storage of gp_tc_prepared_bytes bytes (device) */
 int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols, int32_t k0,
-                  void *storage, gp_tc_prepared *out);
+                  int digits, void *storage, gp_tc_prepared *out);
 /* Y[r][c] = products of the code operand with a prepared panel; sync = 0 leaves the work
  * queued on ctx->stream and neither clears nor reads ctx->d_err (the caller does both) */
 int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, double *d_Y,
@@ -68,17 +69,18 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
  * SNP-major operand covers every sample in order) */
 int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
                     const int32_t *d_snprec, int32_t nk, gp_tc_codes *out);
-/* Y[r][c] = sum_p sum_k A(r, k) sign_p P_p[k][c] with a prepared code operand */
+/* Y[r][c] = sum_p sum_k A(r, k) sign_p P_p[k][c] with a prepared code operand; ncols <= 1024
+ * with 4 digits, any number with 5 */
 int gp_geno_panel_tc_codes(gp_ctx *ctx, const gp_tc_codes *A, int npanels, const gp_tc_panel *pp,
-                           int32_t ncols, double *d_Y, int64_t ldy);
+                           int32_t ncols, int digits, double *d_Y, int64_t ldy);
 
 /*
  * sum_over_snps = 1: Y[q][c] = sum_p sum_{s < nk} A_p(samp[q], snprec[s]) sign_p P_p[s][c]
  * sum_over_snps = 0: Y[s][c] = sum_p sum_{q < nsamp} A_p(samp[q], snprec[s]) sign_p P_p[q][c]
  * npanels (1 or 2) panels share the k extent and are concatenated along k with one joint
- * column scale.  Y is device FP64 with row stride ldy; ncols <= 1024.  Uses scratch2.
+ * column scale.  Y is device FP64 with row stride ldy.  Uses scratch2.
  */
 int gp_geno_panel_tc(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
                      const int32_t *d_snprec, int32_t nk, int npanels, const gp_tc_panel *pp,
-                     int32_t ncols, double *d_Y, int64_t ldy);
+                     int32_t ncols, int digits, double *d_Y, int64_t ldy);
 #endif

@@ -770,12 +770,15 @@ extern "C" int64_t gp_smartpca_footprint(int32_t nind, int64_t nsnp, int32_t pre
                       8 * (nt * (nt + 1) / 2 * 64 * 64 + 27 * nt * 64 + 3 * nt) + 5 * nt * nt;
   int64_t work;
   if (precision == GP_PREC_FP64) {
-    /* lsqproject's panel of pair products, or the exact Gram: its right operand (20 bytes per
-     * genotype, at most 2 GiB at a time), integer sums and sample-major codes */
+    /* lsqproject's panel of pair products and its slices (256 columns at a time), the SNP-major
+     * sums of the weights, or the exact Gram: its right operand (20 bytes per genotype, at most
+     * 2 GiB at a time), integer sums and sample-major codes */
     int64_t slices = 20 * (n + 48) * (m + 64);
     if (slices > (int64_t)2 << 30) slices = (int64_t)2 << 30;
-    work = 8 * m * (k * (k + 1) / 2 + 1) + 8 * n * 256 + slices + 8 * (n + 256) * (n + 304) +
-           npad * (m / 4 + 16);
+    const int64_t cols5 = 5 * (k * (k + 1) / 2 + 1) < 1280 ? 5 * (k * (k + 1) / 2 + 1) + 127 : 1280;
+    if (slices < 2 * m * cols5) slices = 2 * m * cols5;
+    work = 8 * m * (k * (k + 1) / 2 + 1) + 8 * n * 1280 + slices + 8 * m * (9 * k + 127) +
+           8 * (n + 256) * (n + 304) + npad * (m / 4 + 16);
   } else {
     int64_t split = 4 * npad * m;
     if (split > (int64_t)24 << 30) split = (int64_t)24 << 30;
@@ -900,7 +903,8 @@ extern "C" int gp_serve_open(gp_ctx *src, const gp_serve_opts *o, gp_server **ou
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&s->h_err[i], sizeof(int) * 4, 0);
   }
   if (!s->fp64_serial) {
-    size_t b1 = gp_tc_prepared_bytes(1, s->ldp, s->nk), b2 = gp_tc_prepared_bytes(2, K, s->nk);
+    size_t b1 = gp_tc_prepared_bytes(1, s->ldp, s->nk, 4),
+           b2 = gp_tc_prepared_bytes(2, K, s->nk, 4);
     SALLOC(s->stor_co, b1);
     SALLOC(s->stor_rr, b2);
   }
@@ -963,9 +967,9 @@ extern "C" int gp_serve_open(gp_ctx *src, const gp_serve_opts *o, gp_server **ou
   }
   if (!s->fp64_serial && s->nk > 0) {
     gp_tc_panel pc = {s->d_P, s->ldp, 1.0, 0};
-    rc = gp_tc_prepare(ctx, 1, &pc, s->ldp, s->nk, s->stor_co, &s->Pco);
+    rc = gp_tc_prepare(ctx, 1, &pc, s->ldp, s->nk, 4, s->stor_co, &s->Pco);
     gp_tc_panel pr[2] = {{s->d_fE, K, 1.0, 1}, {s->d_mE, K, -1.0, 0}};
-    if (!rc) rc = gp_tc_prepare(ctx, 2, pr, K, s->nk, s->stor_rr, &s->Prr);
+    if (!rc) rc = gp_tc_prepare(ctx, 2, pr, K, s->nk, 4, s->stor_rr, &s->Prr);
     /* the products' slice-column buffer, sized once for the largest batch */
     void *z;
     if (!rc) rc = gp_scratch5(ctx, (size_t)s->max_batch * s->Pco.ncols4_pad * 8 + 256, &z);
