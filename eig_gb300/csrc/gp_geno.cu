@@ -367,58 +367,70 @@ __global__ void k_snp_valid(const uint8_t *geno, int64_t rlen_dev, int64_t nsnp,
   }
 }
 
-/* per sample: number of non-missing genotypes over the used SNPs.  Thread = one word of
- * 16 samples, looping over a slice of SNPs eight records at a time (loads first; an unused
- * SNP reads as all-missing); the observed bits are summed in 4-bit fields of two words
- * (fields 0, 2, .. and 1, 3, ..), flushed into per-sample counts every 15 SNPs; partial
- * counts are summed with atomics. */
-__global__ void k_sample_valid(const uint8_t *geno, int64_t rlen_dev, int64_t nsnp,
-                               const uint8_t *snp_use, int32_t nind, int32_t *out,
-                               int64_t snps_per_slice)
+/* per sample: number of non-missing genotypes over the used SNPs.  A CTA takes 32 words (of 16
+ * samples) of a slice of the SNPs, a warp per eighth of it, so that a warp reads 128 contiguous
+ * bytes of a record; eight records at a time (loads first; an unused SNP reads as all-missing).
+ * The observed bits are summed in 4-bit fields of two words (fields 0, 2, .. and 1, 3, ..),
+ * flushed into per-sample counts every 15 SNPs; the warps' counts are added in shared memory and
+ * the slices' with atomics.  HBM or, on short panels, latency bounds it: the slices are as short
+ * as gives every SM four CTAs (slices of 4,096 SNPs, one CTA per 2,048 samples, left a panel of
+ * 180 x 2,500 to one CTA: 245 us, now 5; 5,000 x 100,000: 44 us). */
+#define SV_WARPS 8
+__global__ void __launch_bounds__(32 * SV_WARPS)
+k_sample_valid(const uint8_t *geno, int64_t rlen_dev, int64_t nsnp, const uint8_t *snp_use,
+               int32_t nind, int32_t *out, int64_t snps_per_slice)
 {
-  int64_t words = rlen_dev >> 2;
-  int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (w >= words) return;
-  int64_t s0 = (int64_t)blockIdx.y * snps_per_slice;
-  int64_t s1 = s0 + snps_per_slice < nsnp ? s0 + snps_per_slice : nsnp;
-  int32_t cnt[16];
+  __shared__ int32_t sum[16][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 16 * 33; i += blockDim.x) (&sum[0][0])[i] = 0;
+  __syncthreads();
+  const int64_t words = rlen_dev >> 2, w = blockIdx.x * (int64_t)32 + lane;
+  const int64_t s0 = (int64_t)blockIdx.y * snps_per_slice;
+  const int64_t s1 = s0 + snps_per_slice < nsnp ? s0 + snps_per_slice : nsnp;
+  if (w < words) {
+    int32_t cnt[16];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) cnt[j] = 0;
-  uint32_t acc_a = 0, acc_b = 0;
-  int pend = 0;
-  auto flush = [&]() {
+    for (int j = 0; j < 16; ++j) cnt[j] = 0;
+    uint32_t acc_a = 0, acc_b = 0;
+    int pend = 0;
+    auto flush = [&]() {
 #pragma unroll
-    for (int f = 0; f < 16; ++f) {
-      /* field f (bits 2f, 2f+1) is sample (f >> 2) * 4 + 3 - (f & 3) of the word */
-      const uint32_t v = ((f & 1) ? acc_b : acc_a) >> (4 * (f >> 1));
-      cnt[(f >> 2) * 4 + 3 - (f & 3)] += (int32_t)(v & 0xFu);
+      for (int f = 0; f < 16; ++f) {
+        /* field f (bits 2f, 2f+1) is sample (f >> 2) * 4 + 3 - (f & 3) of the word */
+        const uint32_t v = ((f & 1) ? acc_b : acc_a) >> (4 * (f >> 1));
+        cnt[(f >> 2) * 4 + 3 - (f & 3)] += (int32_t)(v & 0xFu);
+      }
+      acc_a = acc_b = 0;
+      pend = 0;
+    };
+    const uint32_t *col = (const uint32_t *)geno + w;
+    const int64_t stride = rlen_dev >> 2;
+    for (int64_t s = s0 + 8 * warp; s < s1; s += 8 * SV_WARPS) {
+      uint32_t v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int64_t su = s + u;
+        v[u] = su < s1 ? __ldg(col + su * stride) : 0xFFFFFFFFu;
+        if (snp_use && su < s1 && !snp_use[su]) v[u] = 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t ok = ~((v[u] >> 1) & v[u]) & 0x55555555u;
+        acc_a += ok & 0x11111111u;
+        acc_b += (ok >> 2) & 0x11111111u;
+        if (++pend == 15) flush();
+      }
     }
-    acc_a = acc_b = 0;
-    pend = 0;
-  };
-  const uint32_t *col = (const uint32_t *)geno + w;
-  const int64_t stride = rlen_dev >> 2;
-  for (int64_t s = s0; s < s1; s += 8) {
-    uint32_t v[8];
+    flush();
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int64_t su = s + u;
-      v[u] = su < s1 ? __ldg(col + su * stride) : 0xFFFFFFFFu;
-      if (snp_use && su < s1 && !snp_use[su]) v[u] = 0xFFFFFFFFu;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const uint32_t ok = ~((v[u] >> 1) & v[u]) & 0x55555555u;
-      acc_a += ok & 0x11111111u;
-      acc_b += (ok >> 2) & 0x11111111u;
-      if (++pend == 15) flush();
-    }
+    for (int j = 0; j < 16; ++j)
+      if (cnt[j]) atomicAdd(&sum[j][lane], cnt[j]);
   }
-  flush();
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    int64_t k = w * 16 + j;
-    if (k < nind && cnt[j]) atomicAdd(&out[k], cnt[j]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * 32; i += blockDim.x) {
+    const int64_t k = blockIdx.x * (int64_t)512 + i;
+    const int32_t c = sum[i & 15][i >> 4];
+    if (k < nind && c) atomicAdd(&out[k], c);
   }
 }
 
@@ -460,9 +472,12 @@ extern "C" int gp_valid_counts(gp_ctx *ctx, const uint8_t *sample_use, const uin
   }
   if (sample_valid) {
     GP_CUDA(ctx, cudaMemsetAsync(d_iv, 0, sizeof(int32_t) * (size_t)ctx->nind_all, ctx->stream));
-    int64_t slice = 4096;
-    dim3 grid((unsigned)((nwords + 127) / 128), (unsigned)((nsnp + slice - 1) / slice));
-    k_sample_valid<<<grid, 128, 0, ctx->stream>>>(ctx->d_geno, ctx->rlen_dev, nsnp,
+    const int64_t gx = (nwords + 31) / 32;
+    int64_t slice = (nsnp * gx + 4 * ctx->num_sms - 1) / (4 * ctx->num_sms);
+    slice = (slice + 8 * SV_WARPS - 1) / (8 * SV_WARPS) * (8 * SV_WARPS);
+    while ((nsnp + slice - 1) / slice > 65535) slice *= 2;
+    dim3 grid((unsigned)gx, (unsigned)((nsnp + slice - 1) / slice));
+    k_sample_valid<<<grid, 32 * SV_WARPS, 0, ctx->stream>>>(ctx->d_geno, ctx->rlen_dev, nsnp,
                                                   snp_use ? d_su : NULL, ctx->nind_all, d_iv,
                                                   slice);
     GP_LAUNCH_CHECK(ctx, "k_sample_valid");
