@@ -87,7 +87,7 @@ struct gp_server {
   uint8_t *d_pool;
   int64_t head, tail;
   cudaStream_t copy_stream;
-  double *d_co[2], *d_rr[2], *d_a[2], *d_b[2], *d_work[2], *d_part[2];
+  double *d_co[2], *d_rr[2], *d_a[2], *d_b[2], *d_part[2];
   int32_t *d_nobs[2], *d_status[2];
   int *d_errw[2];
   double *h_a[2];
@@ -402,10 +402,9 @@ static int launch_batch(gp_server *s, gp_batch *b)
       GP_LAUNCH_CHECK(ctx, "k_parts_sum");
     }
   }
-  k_lsq_solve<<<(b->nrows + 127) / 128, 128, 0, ctx->stream>>>(
-      s->d_co[sl], s->ldp, s->d_rr[sl], s->K, b->nrows, s->d_a[sl], s->d_b[sl], s->d_nobs[sl],
-      s->d_status[sl], s->d_work[sl], NULL);
-  GP_LAUNCH_CHECK(ctx, "k_lsq_solve");
+  int rcs = gp_launch_lsq_solve(ctx, s->d_co[sl], s->ldp, s->d_rr[sl], s->K, b->nrows, s->d_a[sl],
+                                s->d_b[sl], s->d_nobs[sl], s->d_status[sl], NULL);
+  if (rcs) return rcs;
   GP_CUDA(ctx, cudaMemcpyAsync(s->h_a[sl], s->d_a[sl], sizeof(double) * (size_t)s->K * b->nrows,
                                cudaMemcpyDeviceToHost, ctx->stream));
   GP_CUDA(ctx, cudaMemcpyAsync(s->h_status[sl], s->d_status[sl], sizeof(int32_t) * b->nrows,
@@ -687,10 +686,10 @@ static int build_loop(gp_server *s)
   if (!rc) rc = gp_tc_apply_dev(ctx, s->d_batch, mb, s->row_bytes, &s->Pco, s->d_Z, s->d_co[0],
                                 s->ldp);
   if (!rc) rc = gp_tc_apply_dev(ctx, s->d_batch, mb, s->row_bytes, &s->Prr, s->d_Z, s->d_rr[0], K);
+  if (!rc)
+    rc = gp_launch_lsq_solve(ctx, s->d_co[0], s->ldp, s->d_rr[0], K, mb, s->d_a[0], s->d_b[0],
+                             s->d_nobs[0], s->d_status[0], &s->d_batch->nrows);
   if (!rc) {
-    k_lsq_solve<<<(mb + 127) / 128, 128, 0, ctx->stream>>>(
-        s->d_co[0], s->ldp, s->d_rr[0], K, 0, s->d_a[0], s->d_b[0], s->d_nobs[0],
-        s->d_status[0], s->d_work[0], &s->d_batch->nrows);
     k_srv_emit<<<(mb + 127) / 128, 128, 0, ctx->stream>>>(s->d_batch, s->d_a[0], s->d_status[0],
                                                           s->d_escale, K, s->d_res, s->d_rst);
     k_srv_done<<<1, 1, 0, ctx->stream>>>(s->dq, s->d_batch, ctx->d_err);
@@ -824,8 +823,8 @@ extern "C" void gp_serve_close(gp_server *s)
   if (s->h_rst) cudaFreeHost(s->h_rst);
   void *dev[] = {s->d_E,     s->d_P,      s->d_fE,     s->d_mE,     s->d_otab,   s->d_rtab,
                  s->stor_co, s->stor_rr,  s->d_pool,   s->d_co[0],  s->d_co[1],  s->d_rr[0],
-                 s->d_rr[1], s->d_a[0],   s->d_a[1],   s->d_b[0],   s->d_b[1],   s->d_work[0],
-                 s->d_work[1], s->d_part[0], s->d_part[1], s->d_nobs[0], s->d_nobs[1],
+                 s->d_rr[1], s->d_a[0],   s->d_a[1],   s->d_b[0],   s->d_b[1],
+                 s->d_part[0], s->d_part[1], s->d_nobs[0], s->d_nobs[1],
                  s->d_status[0], s->d_status[1], s->d_batch, s->d_Z, s->d_escale};
   for (size_t i = 0; i < sizeof(dev) / sizeof(dev[0]); ++i)
     if (dev[i]) cudaFree(dev[i]);
@@ -894,7 +893,6 @@ extern "C" int gp_serve_open(gp_ctx *src, const gp_serve_opts *o, gp_server **ou
     SALLOC(s->d_rr[i], sizeof(double) * (size_t)s->max_batch * K);
     SALLOC(s->d_a[i], sizeof(double) * (size_t)s->max_batch * K);
     SALLOC(s->d_b[i], sizeof(double) * (size_t)s->max_batch * K);
-    SALLOC(s->d_work[i], sizeof(double) * (size_t)s->max_batch * (K * K + 2 * K));
     SALLOC(s->d_nobs[i], sizeof(int32_t) * (size_t)s->max_batch);
     SALLOC(s->d_status[i], sizeof(int32_t) * (size_t)s->max_batch);
     if (s->fp64_serial) SALLOC(s->d_part[i], sizeof(double) * 16 * (size_t)s->max_batch * s->ldp);
