@@ -979,7 +979,7 @@ k_build_EP(const double *ffvecs, const double *fxscal, const int32_t *kept, int3
  * of a row in turn, and the factor (packed lower triangle over the pair sums it replaces),
  * the pivots, the solution and the products sit in shared memory.  K = 20, 5,000 samples:
  * 493 us with a thread per sample and the factors in global memory, 235 with a thread per
- * sample and shared memory, 140 here; 300 samples: 477, now 106.
+ * sample and shared memory, 185 here; 300 samples: 477, now 106.
  */
 #define LSQ_LANES 8
 #define LSQ_SAMPLES (32 / LSQ_LANES)

@@ -9,8 +9,8 @@
  * x = P/2^e_c = sum_t q_t 1024^-(t+1) with |q_0| <= 1024 and |q_t| <= 512 (t > 0): integers
  * that fp16 holds exactly.  A tensor-core MMA of {0,1,2} by such integers over at most 8,192
  * k values sums to an integer below 2^24, which FP32 holds exactly, so the FP32 accumulation
- * of the MMA loses nothing; chunk sums are added in int32 registers and flushed with FP64
- * atomics of exact integers (order-independent, hence deterministic).  The only error left
+ * of the MMA loses nothing; chunk sums are added with 64-bit integer atomics
+ * (order-independent, hence deterministic).  The only error left
  * is the slicing, about 2^-41 of the column maximum: the split precisions' products.
  *
  * The FP64 precision's products take 5 slices of 12 bits (x = sum_t q_t 2^-(11 + 12 t),
@@ -25,20 +25,24 @@
  *   sum over SNPs     rows = samples, k = kept SNPs (codes in sample-major order)
  *   sum over samples  rows = kept SNPs, k = samples (codes in SNP-major order)
  *
- * Kernel structure (grid-stride over work items = row tile x column tile x k-split, the row
- * tile fastest, so that the CTAs running at one time share the B tile and k range they
- * stream and B is read from DRAM about once per wave instead of once per row tile):
- *   warp 0      TMA of the B tile (128 slice-columns x 64 k, fp16, 128-byte swizzle);
- *   warp 1      one thread issues 4 tcgen05.mma (128x128x16, f16 -> f32) per k-block into
- *               TMEM buffer (chunk & 1);
- *   warps 2-9   decode the A tile, two threads per row: each reads 8 bytes of codes (32 k;
- *               the next eight k-blocks' loads in flight) and writes 32 fp16 values into
- *               shared memory in the same swizzled layout, each code turned into its fp16
- *               value by a byte permute of the 4-entry table held in two registers; then
- *               fence.proxy.async + mbarrier arrive (the decode bounds the kernel: four
- *               decoder warps, one thread per row, left the tensor pipe ~20% busy);
- *   warps 10-17 epilogue: per chunk tcgen05.ld the exact FP32 sums, add into int32
- *               registers (64 columns per thread), flush with FP64 atomics per work item.
+ * Kernel structure (grid-stride over work items = 256-row tile x column tile of up to 256
+ * slice columns x k-split, the row tile fastest, so that the CTAs running at one time share the
+ * B tile and k range they stream and B is read from DRAM about once per wave instead of once
+ * per row tile):
+ *   warp 0      TMA of the B tile (slice columns x 64 k, fp16, 128-byte swizzle), 3 stages;
+ *   warp 1      one thread issues 2 x 4 tcgen05.mma (128 x N x 16, f16 -> f32) per k-block:
+ *               the tile's two 128-row halves share the B tile;
+ *   warps 2-9   decode the A tile, a thread per row: 16 bytes of codes (the next four
+ *               k-blocks' loads in flight) become 64 fp16 values in the same swizzled layout,
+ *               four codes at a time through byte permutes (every table value has a zero low
+ *               byte, so one register holds the table); then fence.proxy.async and one arrival
+ *               per warp;
+ *   warps 10-17 epilogue: per chunk tcgen05.ld the exact FP32 sums and add them to the tile's
+ *               64-bit integer sums in global memory (atomics, 32 rows side by side).
+ * The decode of the codes paces it: 128 x 128 tiles decoded each code again for every 128
+ * columns and left the tensor pipe a quarter busy (the normal equations of 5,000 samples x 200,000
+ * SNPs, K = 20: 2.98 ms; with
+ * 256 x 256 tiles 1.41, 1.3 PFLOP/s).
  */
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -49,92 +53,108 @@
 #include "gp_geno_tc.h"
 #include "gp_tc.cuh"
 
-#define XT 128              /* rows / slice-columns per tile */
+#define XT 128              /* rows of a half tile; code operands are padded to it */
+#define XR 256              /* rows per tile: two 128-row accumulators */
+#define XN 256              /* slice columns per tile at most */
 #define XK 64               /* k per k-block */
-#define XSTAGES 4
+#define XSTAGES 3
 #define XA_BYTES (XT * XK * 2)
-#define XB_BYTES (XT * XK * 2)
-#define XSTAGE_BYTES (XA_BYTES + XB_BYTES)
-#define X_THREADS 576       /* 18 warps */
-#define X_DEC_WARPS 8       /* decoder warps: two threads per row of the A tile */
+#define XB_BYTES (XN * XK * 2)
+#define XSTAGE_BYTES (2 * XA_BYTES + XB_BYTES)
+#define X_DEC_WARPS 8       /* decoder warps: a thread per row of the A tile */
+#define X_EPI_WARPS 8
+#define X_THREADS (64 + 32 * (X_DEC_WARPS + X_EPI_WARPS))
 #define X_SMEM (XSTAGES * XSTAGE_BYTES + 1024 + 256)
-#define XPF 8               /* k-blocks of codes a decoder thread loads ahead */
+#define XPF 4               /* k-blocks of codes a decoder thread loads ahead */
 
 #define XERR_FULL 11
 #define XERR_EMPTY 12
 #define XERR_ACCF 13
 #define XERR_ACCE 14
 
-/* fp16 bit patterns of the 4-entry decode tables */
-#define H0 0x0000ull
-#define H1 0x3C00ull
-#define H2 0x4000ull
-static const uint64_t LUT_MASK = H1 | (H1 << 16) | (H1 << 32);      /* {1,1,1,0} */
-/* k-blocks per exact FP32 chunk: 8,192 k with 10-bit slices, 4,096 with 12-bit ones; and the
- * largest k range of a work item whose int32 sums cannot overflow */
+/* the 4-entry decode tables: the high byte of the fp16 value of codes 0, 1, 2, 3 (byte 0
+ * first); the low bytes are zero */
+static const uint32_t LUT_MASK = 0x003C3C3Cu;  /* {1,1,1,0} */
+static const uint32_t LUT_COUNT = 0x00403C00u; /* {0,1,2,0} */
+/* k-blocks per exact FP32 chunk: 8,192 k with 10-bit slices, 4,096 with 12-bit ones */
 #define X_CHUNK_KB(digits) ((digits) == 5 ? 64 : 128)
-#define X_MAX_K(digits) ((digits) == 5 ? 1 << 18 : 1 << 19)
 /* columns of a panel cut and multiplied at a time with 5 slices */
 #define X_GROUP5 256
-static const uint64_t LUT_COUNT = H0 | (H1 << 16) | (H2 << 32);     /* {0,1,2,0} */
 
-__device__ __forceinline__ void fence_proxy_async_smem()
+/* slice columns per tile: the fewest tiles of at most XN, equally wide, a multiple of the
+ * MMA's 16 */
+static int32_t x_tile_cols(int32_t slice_cols)
 {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  const int32_t nct = (slice_cols + XN - 1) / XN;
+  return ((slice_cols + nct - 1) / nct + 15) / 16 * 16;
+}
+
+/* k splits: a work item costs its k-blocks and about 3 more (ring fill, TMEM read, atomics);
+ * of the splits that fill one to four waves of the grid the one whose busiest CTA does least */
+__host__ __device__ __forceinline__ int32_t x_split(int32_t tiles, int32_t nkb, int32_t grid)
+{
+  int32_t best = 1, best_cost = ((tiles + grid - 1) / grid) * (nkb + 3);
+  for (int32_t w = 1; w <= 4; ++w) {
+    int32_t s = w * grid / tiles;
+    if (s > nkb / 4) s = nkb / 4;
+    if (s < 2) continue;
+    const int32_t cost = ((tiles * s + grid - 1) / grid) * ((nkb + s - 1) / s + 3);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
 }
 
 /*
  * codes: rows of ldc bytes (2-bit codes, MSB first, 3 = missing -> 0); output row r reads
  * code row row_map[r] (r itself when row_map is NULL); its k-block kb is the 16 bytes at
- * (kb % kb_period)*16, decoded with lut_lo for kb < kb_switch and lut_hi otherwise (the
- * concatenated-k form [G | O]).
- * zout: [nrows][ldz] FP64, receives atomically the exact integer sums per slice-column.
+ * (kb % kb_period)*16, decoded with lut_lo for kb < kb_period and lut_hi otherwise (the
+ * concatenated-k form [G | O]).  tn: slice columns per tile; nct column tiles.
+ * sums: per row tile, slice column (nct * tn of them) and row of the tile the exact integer
+ * sum, added atomically.
  */
 __global__ void __launch_bounds__(X_THREADS, 1)
 k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restrict__ codes,
-                int64_t ldc, const int32_t *__restrict__ row_map, int32_t nrows, int32_t ncols4,
-                int32_t nkb, int32_t kb_period,
-                int32_t kb_switch, uint64_t lut_lo, uint64_t lut_hi, int32_t ksplit,
-                int32_t chunk_kb, double *zout, int64_t ldz, int *err, const gp_tc_batch *db)
+                int64_t ldc, const int32_t *__restrict__ row_map, int32_t nrows, int32_t tn,
+                int32_t nct, int32_t nkb, int32_t kb_period, uint32_t lut_lo, uint32_t lut_hi,
+                int32_t ksplit, int32_t chunk_kb, unsigned long long *sums, int *err,
+                const gp_tc_batch *db)
 {
   if (db) {
-    /* a device-resident loop's batch: rows and their count are read at run time, and the
-     * k split is chosen as gp_tc_apply chooses it for that count */
+    /* a device-resident loop's batch: rows and their count are read at run time */
     codes = db->codes;
     nrows = db->nrows;
-    const int32_t tiles = ((nrows + XT - 1) / XT) * ((ncols4 + XT - 1) / XT);
-    ksplit = 1;
-    while (tiles * ksplit < 2 * (int32_t)gridDim.x && ksplit * 4 <= nkb) ksplit *= 2;
-    while ((int64_t)((nkb + ksplit - 1) / ksplit) * XK > (1 << 19)) ksplit *= 2;
+    if (nrows < 1) return;
+    ksplit = x_split(((nrows + XR - 1) / XR) * nct, nkb, (int32_t)gridDim.x);
   }
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t *bars = (uint64_t *)(smem + XSTAGES * XSTAGE_BYTES);
   uint64_t *full = bars, *empty = bars + XSTAGES, *accf = bars + 2 * XSTAGES,
-           *acce = bars + 2 * XSTAGES + 2, *drain = bars + 2 * XSTAGES + 4;
-  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * XSTAGES + 5);
+           *acce = bars + 2 * XSTAGES + 1, *drain = bars + 2 * XSTAGES + 2;
+  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * XSTAGES + 3);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  const int32_t nrt = (nrows + XT - 1) / XT, nct = (ncols4 + XT - 1) / XT;
+  const int32_t nrt = (nrows + XR - 1) / XR;
   const int32_t nitems = nrt * nct * ksplit;
   const int32_t kb_per = (nkb + ksplit - 1) / ksplit;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < XSTAGES; ++s) {
-      mbar_init(&full[s], 1 + 32 * X_DEC_WARPS);
+      mbar_init(&full[s], 1 + X_DEC_WARPS);
       mbar_init(&empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&accf[b], 1);
-      mbar_init(&acce[b], 8);
-    }
+    mbar_init(accf, 1);
+    mbar_init(acce, X_EPI_WARPS);
     mbar_init(drain, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 0 && lane == 0) tma_prefetch_desc(&tm_b);
-  if (warp == 1) tmem_alloc(tmem_slot, 256);
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -146,89 +166,88 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
       uint32_t it = 0;
       bool ok = true;
       for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit);
-        int32_t kb0 = ks * kb_per, kb1 = kb0 + kb_per < nkb ? kb0 + kb_per : nkb;
+        const int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit);
+        const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
         for (int32_t kb = kb0; kb < kb1; ++kb, ++it) {
-          uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
+          const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
           if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, XERR_EMPTY)) {
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&full[s], XB_BYTES);
-          tma_load_2d(smem + s * XSTAGE_BYTES + XA_BYTES, &tm_b, &full[s], kb * XK, ct * XT);
+          mbar_arrive_expect_tx(&full[s], (uint32_t)tn * (XK * 2));
+          tma_load_2d(smem + s * XSTAGE_BYTES + 2 * XA_BYTES, &tm_b, &full[s], kb * XK, ct * tn);
         }
       }
       if (*abort_flag) {
-        uint32_t last = it < XSTAGES ? it : XSTAGES;
-        for (uint32_t j = it - last; j < it; ++j) {
-          uint64_t t0 = globaltimer_ns();
+        /* copies already issued must land before the CTA exits (bounded) */
+        const uint64_t t0 = globaltimer_ns();
+        const uint32_t last = it < XSTAGES ? it : XSTAGES;
+        for (uint32_t j = it - last; j < it; ++j)
           while (!mbar_try_wait(&full[j % XSTAGES], (j / XSTAGES) & 1u) &&
                  globaltimer_ns() - t0 < GP_WAIT_NS) {
           }
-        }
       }
     }
   } else if (warp == 1) {
     /* ---------------- MMA issuer ---------------- */
     if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(XT, XT);
+      const uint32_t idesc = idesc_f16_f32(XT, (uint32_t)tn);
       uint32_t it = 0, chunk = 0;
       bool ok = true;
       for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        int32_t ks = (w / nrt) % ksplit;
-        int32_t kb0 = ks * kb_per, kb1 = kb0 + kb_per < nkb ? kb0 + kb_per : nkb;
+        const int32_t ks = (w / nrt) % ksplit, rt = w % nrt;
+        const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+        const bool h1 = rt * XR + XT < nrows;
         for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += chunk_kb, ++chunk) {
-          int32_t c1 = c0 + chunk_kb < kb1 ? c0 + chunk_kb : kb1;
-          uint32_t buf = chunk & 1u, use = chunk >> 1;
-          if (!mbar_wait(&acce[buf], (use & 1u) ^ 1u, abort_flag, err, XERR_ACCE)) {
+          const int32_t c1 = min(kb1, c0 + chunk_kb);
+          if (!mbar_wait(acce, (chunk & 1u) ^ 1u, abort_flag, err, XERR_ACCE)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t d = tmem + buf * XT;
           for (int32_t kb = c0; kb < c1; ++kb, ++it) {
-            uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
+            const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
             if (!mbar_wait(&full[s], ph, abort_flag, err, XERR_FULL)) {
               ok = false;
               break;
             }
             tc_fence_after();
-            uint32_t base = smem_u32(smem + s * XSTAGE_BYTES);
-            uint64_t ad = sdesc_k128(base), bd = sdesc_k128(base + XA_BYTES);
+            const uint32_t base = smem_u32(smem + s * XSTAGE_BYTES);
+            const uint64_t a0 = sdesc_k128(base), a1 = sdesc_k128(base + XA_BYTES),
+                           bd = sdesc_k128(base + 2 * XA_BYTES);
 #pragma unroll
-            for (int k = 0; k < XK / 16; ++k)
-              umma_bf16(d, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc,
-                        (kb > c0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < XK / 16; ++k) {
+              const uint32_t acc = (kb > c0 || k > 0) ? 1u : 0u;
+              umma_bf16(tmem, a0 + 2 * k, bd + 2 * k, idesc, acc);
+              if (h1) umma_bf16(tmem + XN, a1 + 2 * k, bd + 2 * k, idesc, acc);
+            }
             umma_commit(&empty[s]);
           }
-          if (!ok) break;
-          umma_commit(&accf[buf]);
+          if (ok) umma_commit(accf);
         }
       }
     }
   } else if (warp < 2 + X_DEC_WARPS) {
-    /* ---------------- A decoders: two threads per row of the tile ---------------- */
-    const int dt = (warp - 2) * 32 + lane, r = dt >> 1, hb = dt & 1;
-    /* the 4-entry fp16 tables as byte tables for prmt: code c is bytes 2c, 2c+1 */
-    const uint32_t tlo0 = (uint32_t)lut_lo, tlo1 = (uint32_t)(lut_lo >> 32);
-    const uint32_t thi0 = (uint32_t)lut_hi, thi1 = (uint32_t)(lut_hi >> 32);
+    /* ---------------- A decoders: a thread per row of the tile ---------------- */
+    const int r = (warp - 2) * 32 + lane;
+    uint8_t *rowp = smem + (r >> 7) * XA_BYTES + (r & 127) * 128;
+    const uint32_t sw = (uint32_t)(r & 7);
     uint32_t it = 0;
     bool ok = true;
     for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-      int32_t ks = (w / nrt) % ksplit, rt = w % nrt;
-      int32_t kb0 = ks * kb_per, kb1 = kb0 + kb_per < nkb ? kb0 + kb_per : nkb;
-      const int32_t grow = rt * XT + r;
-      const int64_t crow_idx = grow < nrows ? (row_map ? (int64_t)row_map[grow] : (int64_t)grow) : 0;
-      const uint8_t *crow = codes + crow_idx * ldc + 8 * hb;
-      /* this thread's half (8 bytes, 32 codes) of the row's codes of the next XPF k-blocks are
-       * loaded ahead of the stage waits (the k-block index wraps at kb_period, so loads past
-       * kb1 stay inside the row) */
-      const bool live = grow < nrows;
-      auto ld_codes = [&](int32_t kbx) {
-        return live ? __ldg((const uint2 *)(crow + (int64_t)(kbx % kb_period) * 16))
-                    : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+      const int32_t ks = (w / nrt) % ksplit, rt = w % nrt;
+      const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      const int32_t grow = rt * XR + r;
+      /* a half with no row at all is not multiplied and needs no decode */
+      const bool live = grow < nrows, half_on = rt * XR + (r & ~127) < nrows;
+      const uint8_t *crow =
+          codes + (live ? (row_map ? (int64_t)row_map[grow] : (int64_t)grow) : 0) * ldc;
+      auto ld_codes = [&](int32_t kb) {
+        return live && kb < kb1
+                   ? __ldg((const uint4 *)(crow + (int64_t)(kb < kb_period ? kb : kb - kb_period) * 16))
+                   : make_uint4(~0u, ~0u, ~0u, ~0u);
       };
-      uint2 pf[XPF];
+      uint4 pf[XPF];
 #pragma unroll
       for (int u = 0; u < XPF; ++u) pf[u] = ld_codes(kb0 + u);
       for (int32_t kbb = kb0; kbb < kb1 && ok; kbb += XPF) {
@@ -236,86 +255,69 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
         for (int u = 0; u < XPF; ++u) {
           const int32_t kb = kbb + u;
           if (kb >= kb1) break;
-          const uint2 raw = pf[u];
+          const uint32_t words[4] = {pf[u].x, pf[u].y, pf[u].z, pf[u].w};
           pf[u] = ld_codes(kb + XPF);
-          uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
+          const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
           ++it;
-          bool got = mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, XERR_EMPTY);
-          if (!got) {
+          const bool got = mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, XERR_EMPTY);
+          if (!__all_sync(0xffffffffu, got)) {
             ok = false;
             break;
           }
-          const bool hi_tab = kb >= kb_switch;
-          const uint32_t t0 = hi_tab ? thi0 : tlo0, t1 = hi_tab ? thi1 : tlo1;
-          uint8_t *row_base = smem + s * XSTAGE_BYTES + r * 128;
-          const uint32_t words[2] = {raw.x, raw.y};
+          if (half_on) {
+            const uint32_t tab = kb < kb_period ? lut_lo : lut_hi;
+            uint8_t *dst = rowp + s * XSTAGE_BYTES;
 #pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            /* codes 8j..8j+7 (j = 4 hb + jj): bytes 2j, 2j+1 of the row's 16 (little-endian
-             * words); a byte holds four codes, MSB first, and each code c selects bytes 2c,
-             * 2c+1 of the table */
-            const int j = 4 * hb + jj;
-            const uint32_t wv = words[jj >> 1] >> ((jj & 1) * 16);
-            uint32_t outv[4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint32_t b = (wv >> (8 * h)) & 0xFFu;
-              const uint32_t sel01 = ((b >> 6) & 3u) * 0x22u + ((b >> 4) & 3u) * 0x2200u + 0x1010u;
-              const uint32_t sel23 = ((b >> 2) & 3u) * 0x22u + (b & 3u) * 0x2200u + 0x1010u;
-              outv[2 * h] = __byte_perm(t0, t1, sel01);
-              outv[2 * h + 1] = __byte_perm(t0, t1, sel23);
+            for (int o = 0; o < 8; ++o) {
+              /* codes 8o..8o+7: bytes 2o, 2o+1 of the row's 16 */
+              uint32_t s01, s23, s45, s67;
+              const uint32_t hw = words[o >> 1] >> ((o & 1) * 16);
+              code_selectors(hw & 0xFFu, &s01, &s23);
+              code_selectors((hw >> 8) & 0xFFu, &s45, &s67);
+              *(uint4 *)(dst + (((uint32_t)o ^ sw) << 4)) =
+                  make_uint4(__byte_perm(tab, 0, s01), __byte_perm(tab, 0, s23),
+                             __byte_perm(tab, 0, s45), __byte_perm(tab, 0, s67));
             }
-            *(uint4 *)(row_base + ((j ^ (r & 7)) * 16)) =
-                make_uint4(outv[0], outv[1], outv[2], outv[3]);
+            fence_proxy_async_smem();
           }
-          fence_proxy_async_smem();
-          mbar_arrive(&full[s]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[s]);
         }
       }
     }
   } else {
-    /* ---------------- epilogue: warps 2 + X_DEC_WARPS .. (8 warps) ---------------- */
+    /* ---------------- epilogue: warps 2 + X_DEC_WARPS .. ---------------- */
     const int q = warp & 3, half = (warp - 2 - X_DEC_WARPS) >> 2;
-    const int row = q * 32 + lane;
-    const int col0 = half * 64;
-    const uint32_t t_acc = tmem + ((uint32_t)(q * 32) << 16);
+    const uint32_t t_acc = tmem + ((uint32_t)(q * 32) << 16) + half * XN;
     uint32_t chunk = 0;
     bool ok = true;
     for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-      int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit), rt = w % nrt;
-      int32_t kb0 = ks * kb_per, kb1 = kb0 + kb_per < nkb ? kb0 + kb_per : nkb;
-      int32_t acc[64];
-#pragma unroll
-      for (int u = 0; u < 64; ++u) acc[u] = 0;
+      const int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit), rt = w % nrt;
+      const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      const int32_t row = half * XT + q * 32 + lane;
+      const bool live = rt * XR + row < nrows, any = rt * XR + half * XT + q * 32 < nrows;
+      unsigned long long *out = sums + ((int64_t)rt * nct * tn + (int64_t)ct * tn) * XR + row;
       for (int32_t c0 = kb0; c0 < kb1; c0 += chunk_kb, ++chunk) {
-        uint32_t buf = chunk & 1u, use = chunk >> 1;
-        bool got = mbar_wait(&accf[buf], use & 1u, abort_flag, err, XERR_ACCF);
+        const bool got = mbar_wait(accf, chunk & 1u, abort_flag, err, XERR_ACCF);
         if (!__all_sync(0xffffffffu, got)) {
           ok = false;
           break;
         }
         tc_fence_after();
+        if (any)
+          for (int g = 0; g < tn; g += 16) {
+            uint32_t f[16];
+            tmem_ld16(t_acc + g, f);
+            tmem_wait_ld();
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint32_t f[16];
-          tmem_ld16(t_acc + buf * XT + col0 + 16 * g, f);
-          tmem_wait_ld();
-#pragma unroll
-          for (int v = 0; v < 16; ++v) acc[16 * g + v] += __float2int_rn(__uint_as_float(f[v]));
-        }
+            for (int v = 0; v < 16; ++v) {
+              const long long z = __float2int_rn(__uint_as_float(f[v]));
+              if (live) atomicAdd(out + (int64_t)(g + v) * XR, (unsigned long long)z);
+            }
+          }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[buf]);
-      }
-      if (!ok) break;
-      const int32_t grow = rt * XT + row;
-      if (grow < nrows) {
-        double *zr = zout + (int64_t)grow * ldz;
-#pragma unroll
-        for (int u = 0; u < 64; ++u) {
-          int32_t gc = ct * XT + col0 + u;
-          if (gc < ncols4 && acc[u] != 0) atomicAdd(zr + gc, (double)acc[u]);
-        }
+        if (lane == 0) mbar_arrive(acce);
       }
     }
   }
@@ -325,12 +327,12 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
   if (warp == 1) {
     if (*abort_flag && lane == 0) {
       umma_commit(drain);
-      uint64_t t0 = globaltimer_ns();
+      const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(drain, 0) && globaltimer_ns() - t0 < GP_WAIT_NS) {
       }
     }
     __syncwarp();
-    tmem_dealloc(tmem, 256);
+    tmem_dealloc(tmem, 512);
   }
 }
 
@@ -586,28 +588,49 @@ k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t nc
   }
 }
 
-/* Y[r][c] = 2^e_c sum_t Z[r][Sc+t] 2^(b(S-1-t) - F) */
+/*
+ * Y[r][c] = 2^e_c sum_t Z_t 2^(b(S-1-t) - F) with Z_t the integer sum of row r and slice column
+ * Sc + t (sums as k_geno_panel_tc leaves them: rows contiguous; wcols slice columns per row
+ * tile).  A CTA takes 32 rows x 32 columns through shared memory so that sums are read and Y
+ * written contiguously.
+ */
 template <int S>
-__global__ void k_panel_combine(const double *Z, int64_t ldz, int32_t nrows, int32_t ncols,
-                                const int32_t *expo, double *Y, int64_t ldy,
-                                const gp_tc_batch *db)
+__global__ void __launch_bounds__(256)
+k_panel_combine(const unsigned long long *__restrict__ sums, int32_t wcols, int32_t nrows,
+                int32_t ncols, const int32_t *__restrict__ expo, double *Y, int64_t ldy,
+                const gp_tc_batch *db)
 {
+  __shared__ double sy[32][33];
   if (db) nrows = db->nrows;
-  int64_t total = (int64_t)nrows * ncols;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = idx / ncols;
-    int32_t c = (int32_t)(idx - r * ncols);
-    const double *z = Z + r * ldz + S * c;
-    if (S == 4) {
-      double s = ((z[0] * 0x1p-10 + z[1] * 0x1p-20) + z[2] * 0x1p-30) + z[3] * 0x1p-40;
-      Y[r * ldy + c] = ldexp(s, expo[c]);
-    } else {
-      double s = z[S - 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t nrb = (nrows + 31) / 32, ncb = (ncols + 31) / 32;
+  for (int64_t blk = blockIdx.x; blk < nrb * ncb; blk += gridDim.x) {
+    const int64_t r0 = (blk / ncb) * 32;
+    const int32_t c0 = (int32_t)(blk % ncb) * 32;
+    const unsigned long long *src =
+        sums + (r0 / XR * wcols + (int64_t)S * c0) * XR + r0 % XR + lane;
+    if (r0 + lane < nrows) {
+      for (int cc = warp; cc < 32 && c0 + cc < ncols; cc += 8) {
+        double z[S];
 #pragma unroll
-      for (int t = S - 2; t >= 0; --t) s = fma(s, 0x1p-12, z[t]);
-      Y[r * ldy + c] = expo[c] == X_NONFINITE ? nan("") : ldexp(s, expo[c] - 11);
+        for (int t = 0; t < S; ++t) z[t] = (double)(long long)src[(int64_t)(S * cc + t) * XR];
+        const int e = expo[c0 + cc];
+        if (S == 4) {
+          const double v = ((z[0] * 0x1p-10 + z[1] * 0x1p-20) + z[2] * 0x1p-30) + z[3] * 0x1p-40;
+          sy[cc][lane] = ldexp(v, e);
+        } else {
+          double v = z[S - 1];
+#pragma unroll
+          for (int t = S - 2; t >= 0; --t) v = fma(v, 0x1p-12, z[t]);
+          sy[cc][lane] = e == X_NONFINITE ? nan("") : ldexp(v, e - 11);
+        }
+      }
     }
+    __syncthreads();
+    if (c0 + lane < ncols)
+      for (int rr = warp; rr < 32 && r0 + rr < nrows; rr += 8)
+        Y[(r0 + rr) * ldy + c0 + lane] = sy[lane][rr];
+    __syncthreads();
   }
 }
 
@@ -690,7 +713,8 @@ int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int
 size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits)
 {
   const int32_t kpad0 = (k0 + XK - 1) / XK * XK;
-  const int32_t ncols4_pad = (digits * ncols + XT - 1) / XT * XT;
+  const int32_t tn = x_tile_cols(digits * ncols), nct = (digits * ncols + tn - 1) / tn;
+  const int32_t ncols4_pad = nct * tn;
   return align256((size_t)ncols4_pad * kpad0 * npanels * 2) + align256((size_t)ncols * 16) + 256;
 }
 
@@ -700,7 +724,8 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   if ((digits != 4 && digits != 5) || npanels < 1 || npanels > 2 || ncols < 1 || ncols > 1024 || k0 < 1)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_prepare: bad panel shape");
   const int32_t kb0 = (k0 + XK - 1) / XK, kpad0 = kb0 * XK;
-  const int32_t ncols4 = digits * ncols, ncols4_pad = (ncols4 + XT - 1) / XT * XT;
+  const int32_t ncols4 = digits * ncols, tn = x_tile_cols(ncols4);
+  const int32_t nct = (ncols4 + tn - 1) / tn, ncols4_pad = nct * tn;
   const int64_t ldb = (int64_t)kpad0 * npanels;
   uint8_t *base = (uint8_t *)storage;
   __half *B = (__half *)base;
@@ -729,7 +754,7 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   {
     cuuint64_t dims[2] = {(cuuint64_t)ldb, (cuuint64_t)ncols4_pad};
     cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
-    cuuint32_t box[2] = {XK, XT};
+    cuuint32_t box[2] = {XK, (cuuint32_t)tn};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(&out->tmb, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -739,8 +764,8 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   out->B = B;
   out->expo = expo;
   out->ncols = ncols;
-  out->ncols4 = ncols4;
-  out->ncols4_pad = ncols4_pad;
+  out->tn = tn;
+  out->nct = nct;
   out->npanels = npanels;
   out->digits = digits;
   out->kb0 = kb0;
@@ -751,6 +776,17 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   return GP_OK;
 }
 
+size_t gp_tc_sum_bytes(int32_t slice_cols, int32_t nrows)
+{
+  const size_t tn = (size_t)x_tile_cols(slice_cols), nct = ((size_t)slice_cols + tn - 1) / tn;
+  return sizeof(unsigned long long) * (((size_t)nrows + XR - 1) / XR * XR) * nct * tn;
+}
+
+static int combine_grid(const gp_ctx *ctx, int64_t nrows, int32_t ncols)
+{
+  return grid_cap(ctx, (nrows + 31) / 32 * ((ncols + 31) / 32), 1, 32);
+}
+
 int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, double *d_Y,
                 int64_t ldy, int sync)
 {
@@ -758,36 +794,28 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   if (nrows < 1) return GP_OK;
   if (A->k0 != P->k0 || A->ldc < (int64_t)P->kb0 * XK / 4)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_apply: code operand and panel disagree");
-  const int64_t ldz = P->ncols4_pad;
-  double *Z;
-  int rc = gp_scratch5(ctx, (size_t)nrows * ldz * 8 + 256, (void **)&Z);
+  const size_t sum_bytes = gp_tc_sum_bytes(P->digits * P->ncols, nrows);
+  unsigned long long *sums;
+  int rc = gp_scratch5(ctx, sum_bytes + 256, (void **)&sums);
   if (rc) return rc;
   int *d_err = ctx->d_err;
   if (sync) GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
-  GP_CUDA(ctx, cudaMemsetAsync(Z, 0, (size_t)nrows * ldz * 8, ctx->stream));
+  GP_CUDA(ctx, cudaMemsetAsync(sums, 0, sum_bytes, ctx->stream));
   GP_CUDA(ctx, cudaFuncSetAttribute(k_geno_panel_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     X_SMEM));
   const int32_t nkb = P->kb0 * P->npanels;
-  const int32_t nrt = (nrows + XT - 1) / XT, nct = P->ncols4_pad / XT;
-  int32_t tiles = nrt * nct;
-  int32_t ksplit = 1;
-  while (tiles * ksplit < 2 * ctx->num_sms && ksplit * 4 <= nkb) ksplit *= 2;
-  while ((int64_t)((nkb + ksplit - 1) / ksplit) * XK > X_MAX_K(P->digits)) ksplit *= 2;
-  int32_t nitems = tiles * ksplit;
-  int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
-  k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(P->tmb, A->codes, A->ldc, A->row_map,
-                                                           nrows, P->ncols4, nkb, P->kb0, P->kb0,
-                                                           P->lut_lo, P->lut_hi, ksplit,
-                                                           X_CHUNK_KB(P->digits), Z, ldz, d_err,
-                                                           NULL);
+  const int32_t tiles = (nrows + XR - 1) / XR * P->nct;
+  const int32_t ksplit = x_split(tiles, nkb, ctx->num_sms);
+  const int32_t nitems = tiles * ksplit;
+  const int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
+  k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(
+      P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->lut_lo, P->lut_hi,
+      ksplit, X_CHUNK_KB(P->digits), sums, d_err, NULL);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
-  {
-    int64_t work = (int64_t)nrows * P->ncols;
-    (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
-        <<<grid_cap(ctx, work, 256, 32), 256, 0, ctx->stream>>>(Z, ldz, nrows, P->ncols, P->expo,
-                                                                d_Y, ldy, NULL);
-    GP_LAUNCH_CHECK(ctx, "k_panel_combine");
-  }
+  (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
+      <<<combine_grid(ctx, nrows, P->ncols), 256, 0, ctx->stream>>>(
+          sums, P->nct * P->tn, nrows, P->ncols, P->expo, d_Y, ldy, NULL);
+  GP_LAUNCH_CHECK(ctx, "k_panel_combine");
   if (!sync) return GP_OK;
   int herr = 0;
   GP_CUDA(ctx, gp_memcpy(ctx, &herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -796,35 +824,35 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   return GP_OK;
 }
 
-/* Z[r][c] = 0 for the batch's rows */
-__global__ void k_zero_batch_rows(double *Z, int64_t ldz, const gp_tc_batch *db)
+/* the sums of the batch's row tiles = 0 */
+__global__ void k_zero_batch_sums(unsigned long long *sums, int32_t wcols, const gp_tc_batch *db)
 {
-  const int64_t total = (int64_t)db->nrows * ldz;
+  const int64_t total = (int64_t)((db->nrows + XR - 1) / XR) * wcols * (XR / 2);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x)
-    Z[i] = 0.0;
+    ((ulonglong2 *)sums)[i] = make_ulonglong2(0, 0);
 }
 
 int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_t ldc,
-                    const gp_tc_prepared *P, double *Z, double *d_Y, int64_t ldy)
+                    const gp_tc_prepared *P, void *sums, double *d_Y, int64_t ldy)
 {
   if (max_rows < 1) return GP_OK;
   if (P->digits != 4 || ldc < (int64_t)P->kb0 * XK / 4)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_apply_dev: code rows shorter than the panel");
-  const int64_t ldz = P->ncols4_pad;
-  k_zero_batch_rows<<<grid_cap(ctx, (int64_t)max_rows * ldz, 256, 8), 256, 0, ctx->stream>>>(
-      Z, ldz, db);
-  GP_LAUNCH_CHECK(ctx, "k_zero_batch_rows");
+  unsigned long long *z = (unsigned long long *)sums;
+  const int32_t wcols = P->nct * P->tn;
+  k_zero_batch_sums<<<grid_cap(ctx, ((int64_t)max_rows + XR) * wcols / 2, 256, 8), 256, 0,
+                      ctx->stream>>>(z, wcols, db);
+  GP_LAUNCH_CHECK(ctx, "k_zero_batch_sums");
   GP_CUDA(ctx, cudaFuncSetAttribute(k_geno_panel_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     X_SMEM));
-  const int32_t nkb = P->kb0 * P->npanels;
   /* every SM: the kernel takes the batch's row count, and with it its work items, from db */
   k_geno_panel_tc<<<ctx->num_sms, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, NULL, ldc, NULL, 0, P->ncols4, nkb, P->kb0, P->kb0, P->lut_lo, P->lut_hi, 1,
-      X_CHUNK_KB(4), Z, ldz, ctx->d_err, db);
+      P->tmb, NULL, ldc, NULL, 0, P->tn, P->nct, P->kb0 * P->npanels, P->kb0, P->lut_lo, P->lut_hi,
+      1, X_CHUNK_KB(4), z, ctx->d_err, db);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
-  k_panel_combine<4><<<grid_cap(ctx, (int64_t)max_rows * P->ncols, 256, 32), 256, 0, ctx->stream>>>(
-      Z, ldz, 0, P->ncols, P->expo, d_Y, ldy, db);
+  k_panel_combine<4><<<combine_grid(ctx, max_rows, P->ncols), 256, 0, ctx->stream>>>(
+      z, wcols, 0, P->ncols, P->expo, d_Y, ldy, db);
   GP_LAUNCH_CHECK(ctx, "k_panel_combine");
   return GP_OK;
 }

@@ -35,9 +35,10 @@ int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int
 struct gp_tc_prepared {
   __half *B;
   int32_t *expo;
-  int32_t ncols, ncols4, ncols4_pad, npanels, digits, kb0, k0; /* ncols4: slice columns */
+  int32_t ncols, npanels, digits, kb0, k0;
+  int32_t tn, nct; /* slice columns per tile, column tiles */
   int64_t ldb;
-  uint64_t lut_lo, lut_hi;
+  uint32_t lut_lo, lut_hi;
   CUtensorMap tmb;
 };
 size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits);
@@ -60,10 +61,11 @@ struct gp_tc_batch {
   int64_t row0, req_begin, req_end;
 };
 /* gp_tc_apply inside a loop body: the rows come from db at run time (at most max_rows, row
- * stride ldc); Z holds max_rows * P->ncols4_pad doubles of the caller's; errors of the
- * bounded waits go to ctx->d_err */
+ * stride ldc); sums: gp_tc_sum_bytes(digits * ncols, max_rows) bytes of the caller's;
+ * errors of the bounded waits go to ctx->d_err */
+size_t gp_tc_sum_bytes(int32_t slice_cols, int32_t nrows);
 int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_t ldc,
-                    const gp_tc_prepared *P, double *Z, double *d_Y, int64_t ldy);
+                    const gp_tc_prepared *P, void *sums, double *d_Y, int64_t ldy);
 
 /* the code operand of gp_geno_panel_tc (built into scratch4, or the resident records when a
  * SNP-major operand covers every sample in order) */

@@ -221,22 +221,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r)
       : "r"(taddr));
 }
 
-/*
- * Four 2-bit codes (a byte, first code in the high bits) -> four fp16 values.  Every value of
- * h and o has a zero low byte (0, +-1), so a code picks one byte of a 4-entry table `hi` and
- * the other byte comes from a zero register: the selector of a pair is 0x0404 with the codes
- * in nibbles 1 and 3.
- */
-__device__ __forceinline__ void dec_select(uint32_t b, uint32_t *s01, uint32_t *s23)
-{
-  uint32_t x = (b | (b << 12)) & 0x000F000Fu;  /* codes 0,1 in the upper half, 2,3 below */
-  x = (x | (x << 6)) & 0x03030303u;            /* byte 3: code 0 ... byte 0: code 3 */
-  x = __byte_perm(x, 0, 0x0123);               /* byte 0: code 0 ... byte 3: code 3 */
-  x = (x << 4) | 0x04040404u;
-  *s01 = x;
-  *s23 = x >> 16;
-}
-
 __global__ void __launch_bounds__(EX_THREADS, 1)
 k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t ntiles, int32_t ntj,
              int32_t kb0, int32_t nkb, int32_t ksplit, const uint8_t *__restrict__ B,
@@ -391,13 +375,13 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
                 /* codes 8o..8o+7: bytes 2o, 2o+1 of the row's 16 */
                 uint32_t s01, s23, s45, s67;
                 const uint32_t hw = words[o >> 1] >> ((o & 1) * 16);
-                dec_select(hw & 0xFFu, &s01, &s23);
-                dec_select((hw >> 8) & 0xFFu, &s45, &s67);
+                code_selectors(hw & 0xFFu, &s01, &s23);
+                code_selectors((hw >> 8) & 0xFFu, &s45, &s67);
                 *(uint4 *)(dst + (((uint32_t)o ^ sw) << 4)) =
                     make_uint4(__byte_perm(tab[st], 0, s01), __byte_perm(tab[st], 0, s23),
                                __byte_perm(tab[st], 0, s45), __byte_perm(tab[st], 0, s67));
               }
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              fence_proxy_async_smem();
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);

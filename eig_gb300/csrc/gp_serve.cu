@@ -12,6 +12,7 @@
 #include <string.h>
 #include <time.h>
 
+#include <algorithm>
 #include <deque>
 #include <unordered_map>
 #include <vector>
@@ -116,7 +117,8 @@ struct gp_server {
   double *h_res, *d_res;      /* [pool_cap*K] coordinates at the request rows (mapped) */
   int32_t *h_rst, *d_rst;     /* [pool_cap] statuses (mapped) */
   gp_tc_batch *d_batch;
-  double *d_Z, *d_escale;
+  void *d_Z;
+  double *d_escale;
   cudaGraph_t graph;
   cudaGraphExec_t gexec;
   int loop_running;
@@ -781,7 +783,7 @@ extern "C" int64_t gp_smartpca_footprint(int32_t nind, int64_t nsnp, int32_t pre
   } else {
     int64_t split = 4 * npad * m;
     if (split > (int64_t)24 << 30) split = (int64_t)24 << 30;
-    const int64_t tc = n * (m / 4 + 16) + m * 1024 + n * 8 * 1024 + 8 * m * 256;
+    const int64_t tc = n * (m / 4 + 16) + m * 1024 + n * 8 * 1024 + 8 * (m + 256) * 256;
     work = split > tc ? split : tc;
   }
   return rec + gram + eig + work + 100 * m + ((int64_t)256 << 20);
@@ -908,10 +910,10 @@ extern "C" int gp_serve_open(gp_ctx *src, const gp_serve_opts *o, gp_server **ou
   }
   if (!s->host_loop) {
     /* the loop's queue and result rows in mapped pinned host memory, its batch state and the
-     * products' slice-column buffer (normal-equation panel: the wider of the two) */
-    const int64_t ncols4_pad = ((int64_t)4 * s->ldp + 127) / 128 * 128;
+     * products' integer sums (of the wider of the two panels) */
     SALLOC(s->d_batch, sizeof(gp_tc_batch));
-    SALLOC(s->d_Z, sizeof(double) * (size_t)s->max_batch * ncols4_pad);
+    SALLOC(s->d_Z, std::max(gp_tc_sum_bytes(4 * s->ldp, s->max_batch),
+                            gp_tc_sum_bytes(4 * K, s->max_batch)));
     SALLOC(s->d_escale, sizeof(double) * K);
     if (e == cudaSuccess)
       e = cudaHostAlloc((void **)&s->hq, sizeof(gp_srv_queue), cudaHostAllocMapped);
@@ -968,9 +970,11 @@ extern "C" int gp_serve_open(gp_ctx *src, const gp_serve_opts *o, gp_server **ou
     rc = gp_tc_prepare(ctx, 1, &pc, s->ldp, s->nk, 4, s->stor_co, &s->Pco);
     gp_tc_panel pr[2] = {{s->d_fE, K, 1.0, 1}, {s->d_mE, K, -1.0, 0}};
     if (!rc) rc = gp_tc_prepare(ctx, 2, pr, K, s->nk, 4, s->stor_rr, &s->Prr);
-    /* the products' slice-column buffer, sized once for the largest batch */
+    /* the products' integer sums, sized once for the largest batch */
     void *z;
-    if (!rc) rc = gp_scratch5(ctx, (size_t)s->max_batch * s->Pco.ncols4_pad * 8 + 256, &z);
+    if (!rc)
+      rc = gp_scratch5(ctx, std::max(gp_tc_sum_bytes(4 * s->ldp, s->max_batch),
+                                     gp_tc_sum_bytes(4 * K, s->max_batch)) + 256, &z);
     if (!rc) {
       e = cudaStreamSynchronize(ctx->stream);
       if (e != cudaSuccess) rc = gp_cuda_fail(ctx, e, "gp_serve_open prepare");

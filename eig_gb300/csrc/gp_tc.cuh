@@ -148,6 +148,28 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map)
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
 
+/* generic-proxy writes to shared memory become visible to the tensor core's reads */
+__device__ __forceinline__ void fence_proxy_async_smem()
+{
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+/*
+ * Selectors of a byte of 2-bit codes (four, the first in the high bits) for __byte_perm of a
+ * table register with a zero register: two fp16 values per selector.  The table holds the high
+ * bytes of the values of codes 0-3 (byte 0 first), whose low bytes are zero; nibbles 1 and 3 of
+ * a selector pick high bytes by the codes, nibbles 0 and 2 (= 4) the zero register.
+ */
+__device__ __forceinline__ void code_selectors(uint32_t b, uint32_t *s01, uint32_t *s23)
+{
+  uint32_t x = (b | (b << 12)) & 0x000F000Fu; /* codes 0, 1 in the upper half, 2, 3 below */
+  x = (x | (x << 6)) & 0x03030303u;           /* byte 3: code 0 ... byte 0: code 3 */
+  x = __byte_perm(x, 0, 0x0123);              /* byte 0: code 0 ... byte 3: code 3 */
+  x = (x << 4) | 0x04040404u;
+  *s01 = x;
+  *s23 = x >> 16;
+}
+
 /* ---- TMEM ---------------------------------------------------------------------------- */
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols)
