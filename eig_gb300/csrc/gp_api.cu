@@ -798,17 +798,41 @@ static int grid16(const gp_ctx *ctx, int64_t work)
   return (int)(b < ctx->num_sms * 16 ? b : ctx->num_sms * 16);
 }
 
+/* out[rows[r]][j] = w[r][j] */
+__global__ void k_spread_rows(double *out, const double *w, const int32_t *rows, int32_t n, int32_t K)
+{
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < (int64_t)n * K;
+       idx += (int64_t)gridDim.x * blockDim.x)
+    out[(int64_t)rows[idx / K] * K + idx % K] = w[idx];
+}
+
 /* ffvT [nk][K] = fancy (G^T W) - xmean (O^T W) */
 static int weights_tc(gp_ctx *ctx, const kept_tables *kt, const double *d_W, int32_t K, double *d_ffvT)
 {
-  const int32_t n = ctx->nrows, nk = ctx->nkept;
+  const int32_t n = ctx->nrows, nk = ctx->nkept, ni = ctx->nind_all;
+  /* rows that are part of the samples: the resident records serve as the operand all the same,
+   * W zero for the other samples, which cost a product term each; gathering the rows' codes of
+   * every SNP costs about eight (4,000 of 5,000 samples x 200,000 SNPs: 2.7 ms, the products of
+   * all 5,000 0.27 ms each) */
+  const bool spread = n < ni && ni <= 8 * (int64_t)n;
   double *d_yg;
-  int rc = gp_scratch_aux(ctx, sizeof(double) * 2 * (size_t)nk * K, (void **)&d_yg);
+  int rc = gp_scratch_aux(ctx, sizeof(double) * (2 * (size_t)nk + (spread ? ni : 0)) * K,
+                          (void **)&d_yg);
   if (rc) return rc;
   double *d_yo = d_yg + (size_t)nk * K;
   gp_tc_codes A;
-  rc = gp_tc_codes_for(ctx, 0, ctx->d_rows, n, kt->snprec, nk, &A);
-  if (rc) return rc;
+  if (spread) {
+    double *d_Wa = d_yo + (size_t)nk * K;
+    GP_CUDA(ctx, cudaMemsetAsync(d_Wa, 0, sizeof(double) * (size_t)ni * K, ctx->stream));
+    k_spread_rows<<<grid16(ctx, (int64_t)n * K), 256, 0, ctx->stream>>>(d_Wa, d_W, ctx->d_rows, n,
+                                                                        K);
+    GP_LAUNCH_CHECK(ctx, "k_spread_rows");
+    d_W = d_Wa;
+    A = {ctx->d_geno, ctx->rlen_dev, kt->snprec, nk, ni};
+  } else {
+    rc = gp_tc_codes_for(ctx, 0, ctx->d_rows, n, kt->snprec, nk, 1, &A);
+    if (rc) return rc;
+  }
   gp_tc_panel pw = {d_W, K, 1.0, 1};
   rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pw, K, tc_digits(ctx), d_yg, K);
   if (rc) return rc;
@@ -890,7 +914,7 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   /* fxvecs^T[i][j] = xrow_i . ffvecs_j  (fixxrow values g fancy - xmean) */
   if (tc) {
     gp_tc_codes A;
-    rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, kt.snprec, nk, &A);
+    rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, kt.snprec, nk, 1, &A);
     if (!rc) rc = scores_tc(ctx, &A, d_ffvT, K, d_fxT);
     if (rc == GP_ERR_NOMEM && ctx->precision == GP_PREC_FP64) {
       cudaGetLastError();
@@ -1172,7 +1196,9 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
     if (nproj == ctx->nrows && ctx->h_rows &&
         memcmp(samples, ctx->h_rows, sizeof(int32_t) * (size_t)nproj) == 0)
       d_list = ctx->d_rows;
-    rc = gp_tc_codes_for(ctx, 1, d_list, nproj, kt.snprec, nk, &A);
+    int ascending = 1;
+    for (int32_t q = 1; q < nproj; ++q) ascending &= samples[q] > samples[q - 1];
+    rc = gp_tc_codes_for(ctx, 1, d_list, nproj, kt.snprec, nk, ascending, &A);
     gp_tc_panel pc = {d_P, ldp, 1.0, 0};
     if (!rc) rc = gp_geno_panel_tc_codes(ctx, &A, 1, &pc, ldp, tc_digits(ctx), d_co, ldp);
     if (!rc) rc = scores_tc(ctx, &A, d_E, K, d_rr);

@@ -494,7 +494,7 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
     int32_t rows_pad;
     gp_tc_code_bytes(1, n, nk, &ldc, &rows_pad);
     GP_CUDA(ctx, B.get(&codes_samp, (size_t)rows_pad * ldc));
-    rc = gp_tc_build_codes(ctx, 1, ctx->d_rows, n, d_snprec, nk, codes_samp, &A_samp);
+    rc = gp_tc_build_codes(ctx, 1, ctx->d_rows, n, d_snprec, nk, NULL, codes_samp, &A_samp);
     if (rc) return rc;
     if (n == ctx->nind_all) {
       A_snp.codes = ctx->d_geno;
@@ -507,7 +507,7 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
       e = B.get(&codes_snp, (size_t)rows_pad * ldc);
       if (e != cudaSuccess)
         return gp_fail(ctx, GP_ERR_NOMEM, "gp_fastpca: code operand allocation failed");
-      rc = gp_tc_build_codes(ctx, 0, ctx->d_rows, n, d_snprec, nk, codes_snp, &A_snp);
+      rc = gp_tc_build_codes(ctx, 0, ctx->d_rows, n, d_snprec, nk, NULL, codes_snp, &A_snp);
       if (rc) return rc;
     }
   }

@@ -40,9 +40,8 @@
  *   warps 10-17 epilogue: per chunk tcgen05.ld the exact FP32 sums and add them to the tile's
  *               64-bit integer sums in global memory (atomics, 32 rows side by side).
  * The decode of the codes paces it: 128 x 128 tiles decoded each code again for every 128
- * columns and left the tensor pipe a quarter busy (the normal equations of 5,000 samples x 200,000
- * SNPs, K = 20: 2.98 ms; with
- * 256 x 256 tiles 1.41, 1.3 PFLOP/s).
+ * columns and left the tensor pipe a quarter busy (the normal equations of 5,000 samples x
+ * 200,000 SNPs, K = 20: 2.98 ms; with 256 x 256 tiles 1.41, 1.3 PFLOP/s).
  */
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -412,6 +411,80 @@ k_codes_by_sample(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
   }
 }
 
+/* inv[samp[r]] = r (inv preset to -1) */
+__global__ void k_invert_rows(const int32_t *samp, int32_t nsamp, int32_t *inv)
+{
+  for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nsamp; r += gridDim.x * blockDim.x)
+    inv[samp[r]] = r;
+}
+
+/*
+ * The same operand for rows that are distinct samples: all samples are transposed, the selected
+ * ones written to their rows (inv).  A CTA covers 512 samples x 128 SNPs; a thread holds a word
+ * (16 samples) of 16 SNPs and transposes the 16 x 16 codes in registers: the 4 x 4 bytes of
+ * words 4 apart by byte permutes, then the 4 x 4 codes of neighbouring words by masked swaps,
+ * about half an instruction per code; pieces of 32 bytes per row leave through shared memory.
+ * HBM bounds it (5,000 x 200,000: 120 us for 500 MB; a code at a time as below: 734).
+ */
+#define CT_W 32
+__global__ void __launch_bounds__(256)
+k_codes_transpose(const uint8_t *__restrict__ geno, int64_t rlen, int32_t nind,
+                  const int32_t *__restrict__ inv, const int32_t *__restrict__ snprec, int32_t nk,
+                  int64_t ldc, uint8_t *codes)
+{
+  __shared__ uint32_t so[16 * CT_W][9];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int32_t k0 = (int32_t)blockIdx.x * 128;
+  const int64_t w = (int64_t)blockIdx.y * CT_W + lane;
+  const bool in = w < (rlen >> 2);
+  uint32_t a[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int32_t k = k0 + 16 * g + i;
+    a[i] = in && k < nk ? __ldg((const uint32_t *)(geno + (int64_t)snprec[k] * rlen) + w)
+                        : 0xFFFFFFFFu;
+  }
+  /* x[J][ii]: byte I = byte J of word 4 I + ii */
+  uint32_t x[4][4];
+#pragma unroll
+  for (int ii = 0; ii < 4; ++ii) {
+    const uint32_t p0 = __byte_perm(a[ii], a[4 + ii], 0x5140), p1 = __byte_perm(a[8 + ii], a[12 + ii], 0x5140);
+    const uint32_t q0 = __byte_perm(a[ii], a[4 + ii], 0x7362), q1 = __byte_perm(a[8 + ii], a[12 + ii], 0x7362);
+    x[0][ii] = __byte_perm(p0, p1, 0x5410);
+    x[1][ii] = __byte_perm(p0, p1, 0x7632);
+    x[2][ii] = __byte_perm(q0, q1, 0x5410);
+    x[3][ii] = __byte_perm(q0, q1, 0x7632);
+  }
+#pragma unroll
+  for (int J = 0; J < 4; ++J) {
+#pragma unroll
+    for (int ii = 0; ii < 2; ++ii) { /* codes 2, 3 of word ii and 0, 1 of word ii + 2 */
+      const uint32_t t = ((x[J][ii + 2] >> 4) ^ x[J][ii]) & 0x0F0F0F0Fu;
+      x[J][ii] ^= t;
+      x[J][ii + 2] ^= t << 4;
+    }
+#pragma unroll
+    for (int ii = 0; ii < 4; ii += 2) { /* codes 1, 3 of word ii and 0, 2 of word ii + 1 */
+      const uint32_t t = ((x[J][ii + 1] >> 2) ^ x[J][ii]) & 0x33333333u;
+      x[J][ii] ^= t;
+      x[J][ii + 1] ^= t << 2;
+    }
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) so[(4 * J + jj) * CT_W + lane][g] = x[J][jj];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * 16 * CT_W; i += blockDim.x) {
+    const int idx = i >> 1, half = i & 1;
+    const int64_t q = ((int64_t)blockIdx.y * CT_W + (idx & (CT_W - 1))) * 16 + idx / CT_W;
+    const int64_t at = (k0 >> 2) + 16 * half;
+    if (q >= nind || at >= ldc) continue;
+    const int32_t r = inv[q];
+    if (r < 0) continue;
+    const uint32_t *o = so[idx] + 4 * half;
+    *(uint4 *)(codes + (int64_t)r * ldc + at) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 /*
  * sum over samples: codes[k][j] = code of sample samp[j] at kept SNP k; one row per kept
  * SNP, j over the nsamp samples; pad j and pad rows are 3.  One warp per SNP row: the
@@ -673,12 +746,24 @@ int gp_tc_code_bytes(int sum_over_snps, int32_t nsamp, int32_t nk, int64_t *ldc,
 }
 
 int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                      const int32_t *d_snprec, int32_t nk, uint8_t *codes, gp_tc_codes *out)
+                      const int32_t *d_snprec, int32_t nk, int32_t *inv, uint8_t *codes,
+                      gp_tc_codes *out)
 {
   int64_t ldc;
   int32_t nrows_pad;
   gp_tc_code_bytes(sum_over_snps, nsamp, nk, &ldc, &nrows_pad);
-  if (sum_over_snps) {
+  /* transposing every sample reads and shuffles nind_all / nsamp times the codes that are kept;
+   * measured six times as fast per code as gathering them (all of 5,000 x 200,000: 120 us and
+   * 734) */
+  if (sum_over_snps && inv && ctx->nind_all <= 4 * (int64_t)nsamp) {
+    GP_CUDA(ctx, cudaMemsetAsync(inv, 0xFF, sizeof(int32_t) * (size_t)ctx->nind_all, ctx->stream));
+    k_invert_rows<<<grid_cap(ctx, nsamp, 256, 4), 256, 0, ctx->stream>>>(d_samp, nsamp, inv);
+    GP_LAUNCH_CHECK(ctx, "k_invert_rows");
+    dim3 grid((unsigned)((ldc * 4 + 127) / 128),
+              (unsigned)((ctx->rlen_dev / 4 + CT_W - 1) / CT_W));
+    k_codes_transpose<<<grid, 256, 0, ctx->stream>>>(ctx->d_geno, ctx->rlen_dev, ctx->nind_all, inv,
+                                                     d_snprec, nk, ldc, codes);
+  } else if (sum_over_snps) {
     /* about 16 CTAs per SM in all; each walks the SNP tiles of its row block */
     const int64_t nkt = (ldc * 4 + CB_SNP - 1) / CB_SNP, nrb = (nrows_pad + CB_ROWS - 1) / CB_ROWS;
     int64_t gx = ((int64_t)ctx->num_sms * 16 + nrb - 1) / nrb;
@@ -882,7 +967,7 @@ int gp_geno_panel_tc_codes(gp_ctx *ctx, const gp_tc_codes *A, int npanels, const
 }
 
 int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                    const int32_t *d_snprec, int32_t nk, gp_tc_codes *out)
+                    const int32_t *d_snprec, int32_t nk, int distinct, gp_tc_codes *out)
 {
   const int current_rows = sum_over_snps && d_samp == ctx->d_rows && nsamp == ctx->nrows &&
                            nk == ctx->nkept;
@@ -911,20 +996,11 @@ int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32
   int32_t rows_pad;
   gp_tc_code_bytes(sum_over_snps, nsamp, nk, &ldc, &rows_pad);
   uint8_t *codes;
-  int rc = gp_scratch4(ctx, (size_t)rows_pad * ldc + 256, (void **)&codes);
+  const size_t cb = align256((size_t)rows_pad * ldc + 256);
+  int rc = gp_scratch4(ctx, cb + sizeof(int32_t) * (size_t)ctx->nind_all, (void **)&codes);
   if (rc) return rc;
-  rc = gp_tc_build_codes(ctx, sum_over_snps, d_samp, nsamp, d_snprec, nk, codes, out);
+  rc = gp_tc_build_codes(ctx, sum_over_snps, d_samp, nsamp, d_snprec, nk,
+                         distinct ? (int32_t *)(codes + cb) : NULL, codes, out);
   if (!rc && current_rows) ctx->codes4_rows = 1;
   return rc;
-}
-
-int gp_geno_panel_tc(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                     const int32_t *d_snprec, int32_t nk, int npanels, const gp_tc_panel *pp,
-                     int32_t ncols, int digits, double *d_Y, int64_t ldy)
-{
-  if ((sum_over_snps ? nsamp : nk) < 1 || (sum_over_snps ? nk : nsamp) < 1) return GP_OK;
-  gp_tc_codes A;
-  int rc = gp_tc_codes_for(ctx, sum_over_snps, d_samp, nsamp, d_snprec, nk, &A);
-  if (rc) return rc;
-  return gp_geno_panel_tc_codes(ctx, &A, npanels, pp, ncols, digits, d_Y, ldy);
 }

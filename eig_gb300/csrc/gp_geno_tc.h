@@ -26,10 +26,13 @@ struct gp_tc_codes {
   int32_t k0;
 };
 
+/* inv: room for nind_all integers when the samples of a sum over SNPs are distinct (the faster
+ * transpose then applies), or NULL */
 /* bytes of the code operand built by gp_tc_build_codes: rows_pad * ldc */
 int gp_tc_code_bytes(int sum_over_snps, int32_t nsamp, int32_t nk, int64_t *ldc, int32_t *rows_pad);
 int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                      const int32_t *d_snprec, int32_t nk, uint8_t *codes, gp_tc_codes *out);
+                      const int32_t *d_snprec, int32_t nk, int32_t *inv, uint8_t *codes,
+                      gp_tc_codes *out);
 /* a panel cut into fp16 slices once (B operand + column exponents + its tensor map): `digits`
  * slices, 4 of 10 bits (the split precisions) or 5 of 12 bits (FP64) */
 struct gp_tc_prepared {
@@ -67,22 +70,16 @@ size_t gp_tc_sum_bytes(int32_t slice_cols, int32_t nrows);
 int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_t ldc,
                     const gp_tc_prepared *P, void *sums, double *d_Y, int64_t ldy);
 
-/* the code operand of gp_geno_panel_tc (built into scratch4, or the resident records when a
- * SNP-major operand covers every sample in order) */
+/* the code operand of a sum over SNPs (rows = samples d_samp) or over samples (rows = SNPs),
+ * built into scratch4, or the resident records when a SNP-major operand covers every sample in
+ * order; distinct: no sample occurs twice in d_samp */
 int gp_tc_codes_for(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                    const int32_t *d_snprec, int32_t nk, gp_tc_codes *out);
-/* Y[r][c] = sum_p sum_k A(r, k) sign_p P_p[k][c] with a prepared code operand; ncols <= 1024
- * with 4 digits, any number with 5 */
+                    const int32_t *d_snprec, int32_t nk, int distinct, gp_tc_codes *out);
+/* Y[r][c] = sum_p sum_k A_p(r, k) sign_p P_p[k][c] with a prepared code operand: npanels (1 or
+ * 2) panels share the k extent and are concatenated along k with one joint column scale; Y is
+ * device FP64 with row stride ldy; ncols <= 1024 with 4 digits, any number with 5.  Uses
+ * scratch2 and scratch5. */
 int gp_geno_panel_tc_codes(gp_ctx *ctx, const gp_tc_codes *A, int npanels, const gp_tc_panel *pp,
                            int32_t ncols, int digits, double *d_Y, int64_t ldy);
 
-/*
- * sum_over_snps = 1: Y[q][c] = sum_p sum_{s < nk} A_p(samp[q], snprec[s]) sign_p P_p[s][c]
- * sum_over_snps = 0: Y[s][c] = sum_p sum_{q < nsamp} A_p(samp[q], snprec[s]) sign_p P_p[q][c]
- * npanels (1 or 2) panels share the k extent and are concatenated along k with one joint
- * column scale.  Y is device FP64 with row stride ldy.  Uses scratch2.
- */
-int gp_geno_panel_tc(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
-                     const int32_t *d_snprec, int32_t nk, int npanels, const gp_tc_panel *pp,
-                     int32_t ncols, int digits, double *d_Y, int64_t ldy);
 #endif

@@ -552,7 +552,7 @@ int gp_gram_exact(gp_ctx *ctx)
                                                ctx->d_xfancy, snprec, mx);
   GP_LAUNCH_CHECK(ctx, "k_exact_max");
   gp_tc_codes A;
-  rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, snprec, nk, &A);
+  rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, snprec, nk, 1, &A);
   if (rc) return rc;
   GP_CUDA(ctx, cudaFuncSetAttribute(k_gram_exact, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     EX_SMEM));
