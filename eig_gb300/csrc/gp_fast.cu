@@ -125,36 +125,40 @@ __global__ void k_fast_vtab(const int32_t *kept, int32_t nk, const int32_t *cols
   }
 }
 
-#define TSG_T 32     /* cross-product tile edge */
+#define TSG_T 32     /* cross-product tile edge at most */
 #define TSG_R 64     /* rows staged per step */
 
 /*
  * Partial cross products of two tall-skinny row-major matrices A (n x ca, row stride lda) and
- * B (n x cb, row stride ldb): CTA (p, q) computes the 32 x 32 tile p of A^T B over the rows of
+ * B (n x cb, row stride ldb): CTA (p, q) computes the tile p of A^T B over the rows of
  * chunk q and writes it to part[q][i][j] (ca x cb); k_ts_reduce sums the chunks in order
- * (deterministic).
+ * (deterministic).  The FP64 pipe bounds it, so a tile is no wider than the matrix: th x tw
+ * threads of 2 x 2 outputs, 10 x 10 for blocks of 20 columns (a fixed 16 x 16 spent 2.6 times
+ * the multiplications there), and the chunks are short enough for eight CTAs per SM (with
+ * chunks of at least 2,048 rows a 20 x 20 product over 100,000 rows had 49 CTAs: 642 us, now
+ * 113).
  */
 __global__ void __launch_bounds__(256)
 k_ts_cross(const double *__restrict__ A, int64_t lda, int32_t ca, const double *__restrict__ B,
-           int64_t ldb, int32_t cb, int64_t n, int64_t chunk, double *part)
+           int64_t ldb, int32_t cb, int64_t n, int64_t chunk, int32_t th, int32_t tw, double *part)
 {
   __shared__ double As[TSG_R][TSG_T + 1];
   __shared__ double Bs[TSG_R][TSG_T + 1];
-  const int32_t tb = (cb + TSG_T - 1) / TSG_T;
+  const int32_t tb = (cb + 2 * tw - 1) / (2 * tw);
   const int32_t ti = (int32_t)blockIdx.x / tb, tj = (int32_t)blockIdx.x - ti * tb;
-  const int32_t c0 = ti * TSG_T, d0 = tj * TSG_T;
+  const int32_t c0 = ti * 2 * th, d0 = tj * 2 * tw;
   const int64_t r0 = (int64_t)blockIdx.y * chunk;
   const int64_t r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x, ty = tid / tw, tx = tid - ty * tw;
   double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
   for (int64_t rs = r0; rs < r1; rs += TSG_R) {
-    for (int e = tid; e < TSG_R * TSG_T; e += 256) {
+    for (int e = tid; e < TSG_R * TSG_T; e += blockDim.x) {
       const int rr = e / TSG_T, cc = e - rr * TSG_T;
       const int64_t r = rs + rr;
       double va = 0.0, vb = 0.0;
       if (r < r1) {
-        if (c0 + cc < ca) va = A[r * lda + c0 + cc];
-        if (d0 + cc < cb) vb = B[r * ldb + d0 + cc];
+        if (cc < 2 * th && c0 + cc < ca) va = A[r * lda + c0 + cc];
+        if (cc < 2 * tw && d0 + cc < cb) vb = B[r * ldb + d0 + cc];
       }
       As[rr][cc] = va;
       Bs[rr][cc] = vb;
@@ -162,8 +166,8 @@ k_ts_cross(const double *__restrict__ A, int64_t lda, int32_t ca, const double *
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < TSG_R; ++k) {
-      const double a0 = As[k][ty], a1 = As[k][ty + 16];
-      const double b0 = Bs[k][tx], b1 = Bs[k][tx + 16];
+      const double a0 = As[k][ty], a1 = As[k][ty + th];
+      const double b0 = Bs[k][tx], b1 = Bs[k][tx + tw];
       acc[0][0] = fma(a0, b0, acc[0][0]);
       acc[0][1] = fma(a0, b1, acc[0][1]);
       acc[1][0] = fma(a1, b0, acc[1][0]);
@@ -176,18 +180,28 @@ k_ts_cross(const double *__restrict__ A, int64_t lda, int32_t ca, const double *
   for (int u = 0; u < 2; ++u)
 #pragma unroll
     for (int v = 0; v < 2; ++v) {
-      const int32_t i = c0 + ty + 16 * u, j = d0 + tx + 16 * v;
+      const int32_t i = c0 + ty + th * u, j = d0 + tx + tw * v;
       if (i < ca && j < cb) o[(int64_t)i * cb + j] = acc[u][v];
     }
 }
 
-/* out[i][j] = sum over the chunks, in order, of part[q][i][j] (count = ca * cb) */
-__global__ void k_ts_reduce(double *out, const double *part, int32_t nchunk, int64_t count)
+/* out[i][j] = sum over the chunks of part[q][i][j] (count = ca * cb): a CTA takes 32 entries,
+ * each of its 8 warps an eighth of the chunks in order, then the eighths in order */
+__global__ void __launch_bounds__(256)
+k_ts_reduce(double *out, const double *part, int32_t nchunk, int64_t count)
 {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < count;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (int32_t q = 0; q < nchunk; ++q) acc += part[(int64_t)q * count + idx];
+  __shared__ double sp[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t idx = blockIdx.x * (int64_t)32 + lane;
+  const int32_t per = (nchunk + 7) / 8, q0 = warp * per;
+  const int32_t q1 = q0 + per < nchunk ? q0 + per : nchunk;
+  double acc = 0.0;
+  if (idx < count)
+    for (int32_t q = q0; q < q1; ++q) acc += part[(int64_t)q * count + idx];
+  sp[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0 && idx < count) {
+    for (int w = 1; w < 8; ++w) acc += sp[w][lane];
     out[idx] = acc;
   }
 }
@@ -210,70 +224,91 @@ __global__ void k_ts_project(double *Q, const double *__restrict__ Qp, int64_t l
 #define JAC_MAX 64 /* largest block width of the Jacobi kernel */
 
 /*
- * One block: the L x L matrix W (symmetrised) is diagonalised by cyclic Jacobi rotations
- * (Golub & Van Loan, Matrix Computations, 8.5: the symmetric Schur decomposition of each
- * 2 x 2 pivot), W = V diag(s) V^T, and T = V diag(s^-1/2) is written for the directions with
+ * One block: the L x L matrix W (symmetrised) is diagonalised by Jacobi rotations (Golub & Van
+ * Loan, Matrix Computations, 8.5: the symmetric Schur decomposition of each 2 x 2 pivot),
+ * W = V diag(s) V^T, and T = V diag(s^-1/2) is written for the directions with
  * s > tol * max(pre[j][j]) (max(W[j][j]) when pre is NULL; zero columns for the others).  A
  * pivot is rotated while |W_pq| > 1e-15 sqrt(|W_pp W_qq|), the threshold that keeps the small
  * eigenvalues of a positive semidefinite W to high relative accuracy (Demmel & Veselic, 1992);
- * the sweeps stop after one without a rotation, at most 40.
+ * the sweeps stop after one without a rotation, at most 40.  A sweep runs in the rounds of a
+ * round-robin tournament (the parallel ordering of Brent & Luk): L/2 disjoint pivots at once,
+ * their rotations side by side, then every 2 x 2 block of W by its two pivots' rotations.  The
+ * latency of the FP64 square roots and divisions bounds it: one pivot after another, L = 20
+ * took 3.3 ms, now 0.46.
  */
-__global__ void __launch_bounds__(JAC_MAX)
+#define JAC_THREADS 256
+__global__ void __launch_bounds__(JAC_THREADS)
 k_block_orth(const double *__restrict__ Wg, const double *__restrict__ pre, int32_t L,
              double tol, double *T)
 {
   __shared__ double W[JAC_MAX][JAC_MAX + 1];
   __shared__ double V[JAC_MAX][JAC_MAX + 1];
-  __shared__ double cs[2];
-  __shared__ int nrot;
+  __shared__ double sc[JAC_MAX / 2], ss[JAC_MAX / 2];
+  __shared__ int sp[JAC_MAX / 2], sq[JAC_MAX / 2];
   const int t = threadIdx.x;
-  for (int i = 0; i < L; ++i)
-    if (t < L) {
-      W[i][t] = 0.5 * (Wg[(int64_t)i * L + t] + Wg[(int64_t)t * L + i]);
-      V[i][t] = i == t ? 1.0 : 0.0;
-    }
+  const int np = (L + 1) / 2, M = 2 * np - 1; /* pairs per round, rounds; index L: a bye */
+  for (int e = t; e < L * L; e += blockDim.x) {
+    const int i = e / L, j = e - i * L;
+    W[i][j] = 0.5 * (Wg[(int64_t)i * L + j] + Wg[(int64_t)j * L + i]);
+    V[i][j] = i == j ? 1.0 : 0.0;
+  }
   __syncthreads();
   for (int sweep = 0; sweep < 40; ++sweep) {
-    if (t == 0) nrot = 0;
-    __syncthreads();
-    for (int p = 0; p < L - 1; ++p)
-      for (int q = p + 1; q < L; ++q) {
-        if (t == 0) {
+    int rotated = 0;
+    for (int r = 0; r < M; ++r) {
+      int rot = 0;
+      if (t < np) {
+        int p = t == 0 ? M : (r + t) % M, q = t == 0 ? r : (r - t + M) % M;
+        if (p > q) {
+          const int o = p;
+          p = q;
+          q = o;
+        }
+        double c = 1.0, sn = 0.0;
+        if (q < L) {
           const double apq = W[p][q];
-          double c = 1.0, sn = 0.0;
           if (apq != 0.0 && fabs(apq) > 1e-15 * sqrt(fabs(W[p][p] * W[q][q]))) {
             const double tau = (W[q][q] - W[p][p]) / (2.0 * apq);
             const double tt = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
             c = 1.0 / sqrt(1.0 + tt * tt);
             sn = tt * c;
-            ++nrot;
-          }
-          cs[0] = c;
-          cs[1] = sn;
-        }
-        __syncthreads();
-        const double c = cs[0], sn = cs[1];
-        if (sn != 0.0) {
-          if (t < L) { /* rows p, q: W := J^T W */
-            const double wp = W[p][t], wq = W[q][t];
-            W[p][t] = c * wp - sn * wq;
-            W[q][t] = sn * wp + c * wq;
-          }
-          __syncthreads();
-          if (t < L) { /* columns p, q: W := W J, V := V J */
-            const double wp = W[t][p], wq = W[t][q];
-            W[t][p] = c * wp - sn * wq;
-            W[t][q] = sn * wp + c * wq;
-            const double vp = V[t][p], vq = V[t][q];
-            V[t][p] = c * vp - sn * vq;
-            V[t][q] = sn * vp + c * vq;
+            rot = 1;
           }
         }
-        __syncthreads();
+        sc[t] = c;
+        ss[t] = sn;
+        sp[t] = p;
+        sq[t] = q;
       }
-    const bool done = nrot == 0;
-    __syncthreads();
-    if (done) break;
+      if (!__syncthreads_or(rot)) continue;
+      rotated = 1;
+      /* W := J^T W J: the block of pairs (a, b) belongs to one thread */
+      for (int e = t; e < np * np; e += blockDim.x) {
+        const int a = e / np, b = e - a * np;
+        const double ca = sc[a], sa = ss[a], cb = sc[b], sb = ss[b];
+        if (sa == 0.0 && sb == 0.0) continue;
+        const int p = sp[a], q = sq[a], u = sp[b], v = sq[b];
+        const bool hq = q < L, hv = v < L;
+        double wpu = W[p][u], wpv = hv ? W[p][v] : 0.0;
+        double wqu = hq ? W[q][u] : 0.0, wqv = hq && hv ? W[q][v] : 0.0;
+        const double pu = ca * wpu - sa * wqu, qu = sa * wpu + ca * wqu;
+        const double pv = ca * wpv - sa * wqv, qv = sa * wpv + ca * wqv;
+        W[p][u] = cb * pu - sb * pv;
+        if (hv) W[p][v] = sb * pu + cb * pv;
+        if (hq) W[q][u] = cb * qu - sb * qv;
+        if (hq && hv) W[q][v] = sb * qu + cb * qv;
+      }
+      for (int e = t; e < np * L; e += blockDim.x) { /* V := V J */
+        const int i = e / np, a = e - i * np;
+        const double sn = ss[a], c = sc[a];
+        if (sn == 0.0) continue;
+        const double vp = V[i][sp[a]], vq = V[i][sq[a]];
+        V[i][sp[a]] = c * vp - sn * vq;
+        V[i][sq[a]] = sn * vp + c * vq;
+      }
+      __syncthreads();
+    }
+    if (!rotated) break; /* the same for every thread */
   }
   double pmax = 0.0;
   for (int i = 0; i < L; ++i)
@@ -359,21 +394,20 @@ static int ts_cross(gp_ctx *ctx, const double *A, int64_t lda, int32_t ca, const
                     int64_t ldb, int32_t cb, int64_t n, double *part, size_t part_cap,
                     double *out)
 {
-  const int32_t ntiles = ((ca + TSG_T - 1) / TSG_T) * ((cb + TSG_T - 1) / TSG_T);
-  int64_t want = ((int64_t)ctx->num_sms * 4 + ntiles - 1) / ntiles;
-  int64_t chunk = (n + want - 1) / want;
-  if (chunk < 2048) chunk = 2048;
+  const int32_t th = ((ca < TSG_T ? ca : TSG_T) + 1) / 2, tw = ((cb < TSG_T ? cb : TSG_T) + 1) / 2;
+  const int32_t ntiles = ((ca + 2 * th - 1) / (2 * th)) * ((cb + 2 * tw - 1) / (2 * tw));
+  int64_t want = ((int64_t)ctx->num_sms * 8 + ntiles - 1) / ntiles;
+  int64_t chunk = ((n + want - 1) / want + TSG_R - 1) / TSG_R * TSG_R;
   int64_t nchunk = (n + chunk - 1) / chunk;
   while ((size_t)(nchunk * ca * cb) > part_cap) { /* fewer, longer chunks when space is short */
     chunk *= 2;
     nchunk = (n + chunk - 1) / chunk;
   }
   dim3 grid((unsigned)ntiles, (unsigned)nchunk);
-  k_ts_cross<<<grid, 256, 0, ctx->stream>>>(A, lda, ca, B, ldb, cb, n, chunk, part);
+  k_ts_cross<<<grid, th * tw, 0, ctx->stream>>>(A, lda, ca, B, ldb, cb, n, chunk, th, tw, part);
   GP_LAUNCH_CHECK(ctx, "k_ts_cross");
-  k_ts_reduce<<<grid_for_fast(ctx, (int64_t)ca * cb), 256, 0, ctx->stream>>>(out, part,
-                                                                             (int32_t)nchunk,
-                                                                             (int64_t)ca * cb);
+  k_ts_reduce<<<(unsigned)(((int64_t)ca * cb + 31) / 32), 256, 0, ctx->stream>>>(
+      out, part, (int32_t)nchunk, (int64_t)ca * cb);
   GP_LAUNCH_CHECK(ctx, "k_ts_reduce");
   return GP_OK;
 }
@@ -382,21 +416,16 @@ static int ts_cross(gp_ctx *ctx, const double *A, int64_t lda, int32_t ca, const
  * projection is below 1e-10 of the block's norm before it (s is a squared norm) */
 #define GP_FAST_DEP_TOL 1e-20
 
-/* device buffers of one gp_fastpca call, freed together */
+/* the device buffers of one gp_fastpca call, side by side in the handle's aux scratch (kept
+ * there for the next call instead of 17 allocations and releases per call): counted with
+ * base == NULL, then placed */
 struct fast_bufs {
-  std::vector<void *> p;
-  ~fast_bufs()
+  uint8_t *base = NULL;
+  size_t used = 0;
+  template <class T> void get(T **out, size_t count)
   {
-    for (void *q : p)
-      if (q) cudaFree(q);
-  }
-  template <class T> cudaError_t get(T **out, size_t count)
-  {
-    void *q = NULL;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T) + 256);
-    p.push_back(q);
-    *out = (T *)q;
-    return e;
+    *out = (T *)(base + used);
+    used += (count * sizeof(T) + 255) / 256 * 256;
   }
 };
 
@@ -441,33 +470,45 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
    * partials and the small matrices */
   const size_t nG = (size_t)n * L, nQ = (size_t)nk * L;
   const int64_t nmax = n > nk ? n : nk;
-  /* chunk partials: ts_cross takes chunks of at least 2,048 rows and about four CTAs per SM
-   * (it lengthens the chunks when this is short) */
+  /* chunk partials of about eight CTAs per SM (ts_cross lengthens the chunks when this is
+   * short) */
   const size_t part_cap = (size_t)c4 * c4 + ((size_t)nmax / 2048 + 2) * (size_t)c4 * L +
-                          (size_t)4 * ctx->num_sms * TSG_T * TSG_T + 4096;
+                          (size_t)8 * ctx->num_sms * TSG_T * TSG_T + 4096;
   fast_bufs B;
   double *d_Qp, *d_Hp, *d_G, *d_Q, *d_Y1, *d_Y2, *d_part, *d_C, *d_W, *d_pre, *d_T, *d_mu,
       *d_U, *d_ev, *d_vt;
   int32_t *d_snprec;
-  cudaError_t e = B.get(&d_Qp, (size_t)nk * c4);
-  if (e == cudaSuccess) e = B.get(&d_Hp, (size_t)n * c4);
-  if (e == cudaSuccess) e = B.get(&d_G, nG);
-  if (e == cudaSuccess) e = B.get(&d_Q, nQ);
-  if (e == cudaSuccess) e = B.get(&d_Y1, nQ);
-  if (e == cudaSuccess) e = B.get(&d_Y2, nQ);
-  if (e == cudaSuccess) e = B.get(&d_part, part_cap);
-  if (e == cudaSuccess) e = B.get(&d_C, (size_t)c4 * c4);
-  if (e == cudaSuccess) e = B.get(&d_W, (size_t)L * L);
-  if (e == cudaSuccess) e = B.get(&d_pre, (size_t)L * L);
-  if (e == cudaSuccess) e = B.get(&d_T, (size_t)L * L);
-  if (e == cudaSuccess) e = B.get(&d_mu, (size_t)c4);
-  if (e == cudaSuccess) e = B.get(&d_U, (size_t)K * c4);
-  if (e == cudaSuccess) e = B.get(&d_ev, (size_t)n * K);
-  if (e == cudaSuccess) e = B.get(&d_vt, 4 * (size_t)nk);
-  if (e == cudaSuccess) e = B.get(&d_snprec, (size_t)nk);
-  if (e != cudaSuccess)
-    return gp_fail(ctx, GP_ERR_NOMEM, "gp_fastpca: device allocation failed: %s",
-                   cudaGetErrorString(e));
+  uint8_t *codes_samp = NULL, *codes_snp = NULL;
+  int64_t ldc_samp, ldc_snp;
+  int32_t pad_samp, pad_snp, *d_inv = NULL;
+  gp_tc_code_bytes(1, n, nk, &ldc_samp, &pad_samp);
+  gp_tc_code_bytes(0, n, nk, &ldc_snp, &pad_snp);
+  for (int pass = 0; pass < 2; ++pass) {
+    B.used = 0;
+    B.get(&d_Qp, (size_t)nk * c4);
+    B.get(&d_Hp, (size_t)n * c4);
+    B.get(&d_G, nG);
+    B.get(&d_Q, nQ);
+    B.get(&d_Y1, nQ);
+    B.get(&d_Y2, nQ);
+    B.get(&d_part, part_cap);
+    B.get(&d_C, (size_t)c4 * c4);
+    B.get(&d_W, (size_t)L * L);
+    B.get(&d_pre, (size_t)L * L);
+    B.get(&d_T, (size_t)L * L);
+    B.get(&d_mu, (size_t)c4);
+    B.get(&d_U, (size_t)K * c4);
+    B.get(&d_ev, (size_t)n * K);
+    B.get(&d_vt, 4 * (size_t)nk);
+    B.get(&d_snprec, (size_t)nk);
+    if (use_tc) B.get(&d_inv, (size_t)ctx->nind_all);
+    if (use_tc) B.get(&codes_samp, (size_t)pad_samp * ldc_samp);
+    if (use_tc && n != ctx->nind_all) B.get(&codes_snp, (size_t)pad_snp * ldc_snp);
+    if (pass == 0) {
+      rc = gp_scratch_aux(ctx, B.used, (void **)&B.base);
+      if (rc) return rc;
+    }
+  }
 
   k_fast_vtab<<<grid_for_fast(ctx, nk), 256, 0, ctx->stream>>>(ctx->d_kept, nk, ctx->d_cols,
                                                               ctx->d_vtab, d_snprec, d_vt);
@@ -488,13 +529,8 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
   /* code operands: X G reads SNP rows (the device records when every sample is selected, in
    * order), X^T Q reads sample rows */
   gp_tc_codes A_snp, A_samp;
-  uint8_t *codes_samp = NULL, *codes_snp = NULL;
   if (use_tc) {
-    int64_t ldc;
-    int32_t rows_pad;
-    gp_tc_code_bytes(1, n, nk, &ldc, &rows_pad);
-    GP_CUDA(ctx, B.get(&codes_samp, (size_t)rows_pad * ldc));
-    rc = gp_tc_build_codes(ctx, 1, ctx->d_rows, n, d_snprec, nk, NULL, codes_samp, &A_samp);
+    rc = gp_tc_build_codes(ctx, 1, ctx->d_rows, n, d_snprec, nk, d_inv, codes_samp, &A_samp);
     if (rc) return rc;
     if (n == ctx->nind_all) {
       A_snp.codes = ctx->d_geno;
@@ -503,10 +539,6 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
       A_snp.nrows = nk;
       A_snp.k0 = n;
     } else {
-      gp_tc_code_bytes(0, n, nk, &ldc, &rows_pad);
-      e = B.get(&codes_snp, (size_t)rows_pad * ldc);
-      if (e != cudaSuccess)
-        return gp_fail(ctx, GP_ERR_NOMEM, "gp_fastpca: code operand allocation failed");
       rc = gp_tc_build_codes(ctx, 0, ctx->d_rows, n, d_snprec, nk, NULL, codes_snp, &A_snp);
       if (rc) return rc;
     }
@@ -542,7 +574,7 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
       }
       rc = ts_cross(ctx, d_Q, L, L, d_Q, L, L, nk, d_part, part_cap, d_W);
       if (rc) return rc;
-      k_block_orth<<<1, JAC_MAX, 0, ctx->stream>>>(d_W, pass == 0 ? d_pre : NULL, L,
+      k_block_orth<<<1, JAC_THREADS, 0, ctx->stream>>>(d_W, pass == 0 ? d_pre : NULL, L,
                                                   GP_FAST_DEP_TOL, d_T);
       GP_LAUNCH_CHECK(ctx, "k_block_orth");
       k_block_apply<<<grid_for_fast(ctx, (int64_t)nQ), 256, 0, ctx->stream>>>(
