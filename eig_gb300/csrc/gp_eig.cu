@@ -3,8 +3,9 @@
  * and the top nvec eigenvectors (the reference computes every eigenpair with LAPACK dspev,
  * src/eigensrc/eigx.c:97-117, but prints all eigenvalues and uses only the top vectors).
  *
- *   1. Householder tridiagonalisation A = Q T Q^T (k_tridiag below: one cooperative launch,
- *      LAPACK dsytd2's reflectors and storage; cuSOLVER sytrd beyond 8,533 rows);
+ *   1. Householder tridiagonalisation A = Q T Q^T (k_tridiag_tiled or k_tridiag while the
+ *      trailing matrix is large, then k_tridiag_smem: LAPACK dsytd2's reflectors and storage;
+ *      cuSOLVER sytrd beyond 8,533 rows);
  *   2. all eigenvalues of T by multisection on Sturm counts (the published bisection method:
  *      the count of negative pivots of the LDL^T factorisation of T - x I equals the number
  *      of eigenvalues below x), several lanes per eigenvalue index: FP32 brackets first,
@@ -426,49 +427,6 @@ __device__ __forceinline__ bool tr_grid_sync(unsigned *count, unsigned target, i
   return s_ok != 0;
 }
 
-/* sum of the G block partials in a fixed order (warp 0), broadcast through shared memory */
-__device__ __forceinline__ double tr_sum_partials(const double *part, int G, double *slot)
-{
-  if (threadIdx.x < 32) {
-    double s = 0.0;
-    for (int g = threadIdx.x; g < G; g += 32) s += part[g];
-    for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, o);
-    if (threadIdx.x == 0) *slot = s;
-  }
-  __syncthreads();
-  const double r = *slot;
-  __syncthreads();
-  return r;
-}
-
-/* block sum of one value per thread (fixed order), result valid in thread 0 */
-__device__ __forceinline__ double tr_block_sum(double v, double *red)
-{
-  for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < TR_WARPS; ++w) s += red[w];
-  __syncthreads();
-  return s;
-}
-
-/* sum of the G float-float block partials in a fixed order (warp 0), broadcast */
-__device__ __forceinline__ ff2 ff_sum_partials(const double *part, int G, ff2 *slot)
-{
-  if (threadIdx.x < 32) {
-    ff2 s = ff_make(0.f, 0.f);
-    for (int g = threadIdx.x; g < G; g += 32) s = ff_add(s, ff_load(part + g));
-    for (int o = 16; o; o >>= 1) s = ff_add(s, ff_shfl_xor(s, o));
-    if (threadIdx.x == 0) *slot = s;
-  }
-  __syncthreads();
-  const ff2 r = *slot;
-  __syncthreads();
-  return r;
-}
-
 /* block sum of one float-float per thread (fixed order: warp shuffles, then warp 0's
  * shuffle tree over the warps' sums), as float-float in thread 0 */
 __device__ __forceinline__ ff2 ff_block_sum2(ff2 v, ff2 *red)
@@ -486,20 +444,86 @@ __device__ __forceinline__ ff2 ff_block_sum2(ff2 v, ff2 *red)
   return t;
 }
 
-/* block sum of one float-float per thread (fixed order), as a double in thread 0 */
-__device__ __forceinline__ double ff_block_sum(ff2 v, ff2 *red)
+/* a - (p q + r s) in float-float (the rank-2 update of one element): the two high products
+ * exactly (TwoProd with FMA), their cross terms and the errors of two TwoSums gathered in one
+ * FP32 term, one renormalisation: 27 FP32 operations against 30 for two ff_fma, of the same
+ * error order.  With p = r = 0 or q = s = 0 it returns a normalised a unchanged. */
+__device__ __forceinline__ ff2 ff_sub2prod(ff2 a, ff2 p, ff2 q, ff2 r, ff2 s)
 {
-  for (int o = 16; o; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0) {
-    ff2 t = red[0];
-    for (int w = 1; w < TR_WARPS; ++w) t = ff_add(t, red[w]);
-    s = ff_to_double(t);
+  const float p1 = __fmul_rn(p.h, q.h);
+  float e = __fmaf_rn(p.h, q.h, -p1);
+  e = __fmaf_rn(p.h, q.l, e);
+  e = __fmaf_rn(p.l, q.h, e);
+  const float p2 = __fmul_rn(r.h, s.h);
+  e = __fadd_rn(__fmaf_rn(r.h, s.h, -p2), e);
+  e = __fmaf_rn(r.h, s.l, e);
+  e = __fmaf_rn(r.l, s.h, e);
+  const float t1 = __fsub_rn(a.h, p1);
+  const float b1 = __fsub_rn(t1, a.h);
+  const float r1 = __fadd_rn(__fsub_rn(a.h, __fsub_rn(t1, b1)), __fsub_rn(-p1, b1));
+  const float t2 = __fsub_rn(t1, p2);
+  const float b2 = __fsub_rn(t2, t1);
+  const float r2 = __fadd_rn(__fsub_rn(t1, __fsub_rn(t2, b2)), __fsub_rn(-p2, b2));
+  const float low = __fadd_rn(__fsub_rn(a.l, e), __fadd_rn(r1, r2));
+  const float h = __fadd_rn(t2, low);
+  return ff_make(h, __fsub_rn(low, __fsub_rn(h, t2)));
+}
+
+/* a x + b y in float-float: two exact high products, one TwoSum, the cross terms and errors
+ * in one FP32 term (19 FP32 operations against 22 for ff_mul + ff_fma) */
+__device__ __forceinline__ ff2 ff_dot2(ff2 a, ff2 x, ff2 b, ff2 y)
+{
+  const float p1 = __fmul_rn(a.h, x.h);
+  float e = __fmaf_rn(a.h, x.h, -p1);
+  e = __fmaf_rn(a.h, x.l, e);
+  e = __fmaf_rn(a.l, x.h, e);
+  const float p2 = __fmul_rn(b.h, y.h);
+  e = __fadd_rn(__fmaf_rn(b.h, y.h, -p2), e);
+  e = __fmaf_rn(b.h, y.l, e);
+  e = __fmaf_rn(b.l, y.h, e);
+  const float s = __fadd_rn(p1, p2);
+  const float bb = __fsub_rn(s, p1);
+  const float er = __fadd_rn(__fsub_rn(p1, __fsub_rn(s, bb)), __fsub_rn(p2, bb));
+  const float low = __fadd_rn(e, er);
+  const float h = __fadd_rn(s, low);
+  return ff_make(h, __fsub_rn(low, __fsub_rn(h, s)));
+}
+
+/* acc += a x with the accumulator left unnormalised (acc.h the running TwoSum of the high
+ * products, acc.l every lower-order term): 12 FP32 operations against 15 for ff_fma; over a
+ * short dot (16 terms here) its error stays of the order of the normalised accumulation's.
+ * ff_renorm makes the pair normalised again. */
+__device__ __forceinline__ ff2 ff_acc_lazy(ff2 acc, ff2 a, ff2 x)
+{
+  const float p = __fmul_rn(a.h, x.h);
+  float e = __fmaf_rn(a.h, x.h, -p);
+  e = __fmaf_rn(a.h, x.l, e);
+  e = __fmaf_rn(a.l, x.h, e);
+  const float s = __fadd_rn(acc.h, p);
+  const float bb = __fsub_rn(s, acc.h);
+  const float er = __fadd_rn(__fsub_rn(acc.h, __fsub_rn(s, bb)), __fsub_rn(p, bb));
+  return ff_make(s, __fadd_rn(acc.l, __fadd_rn(e, er)));
+}
+__device__ __forceinline__ ff2 ff_renorm(ff2 a)
+{
+  const float h = __fadd_rn(a.h, a.l);
+  return ff_make(h, __fsub_rn(a.l, __fsub_rn(h, a.h)));
+}
+
+/* sum over the warp, the same in every lane: the high parts by TwoSum, the lower-order terms
+ * kept aside and added once at the end, so that a level costs a shuffle and one addition of
+ * latency */
+__device__ __forceinline__ ff2 ff_warp_sum(ff2 v)
+{
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xFFFFFFFFu, v.h, o), ol = __shfl_xor_sync(0xFFFFFFFFu, v.l, o);
+    const float s = __fadd_rn(v.h, oh);
+    const float bb = __fsub_rn(s, v.h);
+    const float er = __fadd_rn(__fsub_rn(v.h, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
+    v = ff_make(s, __fadd_rn(__fadd_rn(v.l, ol), er));
   }
-  __syncthreads();
-  return s;
+  return ff_renorm(v);
 }
 
 /* the (symmetric, full) double matrix to float-float pairs, in place */
@@ -526,8 +550,8 @@ struct tr_step {
  * dormtr (lower) reads them; the upper triangle is left in float-float form.
  */
 /*
- * Steps c_begin .. n-2 of the whole-matrix reduction (k_tridiag's step; the tail steps of
- * k_tridiag_tiled): A holds the trailing matrix (indices >= c_begin) as float-float pairs in
+ * Steps c_begin .. c_end - 1 (at most n-2) of the whole-matrix reduction (k_tridiag's steps; after
+ * the tiled steps k_tridiag_tiled's): A holds the trailing matrix (indices >= c_begin) as float-float pairs in
  * whole columns, both triangles.  svp/swp/svc: the block's vectors in shared memory (at least
  * n pairs each).  tau_pf, scale_pf, e_pf, have_p and target carry the previous step's state.
  * dot0 (when not NULL) holds the previous step's y.v parts at [dot0_k0, dot0_k1) instead of
@@ -535,7 +559,8 @@ struct tr_step {
  * NULL): phase times as in k_tridiag, sph[5] the last time stamp.  False when the grid
  * barrier failed.
  */
-__device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, double *d, double *e,
+__device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int c_end, double *d,
+                                              double *e,
                                               double *tau, double *vbuf, double *wbuf,
                                               double *ybuf, double *part_dot2, unsigned *count,
                                               unsigned &target, int *err, double *svp,
@@ -559,7 +584,7 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, dou
     sph[5] = t_now;                                    \
   }
   const int early = (int)((3LL * n) / 10);
-  for (int c = c_begin; c < n - 1; ++c) {
+  for (int c = c_begin; c < c_end; ++c) {
     /* ---- A (every block, no grid barrier): v and w of step c-1, the pending update of
      * column c and its norm, rebuilt from y, the stored x of step c-1 and column c; each
      * block also writes its share of the reflector storage and of x_c (double buffer) ---- */
@@ -740,36 +765,402 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, dou
   return true;
 }
 
-/* the last diagonal entry and the storage of the last reflector after the whole-matrix steps
- * (block 0) */
-__device__ __forceinline__ void tr_full_last(double *A, int n, double *d, double *ybuf,
-                                             double *part_dot2, ff2 tau_pf, ff2 e_pf,
-                                             bool have_p)
+/*
+ * sqrt(a), a > 0, and a / b from the approximate FP32 reciprocal (square root): two
+ * corrections from the float-float remainder (Karp & Markstein 1997) reach the pair's
+ * precision; they replace ff_sqrt and ff_div on one thread's critical path, whose rounded FP32
+ * divisions are several times longer chains.
+ */
+__device__ __forceinline__ ff2 ff_sqrt_fast(ff2 a)
 {
-  __shared__ ff2 s_slotf;
-  const int G = gridDim.x, b = blockIdx.x;
-  const ff2 ZERO = ff_make(0.f, 0.f);
-  if (b == 0) {
-    ff2 dsum = ZERO;
-    if (have_p) dsum = ff_sum_partials(part_dot2 + (size_t)((n - 2) & 1) * G, G, &s_slotf);
-    if (threadIdx.x == 0) {
-      ff2 a = ff_load(A + (int64_t)(n - 1) * n + n - 1);
-      if (have_p) {
-        const ff2 alpha_p = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), dsum), -0.5f);
-        const ff2 wp =
-            ff_fma(tau_pf, ff_load(ybuf + (int64_t)((n - 2) & 1) * n + n - 1), alpha_p);
-        a = ff_add(a, ff_neg(wp));
-        a = ff_add(a, ff_neg(wp));
-        A[(int64_t)(n - 2) * n + n - 1] = ff_to_double(e_pf);
-      }
-      d[n - 1] = ff_to_double(a);
-    }
-  }
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a.h));
+  const float s = a.h * r, hr = 0.5f * r;
+  ff2 x = ff_make(s, 0.f);
+  ff2 t = ff_fma(ff_neg(x), x, a);
+  x = ff_add(x, ff_make(t.h * hr, 0.f));
+  t = ff_fma(ff_neg(x), x, a);
+  return ff_add(x, ff_make(t.h * hr, 0.f));
+}
+__device__ __forceinline__ ff2 ff_div_fast(ff2 a, ff2 b)
+{
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b.h));
+  ff2 q = ff_make(a.h * r, 0.f);
+  ff2 t = ff_fma(ff_neg(b), q, a);
+  q = ff_add(q, ff_make(t.h * r, 0.f));
+  t = ff_fma(ff_neg(b), q, a);
+  return ff_add(q, ff_make(t.h * r, 0.f));
 }
 
+/*
+ * A float-float value that carries its step: each half next to the step's tag in a 64-bit word
+ * (64-bit accesses are not torn), so that a reader polls for the value itself and needs no
+ * barrier, fence or second trip to L2 for it.  Tags are c + 1 for values of step c, never 0.
+ */
+__device__ __forceinline__ void tag_store(uint4 *p, ff2 v, unsigned tag)
+{
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p),
+               "r"(__float_as_uint(v.h)), "r"(tag), "r"(__float_as_uint(v.l)), "r"(tag)
+               : "memory");
+}
+__device__ __forceinline__ uint4 tag_load(const uint4 *p)
+{
+  uint4 r;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
+/*
+ * y and x of the rows q0 + u step (u < RPT, below n): all the loads of a round are in flight
+ * together, and a round asks for what is missing only.  False when the wait ran out or another
+ * block gave up.
+ */
+template <int RPT>
+__device__ __forceinline__ bool tag_wait(const uint4 *yt, const uint4 *xt, int q0, int step, int n,
+                                         unsigned tag, ff2 *y, ff2 *x, int *err)
+{
+  unsigned need = 0;
+#pragma unroll
+  for (int u = 0; u < RPT; ++u)
+    if (q0 + u * step < n) need |= 3u << (2 * u);
+  uint64_t t0 = 0;
+  for (unsigned it = 0; need; ++it) {
+    uint4 ry[RPT], rx[RPT];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      if (need & (1u << (2 * u))) ry[u] = tag_load(yt + q0 + u * step);
+      if (need & (2u << (2 * u))) rx[u] = tag_load(xt + q0 + u * step);
+    }
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      if ((need & (1u << (2 * u))) && ry[u].y == tag && ry[u].w == tag) {
+        y[u] = ff_make(__uint_as_float(ry[u].x), __uint_as_float(ry[u].z));
+        need &= ~(1u << (2 * u));
+      }
+      if ((need & (2u << (2 * u))) && rx[u].y == tag && rx[u].w == tag) {
+        x[u] = ff_make(__uint_as_float(rx[u].x), __uint_as_float(rx[u].z));
+        need &= ~(2u << (2 * u));
+      }
+    }
+    if (it == 0) t0 = globaltimer_ns();
+    if ((it & 63u) == 63u) {
+      if (*(volatile int *)err) return false;
+      if (globaltimer_ns() - t0 > GP_WAIT_NS) {
+        atomicExch(err, TR_ERR_BARRIER);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
+/* one level of ff_warp_sum */
+__device__ __forceinline__ ff2 ff_lazy_xor(ff2 v, int o)
+{
+  const float oh = __shfl_xor_sync(0xFFFFFFFFu, v.h, o), ol = __shfl_xor_sync(0xFFFFFFFFu, v.l, o);
+  const float s = __fadd_rn(v.h, oh);
+  const float bb = __fsub_rn(s, v.h);
+  const float er = __fadd_rn(__fsub_rn(v.h, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
+  return ff_make(s, __fadd_rn(__fadd_rn(v.l, ol), er));
+}
+
+/*
+ * Steps c0 .. n-2 with the trailing matrix (order m = n - c0 <= NT RPT) in shared memory, and
+ * the last diagonal entry: block b holds whole columns r = c0 + b, c0 + b + G, .. (both
+ * triangles, as float-float pairs; at most 32 columns).  Per step:
+ *   A   every block redundantly: y of step c-1 and column c are polled for in global memory
+ *       (tagged values, double-buffered); x of step c-1 is still in svc, unscaled, with alpha - beta in the
+ *       pivot's place: v = scale x; then y.v, w, the pending update of column c, its norm and
+ *       the reflector
+ *   B   each warp takes a segment of rows of two owned columns: pending update, written back,
+ *       and the dots with x; the owner of column c + 1 publishes it; then the first warp adds
+ *       the segments and publishes y = scale (A x)
+ * No barrier over the blocks: a block cannot start step c before every block's y of step c-1
+ * is there, and a block publishes y of step c only after it has read all of step c-1, so the
+ * two buffers suffice; a block without a column after c leaves before step c, since nobody
+ * would wait for its reading.  A step is a chain of latencies: four block barriers, one trip
+ * through L2, three sums over the block.  Every warp takes part in those sums, so a block has
+ * few: with 32 warps their instructions alone took half the step.  Reflectors, d, e and tau are stored as pairs and converted at the end (an
+ * FP64 instruction occupies its quarter of the SM for 64 clocks).  n = 1,000: 6.3 ms of
+ * 8.2 with the matrix in L2 and a grid barrier per step; n = 180 on 16 blocks: 0.51 of 1.34; the
+ * last 1,740 columns of 5,000: 4 ms less.
+ * Needs every block resident (a cooperative launch), ytag and ctag [2][n] zero.
+ */
+template <int NT, int RPT>
+__device__ __forceinline__ bool tr_smem_steps(double *A, int n, int c0, double *d, double *e,
+                                              double *tau, const double *xprev,
+                                              const double *yprev0, uint4 *ytag, uint4 *ctag,
+                                              unsigned *count, unsigned &target, int *err,
+                                              double *smm, ff2 tau_p, ff2 scale_p, ff2 e_p,
+                                              bool have_p)
+{
+  constexpr int NW = NT / 32;
+  __shared__ ff2 red[NW], red1[NW];
+  __shared__ ff2 sdot[2 * NW];
+  __shared__ tr_step st;
+  __shared__ ff2 s_yc;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const ff2 ONE = ff_make(1.f, 0.f), ZERO = ff_make(0.f, 0.f);
+  const int m = n - c0;
+  double *svp = smm - c0, *swp = smm + m - c0, *svc = smm + 2 * m - c0; /* indexed by row */
+  double *cols = smm + 3 * (size_t)m - c0;                              /* column j at j m */
+  const int cfirst = have_p ? c0 - 1 : c0; /* first reflector stored as pairs */
+  const int nown = c0 + b < n ? (n - 1 - c0 - b) / G + 1 : 0;
+  for (int j = 0; j < nown; ++j)
+    for (int q = c0 + tid; q < n; q += blockDim.x)
+      cols[(size_t)j * m + q] = A[(int64_t)(c0 + b + j * G) * n + q];
+  for (int q = c0 + tid; q < n; q += blockDim.x)
+    ff_store(svc + q, have_p ? ff_load(xprev + q) : ZERO);
+  int j0 = 0; /* first owned column at or after c + 1 */
+  /* position from the owner of the last column: at step c < n-1 the blocks at positions below
+   * n-1-c own a column after c */
+  const int pos = ((n - 1 - c0) % G - b + G) % G;
+  __syncthreads();
+  bool fail = false;
+  for (int c = c0; pos < max(1, n - 1 - c); ++c) {
+    /* ---- A ---- */
+    const int nact = min(G, max(1, n - 1 - c)); /* blocks in this step */
+    ff2 x[RPT], y[RPT], v[RPT];
+    const uint4 *yt = ytag + (size_t)((c - 1) & 1) * n, *ct = ctag + (size_t)(c & 1) * n;
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int q = c + tid + u * NT;
+      x[u] = y[u] = ZERO;
+      if (q >= n) continue;
+      if (c == c0) {
+        x[u] = ff_load(A + (int64_t)c * n + q);
+        if (have_p) y[u] = ff_load(yprev0 + q);
+      }
+    }
+    if (c > c0) fail = !tag_wait<RPT>(yt, ct, c + tid, NT, n, (unsigned)c, y, x, err);
+    ff2 dacc = ZERO;
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int q = c + tid + u * NT;
+      v[u] = ZERO;
+      if (q < n && have_p) {
+        v[u] = q == c ? ONE : ff_mul(ff_load(svc + q), scale_p);
+        dacc = ff_acc_lazy(dacc, y[u], v[u]);
+      }
+    }
+    dacc = ff_warp_sum(dacc);
+    if (lane == 0) red1[warp] = dacc;
+    if (tid == 0) s_yc = y[0];
+    if (__syncthreads_or(fail)) {
+      fail = true;
+      break;
+    }
+    ff2 dsum = red1[lane & (NW - 1)];
+#pragma unroll
+    for (int o = NW / 2; o; o >>= 1) dsum = ff_lazy_xor(dsum, o);
+    dsum = ff_renorm(dsum);
+    const ff2 alpha_p = ff_scale(ff_mul(ff_mul(tau_p, tau_p), dsum), -0.5f);
+    const ff2 wpc = ff_fma(tau_p, s_yc, alpha_p); /* w(c) of step c-1, where v(c) = 1 */
+    ff2 nrm = ZERO;
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int q = c + tid + u * NT;
+      if (q >= n) continue;
+      ff2 w = ZERO;
+      if (have_p) {
+        w = ff_fma(tau_p, y[u], ff_mul(alpha_p, v[u]));
+        x[u] = ff_fma(ff_neg(v[u]), wpc, x[u]);
+        x[u] = ff_add(x[u], ff_neg(w));
+      }
+      ff_store(svp + q, v[u]);
+      ff_store(swp + q, w);
+      ff_store(svc + q, x[u]);
+      if (q >= c + 2) nrm = ff_acc_lazy(nrm, x[u], x[u]);
+    }
+    nrm = ff_warp_sum(nrm);
+    if (lane == 0) red[warp] = nrm;
+    __syncthreads();
+    if (have_p && warp > 0) {
+      /* the reflector of step c-1, the blocks in turn by rows, while the first warp forms the
+       * next one */
+      for (int q = c + pos + (tid - 32) * nact; q < n; q += (NT - 32) * nact)
+        ff_store(A + (int64_t)(c - 1) * n + q, q == c ? e_p : ff_load(svp + q));
+    }
+    if (c == n - 1) {
+      if (tid == 0) ff_store(d + c, x[0]);
+      break;
+    }
+    if (warp == 0) {
+      ff2 xn2 = red[lane & (NW - 1)];
+#pragma unroll
+      for (int o = NW / 2; o; o >>= 1) xn2 = ff_lazy_xor(xn2, o);
+      xn2 = ff_renorm(xn2);
+      if (lane == 0) {
+        /* the reflector (dlarfg): beta = -sign(alpha) sqrt(alpha^2 + |x|^2), tau = (beta -
+         * alpha) / beta, scale = 1 / (alpha - beta) */
+        const ff2 alpha = ff_load(svc + c + 1);
+        ff2 beta = alpha, tau_c = ZERO, scale_c = ZERO;
+        if (xn2.h != 0.f) {
+          const ff2 sq = ff_fma(alpha, alpha, xn2);
+          /* the approximate instructions flush subnormals: far from them only */
+          const bool fast = sq.h > 1e-28f && sq.h < 1e28f;
+          const ff2 nrm2 = fast ? ff_sqrt_fast(sq) : ff_sqrt(sq);
+          beta = alpha.h >= 0.f ? ff_neg(nrm2) : nrm2;
+          const ff2 am = ff_add(alpha, ff_neg(beta));
+          tau_c = fast ? ff_div_fast(ff_neg(am), beta) : ff_div(ff_neg(am), beta);
+          scale_c = fast ? ff_div_fast(ONE, am) : ff_div(ONE, am);
+          ff_store(svc + c + 1, am);
+        }
+        st.beta = beta;
+        st.tau_c = tau_c;
+        st.scale_c = scale_c;
+        if (pos == 0) {
+          ff_store(d + c, ff_load(svc + c));
+          ff_store(e + c, beta);
+          ff_store(tau + c, tau_c);
+        }
+      }
+    } else if (tid == 32) {
+      /* the owned columns from c + 1 on and the segments of a pair of them: a power of two, as
+       * many as there are warps for, of at least 32 rows */
+      int j = j0;
+      if (c0 + b + j * G < c + 1) ++j;
+      const int npair = (nown - j + 1) >> 1, rows = n - 1 - c;
+      int sh = 0;
+      while ((npair << (sh + 1)) <= NW && (rows >> (sh + 1)) >= 32) ++sh;
+      st.b1_u0 = j;
+      st.b1_u1 = sh;
+    }
+    __syncthreads();
+    const ff2 scale_c = st.scale_c;
+    j0 = st.b1_u0;
+    const int sh = st.b1_u1, S = 1 << sh;
+    tau_p = st.tau_c;
+    scale_p = scale_c;
+    e_p = st.beta;
+    have_p = true;
+    /* ---- B: the owned columns r >= c + 1, two at a time ---- */
+    const int nc = nown - j0, nitem = ((nc + 1) >> 1) << sh;
+    const int seg = (((n - 1 - c + S - 1) >> sh) + 31) & ~31;
+    uint4 *cn = ctag + (size_t)((c + 1) & 1) * n;
+    /* an item per warp; with more pairs than warps (sh = 0) the dots of the later pairs wait
+     * in registers for the slots of the earlier ones: at most two rounds, 32 columns */
+    ff2 dab[2];
+#pragma unroll
+    for (int rd = 0; rd < 2; ++rd) {
+      const int it = warp + rd * NW;
+      ff2 da = ZERO, db = ZERO;
+      if (it < nitem) {
+        const int pi = it >> sh, sg = it & (S - 1);
+        const int ja = j0 + 2 * pi, ra = c0 + b + ja * G, rb = ra + G;
+        const bool two = rb < n;
+        double *ca = cols + (size_t)ja * m, *cb = two ? ca + m : ca;
+        const ff2 vra = ff_load(svp + ra), wra = ff_load(swp + ra);
+        const ff2 vrb = two ? ff_load(svp + rb) : ZERO, wrb = two ? ff_load(swp + rb) : ZERO;
+        const int qs = c + 1 + sg * seg, qe = min(n, qs + seg);
+        const bool next = ra == c + 1; /* the first of its block: never the second of a pair */
+#pragma unroll 2
+        for (int q = qs + lane; q < qe; q += 32) {
+          const ff2 vq = ff_load(svp + q), wq = ff_load(swp + q), xq = ff_load(svc + q);
+          const ff2 a = ff_sub2prod(ff_load(ca + q), vq, wra, wq, vra);
+          ff_store(ca + q, a);
+          if (next) tag_store(cn + q, a, (unsigned)(c + 1));
+          da = ff_acc_lazy(da, a, xq);
+          if (two) {
+            const ff2 a2 = ff_sub2prod(ff_load(cb + q), vq, wrb, wq, vrb);
+            ff_store(cb + q, a2);
+            db = ff_acc_lazy(db, a2, xq);
+          }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          da = ff_lazy_xor(da, o);
+          db = ff_lazy_xor(db, o);
+        }
+      }
+      dab[rd] = lane ? db : da; /* lanes 0 and 1 carry a pair's two sums */
+      if (rd == 0) {
+        if (lane < 2) sdot[2 * warp + lane] = dab[0];
+        if (nitem <= NW) break;
+      }
+    }
+    if (nitem > NW) {
+      /* one segment per pair: a warp's own sums are complete */
+      if (lane < 2)
+#pragma unroll
+        for (int rd = 0; rd < 2; ++rd) {
+          const int col = 2 * (warp + rd * NW) + lane;
+          if (col < nc)
+            tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
+                      ff_mul(ff_renorm(dab[rd]), scale_c), (unsigned)(c + 1));
+        }
+      __syncthreads(); /* the vectors are rewritten by the next step */
+      continue;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      /* the segments of a column, slots 2 (pair S + segment) + column of the pair, by a tree */
+#pragma unroll
+      for (int h = 0; h < (2 * NW + 31) / 32; ++h) {
+        const int slot = lane + 32 * h;
+        ff2 t = slot < 2 * nitem ? sdot[slot] : ZERO;
+        for (int o = 1; o < S; o <<= 1) t = ff_lazy_xor(t, 2 * o);
+        const int col = 2 * (slot >> (sh + 1)) + (slot & 1);
+        if (((slot >> 1) & (S - 1)) == 0 && slot < 2 * nitem && col < nc)
+          tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
+                    ff_mul(ff_renorm(t), scale_c), (unsigned)(c + 1));
+      }
+    }
+  }
+  if (fail) return false;
+  /* when every block's pairs are stored: to FP64 */
+  target += G;
+  if (!tr_grid_sync(count, target, err)) return false;
+  for (int c = cfirst + b; c < n - 1; c += G)
+    for (int q = c + 1 + tid; q < n; q += blockDim.x) {
+      double *p = A + (int64_t)c * n + q;
+      *p = ff_to_double(ff_load(p));
+    }
+  if (b == 0)
+    for (int c = c0 + tid; c < n; c += blockDim.x) {
+      d[c] = ff_to_double(ff_load(d + c));
+      if (c < n - 1) {
+        e[c] = ff_to_double(ff_load(e + c));
+        tau[c] = ff_to_double(ff_load(tau + c));
+      }
+    }
+  return true;
+}
+
+/* what a launch's last step leaves for the next launch's first (float-float pairs) */
+struct tr_state {
+  ff2 tau, scale, e;
+};
+
+/* steps c0 .. n-2: from the start (c0 = 0), or after the steps of another kernel */
+template <int NT, int RPT>
+__global__ void __launch_bounds__(NT, 1)
+k_tridiag_smem(double *A, int n, int c0, double *d, double *e, double *tau, const double *xprev,
+               const double *yprev, uint4 *ytag, uint4 *ctag, const tr_state *state, unsigned *bar,
+               int *err)
+{
+  extern __shared__ double sh[];
+  const ff2 ZERO = ff_make(0.f, 0.f);
+  unsigned target = 0;
+  const bool have_p = c0 > 0;
+  tr_smem_steps<NT, RPT>(A, n, c0, d, e, tau, xprev, yprev, ytag, ctag, bar, target, err, sh,
+                         have_p ? state->tau : ZERO, have_p ? state->scale : ZERO,
+                         have_p ? state->e : ZERO, have_p);
+}
+
+#define TR_SMEM_NT 512 /* threads and rows per thread above TR_SMALL_ORDER rows */
+#define TR_SMEM_RPT 4
+#define TR_SMALL_ORDER 768 /* trailing orders up to this with 256 threads */
+
+/* steps 0 .. c_end - 1 by whole columns in L2 */
 __global__ void __launch_bounds__(TR_THREADS, 1)
-k_tridiag(double *A, int n, double *d, double *e, double *tau, double *vbuf, double *wbuf,
-          double *ybuf, double *part_dot2, unsigned *bar, int *err,
+k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double *vbuf,
+          double *wbuf, double *ybuf, double *part_dot2, tr_state *state, unsigned *bar, int *err,
           unsigned long long *phase_ns)
 {
   extern __shared__ double sh[];
@@ -785,13 +1176,13 @@ k_tridiag(double *A, int n, double *d, double *e, double *tau, double *vbuf, dou
     for (int i = 0; i < 5; ++i) s_ph[i] = 0ull;
     s_ph[5] = globaltimer_ns();
   }
-  if (!tr_full_steps(A, n, 0, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
+  if (!tr_full_steps(A, n, 0, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
                      sh + n, sh + 2 * n, tau_pf, scale_pf, e_pf, have_p, NULL, 0, 0,
                      stamp ? s_ph : NULL))
     return;
   if (stamp)
     for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
-  tr_full_last(A, n, d, ybuf, part_dot2, tau_pf, e_pf, have_p);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *state = {tau_pf, scale_pf, e_pf};
 }
 
 /* ---------------------------------------------------------------------------------- */
@@ -855,72 +1246,6 @@ __global__ void k_tri_to_tiles(const double *A, int n, int nt, double *Tm)
       ff_store(tile + idx, ff_from_double(v));
     }
   }
-}
-
-/* a - (p q + r s) in float-float (the rank-2 update of one element): the two high products
- * exactly (TwoProd with FMA), their cross terms and the errors of two TwoSums gathered in one
- * FP32 term, one renormalisation: 27 FP32 operations against 30 for two ff_fma, of the same
- * error order.  With p = r = 0 or q = s = 0 it returns a normalised a unchanged. */
-__device__ __forceinline__ ff2 ff_sub2prod(ff2 a, ff2 p, ff2 q, ff2 r, ff2 s)
-{
-  const float p1 = __fmul_rn(p.h, q.h);
-  float e = __fmaf_rn(p.h, q.h, -p1);
-  e = __fmaf_rn(p.h, q.l, e);
-  e = __fmaf_rn(p.l, q.h, e);
-  const float p2 = __fmul_rn(r.h, s.h);
-  e = __fadd_rn(__fmaf_rn(r.h, s.h, -p2), e);
-  e = __fmaf_rn(r.h, s.l, e);
-  e = __fmaf_rn(r.l, s.h, e);
-  const float t1 = __fsub_rn(a.h, p1);
-  const float b1 = __fsub_rn(t1, a.h);
-  const float r1 = __fadd_rn(__fsub_rn(a.h, __fsub_rn(t1, b1)), __fsub_rn(-p1, b1));
-  const float t2 = __fsub_rn(t1, p2);
-  const float b2 = __fsub_rn(t2, t1);
-  const float r2 = __fadd_rn(__fsub_rn(t1, __fsub_rn(t2, b2)), __fsub_rn(-p2, b2));
-  const float low = __fadd_rn(__fsub_rn(a.l, e), __fadd_rn(r1, r2));
-  const float h = __fadd_rn(t2, low);
-  return ff_make(h, __fsub_rn(low, __fsub_rn(h, t2)));
-}
-
-/* a x + b y in float-float: two exact high products, one TwoSum, the cross terms and errors
- * in one FP32 term (19 FP32 operations against 22 for ff_mul + ff_fma) */
-__device__ __forceinline__ ff2 ff_dot2(ff2 a, ff2 x, ff2 b, ff2 y)
-{
-  const float p1 = __fmul_rn(a.h, x.h);
-  float e = __fmaf_rn(a.h, x.h, -p1);
-  e = __fmaf_rn(a.h, x.l, e);
-  e = __fmaf_rn(a.l, x.h, e);
-  const float p2 = __fmul_rn(b.h, y.h);
-  e = __fadd_rn(__fmaf_rn(b.h, y.h, -p2), e);
-  e = __fmaf_rn(b.h, y.l, e);
-  e = __fmaf_rn(b.l, y.h, e);
-  const float s = __fadd_rn(p1, p2);
-  const float bb = __fsub_rn(s, p1);
-  const float er = __fadd_rn(__fsub_rn(p1, __fsub_rn(s, bb)), __fsub_rn(p2, bb));
-  const float low = __fadd_rn(e, er);
-  const float h = __fadd_rn(s, low);
-  return ff_make(h, __fsub_rn(low, __fsub_rn(h, s)));
-}
-
-/* acc += a x with the accumulator left unnormalised (acc.h the running TwoSum of the high
- * products, acc.l every lower-order term): 12 FP32 operations against 15 for ff_fma; over a
- * short dot (16 terms here) its error stays of the order of the normalised accumulation's.
- * ff_renorm makes the pair normalised again. */
-__device__ __forceinline__ ff2 ff_acc_lazy(ff2 acc, ff2 a, ff2 x)
-{
-  const float p = __fmul_rn(a.h, x.h);
-  float e = __fmaf_rn(a.h, x.h, -p);
-  e = __fmaf_rn(a.h, x.l, e);
-  e = __fmaf_rn(a.l, x.h, e);
-  const float s = __fadd_rn(acc.h, p);
-  const float bb = __fsub_rn(s, acc.h);
-  const float er = __fadd_rn(__fsub_rn(acc.h, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-  return ff_make(s, __fadd_rn(acc.l, __fadd_rn(e, er)));
-}
-__device__ __forceinline__ ff2 ff_renorm(ff2 a)
-{
-  const float h = __fadd_rn(a.h, a.l);
-  return ff_make(h, __fsub_rn(a.l, __fsub_rn(h, a.h)));
 }
 
 /* one part (TT_U columns from TT*J + j0) of tile (I, J) by one warp: the pending update of
@@ -1003,15 +1328,15 @@ __host__ __device__ inline size_t tt_smem_bytes(int nt, int R, int maxr, int max
  * (row J0 of each table).  prow [nt][pc][TT], pcol [nt*TT_UPT][pr][TT_U]: the published row
  * and column parts; dotp [2][nt]: the index blocks' partial y.v of alternate steps; kcnt [nt]:
  * arrival counters (zero at launch).  maxr/maxc/maxi bound a block's tile rows, column units
- * and parts over all J0; R parts per round.  Steps from cs on run whole columns
- * (tr_full_steps), part_dot2 [2G] their block partials.
+ * and parts over all J0; R parts per round.  Steps cs .. c_end - 1 run whole columns
+ * (tr_full_steps), part_dot2 [2G] their block partials; k_tridiag_smem does the rest.
  */
 __global__ void __launch_bounds__(TR_THREADS, 1)
 k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, int maxc,
                 int maxi, int R, int cs, const unsigned char *rgt, const unsigned char *cgt,
                 double *d, double *e, double *tau, double *vbuf, double *wbuf, double *ybuf,
                 double *prow, double *pcol, double *dotp, unsigned *kcnt, double *part_dot2,
-                unsigned *bar, int *err, unsigned long long *phase_ns)
+                unsigned *bar, int *err, unsigned long long *phase_ns, int c_end, tr_state *state)
 {
   extern __shared__ double sh[];
   const int npad = nt * TT, nu = nt * TT_UPT;
@@ -1318,67 +1643,33 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
     TT_STAMP(4)
     have_p = true;
   }
-  if (cs < n - 1) {
-    /* the switch to whole columns: the trailing block (indices >= cs) of the block's parts
-     * into A as float-float pairs, both triangles (the pending update of step cs-1 is applied
-     * by the first whole-column step) */
-    const int ni = s_ni;
-    for (int64_t idx = threadIdx.x; idx < (int64_t)ni * (TT * TT_U); idx += blockDim.x) {
-      const int u = (int)(idx / (TT * TT_U)), rem = (int)(idx - (int64_t)u * (TT * TT_U));
-      const int j = rem / TT, i = rem - j * TT;
-      const int4 it = items[u];
-      const int J = it.y / TT_UPT, jt = (it.y - J * TT_UPT) * TT_U + j;
-      const int r = it.x * TT + i, q = J * TT + jt;
-      if (r >= cs && q >= cs && r < n && q < n) {
-        const double v = Tm[(tt_tile(it.x, J) * TT + jt) * TT + i];
-        A[(int64_t)q * n + r] = v;
-        if (it.x != J) A[(int64_t)r * n + q] = v;
-      }
+  /* the switch to whole columns: the trailing block (indices >= cs) of the block's parts
+   * into A as float-float pairs, both triangles (the pending update of step cs-1 is applied
+   * by the first whole-column step) */
+  const int ni = s_ni;
+  for (int64_t idx = threadIdx.x; idx < (int64_t)ni * (TT * TT_U); idx += blockDim.x) {
+    const int u = (int)(idx / (TT * TT_U)), rem = (int)(idx - (int64_t)u * (TT * TT_U));
+    const int j = rem / TT, i = rem - j * TT;
+    const int4 it = items[u];
+    const int J = it.y / TT_UPT, jt = (it.y - J * TT_UPT) * TT_U + j;
+    const int r = it.x * TT + i, q = J * TT + jt;
+    if (r >= cs && q >= cs && r < n && q < n) {
+      const double v = Tm[(tt_tile(it.x, J) * TT + jt) * TT + i];
+      A[(int64_t)q * n + r] = v;
+      if (it.x != J) A[(int64_t)r * n + q] = v;
     }
-    target += G;
-    if (!tr_grid_sync(count, target, err)) return;
-    ff2 tau_pf = s_tau_p, scale_pf = s_scale_p, e_pf = s_e_p;
-    if (!tr_full_steps(A, n, cs, d, e, tau, vbuf, wbuf, ybuf, part_dot2, count, target, err, svp,
-                       swp, svc, tau_pf, scale_pf, e_pf, have_p,
-                       dotp + (size_t)((cs + 1) & 1) * nt, cs / TT, nt, stamp ? s_ph : NULL))
-      return;
-    if (stamp)
-      for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
-    tr_full_last(A, n, d, ybuf, part_dot2, tau_pf, e_pf, have_p);
-    return;
   }
+  target += G;
+  if (!tr_grid_sync(count, target, err)) return;
+  ff2 tau_pf = s_tau_p, scale_pf = s_scale_p, e_pf = s_e_p;
+  if (!tr_full_steps(A, n, cs, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, count, target, err,
+                     svp, swp, svc, tau_pf, scale_pf, e_pf, have_p,
+                     dotp + (size_t)((cs + 1) & 1) * nt, cs / TT, nt, stamp ? s_ph : NULL))
+    return;
   if (stamp)
     for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
 #undef TT_STAMP
-  /* last diagonal entry and the storage of the last reflector */
-  if (b == 0) {
-    ff2 dsum = ZERO;
-    if (have_p) {
-      if (threadIdx.x < 32) {
-        ff2 s = ZERO;
-        const double *pl = dotp + (size_t)((n - 2) & 1) * nt;
-        for (int k = (n - 1) / TT + (int)threadIdx.x; k < nt; k += 32) s = ff_add(s, ff_load(pl + k));
-        for (int o = 16; o; o >>= 1) s = ff_add(s, ff_shfl_xor(s, o));
-        if (threadIdx.x == 0) s_slotf = s;
-      }
-      __syncthreads();
-      dsum = s_slotf;
-    }
-    if (threadIdx.x == 0) {
-      const int Il = (n - 1) / TT, il = n - 1 - Il * TT;
-      ff2 a = ff_load(Tm + (tt_tile(Il, Il) * TT + il) * TT + il);
-      const ff2 tau_pf = s_tau_p, e_pf = s_e_p;
-      if (have_p) {
-        const ff2 alpha_p = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), dsum), -0.5f);
-        const ff2 wp =
-            ff_fma(tau_pf, ff_load(ybuf + (int64_t)((n - 2) & 1) * n + n - 1), alpha_p);
-        a = ff_add(a, ff_neg(wp));
-        a = ff_add(a, ff_neg(wp));
-        A[(int64_t)(n - 2) * n + n - 1] = ff_to_double(e_pf);
-      }
-      d[n - 1] = ff_to_double(a);
-    }
-  }
+  if (b == 0 && threadIdx.x == 0) *state = {tau_pf, scale_pf, e_pf};
 }
 
 /* deterministic start vector entry in (-1, 1) */
@@ -1829,6 +2120,28 @@ static void tt_tables(int nt, int pr, int pc, std::vector<unsigned char> &rgt,
   *maxi = mi;
 }
 
+/* dynamic shared memory of tr_smem_steps for trailing order m on G blocks */
+static size_t tr_smem_bytes(int m, int G)
+{
+  return sizeof(double) * (3 * (size_t)m + (size_t)((m + G - 1) / G) * m);
+}
+/* blocks for trailing order m: every block reads all of y and the column in each step, which
+ * costs more the more blocks ask (about 1,900 clocks for 16 of them, 4,000 for 64, 6,700 for
+ * 152 at m = 1,000), so no more than one for 12 columns, unless shared memory needs them
+ * (m = 400: 1.71 ms on 32, 2.18 on 152; m = 1,000: 6.0 on 64, 6.4 on 152) */
+static int tr_smem_blocks(int m, int G)
+{
+  int Gm = std::min(G, std::max(m / 12, (m + 31) / 32));
+  while (Gm < G && tr_smem_bytes(m, Gm) > 200 * 1024) ++Gm;
+  return Gm;
+}
+static int tr_smem_order(int G)
+{
+  int m = std::min(32 * G, TR_SMEM_NT * TR_SMEM_RPT);
+  while (m > 1 && tr_smem_bytes(m, G) > 200 * 1024) --m;
+  return m;
+}
+
 int gp_eig_tridiag(gp_ctx *ctx, int32_t n, int32_t nvec, double *d_evals_desc, double *d_vecs)
 {
   return gp_eig_sym(ctx, ctx->d_xtx, n, nvec, d_evals_desc, d_vecs);
@@ -1879,13 +2192,17 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
   int lw = lwork > lwork2 ? lwork : lwork2;
   /* partials + sums of k_apply_q, then the blocks' T from k_wy_tmat */
   const size_t qpart_n = (G + 1) * (size_t)WY_B * nv + nwy * WY_B * WY_B;
-  size_t bytes = sizeof(double) * (9 * nd + 2 * G + (size_t)lw + 6 * nd * nv + 80 + qpart_n) +
+  size_t bytes = sizeof(double) * (18 * nd + 2 * G + (size_t)lw + 6 * nd * nv + 80 + qpart_n) +
                  sizeof(int) * 64;
   double *base;
   int rc = gp_scratch(ctx, bytes, (void **)&base);
   if (rc) return rc;
   double *d = base, *e = d + nd, *tau = e + nd, *e2 = tau + nd, *w = e2 + nd;
-  double *wbuf = w + nd, *ybuf = wbuf + nd, *vbuf = ybuf + 2 * nd, *parts = vbuf + nd;
+  double *wbuf = w + nd, *ybuf = wbuf + nd, *vbuf = ybuf + 2 * nd;
+  /* the shared-memory steps' tagged y and columns, [2][n] of 16 bytes each (d.. + 10 nd: 16-byte
+   * aligned in the 256-byte aligned scratch) */
+  uint4 *ytag = (uint4 *)(base + 10 * nd);
+  double *parts = base + 18 * nd;
   unsigned *bar = (unsigned *)(parts + 2 * G);
   double *ws = parts + 2 * G + 16, *iw = ws + lw; /* 16 doubles: barrier words + phase timers */
   int *d_info = (int *)(iw + 6 * nd * nv + 8);
@@ -1893,6 +2210,10 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
   /* the cooperative tridiagonalisation (k_tridiag) unless GP_EIG_CUSOLVER_SYTRD=1, the
    * vectors do not fit shared memory or the device cannot co-schedule one block per SM */
   const char *senv = getenv("GP_EIG_CUSOLVER_SYTRD");
+  /* the trailing order from which the matrix stays in shared memory (GP_TRIDIAG_SMEM caps it) */
+  const char *m_env = getenv("GP_TRIDIAG_SMEM");
+  int m_smem = tr_smem_order((int)G);
+  if (m_env && m_env[0]) m_smem = std::max(1, std::min(m_smem, atoi(m_env)));
   const size_t tr_smem = 24 * nd;
   int coop = !(senv && senv[0] == '1') && n >= 2 && tr_smem <= 200 * 1024;
   if (coop) {
@@ -1966,43 +2287,79 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     return gp_fail(ctx, GP_ERR_CUDA, "eigensolve: the cooperative tridiagonalisation cannot run");
   GP_EIG_MARK(0);
   int info = 0;
-  if (tiled) {
-    const int64_t ntiles = (int64_t)nt * (nt + 1) / 2;
-    const size_t tile_d = (size_t)ntiles * TT * TT;
-    const size_t part_d = (size_t)(tt_pr + tt_pc) * nt * TT; /* prow + pcol */
-    const size_t tri_bytes = sizeof(double) * (tile_d + part_d + 2 * (size_t)nt) +
-                             sizeof(unsigned) * (size_t)nt;
-    int rc2 = gp_realloc(ctx, (void **)&ctx->d_tri, tri_bytes);
-    if (rc2) return rc2;
-    double *Tm = ctx->d_tri, *prow = Tm + tile_d, *pcol = prow + (size_t)nt * tt_pc * TT;
-    double *dotp = pcol + (size_t)nt * tt_pr * TT;
-    unsigned *kcnt = (unsigned *)(dotp + 2 * (size_t)nt);
+  if (coop) {
     int *d_err = ctx->d_err;
+    double *A = A_in, *pd2 = parts;
+    int nn = n;
+    /* the first steps run in tiles or in L2, those of the last m_smem rows in shared memory */
+    int c_end = std::max(tiled ? tt_cs : 0, n - m_smem);
+    tr_state *state = (tr_state *)((char *)bar + 80);
+    unsigned long long *phase = NULL;
     GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
     GP_CUDA(ctx, cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), ctx->stream));
-    GP_CUDA(ctx, cudaMemsetAsync(kcnt, 0, sizeof(unsigned) * (size_t)nt, ctx->stream));
-    {
-      int blocks = (int)std::min<int64_t>(ntiles, (int64_t)ctx->num_sms * 8);
-      k_tri_to_tiles<<<blocks, 256, 0, ctx->stream>>>(A_in, n, nt, Tm);
-      GP_LAUNCH_CHECK(ctx, "k_tri_to_tiles");
-    }
-    unsigned long long *phase = NULL;
+    GP_CUDA(ctx, cudaMemsetAsync(ytag, 0, sizeof(uint4) * 4 * nd, ctx->stream));
     if (timing) {
       phase = (unsigned long long *)(bar + 8);
       GP_CUDA(ctx, cudaMemsetAsync(phase, 0, 5 * sizeof(unsigned long long), ctx->stream));
     }
-    double *A = A_in, *pd2 = parts;
-    int nn = n, nt_ = nt, cs = tt_cs;
-    const unsigned char *rgt = ctx->d_tt, *cgt = ctx->d_tt + (size_t)nt * nt;
-    void *args[] = {&A,    &Tm,   &nn,   &nt_,  &tt_pr, &tt_pc, &tt_maxr, &tt_maxc,
-                    &tt_maxi, &tt_R, &cs, &rgt, &cgt,  &d,     &e,       &tau,
-                    &vbuf, &wbuf, &ybuf, &prow, &pcol, &dotp,  &kcnt,    &pd2,
-                    &bar,  &d_err, &phase};
-    GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
-    GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag_tiled, dim3((unsigned)G),
-                                             dim3(TR_THREADS), args, tt_smem, ctx->stream));
+    if (tiled) {
+      const int64_t ntiles = (int64_t)nt * (nt + 1) / 2;
+      const size_t tile_d = (size_t)ntiles * TT * TT;
+      const size_t part_d = (size_t)(tt_pr + tt_pc) * nt * TT; /* prow + pcol */
+      const size_t tri_bytes = sizeof(double) * (tile_d + part_d + 2 * (size_t)nt) +
+                               sizeof(unsigned) * (size_t)nt;
+      int rc2 = gp_realloc(ctx, (void **)&ctx->d_tri, tri_bytes);
+      if (rc2) return rc2;
+      double *Tm = ctx->d_tri, *prow = Tm + tile_d, *pcol = prow + (size_t)nt * tt_pc * TT;
+      double *dotp = pcol + (size_t)nt * tt_pr * TT;
+      unsigned *kcnt = (unsigned *)(dotp + 2 * (size_t)nt);
+      GP_CUDA(ctx, cudaMemsetAsync(kcnt, 0, sizeof(unsigned) * (size_t)nt, ctx->stream));
+      int blocks = (int)std::min<int64_t>(ntiles, (int64_t)ctx->num_sms * 8);
+      k_tri_to_tiles<<<blocks, 256, 0, ctx->stream>>>(A_in, n, nt, Tm);
+      GP_LAUNCH_CHECK(ctx, "k_tri_to_tiles");
+      int nt_ = nt, cs = tt_cs;
+      const unsigned char *rgt = ctx->d_tt, *cgt = ctx->d_tt + (size_t)nt * nt;
+      void *args[] = {&A,    &Tm,   &nn,   &nt_,  &tt_pr, &tt_pc, &tt_maxr, &tt_maxc,
+                      &tt_maxi, &tt_R, &cs, &rgt, &cgt,  &d,     &e,       &tau,
+                      &vbuf, &wbuf, &ybuf, &prow, &pcol, &dotp,  &kcnt,    &pd2,
+                      &bar,  &d_err, &phase, &c_end, &state};
+      GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
+      GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag_tiled, dim3((unsigned)G),
+                                               dim3(TR_THREADS), args, tt_smem, ctx->stream));
+      ctx->launches++;
+    } else {
+      int64_t tot = (int64_t)n * n;
+      int blocks = (int)((tot + 255) / 256);
+      if (blocks > ctx->num_sms * 16) blocks = ctx->num_sms * 16;
+      k_tri_to_ff<<<blocks, 256, 0, ctx->stream>>>(A, n);
+      GP_LAUNCH_CHECK(ctx, "k_tri_to_ff");
+      GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
+      if (c_end > 0) {
+        void *args[] = {&A,    &nn,   &c_end, &d,     &e,   &tau,   &vbuf,
+                        &wbuf, &ybuf, &pd2,   &state, &bar, &d_err, &phase};
+        GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag, dim3((unsigned)G),
+                                                 dim3(TR_THREADS), args, tr_smem, ctx->stream));
+        ctx->launches++;
+      }
+    }
+    {
+      const int m = n - c_end, small = m <= TR_SMALL_ORDER;
+      const void *f = small ? (const void *)k_tridiag_smem<256, TR_SMALL_ORDER / 256>
+                            : (const void *)k_tridiag_smem<TR_SMEM_NT, TR_SMEM_RPT>;
+      const int Gm = tr_smem_blocks(m, (int)G);
+      const double *xp = (c_end & 1) ? vbuf : wbuf;
+      const double *yp = ybuf + (int64_t)((c_end + 1) & 1) * n;
+      uint4 *ctag = ytag + 2 * nd;
+      unsigned *bar_s = bar + 1;
+      void *args[] = {&A,  &nn,   &c_end, &d,     &e,     &tau,  &xp,
+                      &yp, &ytag, &ctag,  &state, &bar_s, &d_err};
+      GP_CUDA(ctx, gp_allow_smem(ctx, f));
+      GP_CUDA(ctx, cudaLaunchCooperativeKernel(f, dim3((unsigned)Gm),
+                                               dim3(small ? 256 : TR_SMEM_NT), args,
+                                               tr_smem_bytes(m, Gm), ctx->stream));
+      ctx->launches++;
+    }
     GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr1, ctx->stream));
-    ctx->launches++;
     int herr = 0;
     GP_CUDA(ctx, gp_memcpy(ctx, &herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -2014,49 +2371,6 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "tridiagonalisation grid barrier timed out");
     float tms = 0.f;
     GP_CUDA(ctx, cudaEventElapsedTime(&tms, ctx->ev_tr0, ctx->ev_tr1));
-    if (A_in == ctx->d_xtx) {
-      ctx->tridiag_ms = tms;
-      ctx->tridiag_n = n;
-    }
-    if (timing) {
-      unsigned long long hp[5];
-      cudaMemcpy(hp, phase, sizeof hp, cudaMemcpyDeviceToHost);
-      fprintf(stderr,
-              "k_tridiag_tiled n=%d grid %dx%d, whole columns from step %d (block 0): A %.1f ms, "
-              "B %.1f (first 30%% of steps %.1f), barrier %.1f\n",
-              n, tt_pr, tt_pc, tt_cs, hp[0] * 1e-6, (hp[1] + hp[2]) * 1e-6, hp[2] * 1e-6,
-              hp[4] * 1e-6);
-    }
-  } else if (coop) {
-    int *d_err = ctx->d_err;
-    GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
-    GP_CUDA(ctx, cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), ctx->stream));
-    double *A = A_in, *pd2 = parts;
-    int nn = n;
-    {
-      int64_t tot = (int64_t)n * n;
-      int blocks = (int)((tot + 255) / 256);
-      if (blocks > ctx->num_sms * 16) blocks = ctx->num_sms * 16;
-      k_tri_to_ff<<<blocks, 256, 0, ctx->stream>>>(A, n);
-      GP_LAUNCH_CHECK(ctx, "k_tri_to_ff");
-    }
-    unsigned long long *phase = NULL;
-    if (timing) {
-      phase = (unsigned long long *)(bar + 8);
-      GP_CUDA(ctx, cudaMemsetAsync(phase, 0, 5 * sizeof(unsigned long long), ctx->stream));
-    }
-    void *args[] = {&A, &nn, &d, &e, &tau, &vbuf, &wbuf, &ybuf, &pd2, &bar, &d_err, &phase};
-    GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
-    GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag, dim3((unsigned)G),
-                                             dim3(TR_THREADS), args, tr_smem, ctx->stream));
-    GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr1, ctx->stream));
-    ctx->launches++;
-    int herr = 0;
-    GP_CUDA(ctx, gp_memcpy(ctx, &herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "tridiagonalisation grid barrier timed out");
-    float tms = 0.f;
-    GP_CUDA(ctx, cudaEventElapsedTime(&tms, ctx->ev_tr0, ctx->ev_tr1));
     if (A_in == ctx->d_xtx) { /* the Gram's eigensolve: its time is reported */
       ctx->tridiag_ms = tms;
       ctx->tridiag_n = n;
@@ -2065,9 +2379,9 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       unsigned long long hp[5];
       cudaMemcpy(hp, phase, sizeof hp, cudaMemcpyDeviceToHost);
       fprintf(stderr,
-              "k_tridiag n=%d (block 0): A %.1f ms, B %.1f (first 30%% of steps %.1f), "
-              "barrier %.1f\n",
-              n, hp[0] * 1e-6, (hp[1] + hp[2]) * 1e-6, hp[2] * 1e-6, hp[4] * 1e-6);
+              "tridiagonal n=%d (block 0), steps up to %d: A %.1f ms, B %.1f (first 30%% of "
+              "steps %.1f), barrier %.1f\n",
+              n, c_end, hp[0] * 1e-6, (hp[1] + hp[2]) * 1e-6, hp[2] * 1e-6, hp[4] * 1e-6);
     }
   } else {
     ctx->tridiag_ms = 0.0;
