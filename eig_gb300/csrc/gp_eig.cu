@@ -225,8 +225,11 @@ __device__ __forceinline__ int sturm_count_ff(const float *dh, const float *dl, 
  * A step evaluates P interior points of the bracket at once (one Sturm count per lane) and
  * keeps the sub-interval where the count crosses k: log2(P+1) bits per step.  FP32 counts
  * narrow the bracket to ~4e-7 ||T|| (widened by 64 eps_32 ||T||), float-float counts on the
- * FP32 pipe narrow it to ~1e-12 ||T|| (widened by 64 2^-44 ||T||), two FP64 counts check it
- * (back to the Gershgorin bracket if the check fails), then FP64 counts narrow it to tol.
+ * FP32 pipe narrow it to ~1e-12 ||T|| (widened by 16 2^-44 ||T||).  The first FP64 count takes
+ * the bracket's ends among its points, which checks it (back to the Gershgorin bracket if that
+ * fails), and FP64 counts narrow it to tol: n = 5,000 8.2 ms, of 10.1, and 1,000 0.95, of
+ * 1.13, with a check of its own and a bracket four times as wide.  (Three points per lane in
+ * the FP32 and float-float phases took longer, 12.0 and 1.5 ms: they are bound by issue.)
  * Grid: one CTA of 4 warps per SM; d, e2 and their FP32 hi/lo copies in shared memory
  * (32 N bytes) when they fit (use_smem 2), d, e2 and FP32 copies without the float-float
  * phase (24 N bytes, use_smem 1), else FP64 counts from global memory only.
@@ -314,21 +317,31 @@ k_multisect(const double *gd, const double *ge2, int n, double gl, double gu, do
         glo = nlo;
         ghi = nhi;
       }
-      const double margin2 = 64.0 * 0x1p-44 * tnorm;
+      const double margin2 = 16.0 * 0x1p-44 * tnorm;
       lo = fmax(gl, ff_to_double(glo) - margin2);
       hi = fmin(gu, ff_to_double(ghi) + margin2);
     }
-    int ok = 1;
-    if (sub < 2) {
-      const double x = sub == 0 ? lo : hi;
-      const int c = sturm_count_bits(d, e2, n, x, pivmin);
-      ok = sub == 0 ? (c <= k) : (c > k);
-      if (P == 1) ok = ok && sturm_count_bits(d, e2, n, hi, pivmin) > k; /* one lane: both ends */
-    }
-    const unsigned bad = (__ballot_sync(gmask, !ok) >> gshift) & gbits;
-    if (bad) {
-      lo = gl;
-      hi = gu;
+    if (P == 1) {
+      /* one lane: both ends in turn */
+      if (sturm_count_bits(d, e2, n, lo, pivmin) > k || sturm_count_bits(d, e2, n, hi, pivmin) <= k) {
+        lo = gl;
+        hi = gu;
+      }
+    } else {
+      /* P points from end to end: the ends check the bracket, the others narrow it */
+      const double wdt = hi - lo, den = (double)(P - 1);
+      const double x = sub == P - 1 ? hi : lo + wdt * (double)sub / den;
+      const int flag = sturm_count_bits(d, e2, n, x, pivmin) > k;
+      const unsigned b = (__ballot_sync(gmask, flag) >> gshift) & gbits;
+      if ((b & 1u) || !((b >> (P - 1)) & 1u)) {
+        lo = gl;
+        hi = gu;
+      } else {
+        const int first = __ffs(b) - 1;
+        const double nhi = first == P - 1 ? hi : lo + wdt * (double)first / den;
+        lo = first == 1 ? lo : lo + wdt * (double)(first - 1) / den;
+        hi = nhi;
+      }
     }
   }
   for (int it = 0; it < 200 && hi - lo > tol; ++it) {
@@ -1701,23 +1714,41 @@ __device__ double block_sum(double v, double *red)
   return r;
 }
 
+/* 1/q: rcp_newton and a second Newton step, to the last bits */
+__device__ __forceinline__ double rcp_full(double q)
+{
+  /* rcp_newton's exponent arithmetic holds well inside the normal range only */
+  const double a = fabs(q);
+  if (!(a > 1e-290 && a < 1e290)) return 1.0 / q;
+  const double r = rcp_newton(q);
+  return fma(r, fma(-q, r, 1.0), r);
+}
+
 /*
- * Inverse iteration, one block per top eigenvalue (vector j belongs to w[n-1-j]).
- * The LU factorisation with partial pivoting of T - lam I and the solves are sequential
- * recurrences run by thread 0 with the running values carried in registers (the arrays are
- * only written, or read ahead of the dependency chain); the other threads normalise.
+ * Inverse iteration, one block per top eigenvalue (vector j belongs to w[n-1-j]): the LU
+ * factorisation with partial pivoting of T - lam I and three solves.  The recurrences are
+ * sequential, each step a chain of FP64 instructions, so they run from both ends at once (the
+ * BABE factorisation, "burn at both ends"): lane 0 of the first warp eliminates columns
+ * 0 .. p-1 with rows 0 .. p, lane 0 of the second columns n-1 .. p+2 with rows n-1 .. p+1,
+ * p = (n-2)/2; what remains are two rows in the unknowns p and p+1, solved with pivoting, from
+ * which both substitute outwards.  The multiplier's reciprocal takes two Newton steps on a
+ * 23-bit seed instead of an FP64 division (about 300 clocks of latency against 1,000), and the
+ * solves use rows scaled by their pivots' reciprocals, so that a step's chain is one FMA.
  * With in_smem, the factors, the iterate and (during the factorisation) d and e sit in shared
  * memory, 41 n bytes, so that the recurrences wait on shared-memory rather than L2 latency:
  * d is staged where the iterate goes later and e where the second superdiagonal of U is
  * written, each e(i) being read before DU2(i) overwrites it.  Otherwise work holds the
  * factors (per vector 6n doubles) and the iterate stays in Z.
+ * n = 5,000: 2.57 ms, of 5.3 from one end; n = 1,000: 0.52 of 1.07.
  * Z [nvec][n] (column-major N x nvec).
  */
-__global__ void k_inverse_iteration(const double *__restrict__ d, const double *__restrict__ e,
-                                    int n, const double *__restrict__ w, int nvec, double tnorm,
-                                    double *Z, double *work, int in_smem)
+__global__ void __launch_bounds__(256)
+k_inverse_iteration(const double *__restrict__ d, const double *__restrict__ e, int n,
+                    const double *__restrict__ w, int nvec, double tnorm, double *Z, double *work,
+                    int in_smem)
 {
   __shared__ double red[256];
+  __shared__ double mid[2][3]; /* per side: the last row's entries at p, p + 1; its right side */
   extern __shared__ double ii_sm[];
   const int j = blockIdx.x;
   if (j >= nvec) return;
@@ -1738,43 +1769,59 @@ __global__ void k_inverse_iteration(const double *__restrict__ d, const double *
   }
   const double lam = w[n - 1 - j];
   const double tiny = DBL_EPSILON * tnorm;
-  if (threadIdx.x == 0) {
-    /* dgttrf-style elimination; cur = running diagonal of row i, du = its superdiagonal */
-    double cur = dd[0] - lam;
-    double du = n > 1 ? ee[0] : 0.0;
-    for (int i = 0; i < n - 1; ++i) {
-      const double ei = ee[i];
-      const double dn = dd[i + 1] - lam;               /* row i+1 diagonal */
-      const double en = (i < n - 2) ? ee[i + 1] : 0.0; /* row i+1 superdiagonal */
-      /* one division per step: the pivot's reciprocal, then the multiplier from it */
+  if (n == 1) {
+    if (threadIdx.x == 0) xg[0] = 1.0;
+    return;
+  }
+  const int p = (n - 2) / 2;
+  /* this thread's side: row and column k of it are at R(k); E(k) couples k and k + 1 */
+  const int side = threadIdx.x >> 5, runs = threadIdx.x == 0 || threadIdx.x == 32;
+  const int steps = side ? n - 2 - p : p;
+  auto R = [&](int k) { return side ? n - 1 - k : k; };
+  auto E = [&](int k) { return ee[side ? n - 2 - k : k]; };
+  if (runs) {
+    /* dgttrf-style elimination; cur = running diagonal of row k, du = its next entry */
+    double cur = dd[R(0)] - lam, du = E(0);
+    for (int k = 0; k < steps; ++k) {
+      const int i = R(k);
+      const double ei = E(k);
+      const double dn = dd[R(k + 1)] - lam; /* row k+1: diagonal and next entry */
+      const double en = E(k + 1);
       if (fabs(cur) >= fabs(ei)) {
         if (cur == 0.0) cur = tiny;
-        const double rc = 1.0 / cur;
-        double f = ei * rc;
+        const double rc = rcp_full(cur);
+        const double f = ei * rc;
         DL[i] = f;
         DU[i] = du;
         DU2[i] = 0.0;
         Dinv[i] = rc;
         piv[i] = 0;
-        cur = dn - f * du;
+        cur = fma(-f, du, dn);
         du = en;
       } else {
-        const double re = 1.0 / ei;
-        double f = cur * re;
+        const double re = rcp_full(ei);
+        const double f = cur * re;
         DL[i] = f;
         Dinv[i] = re;
         DU[i] = dn;
         DU2[i] = en;
         piv[i] = 1;
-        cur = du - f * dn;
+        cur = fma(-f, dn, du);
         du = -f * en;
       }
     }
-    if (cur == 0.0) cur = tiny;
-    Dinv[n - 1] = 1.0 / cur;
+    mid[side][side] = cur;
+    mid[side][1 - side] = du;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = start_entry(j, i);
+  /* rows scaled by their pivots' reciprocals */
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    if (i != p && i != p + 1) {
+      DU[i] *= Dinv[i];
+      DU2[i] *= Dinv[i];
+    }
+    x[i] = start_entry(j, i);
+  }
   __syncthreads();
   for (int iter = 0; iter < 3; ++iter) {
     double s2 = 0.0;
@@ -1783,25 +1830,55 @@ __global__ void k_inverse_iteration(const double *__restrict__ d, const double *
     double inv = s2 > 0.0 ? 1.0 / sqrt(s2) : 1.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] *= inv;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      /* forward: apply the row interchanges and L; carry x[i+1] in a register */
-      double xi = x[0];
-      for (int i = 0; i < n - 1; ++i) {
-        double xn = x[i + 1];
+    if (runs) {
+      /* inwards: apply the row interchanges and L; the running value in a register */
+      double xi = x[R(0)];
+      for (int k = 0; k < steps; ++k) {
+        const int i = R(k);
+        const double xn = x[R(k + 1)];
         if (piv[i] == 0) {
           x[i] = xi;
-          xi = xn - DL[i] * xi;
+          xi = fma(-DL[i], xi, xn);
         } else {
           x[i] = xn;
-          xi = xi - DL[i] * xn;
+          xi = fma(-DL[i], xn, xi);
         }
       }
-      x[n - 1] = xi;
-      /* back substitution with U (diag, super, super-super) */
-      double x2 = 0.0, x1 = x[n - 1] * Dinv[n - 1];
-      x[n - 1] = x1;
-      for (int i = n - 2; i >= 0; --i) {
-        double v = (x[i] - DU[i] * x1 - DU2[i] * x2) * Dinv[i];
+      mid[side][2] = xi;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      if (i != p && i != p + 1) x[i] *= Dinv[i];
+    if (threadIdx.x == 0) {
+      /* the two rows [a b | r], [c d | s] in x(p), x(p+1), with pivoting */
+      double a = mid[0][0], b = mid[0][1], r = mid[0][2];
+      double c = mid[1][0], dv = mid[1][1], t = mid[1][2];
+      if (fabs(c) > fabs(a)) {
+        double o = a;
+        a = c;
+        c = o;
+        o = b;
+        b = dv;
+        dv = o;
+        o = r;
+        r = t;
+        t = o;
+      }
+      if (a == 0.0) a = tiny;
+      const double f = c / a;
+      double dd2 = fma(-f, b, dv);
+      if (dd2 == 0.0) dd2 = tiny;
+      const double x1 = fma(-f, r, t) / dd2;
+      x[p + 1] = x1;
+      x[p] = fma(-b, x1, r) / a;
+    }
+    __syncthreads();
+    if (runs) {
+      /* outwards: x(k) = x'(k) - DU' x(k+1) - DU2' x(k+2) */
+      double x1 = x[R(steps)], x2 = x[R(steps + 1)];
+      for (int k = steps - 1; k >= 0; --k) {
+        const int i = R(k);
+        const double v = fma(-DU[i], x1, fma(-DU2[i], x2, x[i]));
         x[i] = v;
         x2 = x1;
         x1 = v;
@@ -1816,10 +1893,61 @@ __global__ void k_inverse_iteration(const double *__restrict__ d, const double *
   for (int i = threadIdx.x; i < n; i += blockDim.x) xg[i] = x[i] * inv;
 }
 
-/* modified Gram-Schmidt over the nvec vectors, in order (one block) */
-__global__ void k_mgs(double *Z, int n, int nvec)
+/*
+ * Orthonormalisation of the nvec vectors in order.  Inverse iteration leaves them orthogonal to
+ * about eps ||T|| / gap; where every product of two is below GS_SMALL, Gram-Schmidt's second-
+ * order terms are below rounding, so z_j - sum_{p<j} (z_p . z_j) z_p with the products of the
+ * vectors as they are is its result: all products at once (a block each), then every row by
+ * itself.  Otherwise one block runs modified Gram-Schmidt, a sum over the block for each pair:
+ * 141 us at n = 180 and 1.0 ms at 5,000 (10 and 20 vectors), with the products first 14
+ * and 35 us.
+ */
+#define GS_SMALL 1e-9
+#define GS_MAX 64
+
+/* S[p * nvec + j] = z_p . z_j for p <= j: block t for the t-th pair; *far = 1 where one is not
+ * small */
+__global__ void __launch_bounds__(256)
+k_gs_products(const double *__restrict__ Z, int n, int nvec, double *S, int *far)
 {
   __shared__ double red[256];
+  int j = 0, t = blockIdx.x;
+  while (t > j) t -= ++j;
+  const double *zp = Z + (int64_t)t * n, *zj = Z + (int64_t)j * n;
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s = fma(zp[i], zj[i], s);
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) {
+    S[t * nvec + j] = s;
+    if (!(t == j ? fabs(s - 1.0) < 1e-6 : fabs(s) < GS_SMALL)) *far = 1;
+  }
+}
+
+__global__ void __launch_bounds__(128)
+k_gs_apply(double *Z, int n, int nvec, const double *__restrict__ S, const int *far)
+{
+  __shared__ double c[GS_MAX * GS_MAX];
+  __shared__ double inv[GS_MAX];
+  if (*far) return;
+  for (int t = threadIdx.x; t < nvec * nvec; t += blockDim.x) c[t] = S[t];
+  __syncthreads();
+  for (int j = threadIdx.x; j < nvec; j += blockDim.x) inv[j] = 1.0 / sqrt(c[j * nvec + j]);
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  for (int j = nvec - 1; j >= 0; --j) { /* the earlier vectors are still as they were */
+    double z = Z[(int64_t)j * n + i];
+    for (int p = 0; p < j; ++p) z = fma(-c[p * nvec + j], Z[(int64_t)p * n + i], z);
+    Z[(int64_t)j * n + i] = z * inv[j];
+  }
+}
+
+/* modified Gram-Schmidt over the nvec vectors, in order (one block); nothing to do unless *far
+ * (NULL: always) */
+__global__ void k_mgs(double *Z, int n, int nvec, const int *far)
+{
+  __shared__ double red[256];
+  if (far && !*far) return;
   for (int j = 0; j < nvec; ++j) {
     double *zj = Z + (int64_t)j * n;
     for (int p = 0; p < j; ++p) {
@@ -2462,7 +2590,17 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
         d, e, n, w, nvec, tnorm, d_vecs, iw, ii_in_smem);
     GP_LAUNCH_CHECK(ctx, "k_inverse_iteration");
     GP_EIG_MARK(5);
-    k_mgs<<<1, 1024, 0, ctx->stream>>>(d_vecs, n, nvec);
+    int *far = NULL;
+    if (nvec <= GS_MAX) {
+      double *S = iw; /* the factors' room: 6 n nvec doubles, nvec <= n */
+      far = (int *)(iw + (size_t)nvec * nvec);
+      GP_CUDA(ctx, cudaMemsetAsync(far, 0, sizeof(int), ctx->stream));
+      k_gs_products<<<nvec * (nvec + 1) / 2, 256, 0, ctx->stream>>>(d_vecs, n, nvec, S, far);
+      GP_LAUNCH_CHECK(ctx, "k_gs_products");
+      k_gs_apply<<<(n + 127) / 128, 128, 0, ctx->stream>>>(d_vecs, n, nvec, S, far);
+      GP_LAUNCH_CHECK(ctx, "k_gs_apply");
+    }
+    k_mgs<<<1, 1024, 0, ctx->stream>>>(d_vecs, n, nvec, far);
     GP_LAUNCH_CHECK(ctx, "k_mgs");
     GP_EIG_MARK(6);
     /* Z := Q Z: the cooperative WY kernel when its row slab fits shared memory, else
@@ -2525,7 +2663,7 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       cudaEventElapsedTime(&t56, ev[5], ev[6]);
     }
     fprintf(stderr, "eig n=%d: tridiagonal %.1f ms, eigenvalues %.1f ms, vectors %.1f ms "
-            "(inverse iteration %.1f, mgs %.1f)\n", n, t01, t23, t34, t35, t56);
+            "(inverse iteration %.1f, Gram-Schmidt %.1f)\n", n, t01, t23, t34, t35, t56);
     for (int i = 0; i < 7; ++i) cudaEventDestroy(ev[i]);
   }
   return GP_OK;

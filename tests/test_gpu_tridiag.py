@@ -59,3 +59,32 @@ def test_rank_deficient(gpu, n, m):
     """reflectors of columns that are zero to rounding"""
     w = solve(gpu, n, m, 5)
     assert np.max(np.abs(w[m:])) <= 1e-11 * w[0]
+
+
+def test_repeated_eigenvalues(gpu):
+    """every sample carries one allele of its own: a multiple of I - 11'/n, whose vectors come
+    out of inverse iteration far from orthogonal"""
+    n = 40
+    gpu.load_genotypes(O.pack(np.eye(n, dtype=np.int8)), n)
+    gpu.set_samples(np.arange(n, dtype=np.int32))
+    gpu.set_snps(np.arange(n, dtype=np.int32))
+    x = gpu.xtx()
+    w, V = gpu.eigvecs(5)
+    A = x["XTX"] * ((n - 1) / x["trace"])
+    assert np.max(np.abs(w[:-1] - 1.0)) <= 1e-12 and abs(w[-1]) <= 1e-12
+    assert np.max(np.abs(V @ V.T - np.eye(5))) <= 1e-12
+    assert np.max(np.abs(A @ V.T - V.T * w[:5])) <= 1e-11
+
+
+def test_more_vectors_than_the_joint_orthonormalisation_takes(gpu):
+    r = np.random.default_rng(8)
+    n, m, k = 120, 900, 70
+    g = r.integers(0, 3, (m, n)).astype(np.int8)
+    gpu.load_genotypes(O.pack(g), n)
+    gpu.set_samples(np.arange(n, dtype=np.int32))
+    gpu.set_snps(np.arange(m, dtype=np.int32))
+    x = gpu.xtx()
+    w, V = gpu.eigvecs(k)
+    A = x["XTX"] * ((n - 1) / x["trace"])
+    assert np.max(np.abs(V @ V.T - np.eye(k))) <= 1e-9
+    assert np.max(np.abs(A @ V.T - V.T * w[:k])) <= 1e-10 * w[0]
