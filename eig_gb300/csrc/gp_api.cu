@@ -358,6 +358,10 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
   if (rc) return rc;
   double tr = 0.0;
   GP_CUDA(ctx, gp_memcpy(ctx, &tr, d_tr, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  if (symmetric) {
+    rc = gp_tc_check(ctx);
+    if (rc) return rc;
+  }
   if (n0 || n1 || nmiss) {
     std::vector<int32_t> cnt((size_t)nc * 3);
     GP_CUDA(ctx, gp_memcpy(ctx, cnt.data(), ctx->d_cnt, sizeof(int32_t) * cnt.size(),
@@ -888,7 +892,10 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   k_fvecs_T<<<blocks, 256, 0, ctx->stream>>>(d_B, ctx->d_evecs, n, K);
   GP_LAUNCH_CHECK(ctx, "k_fvecs_T");
   int tc = tc_products(ctx, nk);
+  const int tc_ran = tc;
   if (tc) {
+    rc = gp_tc_begin(ctx);
+    if (rc) return rc;
     /* tensor-core exact products: X = G fancy - O xmean, so
      * ffvecs^T = fancy (G^T W) - xmean (O^T W) with W = 10 evecs^T over the rows */
     rc = weights_tc(ctx, &kt, d_B, K, d_ffvT);
@@ -925,6 +932,10 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   }
   if (!tc) {
     rc = gp_geno_gemm_f64(ctx, 1, ctx->d_rows, n, kt.snprec, kt.rt, nk, d_ffvT, K, K, d_fxT, K);
+    if (rc) return rc;
+  }
+  if (tc_ran) {
+    rc = gp_tc_check(ctx);
     if (rc) return rc;
   }
   std::vector<double> fx((size_t)n * K);
@@ -1189,7 +1200,10 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
   }
   /* masked normal equations: co = O P (pair sums + observed count), rr = R E */
   int tc = d_raw ? 0 : tc_products(ctx, nk);
+  const int tc_ran = tc;
   if (tc) {
+    rc = gp_tc_begin(ctx);
+    if (rc) return rc;
     gp_tc_codes A;
     /* projecting exactly the analysis rows: the product can reuse their codes */
     const int32_t *d_list = d_samp;
@@ -1226,6 +1240,10 @@ static int lsqproj_impl(gp_ctx *ctx, int32_t numeigs, const int32_t *samples,
   GP_CUDA(ctx, cudaMemsetAsync(d_a, 0, sizeof(double) * nrr, ctx->stream));
   rc = gp_launch_lsq_solve(ctx, d_co, ldp, d_rr, K, nproj, d_a, d_b, d_nobs, d_st, NULL);
   if (rc) return rc;
+  if (tc_ran) {
+    rc = gp_tc_check(ctx);
+    if (rc) return rc;
+  }
   std::vector<int32_t> st((size_t)nproj);
   std::vector<double> ha(nrr);
   GP_CUDA(ctx, gp_memcpy(ctx, ha.data(), d_a, sizeof(double) * nrr, cudaMemcpyDeviceToHost,

@@ -543,6 +543,8 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
       if (rc) return rc;
     }
   }
+  rc = gp_tc_begin(ctx);
+  if (rc) return rc;
   /* the Krylov blocks, orthonormalised as they come: Q_i = X G_i, H_i = X^T Q_i */
   for (int32_t it = 0; it <= I; ++it) {
     if (use_tc) {
@@ -603,6 +605,8 @@ extern "C" int gp_fastpca(gp_ctx *ctx, int32_t K, int32_t L, int32_t I, uint64_t
       GP_LAUNCH_CHECK(ctx, "k_block_next");
     }
   }
+  rc = gp_tc_check(ctx);
+  if (rc) return rc;
   /* B = X^T U = Hp; B^T B = V diag(mu) V^T; eval = mu / M, evec = B v / sqrt(mu) */
   rc = ts_cross(ctx, d_Hp, c4, c4, d_Hp, c4, c4, n, d_part, part_cap, d_C);
   if (rc) return rc;

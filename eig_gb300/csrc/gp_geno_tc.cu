@@ -420,7 +420,7 @@ __global__ void k_invert_rows(const int32_t *samp, int32_t nsamp, int32_t *inv)
 
 /*
  * The same operand for rows that are distinct samples: all samples are transposed, the selected
- * ones written to their rows (inv).  A CTA covers 512 samples x 128 SNPs; a thread holds a word
+ * ones written to their rows (inv; NULL: every sample in order).  A CTA covers 512 samples x 128 SNPs; a thread holds a word
  * (16 samples) of 16 SNPs and transposes the 16 x 16 codes in registers: the 4 x 4 bytes of
  * words 4 apart by byte permutes, then the 4 x 4 codes of neighbouring words by masked swaps,
  * about half an instruction per code; pieces of 32 bytes per row leave through shared memory.
@@ -478,7 +478,7 @@ k_codes_transpose(const uint8_t *__restrict__ geno, int64_t rlen, int32_t nind,
     const int64_t q = ((int64_t)blockIdx.y * CT_W + (idx & (CT_W - 1))) * 16 + idx / CT_W;
     const int64_t at = (k0 >> 2) + 16 * half;
     if (q >= nind || at >= ldc) continue;
-    const int32_t r = inv[q];
+    const int64_t r = inv ? inv[q] : q;
     if (r < 0) continue;
     const uint32_t *o = so[idx] + 4 * half;
     *(uint4 *)(codes + (int64_t)r * ldc + at) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -527,27 +527,33 @@ k_codes_by_snp(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t *__
   }
 }
 
+/* one or two panels as the kernels take them */
+struct x_panels {
+  const double *P[2];
+  int64_t ldp[2];
+  double sign[2];
+};
+
 /*
- * per column c of P [nk][ldp] (FP64): running max of |P[k][c]| as its bit pattern (the
- * order of non-negative doubles), folded into mx[c] with atomicMax; threads keep a fixed
- * column so that a warp reads rows of P contiguously.  Several panels may fold into the
- * same mx (their joint exponent).
+ * per column c of the panels P [nk][ldp] (FP64, blockIdx.y): max of |P[k][c]| as its bit pattern
+ * (the order of non-negative doubles), folded into mx[c] with atomicMax: the panels' joint
+ * scale.  Threads keep a fixed column so that a warp reads rows of P contiguously.
  */
-__global__ void k_panel_absmax(const double *__restrict__ P, int64_t ldp, int32_t nk,
-                               int32_t ncols, unsigned long long *mx)
+__global__ void k_panel_absmax(const x_panels pan, int32_t nk, int32_t ncols,
+                               unsigned long long *mx)
 {
   __shared__ unsigned long long smx[1024];
   for (int c = threadIdx.x; c < ncols; c += blockDim.x) smx[c] = 0ull;
   __syncthreads();
-  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  const int64_t step = nthreads / ncols * ncols;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < step) {
-    const int32_t c = (int32_t)(t % ncols);
+  const double *__restrict__ P = pan.P[blockIdx.y];
+  const int64_t ldp = pan.ldp[blockIdx.y];
+  const int32_t rows = (int32_t)((int64_t)gridDim.x * blockDim.x / ncols); /* per round */
+  const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t k0 = t / ncols, c = t - k0 * ncols;
+  if (k0 < rows) {
     unsigned long long m = 0ull;
-    const int64_t total = (int64_t)nk * ncols;
-    for (int64_t idx = t; idx < total; idx += step) {
-      const int64_t k = idx / ncols;
+#pragma unroll 4
+    for (int64_t k = k0; k < nk; k += rows) {
       const unsigned long long bits =
           (unsigned long long)__double_as_longlong(P[k * ldp + c]) & 0x7FFFFFFFFFFFFFFFull;
       m = bits > m ? bits : m;
@@ -555,22 +561,21 @@ __global__ void k_panel_absmax(const double *__restrict__ P, int64_t ldp, int32_
     if (m) atomicMax(smx + c, m);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < ncols; c += blockDim.x)
-    if (smx[c]) atomicMax(mx + c, smx[c]);
+  for (int i = threadIdx.x; i < ncols; i += blockDim.x)
+    if (smx[i]) atomicMax(mx + i, smx[i]);
 }
 
-/* exponent e_c with max|P| < 2^e_c (frexp), 0 for an all-zero column, X_NONFINITE for one with
- * an infinity or NaN (5 slices: its products are NaN, as FP64 products of 0 and it are) */
+/* exponent e_c with max|P| < 2^e_c (frexp) of a column's mx, 0 for an all-zero column; with 5
+ * slices X_NONFINITE for one with an infinity or NaN (its products are NaN, as FP64 products of
+ * 0 and it are) */
 #define X_NONFINITE (-(1 << 30))
-__global__ void k_panel_expo(const unsigned long long *mx, int32_t ncols, int32_t *expo, int mark)
+template <int S>
+__device__ __forceinline__ int x_exponent(unsigned long long mx)
 {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols; c += gridDim.x * blockDim.x) {
-    const double v = __longlong_as_double((long long)mx[c]);
-    int e = 0;
-    if (v > 0.0) frexp(v, &e); /* v = f 2^e, f in [0.5, 1) -> v < 2^e */
-    if (mark && mx[c] >= 0x7FF0000000000000ull) e = X_NONFINITE;
-    expo[c] = e;
-  }
+  if (S == 5 && mx >= 0x7FF0000000000000ull) return X_NONFINITE;
+  int e = 0;
+  if (mx) frexp(__longlong_as_double((long long)mx), &e); /* v = f 2^e, f in [0.5, 1) */
+  return e;
 }
 
 /*
@@ -613,26 +618,29 @@ __device__ __forceinline__ void slice(double v, int e, bool neg, int d[S])
 }
 
 /*
- * B[(Sc+t)][koff + k] (fp16, row stride ldb elements) = slice t of sign P[k][c] / 2^e_c for
- * k < nk (pad k and pad rows are zero from a memset before).  A tile of 64 k x 32 columns is
- * read row-wise (coalesced) into shared memory and written as 128-byte rows of B.
+ * B[(Sc+t)][p kpad + k] (fp16, row stride ldb elements, rows of them) = slice t of sign P[k][c] /
+ * 2^e_c of panel p = blockIdx.z for k < nk; pad k and pad rows zero.  A tile of 64 k x 32
+ * columns is read row-wise (coalesced) into shared memory and written as 128-byte rows of B.
  */
 #define SL_K 64
 #define SL_C 32
 template <int S>
 __global__ void __launch_bounds__(256)
-k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t ncols,
-               const int32_t *__restrict__ expo, double sign, int64_t koff, __half *B, int64_t ldb)
+k_panel_slices(const x_panels pan, int32_t nk, int32_t ncols,
+               const unsigned long long *__restrict__ mx, __half *B, int64_t ldb, int32_t kpad,
+               int32_t rows)
 {
   __shared__ double sp[SL_K][SL_C + 1];
   __shared__ __align__(16) __half ss[SL_C * S][SL_K + 8];
   __shared__ int sexp[SL_C];
+  const double *__restrict__ P = pan.P[blockIdx.z];
+  const int64_t ldp = pan.ldp[blockIdx.z];
+  const bool neg = pan.sign[blockIdx.z] < 0.0;
   const int tid = threadIdx.x;
   const int32_t kt0 = blockIdx.x * SL_K, ct0 = blockIdx.y * SL_C;
-  const bool neg = sign < 0.0;
   if (tid < SL_C) {
     const int32_t c = ct0 + tid;
-    sexp[tid] = c < ncols ? expo[c] : 0;
+    sexp[tid] = c < ncols ? x_exponent<S>(mx[c]) : 0;
   }
   for (int i = tid; i < SL_K * SL_C; i += blockDim.x) {
     const int kk = i / SL_C, cc = i - kk * SL_C;
@@ -652,11 +660,9 @@ k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t nc
   /* 32 S output rows x 64 halves: 8 threads write one row's 128 bytes */
   for (int i = tid; i < SL_C * S * 8; i += blockDim.x) {
     const int o = i >> 3, seg = i & 7;
-    const int32_t c = ct0 + o / S;
-    if (c >= ncols) continue;
-    const int32_t k = kt0 + seg * 8;
-    if (k >= nk) continue;
-    __half *dst = B + (int64_t)(S * ct0 + o) * ldb + koff + k;
+    const int32_t r = S * ct0 + o;
+    if (r >= rows) continue;
+    __half *dst = B + (int64_t)r * ldb + (int64_t)blockIdx.z * kpad + kt0 + seg * 8;
     *(uint4 *)dst = *(const uint4 *)&ss[o][seg * 8];
   }
 }
@@ -670,7 +676,7 @@ k_panel_slices(const double *__restrict__ P, int64_t ldp, int32_t nk, int32_t nc
 template <int S>
 __global__ void __launch_bounds__(256)
 k_panel_combine(const unsigned long long *__restrict__ sums, int32_t wcols, int32_t nrows,
-                int32_t ncols, const int32_t *__restrict__ expo, double *Y, int64_t ldy,
+                int32_t ncols, const unsigned long long *__restrict__ mx, double *Y, int64_t ldy,
                 const gp_tc_batch *db)
 {
   __shared__ double sy[32][33];
@@ -687,7 +693,7 @@ k_panel_combine(const unsigned long long *__restrict__ sums, int32_t wcols, int3
         double z[S];
 #pragma unroll
         for (int t = 0; t < S; ++t) z[t] = (double)(long long)src[(int64_t)(S * cc + t) * XR];
-        const int e = expo[c0 + cc];
+        const int e = x_exponent<S>(mx[c0 + cc]);
         if (S == 4) {
           const double v = ((z[0] * 0x1p-10 + z[1] * 0x1p-20) + z[2] * 0x1p-30) + z[3] * 0x1p-40;
           sy[cc][lane] = ldexp(v, e);
@@ -756,9 +762,13 @@ int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int
    * measured six times as fast per code as gathering them (all of 5,000 x 200,000: 120 us and
    * 734) */
   if (sum_over_snps && inv && ctx->nind_all <= 4 * (int64_t)nsamp) {
-    GP_CUDA(ctx, cudaMemsetAsync(inv, 0xFF, sizeof(int32_t) * (size_t)ctx->nind_all, ctx->stream));
-    k_invert_rows<<<grid_cap(ctx, nsamp, 256, 4), 256, 0, ctx->stream>>>(d_samp, nsamp, inv);
-    GP_LAUNCH_CHECK(ctx, "k_invert_rows");
+    if (nsamp == ctx->nind_all && d_samp == ctx->d_rows) {
+      inv = NULL; /* every sample, in order */
+    } else {
+      GP_CUDA(ctx, cudaMemsetAsync(inv, 0xFF, sizeof(int32_t) * (size_t)ctx->nind_all, ctx->stream));
+      k_invert_rows<<<grid_cap(ctx, nsamp, 256, 4), 256, 0, ctx->stream>>>(d_samp, nsamp, inv);
+      GP_LAUNCH_CHECK(ctx, "k_invert_rows");
+    }
     dim3 grid((unsigned)((ldc * 4 + 127) / 128),
               (unsigned)((ctx->rlen_dev / 4 + CT_W - 1) / CT_W));
     k_codes_transpose<<<grid, 256, 0, ctx->stream>>>(ctx->d_geno, ctx->rlen_dev, ctx->nind_all, inv,
@@ -800,7 +810,7 @@ size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits)
   const int32_t kpad0 = (k0 + XK - 1) / XK * XK;
   const int32_t tn = x_tile_cols(digits * ncols), nct = (digits * ncols + tn - 1) / tn;
   const int32_t ncols4_pad = nct * tn;
-  return align256((size_t)ncols4_pad * kpad0 * npanels * 2) + align256((size_t)ncols * 16) + 256;
+  return align256((size_t)ncols4_pad * kpad0 * npanels * 2) + align256((size_t)ncols * 8) + 256;
 }
 
 int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols, int32_t k0,
@@ -814,26 +824,26 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   const int64_t ldb = (int64_t)kpad0 * npanels;
   uint8_t *base = (uint8_t *)storage;
   __half *B = (__half *)base;
-  uint8_t *ebase = base + align256((size_t)ncols4_pad * ldb * 2);
-  unsigned long long *mx = (unsigned long long *)ebase; /* [ncols] joint max |P| bits */
-  int32_t *expo = (int32_t *)(ebase + 8 * (size_t)ncols);
+  /* [ncols] joint max |P| bits */
+  unsigned long long *mx = (unsigned long long *)(base + align256((size_t)ncols4_pad * ldb * 2));
+  x_panels pan = {};
+  for (int p = 0; p < npanels; ++p) {
+    pan.P[p] = pp[p].P;
+    pan.ldp[p] = pp[p].ldp;
+    pan.sign[p] = pp[p].sign;
+  }
   GP_CUDA(ctx, cudaMemsetAsync(mx, 0, 8 * (size_t)ncols, ctx->stream));
-  for (int p = 0; p < npanels; ++p) {
-    int blocks = grid_cap(ctx, (int64_t)k0 * ncols, 256 * 16, 8);
-    const int need = (ncols + 255) / 256;
-    if (blocks < need) blocks = need;
-    k_panel_absmax<<<blocks, 256, 0, ctx->stream>>>(pp[p].P, pp[p].ldp, k0, ncols, mx);
-    GP_LAUNCH_CHECK(ctx, "k_panel_absmax");
-  }
-  k_panel_expo<<<(ncols + 255) / 256, 256, 0, ctx->stream>>>(mx, ncols, expo, digits == 5);
-  GP_LAUNCH_CHECK(ctx, "k_panel_expo");
-  GP_CUDA(ctx, cudaMemsetAsync(B, 0, (size_t)ncols4_pad * ldb * 2, ctx->stream));
-  for (int p = 0; p < npanels; ++p) {
-    dim3 sgrid((unsigned)((k0 + SL_K - 1) / SL_K), (unsigned)((ncols + SL_C - 1) / SL_C));
-    (digits == 5 ? k_panel_slices<5> : k_panel_slices<4>)<<<sgrid, 256, 0, ctx->stream>>>(
-        pp[p].P, pp[p].ldp, k0, ncols, expo, pp[p].sign, (int64_t)p * kpad0, B, ldb);
-    GP_LAUNCH_CHECK(ctx, "k_panel_slices");
-  }
+  int blocks = grid_cap(ctx, (int64_t)k0 * ncols, 256 * 16, 8);
+  const int need = (ncols + 255) / 256;
+  if (blocks < need) blocks = need;
+  k_panel_absmax<<<dim3((unsigned)blocks, (unsigned)npanels), 256, 0, ctx->stream>>>(pan, k0, ncols,
+                                                                                    mx);
+  GP_LAUNCH_CHECK(ctx, "k_panel_absmax");
+  dim3 sgrid((unsigned)(kpad0 / SL_K), (unsigned)((ncols4_pad + digits * SL_C - 1) / (digits * SL_C)),
+             (unsigned)npanels);
+  (digits == 5 ? k_panel_slices<5> : k_panel_slices<4>)<<<sgrid, 256, 0, ctx->stream>>>(
+      pan, k0, ncols, mx, B, ldb, kpad0, ncols4_pad);
+  GP_LAUNCH_CHECK(ctx, "k_panel_slices");
   PFN_cuTensorMapEncodeTiled_v12000 enc = tc_encode(ctx);
   if (!enc) return GP_ERR_CUDA;
   {
@@ -847,7 +857,7 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
     if (r != CUDA_SUCCESS) return gp_fail(ctx, GP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   }
   out->B = B;
-  out->expo = expo;
+  out->mx = mx;
   out->ncols = ncols;
   out->tn = tn;
   out->nct = nct;
@@ -872,8 +882,23 @@ static int combine_grid(const gp_ctx *ctx, int64_t nrows, int32_t ncols)
   return grid_cap(ctx, (nrows + 31) / 32 * ((ncols + 31) / 32), 1, 32);
 }
 
+int gp_tc_begin(gp_ctx *ctx)
+{
+  GP_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+  return GP_OK;
+}
+
+int gp_tc_check(gp_ctx *ctx)
+{
+  int herr = 0;
+  GP_CUDA(ctx, gp_memcpy(ctx, &herr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "tensor-core product wait timed out (code %d)", herr);
+  return GP_OK;
+}
+
 int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, double *d_Y,
-                int64_t ldy, int sync)
+                int64_t ldy)
 {
   const int32_t nrows = A->nrows;
   if (nrows < 1) return GP_OK;
@@ -883,8 +908,6 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   unsigned long long *sums;
   int rc = gp_scratch5(ctx, sum_bytes + 256, (void **)&sums);
   if (rc) return rc;
-  int *d_err = ctx->d_err;
-  if (sync) GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
   GP_CUDA(ctx, cudaMemsetAsync(sums, 0, sum_bytes, ctx->stream));
   GP_CUDA(ctx, cudaFuncSetAttribute(k_geno_panel_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     X_SMEM));
@@ -895,17 +918,12 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   const int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
   k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(
       P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->lut_lo, P->lut_hi,
-      ksplit, X_CHUNK_KB(P->digits), sums, d_err, NULL);
+      ksplit, X_CHUNK_KB(P->digits), sums, ctx->d_err, NULL);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
       <<<combine_grid(ctx, nrows, P->ncols), 256, 0, ctx->stream>>>(
-          sums, P->nct * P->tn, nrows, P->ncols, P->expo, d_Y, ldy, NULL);
+          sums, P->nct * P->tn, nrows, P->ncols, P->mx, d_Y, ldy, NULL);
   GP_LAUNCH_CHECK(ctx, "k_panel_combine");
-  if (!sync) return GP_OK;
-  int herr = 0;
-  GP_CUDA(ctx, gp_memcpy(ctx, &herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "tensor-core product wait timed out (code %d)", herr);
   return GP_OK;
 }
 
@@ -937,7 +955,7 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
       1, X_CHUNK_KB(4), z, ctx->d_err, db);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   k_panel_combine<4><<<combine_grid(ctx, max_rows, P->ncols), 256, 0, ctx->stream>>>(
-      z, wcols, 0, P->ncols, P->expo, d_Y, ldy, db);
+      z, wcols, 0, P->ncols, P->mx, d_Y, ldy, db);
   GP_LAUNCH_CHECK(ctx, "k_panel_combine");
   return GP_OK;
 }
@@ -960,7 +978,7 @@ int gp_geno_panel_tc_codes(gp_ctx *ctx, const gp_tc_codes *A, int npanels, const
     if (rc) return rc;
     gp_tc_prepared P;
     rc = gp_tc_prepare(ctx, npanels, pg, nc, A->k0, digits, storage, &P);
-    if (!rc) rc = gp_tc_apply(ctx, A, &P, d_Y + c0, ldy, 1);
+    if (!rc) rc = gp_tc_apply(ctx, A, &P, d_Y + c0, ldy);
     if (rc) return rc;
   }
   return GP_OK;

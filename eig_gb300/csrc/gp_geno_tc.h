@@ -37,7 +37,7 @@ int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int
  * slices, 4 of 10 bits (the split precisions) or 5 of 12 bits (FP64) */
 struct gp_tc_prepared {
   __half *B;
-  int32_t *expo;
+  unsigned long long *mx; /* per column the bits of its largest magnitude: its exponent */
   int32_t ncols, npanels, digits, kb0, k0;
   int32_t tn, nct; /* slice columns per tile, column tiles */
   int64_t ldb;
@@ -48,10 +48,13 @@ size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits);
 /* slice the panels into caller storage of gp_tc_prepared_bytes bytes (device) */
 int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols, int32_t k0,
                   int digits, void *storage, gp_tc_prepared *out);
-/* Y[r][c] = products of the code operand with a prepared panel; sync = 0 leaves the work
- * queued on ctx->stream and neither clears nor reads ctx->d_err (the caller does both) */
+/* Y[r][c] = products of the code operand with a prepared panel, queued on ctx->stream.  Its
+ * bounded waits report through ctx->d_err: gp_tc_begin clears it ahead of any number of
+ * products, gp_tc_check waits for them and returns the error */
 int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, double *d_Y,
-                int64_t ldy, int sync);
+                int64_t ldy);
+int gp_tc_begin(gp_ctx *ctx);
+int gp_tc_check(gp_ctx *ctx);
 
 /* The batch a device-resident loop works on: nrows code rows at codes (ring position row0
  * of the pool), requests [req_begin, req_end) of the loop's queue.  Written on the device

@@ -519,13 +519,14 @@ int gp_gram_exact(gp_ctx *ctx)
   for (int32_t b = 0; b * EX_ROWS < n; ++b) ntiles += ex_row_tiles(b, n);
   uint8_t *base, *B;
   unsigned long long *sums;
-  int rc = gp_scratch(ctx, sizeof(int32_t) * (size_t)nk + 256, (void **)&base);
+  int32_t *snprec;
+  int rc = gp_scratch(ctx, sizeof(int32_t) * (size_t)nk, (void **)&snprec);
   if (rc) return rc;
-  unsigned long long *mx = (unsigned long long *)base;
-  int32_t *snprec = (int32_t *)(base + 256);
   const size_t sum_bytes = sizeof(*sums) * 2 * EX_TILE * (size_t)ntiles;
-  rc = gp_scratch5(ctx, sum_bytes, (void **)&sums);
+  rc = gp_scratch5(ctx, 256 + sum_bytes, (void **)&base);
   if (rc) return rc;
+  unsigned long long *mx = (unsigned long long *)base; /* ahead of the sums: one memset */
+  sums = mx + 32;
   /* the right operand of as many k-blocks as fit the budget, fewer where memory is short */
   const size_t per_kb = 2 * EX_B_BYTES * (size_t)ntj;
   int32_t kbp = (int32_t)(EX_BUDGET / (int64_t)per_kb);
@@ -543,9 +544,9 @@ int gp_gram_exact(gp_ctx *ctx)
   }
   if (rc) return rc;
 
-  GP_CUDA(ctx, cudaMemsetAsync(mx, 0, sizeof(*mx), ctx->stream));
-  GP_CUDA(ctx, cudaMemsetAsync(sums, 0, sum_bytes, ctx->stream));
-  GP_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+  GP_CUDA(ctx, cudaMemsetAsync(mx, 0, 256 + sum_bytes, ctx->stream));
+  rc = gp_tc_begin(ctx);
+  if (rc) return rc;
   int blocks = (nk + 255) / 256;
   if (blocks > ctx->num_sms * 4) blocks = ctx->num_sms * 4;
   k_exact_max<<<blocks, 256, 0, ctx->stream>>>(ctx->d_kept, nk, ctx->d_cols, ctx->d_vtab,
@@ -571,9 +572,5 @@ int gp_gram_exact(gp_ctx *ctx)
   }
   k_exact_finish<<<dim3((unsigned)ntiles, 2, 2), 256, 0, ctx->stream>>>(sums, mx, n, ctx->d_xtx);
   GP_LAUNCH_CHECK(ctx, "k_exact_finish");
-  int herr = 0;
-  GP_CUDA(ctx, gp_memcpy(ctx, &herr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "FP64 Gram kernel wait timed out (code %d)", herr);
   return GP_OK;
 }

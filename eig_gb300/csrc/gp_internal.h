@@ -160,8 +160,9 @@ int gp_lsq_fill_tables(gp_ctx *ctx, const int32_t *d_samp, const int32_t *d_spop
                        int32_t npop, int32_t K, const int32_t *d_snprec, const double *d_ot,
                        int32_t nk, void *work, double **d_raw, double **d_of, double **d_rf);
 int gp_gram_fp64(gp_ctx *ctx);
-/* the FP64 Gram as exact integer sums on the tensor cores (both triangles written); needs at
- * least one kept SNP and no population fill; GP_ERR_NOMEM leaves the Gram untouched */
+/* the FP64 Gram as exact integer sums on the tensor cores (both triangles written), queued on
+ * ctx->stream: gp_tc_check reports its bounded waits; needs at least one kept SNP and no
+ * population fill; GP_ERR_NOMEM leaves the Gram untouched */
 int gp_gram_exact(gp_ctx *ctx);
 int gp_gram_split(gp_ctx *ctx, int precision);
 /* the trace of the Gram; its upper triangle is filled first unless `symmetric` */

@@ -377,8 +377,8 @@ static int launch_batch(gp_server *s, gp_batch *b)
   A.k0 = s->nk;
   int rc;
   if (!s->fp64_serial) {
-    rc = gp_tc_apply(ctx, &A, &s->Pco, s->d_co[sl], s->ldp, 0);
-    if (!rc) rc = gp_tc_apply(ctx, &A, &s->Prr, s->d_rr[sl], s->K, 0);
+    rc = gp_tc_apply(ctx, &A, &s->Pco, s->d_co[sl], s->ldp);
+    if (!rc) rc = gp_tc_apply(ctx, &A, &s->Prr, s->d_rr[sl], s->K);
     if (rc) return rc;
   } else {
     const int32_t n = b->nrows;
