@@ -8,7 +8,12 @@
 #include <math.h>
 #include <stdarg.h>
 #include <stdlib.h>
+#include <sys/mman.h>
+#include <unistd.h>
 #include <algorithm>
+#include <atomic>
+#include <memory>
+#include <thread>
 #include <vector>
 
 #include "gp_geno_gemm.h"
@@ -47,6 +52,93 @@ cudaError_t gp_memcpy(gp_ctx *ctx, void *dst, const void *src, size_t bytes, cud
   if (kind == cudaMemcpyHostToDevice) ctx->h2d_bytes += (int64_t)bytes;
   if (kind == cudaMemcpyDeviceToHost) ctx->d2h_bytes += (int64_t)bytes;
   return cudaMemcpyAsync(dst, src, bytes, kind, stream);
+}
+
+#define OP_PIECE ((size_t)4 << 20)
+#define OP_LEAST ((size_t)8 << 20)
+#define OP_THREADS 4
+
+struct gp_out_pages::impl {
+  std::vector<std::thread> threads;
+  std::atomic<size_t> next{0};
+  std::unique_ptr<std::atomic<uint8_t>[]> done;
+  size_t npieces = 0;
+
+  void run(uint8_t *base, size_t bytes)
+  {
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (size_t i; (i = next.fetch_add(1)) < npieces;) {
+      /* whole pages that begin in the piece (the first piece's partial page stays as it is) */
+      const uintptr_t end = (uintptr_t)base + bytes;
+      uintptr_t a = (uintptr_t)base + i * OP_PIECE, b = a + OP_PIECE < end ? a + OP_PIECE : end;
+      a = (a + page - 1) / page * page;
+      b = (b + page - 1) / page * page;
+      if (b > end) b -= page;
+#ifdef MADV_POPULATE_WRITE
+      if (a < b) (void)madvise((void *)a, b - a, MADV_POPULATE_WRITE); /* a hint: may fail */
+#endif
+      done[i].store(1, std::memory_order_release);
+    }
+  }
+};
+
+gp_out_pages::gp_out_pages(void *dst, size_t n) : base((uint8_t *)dst), bytes(n), im(NULL)
+{
+  if (!dst || n < OP_LEAST) return;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  try {
+    std::unique_ptr<impl> p(new impl);
+    p->npieces = (n + OP_PIECE - 1) / OP_PIECE;
+    p->done.reset(new std::atomic<uint8_t>[p->npieces]);
+    for (size_t i = 0; i < p->npieces; ++i) p->done[i].store(0, std::memory_order_relaxed);
+    impl *q = p.get();
+    p->threads.reserve(OP_THREADS);
+    im = p.release();
+    for (int t = 0; t < OP_THREADS; ++t)
+      im->threads.emplace_back([q, this] { q->run(this->base, this->bytes); });
+  } catch (...) {
+    /* no memory or no thread: the pieces that no thread takes are nobody's to wait for */
+    if (im && im->threads.empty()) {
+      delete im;
+      im = NULL;
+    }
+  }
+}
+
+gp_out_pages::~gp_out_pages()
+{
+  if (!im) return;
+  im->next.store(im->npieces); /* pieces not begun are not needed any more */
+  for (std::thread &t : im->threads) t.join();
+  delete im;
+}
+
+void gp_out_pages::wait(size_t begin, size_t end)
+{
+  if (!im || end <= begin) return;
+  for (size_t i = begin / OP_PIECE; i <= (end - 1) / OP_PIECE; ++i)
+    while (!im->done[i].load(std::memory_order_acquire)) std::this_thread::yield();
+}
+
+cudaError_t gp_copy_out(gp_ctx *ctx, gp_out_pages &pages, size_t offset, const void *src,
+                        size_t bytes)
+{
+  if (!pages.im)
+    return gp_memcpy(ctx, pages.base + offset, src, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+  for (size_t a = 0; a < bytes;) {
+    const size_t n = bytes - a < 4 * OP_PIECE ? bytes - a : 4 * OP_PIECE;
+    pages.wait(offset + a, offset + a + n);
+    cudaError_t e = gp_memcpy(ctx, pages.base + offset + a, (const uint8_t *)src + a, n,
+                              cudaMemcpyDeviceToHost, ctx->stream);
+    if (e != cudaSuccess) return e;
+    a += n;
+  }
+  return cudaSuccess;
 }
 
 int gp_cuda_fail(gp_ctx *ctx, cudaError_t e, const char *what)
@@ -299,6 +391,7 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
   }
   ctx->xtx_valid = ctx->eig_valid = ctx->weights_valid = 0;
   ctx->precision = opts->precision;
+  gp_out_pages out_pages(XTX, XTX ? sizeof(double) * (size_t)need : 0);
   int rc;
   if (ctx->npop > 0) {
     /* usepopsformissing: the observed counts first (the missing-count rule waits for the
@@ -381,8 +474,7 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
     GP_CUDA(ctx, gp_memcpy(ctx, xfancy, ctx->d_xfancy, sizeof(double) * nc,
                                  cudaMemcpyDeviceToHost, ctx->stream));
   if (XTX)
-    GP_CUDA(ctx, gp_memcpy(ctx, XTX, ctx->d_xtx, sizeof(double) * (size_t)need,
-                                 cudaMemcpyDeviceToHost, ctx->stream));
+    GP_CUDA(ctx, gp_copy_out(ctx, out_pages, 0, ctx->d_xtx, sizeof(double) * (size_t)need));
   GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   float gms = 0.f;
   GP_CUDA(ctx, cudaEventElapsedTime(&gms, ctx->ev_g0, ctx->ev_g1));
@@ -876,6 +968,7 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   int rc = gp_realloc(ctx, (void **)&ctx->d_ffvecs, sizeof(double) * (size_t)K * nc);
   if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_fxscal, sizeof(double) * (size_t)K);
   if (rc) return rc;
+  gp_out_pages out_pages(ffvecs, ffvecs ? sizeof(double) * (size_t)K * nc : 0);
   size_t off_tab = kept_tables_bytes(nk);
   size_t bytes = off_tab + sizeof(double) * ((size_t)n * K + (size_t)nk * K + (size_t)n * K) + 256;
   uint8_t *base;
@@ -942,8 +1035,7 @@ extern "C" int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, doub
   GP_CUDA(ctx, gp_memcpy(ctx, fx.data(), d_fxT, sizeof(double) * fx.size(),
                                cudaMemcpyDeviceToHost, ctx->stream));
   if (ffvecs)
-    GP_CUDA(ctx, gp_memcpy(ctx, ffvecs, ctx->d_ffvecs, sizeof(double) * (size_t)K * nc,
-                                 cudaMemcpyDeviceToHost, ctx->stream));
+    GP_CUDA(ctx, gp_copy_out(ctx, out_pages, 0, ctx->d_ffvecs, sizeof(double) * (size_t)K * nc));
   GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   /* fxscal_j = 1/sqrt(sum_i fxvecs^2) in row order (smartpca.c:1504-1525) */
   for (int32_t j = 0; j < K; ++j) {

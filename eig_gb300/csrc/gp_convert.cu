@@ -276,6 +276,7 @@ extern "C" int gp_encode_records(gp_ctx *ctx, int32_t format, const int32_t *sam
       return gp_fail(ctx, GP_ERR_ARG, "gp_encode_records: SNP %lld out of range",
                      (long long)snp_index[i]);
   GP_CUDA(ctx, cudaSetDevice(ctx->device));
+  gp_out_pages out_pages(out_on_device ? NULL : out, out_on_device ? 0 : (size_t)(nsnps * rb));
   /* scratch: sample list, then per chunk the SNP list, flips and (host output) records */
   const int64_t chunk_bytes = (int64_t)64 << 20;
   int64_t chunk = out_on_device ? nsnps : chunk_bytes / rb;
@@ -355,8 +356,7 @@ extern "C" int gp_encode_records(gp_ctx *ctx, int32_t format, const int32_t *sam
     }
     if (out_on_device) GP_CUDA(ctx, cudaEventRecord(ctx->ev_g1, ctx->stream));
     if (!out_on_device)
-      GP_CUDA(ctx, gp_memcpy(ctx, out + s0 * rb, d_rec, (size_t)(nc * rb), cudaMemcpyDeviceToHost,
-                             ctx->stream));
+      GP_CUDA(ctx, gp_copy_out(ctx, out_pages, (size_t)(s0 * rb), d_rec, (size_t)(nc * rb)));
   }
   GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (out_on_device) {
