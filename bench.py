@@ -901,12 +901,8 @@ def unpack_roofline(res, peaks):
 
 def gram_traffic(args):
     """DRAM bytes per launch of the split Gram kernel from the committed ncu summary of the
-    full workload (profiles/gram_split_fp16_full_dram.md, one-CTA schedule), or None for other
-    workloads and for the cluster schedule (not captured: profiler replay of the cluster launch
-    is not used)"""
+    full workload (profiles/gram_split_fp16_full_dram.md), or None for other workloads"""
     if args.config != "full" or args.precision != "fp16":
-        return None
-    if os.environ.get("GP_GRAM_CLUSTER", "4") != "1":
         return None
     p = os.path.join(ROOT, "profiles", "gram_split_fp16_full_dram.md")
     try:
@@ -1063,14 +1059,16 @@ def main():
                 "peak_kind": "bf16 burst, %s" % res["peak_kind"],
                 "kernels": "k_split_transpose + k_gram_split (algorithmic N(N+1)M flop; the "
                            "split scheme issues 3 MMAs per algorithmic FMA)",
-                "traffic_note": "DRAM bytes of the one-CTA schedule from "
-                                "profiles/gram_split_fp16_full_dram.md when GP_GRAM_CLUSTER=1; "
-                                "not captured for the cluster schedule"}
+                "traffic_note": "DRAM bytes per launch of k_gram_split from "
+                                "profiles/gram_split_fp16_full_dram.md"}
     else:
         achieved = res["gram_kernel_flops"] / (res["gram_ms"] * 1e-3) / 1e12
-        roof = {"bound": "fp64", "achieved": achieved, "peak": 1.25, "unit": "TFLOP/s",
-                "frac": achieved / 1.25, "traffic": None,
-                "peak_kind": "nominal GB300 FP64 1.25 TFLOP/s (not in the measured peaks)"}
+        peak = peaks.get("bf16_tflops", 1900.0)
+        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak, "traffic": None,
+                "peak_kind": "bf16 burst, %s" % res["peak_kind"],
+                "kernels": "the exact Gram's kernels (algorithmic N(N+1)M flop; ten fp16 MMAs "
+                           "per algorithmic FMA)"}
     line = {"metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": 1,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": res["step_ms"],
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

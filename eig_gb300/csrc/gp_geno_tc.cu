@@ -161,69 +161,65 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
 
   if (warp == 0) {
     /* ---------------- B producer (TMA) ---------------- */
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        const int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit);
-        const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
-        for (int32_t kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
-          if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, XERR_EMPTY)) {
-            ok = false;
-            break;
-          }
-          mbar_arrive_expect_tx(&full[s], (uint32_t)tn * (XK * 2));
-          tma_load_2d(smem + s * XSTAGE_BYTES + 2 * XA_BYTES, &tm_b, &full[s], kb * XK, ct * tn);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const int32_t ks = (w / nrt) % ksplit, ct = w / (nrt * ksplit);
+      const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      for (int32_t kb = kb0; kb < kb1; ++kb, ++it) {
+        const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
+        if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort_flag, err, XERR_EMPTY)) {
+          ok = false;
+          break;
         }
+        mbar_arrive_expect_tx_warp(&full[s], (uint32_t)tn * (XK * 2));
+        tma_load_2d(smem + s * XSTAGE_BYTES + 2 * XA_BYTES, &tm_b, &full[s], kb * XK, ct * tn);
       }
-      if (*abort_flag) {
-        /* copies already issued must land before the CTA exits (bounded) */
-        const uint64_t t0 = globaltimer_ns();
-        const uint32_t last = it < XSTAGES ? it : XSTAGES;
-        for (uint32_t j = it - last; j < it; ++j)
-          while (!mbar_try_wait(&full[j % XSTAGES], (j / XSTAGES) & 1u) &&
-                 globaltimer_ns() - t0 < GP_WAIT_NS) {
-          }
-      }
+    }
+    if (*abort_flag) {
+      /* copies already issued must land before the CTA exits (bounded) */
+      const uint64_t t0 = globaltimer_ns();
+      const uint32_t last = it < XSTAGES ? it : XSTAGES;
+      for (uint32_t j = it - last; j < it; ++j)
+        while (!mbar_try_wait(&full[j % XSTAGES], (j / XSTAGES) & 1u) &&
+               globaltimer_ns() - t0 < GP_WAIT_NS) {
+        }
     }
   } else if (warp == 1) {
     /* ---------------- MMA issuer ---------------- */
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(XT, (uint32_t)tn);
-      uint32_t it = 0, chunk = 0;
-      bool ok = true;
-      for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        const int32_t ks = (w / nrt) % ksplit, rt = w % nrt;
-        const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
-        const bool h1 = rt * XR + XT < nrows;
-        for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += chunk_kb, ++chunk) {
-          const int32_t c1 = min(kb1, c0 + chunk_kb);
-          if (!mbar_wait(acce, (chunk & 1u) ^ 1u, abort_flag, err, XERR_ACCE)) {
+    const uint32_t idesc = idesc_f16_f32(XT, (uint32_t)tn);
+    uint32_t it = 0, chunk = 0;
+    bool ok = true;
+    for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const int32_t ks = (w / nrt) % ksplit, rt = w % nrt;
+      const int32_t kb0 = ks * kb_per, kb1 = min(nkb, kb0 + kb_per);
+      const bool h1 = rt * XR + XT < nrows;
+      for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += chunk_kb, ++chunk) {
+        const int32_t c1 = min(kb1, c0 + chunk_kb);
+        if (!mbar_wait_warp(acce, (chunk & 1u) ^ 1u, abort_flag, err, XERR_ACCE)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        for (int32_t kb = c0; kb < c1; ++kb, ++it) {
+          const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
+          if (!mbar_wait_warp(&full[s], ph, abort_flag, err, XERR_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          for (int32_t kb = c0; kb < c1; ++kb, ++it) {
-            const uint32_t s = it % XSTAGES, ph = (it / XSTAGES) & 1u;
-            if (!mbar_wait(&full[s], ph, abort_flag, err, XERR_FULL)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t base = smem_u32(smem + s * XSTAGE_BYTES);
-            const uint64_t a0 = sdesc_k128(base), a1 = sdesc_k128(base + XA_BYTES),
-                           bd = sdesc_k128(base + 2 * XA_BYTES);
+          const uint32_t base = smem_u32(smem + s * XSTAGE_BYTES);
+          const uint64_t a0 = sdesc_k128(base), a1 = sdesc_k128(base + XA_BYTES),
+                         bd = sdesc_k128(base + 2 * XA_BYTES);
 #pragma unroll
-            for (int k = 0; k < XK / 16; ++k) {
-              const uint32_t acc = (kb > c0 || k > 0) ? 1u : 0u;
-              umma_bf16(tmem, a0 + 2 * k, bd + 2 * k, idesc, acc);
-              if (h1) umma_bf16(tmem + XN, a1 + 2 * k, bd + 2 * k, idesc, acc);
-            }
-            umma_commit(&empty[s]);
+          for (int k = 0; k < XK / 16; ++k) {
+            const uint32_t acc = (kb > c0 || k > 0) ? 1u : 0u;
+            umma_bf16(tmem, a0 + 2 * k, bd + 2 * k, idesc, acc);
+            if (h1) umma_bf16(tmem + XN, a1 + 2 * k, bd + 2 * k, idesc, acc);
           }
-          if (ok) umma_commit(accf);
+          umma_commit(&empty[s]);
         }
+        if (ok) umma_commit(accf);
       }
     }
   } else if (warp < 2 + X_DEC_WARPS) {
@@ -324,7 +320,7 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
   __syncthreads();
   tc_fence_after();
   if (warp == 1) {
-    if (*abort_flag && lane == 0) {
+    if (*abort_flag) {
       umma_commit(drain);
       const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(drain, 0) && globaltimer_ns() - t0 < GP_WAIT_NS) {

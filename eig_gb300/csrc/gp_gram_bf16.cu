@@ -13,9 +13,10 @@
  * accumulation at FP32 speed (GB300's FP64 rate is a small fraction of its FP32 rate); the
  * tile is written out in FP64.
  *
- * Data layout in HBM: Xhi and Xlo as row-major [Npad][Kc] bf16 (samples x kept SNPs of the
- * current super-chunk), written by k_split_transpose from the packed records; the Gram
- * kernel reads them with TMA as 128-row x 64-SNP boxes in the 128-byte swizzle.
+ * Data layout in HBM: Xhi and Xlo as [Kc / 64][Npad][64] (for each k-block of 64 kept SNPs of
+ * the current super-chunk, the samples' 128-byte rows one after the other), written by
+ * k_split_transpose from the packed records; the Gram kernel reads them with TMA as boxes of
+ * 128 such rows, 16 KB in a piece, in the 128-byte swizzle.
  *
  * Kernel structure (persistent, one CTA per SM, 18 warps):
  *   warp 0      TMA producer: per k-block of 64 SNPs four 16 KB boxes (A hi/lo, B hi/lo)
@@ -27,12 +28,20 @@
  *               release it and add it into registers; every GP_FOLD chunks fold those into
  *               the (hi, lo) running sums in TMEM columns 256-511; after the last chunk of a
  *               tile write the tile to the Gram in FP64.
- * Tiles are the 128x128 blocks of the lower triangle, distributed round-robin over CTAs, or
- * over clusters: four CTAs on a 2 x 2 block of tiles (each loads one box of its tile row and
- * one of its tile column and multicasts it to the two CTAs that share it: half the boxes of
- * the one-CTA kernel) or two CTAs on two tiles of a row (the row's boxes multicast: three
- * quarters).  A stage is then released when every CTA of the cluster has read it
- * (tcgen05.commit multicast to each CTA's empty barrier).
+ * Tiles are the 128x128 blocks of the lower triangle, distributed round-robin over the CTAs;
+ * the tiles of a last wave that would leave half of the CTAs or more without work are cut along
+ * the SNPs into as many parts as there are CTAs for (at fold boundaries, so that every FP32 sum
+ * is the same), and k_gram_parts adds the parts.
+ *
+ * What bounds it is the shared memory's 128 bytes a clock: a 128x128x16 MMA reads 8 KB, so the 12
+ * MMAs of a k-block read 96 KB and its boxes' 64 KB come in: 1,250 clocks, against 768 of tensor
+ * work; measured 1,285 (5,000 x 600,000 in split fp16: 35.7 ms with the transpose, 43.4 before the
+ * warp-wide issue, the k-block layout and the parts).  The pieces of the running sums fill the
+ * TMEM, so a CTA's tile cannot be larger.  Tried and not kept: pairs of CTAs (cta_group::2,
+ * 256x128, 120 KB a k-block) wait for one another's barriers, 1,430 clocks (1,000 with the loads
+ * left out); clusters of four CTAs that share their boxes by multicast halve the L2 reads, which
+ * are not the limit: the same 38.2 ms without the parts, and 2 x 2 blocks of tiles fill the last
+ * wave worse (3,001 samples: 2.04 against 1.46 ms).
  */
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -65,8 +74,8 @@
 #define GP_KERR_TIMEOUT_ACCF 3
 #define GP_KERR_TIMEOUT_ACCE 4
 #define GP_KERR_TIMEOUT_SYNC 5
-#define GP_KERR_CLUSTER 6 /* launched without clusters of the kernel's size */
 #define GRAM_SYNC_KB 64 /* k-blocks between the producers' lockstep points */
+#define GRAM_PART_FOLDS 4 /* folds of the smallest part (4,096 SNPs: 40 us) */
 
 __device__ __forceinline__ int32_t tri_root(int32_t t)
 {
@@ -84,33 +93,6 @@ __device__ __forceinline__ int32_t tri_root(int32_t t)
  * instead of being read from HBM once per tile.
  */
 #define GRAM_GROUP 12
-/* element t of the lower triangle of an nt x nt grid walked in gs x gs groups */
-__device__ __forceinline__ void tri_tile_group(int32_t t, int32_t nt, int32_t gs, int32_t *bi,
-                                               int32_t *bj)
-{
-  const int32_t ng = (nt + gs - 1) / gs;
-  for (int32_t gi = 0; gi < ng; ++gi) {
-    const int32_t r0 = gi * gs, nr = min(nt, r0 + gs) - r0;
-    for (int32_t gj = 0; gj <= gi; ++gj) {
-      const int32_t c0 = gj * gs, nc = min(nt, c0 + gs) - c0;
-      const int32_t cnt = gi == gj ? nr * (nr + 1) / 2 : nr * nc;
-      if (t < cnt) {
-        if (gi == gj) {
-          const int32_t i = tri_root(t);
-          *bi = r0 + i;
-          *bj = c0 + t - i * (i + 1) / 2;
-        } else {
-          *bi = r0 + t / nc;
-          *bj = c0 + t % nc;
-        }
-        return;
-      }
-      t -= cnt;
-    }
-  }
-  *bi = *bj = 0; /* not reached for t < nt (nt + 1) / 2 */
-}
-
 __device__ __forceinline__ void tri_tile(int32_t t, int32_t nt, int32_t *bi, int32_t *bj)
 {
   const int32_t ng = (nt + GRAM_GROUP - 1) / GRAM_GROUP;
@@ -136,102 +118,42 @@ __device__ __forceinline__ void tri_tile(int32_t t, int32_t nt, int32_t *bi, int
   *bi = *bj = 0; /* not reached for t < ntiles */
 }
 
-/*
- * Pair p of tiles for a cluster of two CTAs: the tiles of one tile row are taken two at a time
- * (columns 2q, 2q+1 of the row inside its group block), so the pair shares the row block bi
- * (the A operand).  bj1 = -1 when the row has an odd count and p is its last pair.
- */
-__device__ __forceinline__ void tri_pair(int32_t p, int32_t nt, int32_t *bi, int32_t *bj0,
-                                         int32_t *bj1)
-{
-  const int32_t ng = (nt + GRAM_GROUP - 1) / GRAM_GROUP;
-  for (int32_t gi = 0; gi < ng; ++gi) {
-    const int32_t r0 = gi * GRAM_GROUP, nr = min(nt, r0 + GRAM_GROUP) - r0;
-    for (int32_t gj = 0; gj <= gi; ++gj) {
-      const int32_t c0 = gj * GRAM_GROUP, nc = min(nt, c0 + GRAM_GROUP) - c0;
-      for (int32_t lr = 0; lr < nr; ++lr) {
-        const int32_t len = gi == gj ? lr + 1 : nc;
-        const int32_t np = (len + 1) / 2;
-        if (p < np) {
-          *bi = r0 + lr;
-          *bj0 = c0 + 2 * p;
-          *bj1 = 2 * p + 1 < len ? c0 + 2 * p + 1 : -1;
-          return;
-        }
-        p -= np;
-      }
-    }
-  }
-  *bi = *bj0 = 0; /* not reached for p < npairs */
-  *bj1 = -1;
-}
+/* a CTA's work: nfull whole tiles, then the other tiles in nsplit parts each */
+struct gram_plan {
+  int32_t nt;       /* tile rows */
+  int32_t nfull;    /* tiles done whole: the first ones */
+  int32_t nsplit;   /* parts of each further tile */
+  int32_t nitems;   /* nfull + nsplit (ntiles - nfull) */
+  int32_t nkb;      /* k-blocks */
+  int32_t chunk_kb; /* k-blocks per FP32 accumulation chunk */
+};
 
-/*
- * Quad w: a 2 x 2 block of tiles (tile rows 2I, 2I+1, tile columns 2J, 2J+1, J <= I) for a
- * cluster of four CTAs, quads in GRAM_GROUP/2-square groups (lower triangle of groups, row by
- * row inside a group) like the tiles of tri_tile.
- */
-__device__ __forceinline__ void tri_quad(int32_t w, int32_t nq, int32_t *qi, int32_t *qj)
+/* item w: its tile and its k-blocks [*kb0, *kb1), whole folds unless the last */
+__device__ __forceinline__ void gram_item(const gram_plan &p, int32_t w, int32_t *bi, int32_t *bj,
+                                          int32_t *kb0, int32_t *kb1)
 {
-  tri_tile_group(w, nq, GRAM_GROUP / 2, qi, qj);
-}
-
-/*
- * The tile of work item w for this CTA (cluster rank `rank`): CL = 1 a tile; CL = 2 the
- * rank's tile of pair w (the second CTA of an odd pair computes the first tile again); CL = 4
- * tile (2I + rank/2, 2J + rank%2) of quad w.  *write is false for a stand-in tile (a second
- * tile the pair does not have, or a quad position outside the lower triangle or the matrix);
- * *arow / *bcol are the tile row and column whose boxes the CTA loads (in the matrix always).
- */
-template <int CL>
-__device__ __forceinline__ void gram_work(int32_t w, int32_t nt, uint32_t rank, int32_t *bi,
-                                          int32_t *bj, bool *write)
-{
-  if (CL == 1) {
-    tri_tile(w, nt, bi, bj);
-    *write = true;
-  } else if (CL == 2) {
-    int32_t j0, j1;
-    tri_pair(w, nt, bi, &j0, &j1);
-    *bj = (rank == 0 || j1 < 0) ? j0 : j1;
-    *write = rank == 0 || j1 >= 0;
-  } else {
-    int32_t qi, qj;
-    tri_quad(w, (nt + 1) / 2, &qi, &qj);
-    const int32_t ti = 2 * qi + (int32_t)(rank >> 1), tj = 2 * qj + (int32_t)(rank & 1);
-    *write = ti < nt && tj < nt && tj <= ti;
-    *bi = ti < nt ? ti : 2 * qi;
-    *bj = tj < nt ? tj : 2 * qj;
+  const int32_t u = w - p.nfull;
+  tri_tile(u < 0 ? w : p.nfull + u / p.nsplit, p.nt, bi, bj);
+  *kb0 = 0;
+  *kb1 = p.nkb;
+  if (u >= 0) {
+    const int32_t fold_kb = GP_FOLD * p.chunk_kb, nf = (p.nkb + fold_kb - 1) / fold_kb;
+    const int32_t q = u % p.nsplit;
+    *kb0 = (int32_t)((int64_t)nf * q / p.nsplit) * fold_kb;
+    *kb1 = min(p.nkb, (int32_t)((int64_t)nf * (q + 1) / p.nsplit) * fold_kb);
   }
 }
 
 /*
  * grams: XTX (n x n row-major FP64); accumulate != 0 adds to the values already there
- * (super-chunks after the first).  nkb = k-blocks of this super-chunk; chunk_kb = k-blocks
- * per FP32 accumulation chunk.
+ * (super-chunks after the first).  The items after the whole tiles go to parts, [item][128][128].
  */
-template <int FP16, int NMMA, int CL>
+template <int FP16, int NMMA>
 __global__ void __launch_bounds__(GRAM_THREADS, 1)
 k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
-                  int32_t nwork, int32_t nt_rows, int32_t nkb, int32_t chunk_kb, double *xtx,
-                  int32_t n, int32_t accumulate, unsigned *sync_ctr, int *err)
+             gram_plan p, double *xtx, int32_t n, int32_t accumulate, double *parts,
+             unsigned *sync_ctr, int *err)
 {
-  /* CL = 2: clusters of two CTAs computing two tiles of one tile row; the row block's boxes
-   * (A hi and lo) are multicast to both, one box by each CTA.  CL = 4: clusters of four CTAs
-   * computing a 2 x 2 block of tiles; each CTA loads one of the two boxes of its tile row
-   * (multicast to the row's two CTAs) and one of the two boxes of its tile column
-   * (multicast to the column's two CTAs).  A stage is released when every CTA's MMAs of the
-   * cluster have read it. */
-  /* a cluster kernel run without clusters of its size (for instance a launch that lost the
-   * cluster attribute) would multicast to CTAs that do not exist: it refuses to run */
-  if (CL > 1 && cluster_nctarank() != (uint32_t)CL) {
-    if (threadIdx.x == 0) atomicExch(err, GP_KERR_CLUSTER);
-    return;
-  }
-  const uint32_t rank = CL > 1 ? cluster_ctarank() : 0u;
-  const int32_t w0 = CL > 1 ? (int32_t)cluster_id_x() : (int32_t)blockIdx.x;
-  const int32_t wstride = CL > 1 ? (int32_t)cluster_count_x() : (int32_t)gridDim.x;
-  const uint16_t all_mask = (uint16_t)((1u << CL) - 1u);
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t *bars = (uint64_t *)(smem + NSTAGE * STAGE_BYTES);
@@ -247,7 +169,7 @@ k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CL);
+      mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
@@ -264,129 +186,101 @@ k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
-  if (CL > 1) cluster_sync_all(); /* the peers' barriers are initialised before any multicast */
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int32_t nchunk = (nkb + chunk_kb - 1) / chunk_kb;
 
   if (warp == 0) {
     /* ---------------- TMA producer ---------------- */
-    if (lane == 0) {
-      uint32_t it = 0;
-      const int32_t nsync = (nkb + GRAM_SYNC_KB - 1) / GRAM_SYNC_KB;
-      for (int32_t t = w0; t < nwork && !*abort_flag; t += wstride) {
-        int32_t bi, bj;
-        bool wr;
-        gram_work<CL>(t, nt_rows, rank, &bi, &bj, &wr);
-        /* the CTAs of one wave (work items t / wstride) meet every GRAM_SYNC_KB k-blocks, so
-         * that the boxes one of them loads are still in L2 when the others need them */
-        const int32_t wave = t / wstride;
-        const unsigned wave_n = (unsigned)(min(wstride, nwork - wave * wstride) * CL);
-        for (int32_t kb = 0; kb < nkb; ++kb, ++it) {
-          if (kb > 0 && kb % GRAM_SYNC_KB == 0) {
-            unsigned *ctr = sync_ctr + (int64_t)wave * nsync + kb / GRAM_SYNC_KB;
+    uint32_t it = 0;
+    bool ok = true;
+    const int32_t nsync = (p.nkb + GRAM_SYNC_KB - 1) / GRAM_SYNC_KB;
+    for (int32_t w = blockIdx.x; w < p.nitems && ok; w += gridDim.x) {
+      int32_t bi, bj, kb0, kb1;
+      gram_item(p, w, &bi, &bj, &kb0, &kb1);
+      /* the CTAs of one wave of whole tiles meet every GRAM_SYNC_KB k-blocks, so that the boxes
+       * one of them loads are still in L2 when the others need them */
+      const int32_t wave = w / (int32_t)gridDim.x;
+      const unsigned wave_n = (unsigned)min((int32_t)gridDim.x, p.nfull - wave * (int32_t)gridDim.x);
+      for (int32_t kb = kb0; kb < kb1; ++kb, ++it) {
+        if (w < p.nfull && kb > 0 && kb % GRAM_SYNC_KB == 0) {
+          unsigned *ctr = sync_ctr + (int64_t)wave * nsync + kb / GRAM_SYNC_KB;
+          bool met = true;
+          if (lane == 0) {
             atomicAdd(ctr, 1u);
             volatile unsigned *vc = ctr;
             const uint64_t t0 = globaltimer_ns();
-            bool ok = true;
-            while (*vc < wave_n) {
+            while (met && *vc < wave_n) {
               if (*abort_flag) {
-                ok = false;
-                break;
-              }
-              if (globaltimer_ns() - t0 > GP_WAIT_NS) {
+                met = false;
+              } else if (globaltimer_ns() - t0 > GP_WAIT_NS) {
                 atomicExch(err, GP_KERR_TIMEOUT_SYNC);
                 *abort_flag = 1;
-                ok = false;
-                break;
+                met = false;
               }
             }
-            if (!ok) break;
           }
-          uint32_t s = it % NSTAGE, ph = (it / NSTAGE) & 1u;
-          if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, GP_KERR_TIMEOUT_EMPTY)) break;
-          uint8_t *st = smem + s * STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-          if (CL == 4) {
-            /* rank = 2 a + b: row a's box (hi for b = 0, lo for b = 1) to ranks 2a, 2a+1;
-             * column b's box (hi for a = 0, lo for a = 1) to ranks b, b+2 */
-            const uint32_t a = rank >> 1, b = rank & 1u;
-            const uint16_t rmask = (uint16_t)(3u << (2 * a)), cmask = (uint16_t)(5u << b);
-            tma_load_2d_mc(st + b * BOX_BYTES, b ? &tm_lo : &tm_hi, &full[s], kb * BK, bi * BT,
-                           rmask);
-            tma_load_2d_mc(st + (2 + a) * BOX_BYTES, a ? &tm_lo : &tm_hi, &full[s], kb * BK,
-                           bj * BT, cmask);
-          } else {
-            if (CL == 2) {
-              /* A hi from rank 0 and A lo from rank 1, each into both CTAs */
-              if (rank == 0)
-                tma_load_2d_mc(st, &tm_hi, &full[s], kb * BK, bi * BT, (uint16_t)3);
-              else
-                tma_load_2d_mc(st + BOX_BYTES, &tm_lo, &full[s], kb * BK, bi * BT, (uint16_t)3);
-            } else {
-              tma_load_2d(st, &tm_hi, &full[s], kb * BK, bi * BT);
-              tma_load_2d(st + BOX_BYTES, &tm_lo, &full[s], kb * BK, bi * BT);
-            }
-            tma_load_2d(st + 2 * BOX_BYTES, &tm_hi, &full[s], kb * BK, bj * BT);
-            tma_load_2d(st + 3 * BOX_BYTES, &tm_lo, &full[s], kb * BK, bj * BT);
-          }
+          ok = __all_sync(0xffffffffu, met);
+          if (!ok) break;
         }
+        const uint32_t s = it % NSTAGE, ph = (it / NSTAGE) & 1u;
+        ok = mbar_wait_warp(&empty[s], ph ^ 1u, abort_flag, err, GP_KERR_TIMEOUT_EMPTY);
+        if (!ok) break;
+        uint8_t *st = smem + s * STAGE_BYTES;
+        const int32_t ya = (kb * p.nt + bi) * BT, yb = (kb * p.nt + bj) * BT;
+        mbar_arrive_expect_tx_warp(&full[s], STAGE_BYTES);
+        tma_load_2d(st, &tm_hi, &full[s], 0, ya);
+        tma_load_2d(st + BOX_BYTES, &tm_lo, &full[s], 0, ya);
+        tma_load_2d(st + 2 * BOX_BYTES, &tm_hi, &full[s], 0, yb);
+        tma_load_2d(st + 3 * BOX_BYTES, &tm_lo, &full[s], 0, yb);
       }
-      if (*abort_flag) {
-        /* copies already issued must land before the CTA exits (bounded) */
-        uint32_t last = it < NSTAGE ? it : NSTAGE;
-        for (uint32_t j = it - last; j < it; ++j) {
-          uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(&full[j % NSTAGE], (j / NSTAGE) & 1u) &&
-                 globaltimer_ns() - t0 < GP_WAIT_NS) {
-          }
+    }
+    if (*abort_flag) {
+      /* copies already issued must land before the CTA exits (bounded) */
+      const uint32_t last = it < NSTAGE ? it : NSTAGE;
+      for (uint32_t j = it - last; j < it; ++j) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try_wait(&full[j % NSTAGE], (j / NSTAGE) & 1u) &&
+               globaltimer_ns() - t0 < GP_WAIT_NS) {
         }
       }
     }
   } else if (warp == 1) {
     /* ---------------- MMA issuer ---------------- */
-    if (lane == 0) {
-      const uint32_t idesc = FP16 ? idesc_f16_f32(BT, BT) : idesc_bf16_f32(BT, BT);
-      uint32_t it = 0, chunk = 0;
-      bool ok = true;
-      for (int32_t t = w0; t < nwork && ok; t += wstride) {
-        for (int32_t c = 0; c < nchunk && ok; ++c, ++chunk) {
-          uint32_t buf = chunk & 1u, use = chunk >> 1;
-          if (!mbar_wait(&acce[buf], (use & 1u) ^ 1u, abort_flag, err, GP_KERR_TIMEOUT_ACCE)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t d = tmem + buf * BT;
-          int32_t kb0 = c * chunk_kb, kb1 = kb0 + chunk_kb < nkb ? kb0 + chunk_kb : nkb;
-          for (int32_t kb = kb0; kb < kb1; ++kb, ++it) {
-            uint32_t s = it % NSTAGE, ph = (it / NSTAGE) & 1u;
-            if (!mbar_wait(&full[s], ph, abort_flag, err, GP_KERR_TIMEOUT_FULL)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            uint32_t base = smem_u32(smem + s * STAGE_BYTES);
-            uint64_t ahi = sdesc_k128(base), alo = sdesc_k128(base + BOX_BYTES);
-            uint64_t bhi = sdesc_k128(base + 2 * BOX_BYTES), blo = sdesc_k128(base + 3 * BOX_BYTES);
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-              /* +32 bytes along K per 16 bf16 = +2 in the 16-byte address field */
-              uint64_t o = (uint64_t)(2 * k);
-              uint32_t acc0 = (kb > kb0 || k > 0) ? 1u : 0u;
-              umma_bf16(d, ahi + o, bhi + o, idesc, acc0);
-              umma_bf16(d, ahi + o, blo + o, idesc, 1u);
-              umma_bf16(d, alo + o, bhi + o, idesc, 1u);
-              if (NMMA == 4) umma_bf16(d, alo + o, blo + o, idesc, 1u);
-            }
-            if (CL > 1)
-              umma_commit_mc(&empty[s], all_mask); /* this CTA has read the stage */
-            else
-              umma_commit(&empty[s]);
-          }
+    const uint32_t idesc = FP16 ? idesc_f16_f32(BT, BT) : idesc_bf16_f32(BT, BT);
+    uint32_t it = 0, chunk = 0;
+    bool ok = true;
+    for (int32_t w = blockIdx.x; w < p.nitems && ok; w += gridDim.x) {
+      int32_t bi, bj, kb0, kb1;
+      gram_item(p, w, &bi, &bj, &kb0, &kb1);
+      for (int32_t c0 = kb0; c0 < kb1 && ok; c0 += p.chunk_kb, ++chunk) {
+        const uint32_t buf = chunk & 1u, use = chunk >> 1;
+        ok = mbar_wait_warp(&acce[buf], (use & 1u) ^ 1u, abort_flag, err, GP_KERR_TIMEOUT_ACCE);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem + buf * BT;
+        const int32_t c1 = min(kb1, c0 + p.chunk_kb);
+        for (int32_t kb = c0; kb < c1; ++kb, ++it) {
+          const uint32_t s = it % NSTAGE, ph = (it / NSTAGE) & 1u;
+          ok = mbar_wait_warp(&full[s], ph, abort_flag, err, GP_KERR_TIMEOUT_FULL);
           if (!ok) break;
-          umma_commit(&accf[buf]);
+          tc_fence_after();
+          const uint32_t base = smem_u32(smem + s * STAGE_BYTES);
+          const uint64_t ahi = sdesc_k128(base), alo = sdesc_k128(base + BOX_BYTES);
+          const uint64_t bhi = sdesc_k128(base + 2 * BOX_BYTES);
+          const uint64_t blo = sdesc_k128(base + 3 * BOX_BYTES);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            /* +32 bytes along K per 16 bf16 = +2 in the 16-byte address field */
+            const uint64_t o = (uint64_t)(2 * k);
+            const uint32_t acc0 = (kb > c0 || k > 0) ? 1u : 0u;
+            umma_bf16(d, ahi + o, bhi + o, idesc, acc0);
+            umma_bf16(d, ahi + o, blo + o, idesc, 1u);
+            umma_bf16(d, alo + o, bhi + o, idesc, 1u);
+            if (NMMA == 4) umma_bf16(d, alo + o, blo + o, idesc, 1u);
+          }
+          umma_commit(&empty[s]);
         }
+        if (ok) umma_commit(&accf[buf]);
       }
     }
   } else {
@@ -405,10 +299,10 @@ k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
     const uint32_t t_acc = tmem + lane_addr;
     uint32_t chunk = 0;
     bool ok = true;
-    for (int32_t t = w0; t < nwork && ok; t += wstride) {
-      int32_t bi, bj;
-      bool wr;
-      gram_work<CL>(t, nt_rows, rank, &bi, &bj, &wr);
+    for (int32_t w = blockIdx.x; w < p.nitems && ok; w += gridDim.x) {
+      int32_t bi, bj, kb0, kb1;
+      gram_item(p, w, &bi, &bj, &kb0, &kb1);
+      const int32_t nchunk = (kb1 - kb0 + p.chunk_kb - 1) / p.chunk_kb;
       const int32_t gi = bi * BT + row;
       const int32_t gj0 = bj * BT + col0;
       float A[EPI_COLS];
@@ -469,21 +363,22 @@ k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
         }
       }
       if (!ok) break;
-      /* the tile -> Gram rows in FP64 (super-chunks after the first add to what is there) */
-      double *orow = xtx + (int64_t)gi * n;
+      /* the tile -> Gram rows in FP64 (super-chunks after the first add to what is there), or
+       * the part -> its place */
+      double *orow = w < p.nfull ? xtx + (int64_t)gi * n + gj0
+                                 : parts + ((int64_t)(w - p.nfull) * BT + row) * BT + col0;
+      const int32_t ncol = w >= p.nfull ? EPI_COLS : gi < n ? n - gj0 : 0;
+      const bool add = accumulate && w < p.nfull;
 #pragma unroll
       for (int g = 0; g < EPI_COLS / 16; ++g) {
         uint32_t hs[16], ls[16];
         tmem_ld16(t_acc + 256 + col0 + 16 * g, hs);
         tmem_ld16(t_acc + 384 + col0 + 16 * g, ls);
         tmem_wait_ld();
-        if (wr && gi < n) {
-          for (int v = 0; v < 16; ++v) {
-            int32_t gj = gj0 + 16 * g + v;
-            if (gj < n) {
-              double x = (double)__uint_as_float(hs[v]) + (double)__uint_as_float(ls[v]);
-              orow[gj] = accumulate ? orow[gj] + x : x;
-            }
+        for (int v = 0; v < 16; ++v) {
+          if (16 * g + v < ncol) {
+            double x = (double)__uint_as_float(hs[v]) + (double)__uint_as_float(ls[v]);
+            orow[16 * g + v] = add ? orow[16 * g + v] + x : x;
           }
         }
       }
@@ -492,19 +387,34 @@ k_gram_split(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 1 && lane == 0 && (CL > 1 || *abort_flag)) {
-    /* let MMAs already issued finish (and, in a pair, their arrivals on the peer's
-     * barriers land) before the columns are released and the CTA leaves */
-    umma_commit(drain);
-    uint64_t t0 = globaltimer_ns();
-    while (!mbar_try_wait(drain, 0) && globaltimer_ns() - t0 < GP_WAIT_NS) {
-    }
-  }
-  __syncthreads();
-  if (CL > 1) cluster_sync_all(); /* no multicast or remote arrive targets a CTA that has left */
   if (warp == 1) {
+    if (*abort_flag) {
+      /* let MMAs already issued finish before the columns are released and the CTA leaves */
+      umma_commit(drain);
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(drain, 0) && globaltimer_ns() - t0 < GP_WAIT_NS) {
+      }
+    }
     __syncwarp();
     tmem_dealloc(tmem, 512);
+  }
+}
+
+/* the parts of the tiles after the whole ones, in order, into the Gram: a thread per entry */
+__global__ void __launch_bounds__(256)
+k_gram_parts(gram_plan p, const double *__restrict__ parts, double *xtx, int32_t n,
+             int32_t accumulate)
+{
+  int32_t bi, bj;
+  tri_tile(p.nfull + blockIdx.x, p.nt, &bi, &bj);
+  const double *src = parts + (int64_t)blockIdx.x * p.nsplit * (BT * BT);
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < BT * BT; e += gridDim.y * blockDim.x) {
+    const int32_t gi = bi * BT + e / BT, gj = bj * BT + e % BT;
+    if (gi >= n || gj >= n) continue;
+    double *dst = xtx + (int64_t)gi * n + gj;
+    double x = accumulate ? *dst : 0.0;
+    for (int32_t q = 0; q < p.nsplit; ++q) x += src[(int64_t)q * (BT * BT) + e];
+    *dst = x;
   }
 }
 
@@ -539,8 +449,8 @@ __global__ void k_split_tables(const int32_t *kept, int32_t nkept, const double 
 }
 
 /*
- * Xhi/Xlo [npad][kc] for kept columns [k0, k0 + kc), rows >= nrows and columns >= nkept zero,
- * tile by tile through shared memory (a transpose of the SNP-major records):
+ * Xhi/Xlo [kc / 64][npad][64] for kept columns [k0, k0 + kc), rows >= nrows and columns >= nkept
+ * zero, tile by tile through shared memory (a transpose of the SNP-major records):
  * CTA (kt, rt) covers 64 kept SNPs x 256 output rows.  When the tile's samples span at most
  * 256 record bytes (always when the rows are all samples or a subset with few gaps) the 64
  * records' byte ranges are read once, coalesced, into shared memory; each thread then writes
@@ -554,8 +464,8 @@ __global__ void k_split_tables(const int32_t *kept, int32_t nkept, const double 
 __global__ void __launch_bounds__(256)
 k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t *__restrict__ rows,
                   int32_t nrows, const int32_t *__restrict__ cols, const int32_t *__restrict__ kept,
-                  int32_t nkept, const uint32_t *__restrict__ split, int32_t k0, int32_t kc,
-                  int32_t npad, __nv_bfloat16 *xhi, __nv_bfloat16 *xlo)
+                  int32_t nkept, const uint32_t *__restrict__ split, int32_t k0, int32_t npad,
+                  __nv_bfloat16 *xhi, __nv_bfloat16 *xlo)
 {
   __shared__ uint32_t srec[MT_SNP][MT_PITCH_W];
   __shared__ uint32_t stab[MT_SNP][4];
@@ -615,7 +525,7 @@ k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
         lv[u >> 1] |= (pair >> 16) << ((u & 1) * 16);
       }
     }
-    const int64_t off = (int64_t)r * kc + (int64_t)kt * MT_SNP + g8 * 8;
+    const int64_t off = ((int64_t)kt * npad + r) * MT_SNP + g8 * 8;
     *(uint4 *)(xhi + off) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
     *(uint4 *)(xlo + off) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
   }
@@ -639,28 +549,12 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode(gp_ctx *ctx)
   return fn;
 }
 
-/* number of tile pairs of tri_pair for nt tile rows */
-static int32_t gram_npairs(int32_t nt)
-{
-  const int32_t ng = (nt + GRAM_GROUP - 1) / GRAM_GROUP;
-  int32_t total = 0;
-  for (int32_t gi = 0; gi < ng; ++gi) {
-    const int32_t r0 = gi * GRAM_GROUP, nr = (nt < r0 + GRAM_GROUP ? nt : r0 + GRAM_GROUP) - r0;
-    for (int32_t gj = 0; gj <= gi; ++gj) {
-      const int32_t c0 = gj * GRAM_GROUP, nc = (nt < c0 + GRAM_GROUP ? nt : c0 + GRAM_GROUP) - c0;
-      for (int32_t lr = 0; lr < nr; ++lr) total += ((gi == gj ? lr + 1 : nc) + 1) / 2;
-    }
-  }
-  return total;
-}
-
-static int make_map(gp_ctx *ctx, CUtensorMap *m, void *base, int32_t rows, int32_t cols,
-                    CUtensorMapDataType dt)
+static int make_map(gp_ctx *ctx, CUtensorMap *m, void *base, int64_t rows, CUtensorMapDataType dt)
 {
   PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode(ctx);
   if (!enc) return GP_ERR_CUDA;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+  cuuint64_t dims[2] = {BK, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {BK * 2};
   cuuint32_t box[2] = {BK, BT};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(m, dt, 2, base, dims, strides, box, estr,
@@ -673,6 +567,28 @@ static int make_map(gp_ctx *ctx, CUtensorMap *m, void *base, int32_t rows, int32
 /* FP32 accumulation depth in k-blocks of 64 SNPs before the (hi, lo) add; split budget in bytes */
 #define GP_BF16_CHUNK_KB 2
 #define GP_BF16_BUDGET (24ll << 30)
+
+/*
+ * Whole tiles for the full waves; a last wave that would fill at most half of the nsm CTAs is cut
+ * along the SNPs (5,000 samples x 600,000 SNPs: 60 tiles in two parts, 38.4 -> 35.7 ms; 1,000 x
+ * 60,000: 36 tiles in four, 0.70 -> 0.29), into parts of GRAM_PART_FOLDS folds at least.  nsm = 0:
+ * no parts.
+ */
+static gram_plan gram_make_plan(int32_t nt, int32_t nkb, int32_t chunk_kb, int32_t nsm)
+{
+  const int32_t ntiles = nt * (nt + 1) / 2, rest = nsm ? ntiles % nsm : 0;
+  const int32_t nfold = (nkb + GP_FOLD * chunk_kb - 1) / (GP_FOLD * chunk_kb);
+  gram_plan p = {nt, ntiles, 1, ntiles, nkb, chunk_kb};
+  if (rest > 0) {
+    const int32_t ns = nsm / rest < nfold / GRAM_PART_FOLDS ? nsm / rest : nfold / GRAM_PART_FOLDS;
+    if (ns > 1) {
+      p.nfull = ntiles - rest;
+      p.nsplit = ns;
+      p.nitems = p.nfull + rest * ns;
+    }
+  }
+  return p;
+}
 
 int gp_gram_split(gp_ctx *ctx, int precision)
 {
@@ -701,20 +617,27 @@ int gp_gram_split(gp_ctx *ctx, int precision)
   int32_t kc = (int32_t)(kpad < kc_max ? kpad : kc_max);
   size_t xbytes = (size_t)npad * kc * 2;
   size_t tab_bytes = (size_t)nk * 16 + 256;
-  const int grid0 = ctx->num_sms < ntiles ? ctx->num_sms : ntiles;
-  const size_t nsync = (size_t)((kc / BK + GRAM_SYNC_KB - 1) / GRAM_SYNC_KB);
-  /* lockstep counters for the waves of either kernel (at least one cluster of two) */
-  const size_t waves = (size_t)((ntiles + grid0 - 1) / grid0) > (size_t)gram_npairs(nt)
-                           ? (size_t)((ntiles + grid0 - 1) / grid0)
-                           : (size_t)gram_npairs(nt);
-  const size_t sync_bytes = sizeof(unsigned) * nsync * waves;
-  uint8_t *base;
-  int rc = gp_scratch2(ctx, 2 * xbytes + tab_bytes + sync_bytes + 512, (void **)&base);
+  gram_plan plan;
+  size_t part_bytes = 0, sync_bytes = 0;
+  int grid = 0, rc = GP_OK;
+  uint8_t *base = NULL;
+  for (int split = 1; split >= 0; --split) { /* without parts if there is no memory for them */
+    plan = gram_make_plan(nt, kc / BK, chunk_kb, split ? ctx->num_sms : 0);
+    part_bytes = sizeof(double) * BT * BT * (size_t)(plan.nitems - plan.nfull);
+    grid = ctx->num_sms < plan.nitems ? ctx->num_sms : plan.nitems;
+    sync_bytes = sizeof(unsigned) * (size_t)((kc / BK + GRAM_SYNC_KB - 1) / GRAM_SYNC_KB) *
+                 (size_t)((plan.nitems + grid - 1) / grid);
+    rc = gp_scratch2(ctx, 2 * xbytes + part_bytes + tab_bytes + sync_bytes + 512, (void **)&base);
+    if (rc != GP_ERR_NOMEM || !part_bytes) break;
+  }
   if (rc) return rc;
+  const int32_t nsplit_tiles = ntiles - plan.nfull;
   __nv_bfloat16 *xhi = (__nv_bfloat16 *)base;
   __nv_bfloat16 *xlo = (__nv_bfloat16 *)(base + xbytes);
-  uint32_t *split = (uint32_t *)(base + 2 * xbytes);
-  unsigned *sync_ctr = (unsigned *)(base + ((2 * xbytes + tab_bytes + 255) / 256) * 256);
+  double *parts = (double *)(base + 2 * xbytes);
+  uint32_t *split = (uint32_t *)(base + 2 * xbytes + part_bytes);
+  unsigned *sync_ctr =
+      (unsigned *)(base + ((2 * xbytes + part_bytes + tab_bytes + 255) / 256) * 256);
   int *d_err = ctx->d_err;
   GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
   {
@@ -726,102 +649,37 @@ int gp_gram_split(gp_ctx *ctx, int precision)
       k_split_tables<0><<<blocks, 256, 0, ctx->stream>>>(ctx->d_kept, nk, ctx->d_vtab, split);
     GP_LAUNCH_CHECK(ctx, "k_split_tables");
   }
-  typedef void (*gram_kern_t)(const CUtensorMap, const CUtensorMap, int32_t, int32_t, int32_t,
-                              int32_t, double *, int32_t, int32_t, unsigned *, int *);
-  gram_kern_t kern = fp16 ? k_gram_split<1, 3, 1>
-                          : (nmma == 4 ? k_gram_split<0, 4, 1> : k_gram_split<0, 3, 1>);
-  gram_kern_t kern2 = fp16 ? k_gram_split<1, 3, 2>
-                           : (nmma == 4 ? k_gram_split<0, 4, 2> : k_gram_split<0, 3, 2>);
-  gram_kern_t kern4 = fp16 ? k_gram_split<1, 3, 4>
-                           : (nmma == 4 ? k_gram_split<0, 4, 4> : k_gram_split<0, 3, 4>);
-  /* clusters of four CTAs (2 x 2 tiles sharing row and column boxes), else two (two tiles of
-   * a row sharing its boxes), else one CTA per tile; GP_GRAM_CLUSTER=1|2|4 caps the size.
-   * The next smaller size is used when the cluster launch is refused. */
-  int cl = ctx->gram_cluster_cap > 0 ? ctx->gram_cluster_cap : 4;
-  {
-    const char *ce = getenv("GP_GRAM_CLUSTER");
-    if (ce && atoi(ce) >= 1 && atoi(ce) < cl) cl = atoi(ce) >= 4 ? 4 : (atoi(ce) >= 2 ? 2 : 1);
-  }
-  const int32_t nq = (nt + 1) / 2;
-  const int32_t nwork_cl[5] = {0, ntiles, gram_npairs(nt), 0, nq * (nq + 1) / 2};
-  int32_t ncl = 0;
-  for (; cl > 1; cl /= 2) {
-    gram_kern_t kc = cl == 4 ? kern4 : kern2;
-    GP_CUDA(ctx, cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAM_SMEM));
-    cudaLaunchConfig_t qc = {};
-    qc.gridDim = dim3((unsigned)((ctx->num_sms / cl) * cl));
-    qc.blockDim = dim3(GRAM_THREADS);
-    qc.dynamicSmemBytes = GRAM_SMEM;
-    cudaLaunchAttribute qa[1];
-    qa[0].id = cudaLaunchAttributeClusterDimension;
-    qa[0].val.clusterDim.x = (unsigned)cl;
-    qa[0].val.clusterDim.y = 1;
-    qa[0].val.clusterDim.z = 1;
-    qc.attrs = qa;
-    qc.numAttrs = 1;
-    int maxcl = 0;
-    if (cudaOccupancyMaxActiveClusters(&maxcl, (const void *)kc, &qc) != cudaSuccess) {
-      cudaGetLastError();
-      maxcl = 0;
-    }
-    ncl = maxcl < ctx->num_sms / cl ? maxcl : ctx->num_sms / cl;
-    if (ncl > nwork_cl[cl]) ncl = nwork_cl[cl];
-    if (ncl >= 1) break;
-  }
-  if (cl < 2) ncl = 0;
+  typedef void (*gram_kern_t)(const CUtensorMap, const CUtensorMap, gram_plan, double *, int32_t,
+                              int32_t, double *, unsigned *, int *);
+  gram_kern_t kern = fp16 ? k_gram_split<1, 3> : (nmma == 4 ? k_gram_split<0, 4> : k_gram_split<0, 3>);
   GP_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAM_SMEM));
   CUtensorMap mhi, mlo;
   CUtensorMapDataType dt = fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  rc = make_map(ctx, &mhi, xhi, npad, kc, dt);
-  if (!rc) rc = make_map(ctx, &mlo, xlo, npad, kc, dt);
+  const int64_t xrows = (int64_t)kc / BK * npad;
+  rc = make_map(ctx, &mhi, xhi, xrows, dt);
+  if (!rc) rc = make_map(ctx, &mlo, xlo, xrows, dt);
   if (rc) return rc;
-  int grid = grid0;
   for (int32_t k0 = 0; k0 < kpad; k0 += kc) {
     int32_t kcur = kpad - k0 < kc ? kpad - k0 : kc;
     /* columns beyond kcur in this super-chunk are zero (k >= nkept guard covers the tail) */
     dim3 tgrid((unsigned)(kc / MT_SNP), (unsigned)((npad + MT_ROWS - 1) / MT_ROWS));
     k_split_transpose<<<tgrid, 256, 0, ctx->stream>>>(ctx->d_geno, ctx->rlen_dev, ctx->d_rows, n,
-                                                      ctx->d_cols, ctx->d_kept, nk, split, k0, kc,
+                                                      ctx->d_cols, ctx->d_kept, nk, split, k0,
                                                       npad, xhi, xlo);
     GP_LAUNCH_CHECK(ctx, "k_split_transpose");
     int32_t nkb = kcur / BK;
     GP_CUDA(ctx, cudaMemsetAsync(sync_ctr, 0, sync_bytes, ctx->stream));
     /* cooperative launch: the producers' lockstep points need every CTA resident */
-    int32_t a_nt = ntiles, a_rows = nt, a_nkb = nkb, a_ck = chunk_kb, a_n = n,
-            a_acc = k0 > 0 ? 1 : 0;
+    plan.nkb = nkb;
+    int32_t a_n = n, a_acc = k0 > 0 ? 1 : 0;
     double *a_xtx = ctx->d_xtx;
-    bool launched = false;
-    while (!launched && ncl > 0) {
-      cudaLaunchConfig_t lc = {};
-      lc.gridDim = dim3((unsigned)(cl * ncl));
-      lc.blockDim = dim3(GRAM_THREADS);
-      lc.dynamicSmemBytes = GRAM_SMEM;
-      lc.stream = ctx->stream;
-      cudaLaunchAttribute la[2];
-      la[0].id = cudaLaunchAttributeClusterDimension;
-      la[0].val.clusterDim.x = (unsigned)cl;
-      la[0].val.clusterDim.y = 1;
-      la[0].val.clusterDim.z = 1;
-      la[1].id = cudaLaunchAttributeCooperative;
-      la[1].val.cooperative = 1;
-      lc.attrs = la;
-      lc.numAttrs = 2;
-      cudaError_t le = cudaLaunchKernelEx(&lc, cl == 4 ? kern4 : kern2, mhi, mlo, nwork_cl[cl],
-                                          a_rows, a_nkb, a_ck, a_xtx, a_n, a_acc, sync_ctr, d_err);
-      if (le == cudaSuccess) {
-        launched = true;
-      } else {
-        cudaGetLastError();
-        /* refused: the next smaller cluster (same count of SMs), finally one CTA per tile */
-        cl /= 2;
-        ncl = cl > 1 ? ((ctx->num_sms / cl) < nwork_cl[cl] ? ctx->num_sms / cl : nwork_cl[cl]) : 0;
-      }
-    }
-    if (!launched) {
-      void *args[] = {&mhi, &mlo, &a_nt, &a_rows, &a_nkb, &a_ck, &a_xtx, &a_n, &a_acc, &sync_ctr,
-                      &d_err};
-      GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(GRAM_THREADS),
-                                               args, GRAM_SMEM, ctx->stream));
+    void *args[] = {&mhi, &mlo, &plan, &a_xtx, &a_n, &a_acc, &parts, &sync_ctr, &d_err};
+    GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(GRAM_THREADS),
+                                             args, GRAM_SMEM, ctx->stream));
+    if (nsplit_tiles > 0) {
+      k_gram_parts<<<dim3((unsigned)nsplit_tiles, 8), 256, 0, ctx->stream>>>(plan, parts, ctx->d_xtx,
+                                                                             n, a_acc);
+      GP_LAUNCH_CHECK(ctx, "k_gram_parts");
     }
     ctx->launches++;
     ctx->gram_launches++;
@@ -829,15 +687,6 @@ int gp_gram_split(gp_ctx *ctx, int precision)
   int herr = 0;
   GP_CUDA(ctx, gp_memcpy(ctx, &herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (herr == GP_KERR_CLUSTER) {
-    /* the launch ran without its clusters (every CTA refused before any load or MMA, so
-     * nothing was written): redo the whole Gram on the one-CTA schedule, which needs no
-     * cluster, and keep that schedule for this handle */
-    if (ctx->gram_cluster_cap == 1)
-      return gp_fail(ctx, GP_ERR_CUDA, "split Gram: the cluster launch was not honoured");
-    ctx->gram_cluster_cap = 1;
-    return gp_gram_split(ctx, precision);
-  }
   if (herr) return gp_fail(ctx, GP_ERR_TIMEOUT, "split-BF16 Gram kernel wait timed out (code %d)", herr);
   return GP_OK;
 }

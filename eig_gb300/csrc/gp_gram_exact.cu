@@ -206,7 +206,9 @@ k_exact_slices(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
   asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+      "\n\t}\n" ::"r"(
           smem_u32(dst)),
       "l"((uint64_t)__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
@@ -256,77 +258,73 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
 
   if (warp == 0) {
     /* ---------------- right tiles ---------------- */
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        int32_t bi, jt;
-        ex_tile(w % ntiles, n, &bi, &jt);
-        const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
-        for (int32_t kb = a; kb < b && ok; ++kb) {
-          const uint8_t *src = B + ((int64_t)kb * ntj + jt) * (2 * EX_B_BYTES);
-          for (int st = 0; st < 2; ++st, ++it) {
-            const uint32_t s = it % EX_STAGES, ph = (it / EX_STAGES) & 1u;
-            if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, err, EXERR_EMPTY)) {
-              ok = false;
-              break;
-            }
-            mbar_arrive_expect_tx(&full[s], EX_B_BYTES);
-            bulk_load(smem + s * EX_STAGE_BYTES + 2 * EX_A_BYTES, src + st * EX_B_BYTES,
-                      EX_B_BYTES, &full[s]);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      int32_t bi, jt;
+      ex_tile(w % ntiles, n, &bi, &jt);
+      const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
+      for (int32_t kb = a; kb < b && ok; ++kb) {
+        const uint8_t *src = B + ((int64_t)kb * ntj + jt) * (2 * EX_B_BYTES);
+        for (int st = 0; st < 2; ++st, ++it) {
+          const uint32_t s = it % EX_STAGES, ph = (it / EX_STAGES) & 1u;
+          if (!mbar_wait_warp(&empty[s], ph ^ 1u, abort_flag, err, EXERR_EMPTY)) {
+            ok = false;
+            break;
           }
+          mbar_arrive_expect_tx_warp(&full[s], EX_B_BYTES);
+          bulk_load(smem + s * EX_STAGE_BYTES + 2 * EX_A_BYTES, src + st * EX_B_BYTES,
+                    EX_B_BYTES, &full[s]);
         }
       }
-      if (*abort_flag) {
-        /* copies already issued must land before the CTA exits: a stage's barrier completes
-         * only if the decoders arrived too, so wait for the time a copy can take at most */
-        const uint64_t t0 = globaltimer_ns();
-        const uint32_t last = it < EX_STAGES ? it : EX_STAGES;
-        for (uint32_t j = it - last; j < it; ++j)
-          while (!mbar_try_wait(&full[j % EX_STAGES], (j / EX_STAGES) & 1u) &&
-                 globaltimer_ns() - t0 < GP_WAIT_NS) {
-          }
-      }
+    }
+    if (*abort_flag) {
+      /* copies already issued must land before the CTA exits: a stage's barrier completes
+       * only if the decoders arrived too, so wait for the time a copy can take at most */
+      const uint64_t t0 = globaltimer_ns();
+      const uint32_t last = it < EX_STAGES ? it : EX_STAGES;
+      for (uint32_t j = it - last; j < it; ++j)
+        while (!mbar_try_wait(&full[j % EX_STAGES], (j / EX_STAGES) & 1u) &&
+               globaltimer_ns() - t0 < GP_WAIT_NS) {
+        }
     }
   } else if (warp == 1) {
     /* ---------------- MMA issuer ---------------- */
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16_f32(128, EX_N);
-      uint32_t it = 0, chunk = 0;
-      bool ok = true;
-      for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
-        int32_t bi, jt;
-        bool h0, h1;
-        ex_tile(w % ntiles, n, &bi, &jt);
-        ex_halves(bi, jt, n, &h0, &h1);
-        const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
-        for (int32_t c0 = a; c0 < b && ok; c0 += EX_CHUNK_KB, ++chunk) {
-          const int32_t c1 = min(b, c0 + EX_CHUNK_KB);
-          if (!mbar_wait(acce, (chunk & 1u) ^ 1u, abort_flag, err, EXERR_ACCE)) {
+    const uint32_t idesc = idesc_f16_f32(128, EX_N);
+    uint32_t it = 0, chunk = 0;
+    bool ok = true;
+    for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      int32_t bi, jt;
+      bool h0, h1;
+      ex_tile(w % ntiles, n, &bi, &jt);
+      ex_halves(bi, jt, n, &h0, &h1);
+      const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
+      for (int32_t c0 = a; c0 < b && ok; c0 += EX_CHUNK_KB, ++chunk) {
+        const int32_t c1 = min(b, c0 + EX_CHUNK_KB);
+        if (!mbar_wait_warp(acce, (chunk & 1u) ^ 1u, abort_flag, err, EXERR_ACCE)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        for (int32_t q = 2 * c0; q < 2 * c1; ++q, ++it) {
+          const uint32_t s = it % EX_STAGES, ph = (it / EX_STAGES) & 1u;
+          if (!mbar_wait_warp(&full[s], ph, abort_flag, err, EXERR_FULL)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          for (int32_t q = 2 * c0; q < 2 * c1; ++q, ++it) {
-            const uint32_t s = it % EX_STAGES, ph = (it / EX_STAGES) & 1u;
-            if (!mbar_wait(&full[s], ph, abort_flag, err, EXERR_FULL)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t base = smem_u32(smem + s * EX_STAGE_BYTES);
-            const uint64_t a0 = sdesc_k128(base), a1 = sdesc_k128(base + EX_A_BYTES),
-                           bd = sdesc_k128(base + 2 * EX_A_BYTES);
+          const uint32_t base = smem_u32(smem + s * EX_STAGE_BYTES);
+          const uint64_t a0 = sdesc_k128(base), a1 = sdesc_k128(base + EX_A_BYTES),
+                         bd = sdesc_k128(base + 2 * EX_A_BYTES);
 #pragma unroll
-            for (int k = 0; k < EX_K / 16; ++k) {
-              const uint32_t acc = (q > 2 * c0 || k > 0) ? 1u : 0u;
-              if (h0) umma_bf16(tmem, a0 + 2 * k, bd + 2 * k, idesc, acc);
-              if (h1) umma_bf16(tmem + EX_D1, a1 + 2 * k, bd + 2 * k, idesc, acc);
-            }
-            umma_commit(&empty[s]);
+          for (int k = 0; k < EX_K / 16; ++k) {
+            const uint32_t acc = (q > 2 * c0 || k > 0) ? 1u : 0u;
+            if (h0) umma_bf16(tmem, a0 + 2 * k, bd + 2 * k, idesc, acc);
+            if (h1) umma_bf16(tmem + EX_D1, a1 + 2 * k, bd + 2 * k, idesc, acc);
           }
-          if (ok) umma_commit(accf);
+          umma_commit(&empty[s]);
         }
+        if (ok) umma_commit(accf);
       }
     }
   } else if (warp < 2 + EX_DEC_WARPS) {
@@ -441,7 +439,7 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
   __syncthreads();
   tc_fence_after();
   if (warp == 1) {
-    if (*abort_flag && lane == 0) {
+    if (*abort_flag) {
       umma_commit(drain);
       const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(drain, 0) && globaltimer_ns() - t0 < GP_WAIT_NS) {

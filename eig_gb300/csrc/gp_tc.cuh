@@ -88,59 +88,42 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   }
 }
 
+/* mbar_arrive_expect_tx by one elected lane of a converged warp */
+__device__ __forceinline__ void mbar_arrive_expect_tx_warp(uint64_t *bar, uint32_t bytes)
+{
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}\n" ::"r"(smem_u32(bar)),
+      "r"(bytes)
+      : "memory");
+}
+
+/* mbar_wait by a converged warp, with one answer for all its lanes */
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity,
+                                               volatile int *abort_flag, int *err, int code)
+{
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
+
+/*
+ * What a role's warp issues (copies, their barriers' byte counts, MMAs, commits) is called by the
+ * converged warp and issued by one elected lane.  Inside a single-lane branch every operand is a
+ * per-thread value that has to be moved to a uniform register before each instruction: the split
+ * Gram's 128x128x16 MMAs then came 104 clocks apart whatever their shape and operands, and 94,
+ * the shared memory's pace, in this form (5,000 x 150,000: 11.0 -> 9.7 ms).
+ */
+
 /* ---- TMA ---------------------------------------------------------------------------- */
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar,
                                             int32_t x, int32_t y)
 {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];\n\t}\n" ::"r"(smem_u32(dst)),
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
-}
-
-/* the same box into the same shared-memory offset of every CTA of the cluster in cta_mask,
- * completing bytes on the mbarrier at the same offset in each */
-__device__ __forceinline__ void tma_load_2d_mc(void *dst, const CUtensorMap *map, uint64_t *bar,
-                                               int32_t x, int32_t y, uint16_t cta_mask)
-{
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster"
-      " [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar)), "h"(cta_mask)
-      : "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_ctarank()
-{
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_id_x()
-{
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_nctarank()
-{
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_count_x()
-{
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
-  return r;
-}
-/* every thread of every CTA of the cluster (release / acquire) */
-__device__ __forceinline__ void cluster_sync_all()
-{
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
-               ::: "memory");
 }
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map)
@@ -261,9 +244,10 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
                                           uint32_t idesc, uint32_t accumulate)
 {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
@@ -271,17 +255,9 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
 __device__ __forceinline__ void umma_commit(uint64_t *bar)
 {
   asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(
           smem_u32(bar))
       : "memory");
 }
-/* the commit's arrive on the mbarrier at bar's offset in every CTA of cta_mask */
-__device__ __forceinline__ void umma_commit_mc(uint64_t *bar, uint16_t cta_mask)
-{
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], %1;" ::"r"(smem_u32(bar)), "h"(cta_mask)
-      : "memory");
-}
-
 #endif
