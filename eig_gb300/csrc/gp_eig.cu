@@ -3,8 +3,8 @@
  * and the top nvec eigenvectors (the reference computes every eigenpair with LAPACK dspev,
  * src/eigensrc/eigx.c:97-117, but prints all eigenvalues and uses only the top vectors).
  *
- *   1. Householder tridiagonalisation A = Q T Q^T (k_tridiag_tiled or k_tridiag while the
- *      trailing matrix is large, then k_tridiag_smem: LAPACK dsytd2's reflectors and storage;
+ *   1. Householder tridiagonalisation A = Q T Q^T (k_tridiag_tiled, or k_tridiag above orders of
+ *      about 7,600, while the trailing matrix is large, then k_tridiag_smem: LAPACK dsytd2's reflectors and storage;
  *      cuSOLVER sytrd beyond 8,533 rows);
  *   2. all eigenvalues of T by multisection on Sturm counts (the published bisection method:
  *      the count of negative pivots of the LDL^T factorisation of T - x I equals the number
@@ -563,29 +563,23 @@ struct tr_step {
  * dormtr (lower) reads them; the upper triangle is left in float-float form.
  */
 /*
- * Steps c_begin .. c_end - 1 (at most n-2) of the whole-matrix reduction (k_tridiag's steps; after
- * the tiled steps k_tridiag_tiled's): A holds the trailing matrix (indices >= c_begin) as float-float pairs in
- * whole columns, both triangles.  svp/swp/svc: the block's vectors in shared memory (at least
- * n pairs each).  tau_pf, scale_pf, e_pf, have_p and target carry the previous step's state.
- * dot0 (when not NULL) holds the previous step's y.v parts at [dot0_k0, dot0_k1) instead of
- * part_dot2 (the step before c_begin was a tiled one).  sph (block 0, thread 0 only; else
- * NULL): phase times as in k_tridiag, sph[5] the last time stamp.  False when the grid
- * barrier failed.
+ * Steps 0 .. c_end - 1 (at most n-2) by whole columns.  svp/swp/svc: the block's vectors in shared
+ * memory (n pairs each).  tau_pf, scale_pf, e_pf, have_p and target carry the previous step's
+ * state.  sph (block 0, thread 0 only; else NULL): phase times as in k_tridiag, sph[5] the last
+ * time stamp.  False when the grid barrier failed.
  */
-__device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int c_end, double *d,
-                                              double *e,
+__device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_end, double *d, double *e,
                                               double *tau, double *vbuf, double *wbuf,
                                               double *ybuf, double *part_dot2, unsigned *count,
                                               unsigned &target, int *err, double *svp,
                                               double *swp, double *svc, ff2 &tau_pf,
                                               ff2 &scale_pf, ff2 &e_pf, bool &have_p,
-                                              const double *dot0, int dot0_k0, int dot0_k1,
                                               unsigned long long *sph)
 {
   __shared__ ff2 red[TR_WARPS];
   __shared__ ff2 sdotp[TR_B1_SLOTS];
   __shared__ tr_step st;
-  __shared__ ff2 s_slotf;
+  __shared__ ff2 s_slotf, s_yc;
   const int G = gridDim.x, b = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const ff2 ONE = ff_make(1.f, 0.f), ZERO = ff_make(0.f, 0.f);
@@ -597,7 +591,7 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int
     sph[5] = t_now;                                    \
   }
   const int early = (int)((3LL * n) / 10);
-  for (int c = c_begin; c < c_end; ++c) {
+  for (int c = 0; c < c_end; ++c) {
     /* ---- A (every block, no grid barrier): v and w of step c-1, the pending update of
      * column c and its norm, rebuilt from y, the stored x of step c-1 and column c; each
      * block also writes its share of the reflector storage and of x_c (double buffer) ---- */
@@ -613,14 +607,8 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int
     ff2 pacc = ZERO;
     if (have_p && warp == TR_WARPS - 1) {
       const double *pprev = part_dot2 + (size_t)((c + 1) & 1) * G;
-      int g0 = 0, g1 = G;
-      if (c == c_begin && dot0 != NULL) { /* the previous step was a tiled one */
-        pprev = dot0;
-        g0 = dot0_k0;
-        g1 = dot0_k1;
-      }
 #pragma unroll 4
-      for (int g = g0 + lane; g < g1; g += 32) pacc = ff_add(pacc, ff_load(pprev + g));
+      for (int g = lane; g < G; g += 32) pacc = ff_add(pacc, ff_load(pprev + g));
     }
     /* loads (v_p needs only step c-1's scale; y is kept raw in swp for now) */
 #pragma unroll 4
@@ -629,6 +617,7 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int
       if (have_p) {
         vp = (q == c) ? ONE : ff_mul(ff_load(xprev + q), scale_pf);
         yq = ff_load(yprev + q);
+        if (q == c) s_yc = yq; /* swp(c) changes while other warps still need y(c) */
       }
       ff_store(svp + q, vp);
       ff_store(swp + q, yq);
@@ -644,7 +633,7 @@ __device__ __forceinline__ bool tr_full_steps(double *A, int n, int c_begin, int
       /* every thread forms alpha and w_p(c) of step c-1 from the same values */
       const ff2 dsum = s_slotf;
       alpha_pf = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), dsum), -0.5f);
-      wpc = ff_fma(tau_pf, ff_load(swp + c), alpha_pf); /* w_p(c); v_p(c) = 1 */
+      wpc = ff_fma(tau_pf, s_yc, alpha_pf); /* w_p(c); v_p(c) = 1 */
     }
     {
       const int cnt = n - c, per = (cnt + G - 1) / G;
@@ -1170,7 +1159,7 @@ k_tridiag_smem(double *A, int n, int c0, double *d, double *e, double *tau, cons
 #define TR_SMEM_RPT 4
 #define TR_SMALL_ORDER 768 /* trailing orders up to this with 256 threads */
 
-/* steps 0 .. c_end - 1 by whole columns in L2 */
+/* steps 0 .. c_end - 1 by whole columns in L2: orders whose tiles' shared memory does not fit */
 __global__ void __launch_bounds__(TR_THREADS, 1)
 k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double *vbuf,
           double *wbuf, double *ybuf, double *part_dot2, tr_state *state, unsigned *bar, int *err,
@@ -1189,9 +1178,8 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
     for (int i = 0; i < 5; ++i) s_ph[i] = 0ull;
     s_ph[5] = globaltimer_ns();
   }
-  if (!tr_full_steps(A, n, 0, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
-                     sh + n, sh + 2 * n, tau_pf, scale_pf, e_pf, have_p, NULL, 0, 0,
-                     stamp ? s_ph : NULL))
+  if (!tr_full_steps(A, n, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
+                     sh + n, sh + 2 * n, tau_pf, scale_pf, e_pf, have_p, stamp ? s_ph : NULL))
     return;
   if (stamp)
     for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
@@ -1200,12 +1188,183 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
 
 /* ---------------------------------------------------------------------------------- */
 /*
+ * Pairs of float-float numbers in the packed FP32 instructions (two operations in one issue
+ * slot; each is rounded as its scalar form, so every formula below is the scalar one above it,
+ * twice).
+ */
+typedef unsigned long long f2;
+struct pf2 {
+  f2 h, l;
+};
+__device__ __forceinline__ f2 f2_make(float a, float b)
+{
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(f2 a)
+{
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
+{
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+#define F2_MINUS_ONE 0xBF800000BF800000ull
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) { return f2_fma(b, F2_MINUS_ONE, a); }
+__device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ pf2 pf_make(f2 h, f2 l)
+{
+  pf2 r;
+  r.h = h;
+  r.l = l;
+  return r;
+}
+__device__ __forceinline__ pf2 pf_dup(ff2 a)
+{
+  return pf_make(f2_make(a.h, a.h), f2_make(a.l, a.l));
+}
+__device__ __forceinline__ ff2 pf_even(pf2 a) { return ff_make(f2_get(a.h).x, f2_get(a.l).x); }
+__device__ __forceinline__ ff2 pf_odd(pf2 a) { return ff_make(f2_get(a.h).y, f2_get(a.l).y); }
+__device__ __forceinline__ pf2 pf_join(ff2 e, ff2 o)
+{
+  return pf_make(f2_make(e.h, o.h), f2_make(e.l, o.l));
+}
+/* ff_add */
+__device__ __forceinline__ pf2 pf_add(pf2 a, pf2 b)
+{
+  const f2 s = f2_add(a.h, b.h);
+  const f2 bb = f2_sub(s, a.h);
+  f2 err = f2_add(f2_sub(a.h, f2_sub(s, bb)), f2_sub(b.h, bb));
+  err = f2_add(err, f2_add(a.l, b.l));
+  const f2 h = f2_add(s, err);
+  return pf_make(h, f2_sub(err, f2_sub(h, s)));
+}
+/* ff_mul */
+__device__ __forceinline__ pf2 pf_mul(pf2 a, pf2 b)
+{
+  const f2 p = f2_mul(a.h, b.h);
+  f2 e = f2_fma(a.h, b.h, f2_neg(p));
+  e = f2_fma(a.h, b.l, e);
+  e = f2_fma(a.l, b.h, e);
+  const f2 h = f2_add(p, e);
+  return pf_make(h, f2_sub(e, f2_sub(h, p)));
+}
+/* ff_fma */
+__device__ __forceinline__ pf2 pf_fma(pf2 a, pf2 b, pf2 c)
+{
+  const f2 p = f2_mul(a.h, b.h);
+  f2 pe = f2_fma(a.h, b.h, f2_neg(p));
+  pe = f2_fma(a.h, b.l, pe);
+  pe = f2_fma(a.l, b.h, pe);
+  const f2 s = f2_add(c.h, p);
+  const f2 bb = f2_sub(s, c.h);
+  f2 err = f2_add(f2_sub(c.h, f2_sub(s, bb)), f2_sub(p, bb));
+  err = f2_add(err, f2_add(c.l, pe));
+  const f2 h = f2_add(s, err);
+  return pf_make(h, f2_sub(err, f2_sub(h, s)));
+}
+/* ff_sub2prod, with qn = -q.h and sn = -s.h */
+__device__ __forceinline__ pf2 pf_sub2prod(pf2 a, pf2 p, pf2 q, f2 qn, pf2 r, pf2 s, f2 sn)
+{
+  const f2 m1 = f2_mul(p.h, qn);
+  f2 e = f2_fma(p.h, q.h, m1);
+  e = f2_fma(p.h, q.l, e);
+  e = f2_fma(p.l, q.h, e);
+  const f2 m2 = f2_mul(r.h, sn);
+  e = f2_add(f2_fma(r.h, s.h, m2), e);
+  e = f2_fma(r.h, s.l, e);
+  e = f2_fma(r.l, s.h, e);
+  const f2 t1 = f2_add(a.h, m1);
+  const f2 b1 = f2_sub(t1, a.h);
+  const f2 r1 = f2_add(f2_sub(a.h, f2_sub(t1, b1)), f2_sub(m1, b1));
+  const f2 t2 = f2_add(t1, m2);
+  const f2 b2 = f2_sub(t2, t1);
+  const f2 r2 = f2_add(f2_sub(t1, f2_sub(t2, b2)), f2_sub(m2, b2));
+  const f2 low = f2_add(f2_sub(a.l, e), f2_add(r1, r2));
+  const f2 h = f2_add(t2, low);
+  return pf_make(h, f2_sub(low, f2_sub(h, t2)));
+}
+/* ff_dot2 */
+__device__ __forceinline__ pf2 pf_dot2(pf2 a, pf2 x, pf2 b, pf2 y)
+{
+  const f2 p1 = f2_mul(a.h, x.h);
+  f2 e = f2_fma(a.h, x.h, f2_neg(p1));
+  e = f2_fma(a.h, x.l, e);
+  e = f2_fma(a.l, x.h, e);
+  const f2 p2 = f2_mul(b.h, y.h);
+  e = f2_add(f2_fma(b.h, y.h, f2_neg(p2)), e);
+  e = f2_fma(b.h, y.l, e);
+  e = f2_fma(b.l, y.h, e);
+  const f2 s = f2_add(p1, p2);
+  const f2 bb = f2_sub(s, p1);
+  const f2 er = f2_add(f2_sub(p1, f2_sub(s, bb)), f2_sub(p2, bb));
+  const f2 low = f2_add(e, er);
+  const f2 h = f2_add(s, low);
+  return pf_make(h, f2_sub(low, f2_sub(h, s)));
+}
+/* ff_acc_lazy, with xn = -x.h */
+__device__ __forceinline__ pf2 pf_acc_lazy(pf2 acc, pf2 a, pf2 x, f2 xn)
+{
+  const f2 m = f2_mul(a.h, xn);
+  f2 e = f2_fma(a.h, x.h, m);
+  e = f2_fma(a.h, x.l, e);
+  e = f2_fma(a.l, x.h, e);
+  const f2 s = f2_sub(acc.h, m);
+  const f2 bb = f2_sub(s, acc.h);
+  const f2 er = f2_sub(f2_sub(acc.h, f2_sub(s, bb)), f2_add(m, bb));
+  return pf_make(s, f2_add(acc.l, f2_add(e, er)));
+}
+__device__ __forceinline__ pf2 pf_shfl_xor(pf2 a, int o)
+{
+  return pf_make(__shfl_xor_sync(0xFFFFFFFFu, a.h, o), __shfl_xor_sync(0xFFFFFFFFu, a.l, o));
+}
+/* vectors of pairs: indices 2p and 2p + 1 as 16 bytes h, h', l, l' at double 2p */
+__device__ __forceinline__ pf2 pv_load(const double *v, int p)
+{
+  const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(v + 2 * (size_t)p);
+  return pf_make(x.x, x.y);
+}
+__device__ __forceinline__ void pv_store(double *v, int p, pf2 a)
+{
+  *reinterpret_cast<ulonglong2 *>(v + 2 * (size_t)p) = make_ulonglong2(a.h, a.l);
+}
+__device__ __forceinline__ ff2 pv_get(const double *v, int q)
+{
+  const float *f = reinterpret_cast<const float *>(v + (q & ~1)) + (q & 1);
+  return ff_make(f[0], f[2]);
+}
+__device__ __forceinline__ void pv_put(double *v, int q, ff2 a)
+{
+  float *f = reinterpret_cast<float *>(v + (q & ~1)) + (q & 1);
+  f[0] = a.h;
+  f[2] = a.l;
+}
+
+/*
  * The same reduction (dsytd2, lower) with the trailing matrix held as its lower triangle only,
  * in TT x TT tiles: half the bytes per column step and two thirds of the float-float work of
  * the whole-column step, whose product needs both triangles.  Tile (I, J), I >= J, of the
- * lower triangle is TT*TT float-float pairs at Tm + tt_tile(I, J)*TT*TT, column-major inside
- * the tile (element (i, j) at j*TT + i); diagonal tiles are held in full; rows and columns
- * beyond n are zero padding.
+ * lower triangle is at Tm + tt_tile(I, J)*TT*TT (doubles' storage): 16 bytes per row and pair of
+ * columns, the pairs of columns one after the other (TT rows each), elements (i, 2k), (i, 2k+1)
+ * as h, h', l, l', the operands of the packed FP32 instructions.  Diagonal tiles are held in
+ * full; rows and columns beyond n are zero padding.
  *
  * Work is split into parts: tile row I (TT rows) x column unit u (TT_U columns, u = 0 ..
  * nt*TT/TT_U - 1, in tile column u/(TT/TT_U)).  The blocks form a pr x pc grid: block (a, b)
@@ -1214,12 +1373,12 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
  * block has about the same number of parts).  So the product's index block K (TT indices)
  * has pc row-part contributors (blocks (rg(K), *)) and, for each of its units, pr column-part
  * contributors (blocks (*, cg(u))).  Per step:
- *   A   as in the whole-column step (every block: v and w of step c-1, the pending update of
- *       column c read from the tiles, its norm, the reflector; y.v from the index blocks'
- *       partial dots)
+ *   A   every block: the pending w of step c-1 from its y, the pending update of column c read
+ *       from the tiles, its norm, the reflector; y.v from the index blocks' partial dots.  v of
+ *       step c-1 is still in shared memory
  *   B   each warp takes parts of the block: the pending rank-2 update of step c-1 (written
  *       back), the row dots (two rows per lane) and, off the diagonal, the column dots (a
- *       reduce-scatter over the warp per 4 columns); the block sums its parts per tile row and
+ *       reduce-scatter over the warp per 8 columns); the block sums its parts per tile row and
  *       per column unit in a fixed order and publishes them, one arrival (release) on the
  *       index block's counter per published sum; block K mod G waits (acquire, bounded) for
  *       index block K's pc + (TT/TT_U)*pr arrivals and sums them in a fixed order into y and
@@ -1228,11 +1387,23 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
  * Rows and columns up to c keep their values (the pending-update vectors and v are zero there),
  * so that phase A of a block still reading column c never sees it change.  Every sum has a
  * fixed order.
+ *
+ * What bounds it: in B the FP32 pipe, 53 operations per element and step, and the issue slots.
+ * Packed over two columns the operations take half the slots, and with 16 warps instead of 32 the
+ * registers hold the next columns while these are worked on (parts of an early step of order
+ * 5,000: 69,000 -> 52,000 clocks; 20 and 24 warps spill and are slower).  The chain around them,
+ * some 30,000 clocks a step, is A (14,000: y and the column of every block from L2, then the
+ * vectors, packed too), the sums, the arrivals and their wait (10,000), the terms of y, all read
+ * before any is added (3,000), and the grid barrier (4,000).  Order 5,000: 114 -> 100 ms; 3,600:
+ * 57 -> 52.  Down to the order that fits shared memory these steps beat whole columns (2,500:
+ * 28.4 -> 26.5 ms), which remain for orders whose vectors leave no room for the slots.
  */
 #define TT 64
 #define TT_U 16                /* columns per column unit */
 #define TT_UPT (TT / TT_U)     /* column units per tile column */
 #define TT_MAXG 32             /* row or column groups at most */
+#define TT_THREADS 512
+#define TT_WARPS (TT_THREADS / 32)
 #define TR_ERR_LISTS 12
 #define TR_ERR_WAIT 13
 
@@ -1252,85 +1423,145 @@ __global__ void k_tri_to_tiles(const double *A, int n, int nt, double *Tm)
     while ((int64_t)I * (I + 1) / 2 > t) --I;
     const int J = (int)(t - (int64_t)I * (I + 1) / 2);
     double *tile = Tm + t * (TT * TT);
-    for (int idx = threadIdx.x; idx < TT * TT; idx += blockDim.x) {
-      const int j = idx / TT, i = idx - j * TT;
+    for (int idx = threadIdx.x; idx < TT * TT / 2; idx += blockDim.x) {
+      const int j = idx / TT * 2, i = idx % TT;
       const int r = I * TT + i, q = J * TT + j;
-      const double v = (r < n && q < n) ? A[(int64_t)q * n + r] : 0.0;
-      ff_store(tile + idx, ff_from_double(v));
+      const double v0 = (r < n && q < n) ? A[(int64_t)q * n + r] : 0.0;
+      const double v1 = (r < n && q + 1 < n) ? A[(int64_t)(q + 1) * n + r] : 0.0;
+      pv_store(tile, idx, pf_join(ff_from_double(v0), ff_from_double(v1)));
     }
   }
 }
 
-/* one part (TT_U columns from TT*J + j0) of tile (I, J) by one warp: the pending update of
- * step c-1 (have_p), written back; the row dots with v over these columns into rs[TT] (rows
- * 2 lane, 2 lane + 1); unless the tile is diagonal, the column dots with v over the tile's
- * rows into cs[TT_U] */
-__device__ __forceinline__ void tt_part(double *tile, int I, int J, int j0, bool diag,
-                                        bool have_p, const double *svp, const double *swp,
-                                        const double *svc, double *rs, double *cs, int lane)
+/* a + b left unnormalised (ff_warp_sum's step) */
+__device__ __forceinline__ pf2 pf_add_lazy(pf2 a, pf2 b)
 {
-  const ff2 ZERO = ff_make(0.f, 0.f);
-  const int r = I * TT + 2 * lane;
-  const ff2 vr0 = ff_load(svc + r), vr1 = ff_load(svc + r + 1);
-  const ff2 pr0 = ff_load(svp + r), pr1 = ff_load(svp + r + 1);
-  const ff2 qr0 = ff_load(swp + r), qr1 = ff_load(swp + r + 1);
-  ff2 ra0 = ZERO, ra1 = ZERO;
-  const int col0 = J * TT + j0;
-  double *p0 = tile + (size_t)j0 * TT + 2 * lane;
-#pragma unroll 1
-  for (int cb = 0; cb < TT_U; cb += 4) {
-    float4 a[4];
+  const f2 s = f2_add(a.h, b.h);
+  const f2 bb = f2_sub(s, a.h);
+  const f2 er = f2_add(f2_sub(a.h, f2_sub(s, bb)), f2_sub(b.h, bb));
+  return pf_make(s, f2_add(f2_add(a.l, b.l), er));
+}
+__device__ __forceinline__ ff2 ff_add_lazy(ff2 a, ff2 b)
+{
+  const float s = __fadd_rn(a.h, b.h);
+  const float bb = __fsub_rn(s, a.h);
+  const float er = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
+  return ff_make(s, __fadd_rn(__fadd_rn(a.l, b.l), er));
+}
+/* sum over the lanes of 8 columns' dots (4 pairs), scattered: lanes 4k .. 4k+3 end with column k */
+__device__ __forceinline__ ff2 tt_scatter8(pf2 *cp, int lane)
+{
+  const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] = *reinterpret_cast<const float4 *>(p0 + (size_t)(cb + k) * TT);
-    ff2 cp[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int col = col0 + cb + k;
-      ff2 a0 = ff_make(a[k].x, a[k].y), a1 = ff_make(a[k].z, a[k].w);
-      if (have_p) {
-        const ff2 vpc = ff_load(svp + col), wpc = ff_load(swp + col);
-        a0 = ff_sub2prod(a0, pr0, wpc, qr0, vpc);
-        a1 = ff_sub2prod(a1, pr1, wpc, qr1, vpc);
-        *reinterpret_cast<float4 *>(p0 + (size_t)(cb + k) * TT) = make_float4(a0.h, a0.l, a1.h, a1.l);
-      }
-      const ff2 vc = ff_load(svc + col);
-      ra0 = ff_acc_lazy(ra0, a0, vc);
-      ra1 = ff_acc_lazy(ra1, a1, vc);
-      cp[k] = ff_dot2(a0, vr0, a1, vr1);
-    }
-    if (!diag) {
-      /* reduce-scatter over the warp: lanes 8t..8t+7 end with column cb + t (lane bits 4 and 3
-       * pick the column, bits 2..0 are summed) */
-      const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const ff2 send = b4 ? cp[k] : cp[k + 2];
-        const ff2 keep = b4 ? cp[k + 2] : cp[k];
-        cp[k] = ff_add(keep, ff_shfl_xor(send, 16));
-      }
-      {
-        const ff2 send = b3 ? cp[0] : cp[1];
-        const ff2 keep = b3 ? cp[1] : cp[0];
-        cp[0] = ff_add(keep, ff_shfl_xor(send, 8));
-      }
-      cp[0] = ff_add(cp[0], ff_shfl_xor(cp[0], 4));
-      cp[0] = ff_add(cp[0], ff_shfl_xor(cp[0], 2));
-      cp[0] = ff_add(cp[0], ff_shfl_xor(cp[0], 1));
-      if ((lane & 7) == 0) ff_store(cs + cb + (lane >> 3), cp[0]);
-    }
+  for (int k = 0; k < 2; ++k) {
+    const pf2 send = b4 ? cp[k] : cp[k + 2], keep = b4 ? cp[k + 2] : cp[k];
+    cp[k] = pf_add_lazy(keep, pf_shfl_xor(send, 16));
   }
-  ff_store(rs + 2 * lane, ff_renorm(ra0));
-  ff_store(rs + 2 * lane + 1, ff_renorm(ra1));
+  {
+    const pf2 send = b3 ? cp[0] : cp[1], keep = b3 ? cp[1] : cp[0];
+    cp[0] = pf_add_lazy(keep, pf_shfl_xor(send, 8));
+  }
+  const ff2 e = pf_even(cp[0]), o = pf_odd(cp[0]);
+  const ff2 send = b2 ? e : o, keep = b2 ? o : e;
+  ff2 r = ff_add_lazy(keep, ff_shfl_xor(send, 4));
+  r = ff_add_lazy(r, ff_shfl_xor(r, 2));
+  return ff_renorm(ff_add_lazy(r, ff_shfl_xor(r, 1)));
 }
 
-/* shared-memory bytes of k_tridiag_tiled for round size R (parts per round) and the bounds of
- * a block's tile rows, column units and parts */
-__host__ __device__ inline size_t tt_smem_bytes(int nt, int R, int maxr, int maxc, int maxi)
+/* two pairs of columns of the lane's rows (lane, lane + 32), from the first pair's address */
+__device__ __forceinline__ void tt_load(pf2 a[2][2], const double *p0)
+{
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    a[k][0] = pv_load(p0 + (size_t)k * (2 * TT), 0);
+    a[k][1] = pv_load(p0 + (size_t)k * (2 * TT), 32);
+  }
+}
+
+/* a warp's halves of parts (TT_H columns each), h0 .. h1 - 1 in the order of the block's parts:
+ * the pending update of step c-1, written back; the row dots with v (rows lane and lane + 32),
+ * into one slot rseg[TT] for each tile row that the warp meets, from slot seg on; off the
+ * diagonal the column dots with v over the tile's rows into cslot[h][TT_H].  The next columns are
+ * read while these are worked on. */
+#define TT_H 8
+__device__ __forceinline__ void tt_halves(double *Tm, const int4 *items, int h0, int h1, int seg,
+                                          int dead, const double *svp, const double *swp,
+                                          const double *svc, double *rseg, double *cslot, int lane)
+{
+  if (h0 >= h1) return;
+  const pf2 Z = pf_make(0, 0);
+  Tm += 2 * lane;
+  auto half = [&](int h) { return Tm + (int64_t)items[h >> 1].z * (TT * TT_H) + (h & 1) * (TT * TT_H); };
+  pf2 vr0 = Z, vr1 = Z, pr0 = Z, pr1 = Z, qr0 = Z, qr1 = Z, ra0 = Z, ra1 = Z;
+  int I = -1;
+  double *p0 = half(h0);
+  pf2 a[2][2];
+  tt_load(a, p0);
+  for (int h = h0; h < h1; ++h) {
+    const int4 it = items[h >> 1];
+    if (it.x != I) {
+      if (I >= 0) {
+        ff_store(rseg + seg * TT + lane, ff_add(ff_renorm(pf_even(ra0)), ff_renorm(pf_odd(ra0))));
+        ff_store(rseg + seg * TT + lane + 32,
+                 ff_add(ff_renorm(pf_even(ra1)), ff_renorm(pf_odd(ra1))));
+        ++seg;
+      }
+      I = it.x;
+      const int r = I * TT + lane;
+      vr0 = pf_dup(pv_get(svc, r)), vr1 = pf_dup(pv_get(svc, r + 32));
+      pr0 = pf_dup(pv_get(svp, r)), pr1 = pf_dup(pv_get(svp, r + 32));
+      qr0 = pf_dup(pv_get(swp, r)), qr1 = pf_dup(pv_get(swp, r + 32));
+      ra0 = ra1 = Z;
+    }
+    const int col0 = it.y * TT_U + (h & 1) * TT_H;
+    double *pn = h + 1 < h1 ? half(h + 1) : p0;
+    if (col0 + TT_H <= dead) { /* every column is at or before c */
+      if (lane < TT_H) ff_store(cslot + (size_t)h * TT_H + lane, ff_make(0.f, 0.f));
+      tt_load(a, pn);
+    } else {
+      pf2 cp[4];
+#pragma unroll
+      for (int cb = 0; cb < 4; cb += 2) {
+        pf2 nx[2][2];
+        tt_load(nx, cb ? pn : p0 + 2 * (2 * TT));
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int p = col0 / 2 + cb + k;
+          const pf2 vpc = pv_load(svp, p), wpc = pv_load(swp, p), vc = pv_load(svc, p);
+          const f2 vpn = f2_neg(vpc.h), wpn = f2_neg(wpc.h), vn = f2_neg(vc.h);
+          const pf2 a0 = pf_sub2prod(a[k][0], pr0, wpc, wpn, qr0, vpc, vpn);
+          const pf2 a1 = pf_sub2prod(a[k][1], pr1, wpc, wpn, qr1, vpc, vpn);
+          pv_store(p0 + (size_t)(cb + k) * (2 * TT), 0, a0);
+          pv_store(p0 + (size_t)(cb + k) * (2 * TT), 32, a1);
+          ra0 = pf_acc_lazy(ra0, a0, vc, vn);
+          ra1 = pf_acc_lazy(ra1, a1, vc, vn);
+          cp[cb + k] = pf_dot2(a0, vr0, a1, vr1);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          a[k][0] = nx[k][0];
+          a[k][1] = nx[k][1];
+        }
+      }
+      if (it.w >= 0) {
+        const ff2 t = tt_scatter8(cp, lane);
+        if ((lane & 3) == 0) ff_store(cslot + (size_t)h * TT_H + (lane >> 2), t);
+      }
+    }
+    p0 = pn;
+  }
+  ff_store(rseg + seg * TT + lane, ff_add(ff_renorm(pf_even(ra0)), ff_renorm(pf_odd(ra0))));
+  ff_store(rseg + seg * TT + lane + 32, ff_add(ff_renorm(pf_even(ra1)), ff_renorm(pf_odd(ra1))));
+}
+
+/* shared-memory bytes of k_tridiag_tiled for the bounds of a block's tile rows, column units and
+ * parts */
+__host__ __device__ inline size_t tt_smem_bytes(int nt, int maxr, int maxc, int maxi)
 {
   const size_t npad = (size_t)nt * TT;
-  const size_t dbl = 3 * npad + (size_t)R * (TT + TT_U) + (size_t)maxr * TT + (size_t)maxc * TT_U;
+  const size_t dbl = 3 * npad + (size_t)(maxr + TT_WARPS) * TT + (size_t)maxi * TT_U;
   const size_t bytes = dbl * sizeof(double) + (size_t)maxi * sizeof(int4) +
-                       sizeof(int) * (size_t)(3 * maxr + maxc) + (size_t)nt * (1 + TT_UPT);
+                       sizeof(int) * (size_t)(5 * maxr + maxc) + (size_t)nt * (1 + TT_UPT);
   return (bytes + 15) & ~(size_t)15;
 }
 
@@ -1340,36 +1571,40 @@ __host__ __device__ inline size_t tt_smem_bytes(int nt, int R, int maxr, int max
  * of each tile row and the column group of each column unit for first active tile index J0
  * (row J0 of each table).  prow [nt][pc][TT], pcol [nt*TT_UPT][pr][TT_U]: the published row
  * and column parts; dotp [2][nt]: the index blocks' partial y.v of alternate steps; kcnt [nt]:
- * arrival counters (zero at launch).  maxr/maxc/maxi bound a block's tile rows, column units
- * and parts over all J0; R parts per round.  Steps cs .. c_end - 1 run whole columns
- * (tr_full_steps), part_dot2 [2G] their block partials; k_tridiag_smem does the rest.
+ * arrival counters (zero at launch); yb [2][nt*TT]: y of alternate steps, as a vector of pairs
+ * (zero at launch, as dotp).  maxr/maxc/maxi bound a block's tile rows, column units and parts
+ * over all J0.  After step cs - 1 the trailing matrix (indices >= cs) goes to
+ * A as float-float pairs in whole columns, both triangles, v and y of that step to xlast and
+ * ylast and its scalars to *state (v is scaled already, so its scale is 1): k_tridiag_smem does
+ * the rest.
  */
-__global__ void __launch_bounds__(TR_THREADS, 1)
+__global__ void __launch_bounds__(TT_THREADS, 1)
 k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, int maxc,
-                int maxi, int R, int cs, const unsigned char *rgt, const unsigned char *cgt,
-                double *d, double *e, double *tau, double *vbuf, double *wbuf, double *ybuf,
-                double *prow, double *pcol, double *dotp, unsigned *kcnt, double *part_dot2,
-                unsigned *bar, int *err, unsigned long long *phase_ns, int c_end, tr_state *state)
+                int maxi, int cs, const unsigned char *rgt, const unsigned char *cgt,
+                double *d, double *e, double *tau, double *yb, double *xlast, double *ylast,
+                double *prow, double *pcol, double *dotp, unsigned *kcnt, unsigned *bar, int *err,
+                unsigned long long *phase_ns, tr_state *state)
 {
   extern __shared__ double sh[];
   const int npad = nt * TT, nu = nt * TT_UPT;
-  double *svp = sh, *swp = sh + npad, *svc = sh + 2 * npad; /* float-float pairs */
-  double *rslot = sh + 3 * (size_t)npad;      /* [R][TT] */
-  double *cslot = rslot + (size_t)R * TT;     /* [R][TT_U] */
-  double *racc = cslot + (size_t)R * TT_U;    /* [maxr][TT] */
-  double *cacc = racc + (size_t)maxr * TT;    /* [maxc][TT_U] */
-  int4 *items = reinterpret_cast<int4 *>(cacc + (size_t)maxc * TT_U);
+  double *svp = sh, *swp = sh + npad, *svc = sh + 2 * npad; /* vectors of pairs */
+  double *rseg = sh + 3 * (size_t)npad;                     /* [maxr + TT_WARPS][TT] */
+  double *cslot = rseg + (size_t)(maxr + TT_WARPS) * TT;    /* [maxi][TT_U] */
+  int4 *items = reinterpret_cast<int4 *>(cslot + (size_t)maxi * TT_U);
   int *rowl = reinterpret_cast<int *>(items + maxi); /* tile rows */
   int *rowb = rowl + maxr;                           /* first part of each tile row */
   int *rown = rowb + maxr;                           /* parts of each tile row */
-  int *coll = rown + maxr;                           /* column units */
+  int *segb = rown + maxr;                           /* first row slot of each tile row */
+  int *segn = segb + maxr;                           /* row slots of each tile row */
+  int *coll = segn + maxr;                           /* column units */
   unsigned char *rg = reinterpret_cast<unsigned char *>(coll + maxc);
   unsigned char *cg = rg + nt;
-  __shared__ ff2 red[TR_WARPS];
-  __shared__ ff2 s_dot[TR_WARPS];
+  __shared__ ff2 red[TT_WARPS];
+  __shared__ ff2 s_dot[TT_WARPS];
   __shared__ tr_step st;
-  __shared__ ff2 s_slotf, s_dc;
+  __shared__ ff2 s_slotf, s_dc, s_yc;
   __shared__ int s_nr, s_nc, s_ni, s_ok;
+  __shared__ int s_seg[TT_WARPS]; /* each warp's first row slot */
   const int G = gridDim.x, b = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool active = b < pr * pc;
@@ -1378,8 +1613,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
   unsigned *count = bar;
   unsigned target = 0;
   /* the previous step's reflector scalars (block-uniform, kept in shared memory) */
-  __shared__ ff2 s_tau_p, s_scale_p, s_e_p;
-  bool have_p = false;
+  __shared__ ff2 s_tau_p, s_e_p;
   /* phase_ns (optional, block 0): time in A, B (entry 1; entry 2 for the first 30% of the
    * steps) and the barrier (entry 4), accumulated in shared memory */
   __shared__ unsigned long long s_ph[6];
@@ -1388,7 +1622,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
     for (int i = 0; i < 5; ++i) s_ph[i] = 0ull;
     s_ph[5] = globaltimer_ns();
   }
-  if (threadIdx.x == 0) s_tau_p = s_scale_p = s_e_p = ZERO;
+  if (threadIdx.x == 0) s_tau_p = s_e_p = ZERO;
 #define TT_STAMP(i)                                    \
   if (stamp) {                                         \
     const unsigned long long t_now = globaltimer_ns(); \
@@ -1397,7 +1631,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
   }
   const int early = (int)((3LL * n) / 10);
   const unsigned arrivals = (unsigned)(pc + TT_UPT * pr); /* per index block and step */
-  for (int q = threadIdx.x; q < 3 * npad; q += blockDim.x) sh[q] = 0.0; /* padding stays 0 */
+  for (int q = threadIdx.x; q < 3 * npad; q += TT_THREADS) sh[q] = 0.0; /* padding stays 0 */
   int j0_lists = -1;
   for (int c = 0; c < cs; ++c) {
     const int J0 = (c + 1) / TT;
@@ -1422,12 +1656,28 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
             int k = 0;
             for (; k < nc && coll[k] / TT_UPT <= rowl[kr]; ++k) {
               if (ni < maxi)
-                items[ni++] = make_int4(rowl[kr], coll[k], kr,
+                items[ni++] = make_int4(rowl[kr], coll[k],
+                                        (int)tt_tile(rowl[kr], coll[k] / TT_UPT) * (TT / TT_H) +
+                                            coll[k] % TT_UPT * (TT_U / TT_H),
                                         coll[k] / TT_UPT == rowl[kr] ? -1 : k);
               else
                 bad = 1;
             }
             rown[kr] = k;
+          }
+          /* the warps' shares of the parts' halves in order, and a row slot for every piece of
+           * a tile row in a share */
+          int seg = 0, w = 0;
+          for (int kr = 0; kr < nr; ++kr) {
+            const int ha = 2 * rowb[kr], hb = ha + 2 * rown[kr];
+            segb[kr] = seg;
+            for (int h = ha; h < hb;) {
+              while (2 * ni * (w + 1) / TT_WARPS <= h) ++w;
+              if (2 * ni * w / TT_WARPS >= ha) s_seg[w] = seg; /* the share begins in this row */
+              h = 2 * ni * (w + 1) / TT_WARPS;
+              ++seg;
+            }
+            segn[kr] = seg - segb[kr];
           }
         }
         if (bad) atomicExch(err, TR_ERR_LISTS);
@@ -1438,65 +1688,80 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
       __syncthreads();
       j0_lists = J0;
     }
-    /* ---- A: as in the whole-column step, with column c read from the tiles ---- */
-    const ff2 tau_pf = s_tau_p, scale_pf = s_scale_p, e_pf = s_e_p;
-    double *xcur = (c & 1) ? wbuf : vbuf, *xprev = (c & 1) ? vbuf : wbuf;
-    double *ycur = ybuf + (int64_t)(c & 1) * n, *yprev = ybuf + (int64_t)((c + 1) & 1) * n;
+    /* ---- A ---- (before step 0 every vector and scalar of the "previous step" is zero) */
+    {
+      double *t = svp; /* v of step c-1 */
+      svp = svc;
+      svc = t;
+    }
+    const ff2 tau_pf = s_tau_p, e_pf = s_e_p;
+    double *ycur = yb + (size_t)(c & 1) * npad;
+    const double *yprev = yb + (size_t)((c + 1) & 1) * npad;
+    const int p0 = c / 2, odd = c & 1, np = npad / 2;
     ff2 pacc = ZERO;
-    if (have_p && warp == TR_WARPS - 1) {
+    if (warp == TT_WARPS - 1) {
       /* y.v of step c-1: its index blocks' partial dots (from (c-1+1)/TT on), in order */
       const double *pprev = dotp + (size_t)((c + 1) & 1) * nt;
       for (int k = c / TT + lane; k < nt; k += 32) pacc = ff_add(pacc, ff_load(pprev + k));
     }
     {
-      const int Jc = c / TT, jc = c - Jc * TT;
+      const int Jc = c / TT, kc = (c - Jc * TT) / 2;
 #pragma unroll 4
-      for (int q = c + threadIdx.x; q < n; q += blockDim.x) {
-        ff2 vp = ZERO, yq = ZERO;
-        if (have_p) {
-          vp = (q == c) ? ONE : ff_mul(ff_load(xprev + q), scale_pf);
-          yq = ff_load(yprev + q);
-        }
-        ff_store(svp + q, vp);
-        ff_store(swp + q, yq);
-        const int I = q / TT;
-        ff_store(svc + q, ff_load(Tm + (tt_tile(I, Jc) * TT + jc) * TT + (q - I * TT)));
+      for (int p = p0 + threadIdx.x; p < np; p += TT_THREADS) {
+        const int q = 2 * p, I = q / TT;
+        const float4 *a = reinterpret_cast<const float4 *>(Tm + tt_tile(I, Jc) * (TT * TT)) +
+                          kc * TT + (q - I * TT);
+        const float4 a0 = a[0], a1 = a[1];
+        const pf2 y = pv_load(yprev, p);
+        pv_store(svc, p, pf_make(f2_make(odd ? a0.y : a0.x, odd ? a1.y : a1.x),
+                                 f2_make(odd ? a0.w : a0.z, odd ? a1.w : a1.z)));
+        pv_store(swp, p, y);
+        if (p == p0) s_yc = odd ? pf_odd(y) : pf_even(y);
       }
     }
-    if (have_p && warp == TR_WARPS - 1) {
+    if (warp == TT_WARPS - 1) {
       for (int o = 16; o; o >>= 1) pacc = ff_add(pacc, ff_shfl_xor(pacc, o));
       if (lane == 0) s_slotf = pacc;
     }
     __syncthreads();
-    ff2 wpc = ZERO, alpha_pf = ZERO;
-    if (have_p) {
-      const ff2 dsum = s_slotf;
-      alpha_pf = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), dsum), -0.5f);
-      wpc = ff_fma(tau_pf, ff_load(swp + c), alpha_pf);
-    }
     {
+      const ff2 alpha_pf = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), s_slotf), -0.5f);
+      const ff2 wpc = ff_fma(tau_pf, s_yc, alpha_pf);
+      const pf2 tau2 = pf_dup(tau_pf), alpha2 = pf_dup(alpha_pf), nwpc2 = pf_dup(ff_neg(wpc));
       const int cnt = n - c, per = (cnt + G - 1) / G;
       const int r0 = c + b * per, r1 = min(n, r0 + per);
-      ff2 nrm = ZERO;
-      for (int q = c + threadIdx.x; q < n; q += blockDim.x) {
-        ff2 x = ff_load(svc + q);
-        const bool mine = q >= r0 && q < r1;
-        if (have_p) {
-          const ff2 vp = ff_load(svp + q);
-          const ff2 wp = ff_fma(tau_pf, ff_load(swp + q), ff_mul(alpha_pf, vp));
-          ff_store(swp + q, wp);
-          x = ff_fma(ff_neg(vp), wpc, x);
-          x = ff_add(x, ff_neg(wp));
-          if (mine) A[(int64_t)(c - 1) * n + q] = ff_to_double(q == c ? e_pf : vp);
+      pf2 nrm = pf_make(0, 0);
+#pragma unroll 2
+      for (int p = p0 + threadIdx.x; p < np; p += TT_THREADS) {
+        const pf2 vp = pv_load(svp, p);
+        pf2 wp = pf_fma(tau2, pv_load(swp, p), pf_mul(alpha2, vp));
+        pf2 x = pf_fma(vp, nwpc2, pv_load(svc, p));
+        x = pf_add(x, pf_make(f2_neg(wp.h), f2_neg(wp.l)));
+        if (2 * p < c) { /* index c - 1 takes no part any more */
+          wp = pf_join(ZERO, pf_odd(wp));
+          x = pf_join(ZERO, pf_odd(x));
         }
-        ff_store(svc + q, x);
-        if (mine) ff_store(xcur + q, x);
-        if (q >= c + 2) nrm = ff_fma(x, x, nrm);
+        pv_store(swp, p, wp);
+        pv_store(svc, p, x);
+        if (2 * p + 1 >= r0 && 2 * p < r1 && c > 0) {
+          for (int q = max(2 * p, r0); q < min(2 * p + 2, r1); ++q)
+            A[(int64_t)(c - 1) * n + q] =
+                ff_to_double(q == c ? e_pf : (q & 1) ? pf_odd(vp) : pf_even(vp));
+        }
+        if (2 * p < c + 2) x = pf_join(ZERO, 2 * p + 1 < c + 2 ? ZERO : pf_odd(x));
+        nrm = pf_fma(x, x, nrm);
       }
-      const ff2 xn2 = ff_block_sum2(nrm, red);
+      ff2 t = ff_add(pf_even(nrm), pf_odd(nrm));
+      for (int o = 16; o; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
+      if (lane == 0) red[warp] = t;
+      __syncthreads();
+      if (warp == 0) {
+        t = lane < TT_WARPS ? red[lane] : ZERO;
+        for (int o = 16; o; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
+      }
       if (threadIdx.x == 0) {
-        const ff2 alpha = ff_load(svc + c + 1);
-        s_dc = ff_load(svc + c);
+        const ff2 xn2 = t, alpha = pv_get(svc, c + 1);
+        s_dc = pv_get(svc, c);
         if (xn2.h == 0.f) {
           st.beta = alpha;
           st.tau_c = ZERO;
@@ -1518,81 +1783,59 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
       }
     }
     const ff2 beta = st.beta, tau_c = st.tau_c;
-    const ff2 scale_cf = st.scale_c;
     TT_STAMP(0)
     /* ---- B ---- v of step c; the vectors zero at indices J0*TT .. c (rows and columns up to
      * c keep their values, and take no part in the dots) */
-    for (int q = c + 1 + threadIdx.x; q < n; q += blockDim.x)
-      ff_store(svc + q, (q == c + 1) ? ONE : ff_mul(ff_load(svc + q), scale_cf));
-    for (int q = J0 * TT + threadIdx.x; q <= c; q += blockDim.x) {
-      ff_store(svc + q, ZERO);
-      ff_store(svp + q, ZERO);
-      ff_store(swp + q, ZERO);
+    {
+      const pf2 scale2 = pf_dup(st.scale_c);
+      for (int p = J0 * TT / 2 + threadIdx.x; p < np; p += TT_THREADS) {
+        pf2 v = pf_mul(pv_load(svc, p), scale2);
+        if (2 * p <= c + 1) {
+          const ff2 v0 = 2 * p == c + 1 ? ONE : ZERO;
+          const ff2 v1 = 2 * p + 1 == c + 1 ? ONE : 2 * p + 1 <= c ? ZERO : pf_odd(v);
+          v = pf_join(v0, v1);
+          if (2 * p <= c) {
+            const bool keep = 2 * p + 1 > c;
+            pv_store(svp, p, pf_join(ZERO, keep ? pf_odd(pv_load(svp, p)) : ZERO));
+            pv_store(swp, p, pf_join(ZERO, keep ? pf_odd(pv_load(swp, p)) : ZERO));
+          }
+        }
+        pv_store(svc, p, v);
+      }
     }
     const int nr = s_nr, nc = s_nc, ni = s_ni;
-    for (int idx = threadIdx.x; idx < nr * TT + nc * TT_U; idx += blockDim.x)
-      ff_store(idx < nr * TT ? racc + idx : cacc + (idx - nr * TT), ZERO);
     __syncthreads();
-    for (int rb = 0; rb < ni; rb += R) {
-      const int re = min(ni, rb + R);
-      for (int u = warp; rb + u < re; u += TR_WARPS) {
-        const int4 it = items[rb + u];
-        const int I = it.x, J = it.y / TT_UPT, j0 = (it.y - J * TT_UPT) * TT_U;
-        double *rs = rslot + (size_t)u * TT, *cs_ = cslot + (size_t)u * TT_U;
-        if (J == J0 && J0 * TT + j0 + TT_U <= c + 1) {
-          /* every column of this part is at or before c */
-          ff_store(rs + 2 * lane, ZERO);
-          ff_store(rs + 2 * lane + 1, ZERO);
-          if (lane < TT_U) ff_store(cs_ + lane, ZERO);
-        } else {
-          tt_part(Tm + tt_tile(I, J) * (TT * TT), I, J, j0, I == J, have_p, svp, swp, svc, rs,
-                  cs_, lane);
-        }
-      }
-      __syncthreads();
-      /* the round's parts into the block's sums, in part order: tile row kr owns parts
-       * rowb[kr] .. rowb[kr] + rown[kr] - 1, its k-th column unit at rowb[kr] + k */
-      for (int idx = threadIdx.x; idx < nr * TT; idx += blockDim.x) {
-        const int kr = idx / TT, i = idx - kr * TT;
-        ff2 s = ff_load(racc + idx);
-        const int t0 = max(rb, rowb[kr]), t1 = min(re, rowb[kr] + rown[kr]);
-        for (int t = t0; t < t1; ++t) s = ff_add(s, ff_load(rslot + (size_t)(t - rb) * TT + i));
-        ff_store(racc + idx, s);
-      }
-      for (int idx = threadIdx.x; idx < nc * TT_U; idx += blockDim.x) {
-        const int kc = idx / TT_U, j = idx - kc * TT_U;
-        ff2 s = ff_load(cacc + idx);
-        for (int kr = 0; kr < nr; ++kr) {
-          const int t = rowb[kr] + kc;
-          if (kc < rown[kr] && coll[kc] / TT_UPT != rowl[kr] && t >= rb && t < re)
-            s = ff_add(s, ff_load(cslot + (size_t)(t - rb) * TT_U + j));
-        }
-        ff_store(cacc + idx, s);
-      }
-      __syncthreads();
-    }
-    /* publish the block's sums: row parts of its tile rows, column parts of its units; then
-     * one arrival per published sum on its index block's counter */
+    tt_halves(Tm, items, 2 * ni * warp / TT_WARPS, 2 * ni * (warp + 1) / TT_WARPS, s_seg[warp],
+              c + 1, svp, swp, svc, rseg, cslot, lane);
+    __syncthreads();
+    /* the block's sums, in part order: row parts of its tile rows, column parts of its units
+     * (tile row kr's k-th unit is part rowb[kr] + k); then one arrival per published sum on its
+     * index block's counter */
     if (active) {
-      for (int idx = threadIdx.x; idx < nr * TT; idx += blockDim.x) {
+      for (int idx = threadIdx.x; idx < nr * TT; idx += TT_THREADS) {
         const int kr = idx / TT, i = idx - kr * TT;
-        ff_store(prow + ((size_t)rowl[kr] * pc + gb) * TT + i, ff_load(racc + idx));
+        const double *r = rseg + (size_t)segb[kr] * TT + i;
+        ff2 t = ff_load(r);
+        for (int k = 1; k < segn[kr]; ++k) t = ff_add(t, ff_load(r + (size_t)k * TT));
+        ff_store(prow + ((size_t)rowl[kr] * pc + gb) * TT + i, segn[kr] ? t : ZERO);
       }
-      for (int idx = threadIdx.x; idx < nc * TT_U; idx += blockDim.x) {
-        const int kc = idx / TT_U, j = idx - kc * TT_U;
-        ff_store(pcol + ((size_t)coll[kc] * pr + ga) * TT_U + j, ff_load(cacc + idx));
+      for (int idx = threadIdx.x; idx < nc * TT_U; idx += TT_THREADS) {
+        const int kc = idx / TT_U, j = idx - kc * TT_U, J = coll[kc] / TT_UPT;
+        ff2 t = ZERO;
+        for (int kr = 0; kr < nr; ++kr)
+          if (kc < rown[kr] && J != rowl[kr])
+            t = ff_add(t, ff_load(cslot + (size_t)(rowb[kr] + kc) * TT_U + j));
+        ff_store(pcol + ((size_t)coll[kc] * pr + ga) * TT_U + j, t);
       }
     }
     __syncthreads();
     if (active) {
-      if ((int)threadIdx.x < nr) /* nr, nc <= 512 (host check) */
-        red_release_gpu(kcnt + rowl[threadIdx.x], 1u);
-      else if (threadIdx.x >= 512 && (int)threadIdx.x - 512 < nc)
-        red_release_gpu(kcnt + coll[threadIdx.x - 512] / TT_UPT, 1u);
+      for (int k = threadIdx.x; k < nr + nc; k += TT_THREADS)
+        red_release_gpu(kcnt + (k < nr ? rowl[k] : coll[k - nr] / TT_UPT), 1u);
     }
     /* index blocks K = b, b + G, ...: wait for their arrivals, then y over the TT indices
-     * (pc row parts, then pr column parts of the index's unit, in order: 16 threads per index
-     * with two terms each and a fixed shuffle tree) and the partial y.v */
+     * (pc row parts, then pr column parts of the index's unit, in order: 8 threads per index
+     * with four terms each and a fixed shuffle tree) and the partial y.v */
     {
       const unsigned ktarget = arrivals * (unsigned)(c + 1);
       for (int K = b; K < nt; K += G) {
@@ -1618,27 +1861,37 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
         }
         __syncthreads();
         if (!s_ok) return;
-        const int i = threadIdx.x >> 4, g = threadIdx.x & 15;
+        const int i = threadIdx.x >> 3, g = threadIdx.x & 7;
         const int nterm = pc + pr;
-        ff2 y = ZERO;
-        for (int t = g; t < nterm; t += 16) {
-          const double *src = t < pc ? prow + ((size_t)K * pc + t) * TT + i
+        /* at most 8 terms a thread (pr, pc <= TT_MAXG), read before any is added */
+        ff2 term[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int t = g + 8 * k;
+          term[k] = ZERO;
+          if (t < nterm)
+            term[k] = ff_load(t < pc ? prow + ((size_t)K * pc + t) * TT + i
                                      : pcol + ((size_t)(K * TT_UPT + i / TT_U) * pr + (t - pc)) *
-                                                  TT_U + (i & (TT_U - 1));
-          y = ff_add(y, ff_load(src));
+                                                  TT_U + (i & (TT_U - 1)));
         }
-        for (int o = 8; o; o >>= 1) y = ff_add(y, ff_shfl_xor(y, o));
+        ff2 y = term[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k)
+          if (8 * k < nterm) y = ff_add(y, term[k]);
+        for (int o = 4; o; o >>= 1) y = ff_add(y, ff_shfl_xor(y, o));
         const int q = K * TT + i;
         ff2 dv = ZERO;
         if (g == 0) {
-          if (q < n) ff_store(ycur + q, y);
-          dv = ff_mul(y, ff_load(svc + q));
+          pv_put(ycur, q, y);
+          dv = ff_mul(y, pv_get(svc, q));
         }
-        dv = ff_add(dv, ff_shfl_xor(dv, 16)); /* the warp's two indices, lanes 0 and 16 */
+        /* the warp's four indices, lanes 0, 8, 16 and 24 */
+        dv = ff_add(dv, ff_shfl_xor(dv, 8));
+        dv = ff_add(dv, ff_shfl_xor(dv, 16));
         if (lane == 0) s_dot[warp] = dv;
         __syncthreads();
         if (threadIdx.x < 32) {
-          ff2 t = s_dot[threadIdx.x];
+          ff2 t = lane < TT_WARPS ? s_dot[lane] : ZERO;
           for (int o = 16; o; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
           if (threadIdx.x == 0) ff_store(dotp + (size_t)(c & 1) * nt + K, t);
         }
@@ -1648,41 +1901,37 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
     TT_STAMP(c < early ? 2 : 1)
     if (threadIdx.x == 0) { /* read again only after the grid barrier's block barriers */
       s_tau_p = tau_c;
-      s_scale_p = scale_cf;
       s_e_p = beta;
     }
     target += G;
     if (!tr_grid_sync(count, target, err)) return;
     TT_STAMP(4)
-    have_p = true;
   }
-  /* the switch to whole columns: the trailing block (indices >= cs) of the block's parts
-   * into A as float-float pairs, both triangles (the pending update of step cs-1 is applied
-   * by the first whole-column step) */
+  /* the trailing block (indices >= cs) of the block's parts into A as float-float pairs, both
+   * triangles (the pending update of step cs-1 is applied by the next kernel) */
   const int ni = s_ni;
-  for (int64_t idx = threadIdx.x; idx < (int64_t)ni * (TT * TT_U); idx += blockDim.x) {
+  for (int64_t idx = threadIdx.x; idx < (int64_t)ni * (TT * TT_U); idx += TT_THREADS) {
     const int u = (int)(idx / (TT * TT_U)), rem = (int)(idx - (int64_t)u * (TT * TT_U));
     const int j = rem / TT, i = rem - j * TT;
     const int4 it = items[u];
     const int J = it.y / TT_UPT, jt = (it.y - J * TT_UPT) * TT_U + j;
     const int r = it.x * TT + i, q = J * TT + jt;
     if (r >= cs && q >= cs && r < n && q < n) {
-      const double v = Tm[(tt_tile(it.x, J) * TT + jt) * TT + i];
-      A[(int64_t)q * n + r] = v;
-      if (it.x != J) A[(int64_t)r * n + q] = v;
+      const float *f = reinterpret_cast<const float *>(Tm + tt_tile(it.x, J) * (TT * TT)) +
+                       4 * ((jt / 2) * TT + i) + (jt & 1);
+      const ff2 v = ff_make(f[0], f[2]);
+      ff_store(A + (int64_t)q * n + r, v);
+      if (it.x != J) ff_store(A + (int64_t)r * n + q, v);
     }
   }
-  target += G;
-  if (!tr_grid_sync(count, target, err)) return;
-  ff2 tau_pf = s_tau_p, scale_pf = s_scale_p, e_pf = s_e_p;
-  if (!tr_full_steps(A, n, cs, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, count, target, err,
-                     svp, swp, svc, tau_pf, scale_pf, e_pf, have_p,
-                     dotp + (size_t)((cs + 1) & 1) * nt, cs / TT, nt, stamp ? s_ph : NULL))
-    return;
+  for (int q = cs + b * TT_THREADS + threadIdx.x; q < n; q += G * TT_THREADS) {
+    ff_store(xlast + q, pv_get(svc, q));
+    ff_store(ylast + q, pv_get(yb + (size_t)((cs + 1) & 1) * npad, q));
+  }
   if (stamp)
     for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
 #undef TT_STAMP
-  if (b == 0 && threadIdx.x == 0) *state = {tau_pf, scale_pf, e_pf};
+  if (b == 0 && threadIdx.x == 0) *state = {s_tau_p, ONE, s_e_p};
 }
 
 /* deterministic start vector entry in (-1, 1) */
@@ -2357,18 +2606,17 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
   const int nt = (n + TT - 1) / TT;
   int tt_pr = 0, tt_pc = 0, tt_maxr = 0, tt_maxc = 0, tt_maxi = 0;
   size_t tt_smem = 0;
-  /* the tiled steps run while the trailing order exceeds tt_switch (GP_TRIDIAG_SWITCH), where
-   * the whole-column steps, with more rows per block than tile rows, take over */
+  /* the tiled steps run until the rest fits the shared memories (GP_TRIDIAG_SWITCH: until the
+   * trailing order is at most its value) */
   const char *sw_env = getenv("GP_TRIDIAG_SWITCH");
-  const int tt_switch = sw_env && sw_env[0] ? atoi(sw_env) : 2500;
-  const int tt_cs = n - 1 - std::max(1, tt_switch); /* first whole-column step */
+  const int tt_switch = sw_env && sw_env[0] ? std::max(1, atoi(sw_env)) : n;
+  const int tt_cs = std::max(n - m_smem, n - 1 - tt_switch); /* first step after the tiled ones */
   int tiled = !(senv && senv[0] == '1') && !(tt_env && tt_env[0] == '0') && tt_cs >= 1 &&
               tr_smem <= 200 * 1024;
   if (tiled) {
     tt_grid((int)G, &tt_pr, &tt_pc);
     tiled = tt_pr >= 1 && tt_pc >= 1;
   }
-  int tt_R = 0;
   if (tiled && !(ctx->d_tt && ctx->tt_n == n && ctx->tt_G == (int)G)) {
     /* the assignment tables, once per order and grid */
     std::vector<unsigned char> rgt, cgt;
@@ -2388,23 +2636,15 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     tt_maxr = ctx->tt_maxr;
     tt_maxc = ctx->tt_maxc;
     tt_maxi = ctx->tt_maxi;
-    /* parts per round: all of a block's parts in one round where shared memory allows
-     * (GP_TT_ROUND caps it, to run the several-round path at smaller orders) */
-    tt_R = std::min(128, (tt_maxi + TR_WARPS - 1) / TR_WARPS * TR_WARPS);
-    const char *r_env = getenv("GP_TT_ROUND");
-    if (r_env && atoi(r_env) >= TR_WARPS)
-      tt_R = std::min(tt_R, atoi(r_env) / TR_WARPS * TR_WARPS);
-    while (tt_R > TR_WARPS && tt_smem_bytes(nt, tt_R, tt_maxr, tt_maxc, tt_maxi) > 220 * 1024)
-      tt_R -= TR_WARPS;
-    tt_smem = tt_smem_bytes(nt, tt_R, tt_maxr, tt_maxc, tt_maxi);
-    tiled = tt_maxr <= 512 && tt_maxc <= 512 && tt_smem <= 220 * 1024;
+    tt_smem = tt_smem_bytes(nt, tt_maxr, tt_maxc, tt_maxi);
+    tiled = tt_smem <= 226 * 1024; /* 227 KB less the static part */
   }
   if (tiled) {
     int dev_coop = 0, per_sm = 0;
     cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, ctx->device);
     tiled = dev_coop && gp_allow_smem(ctx, (const void *)k_tridiag_tiled) == cudaSuccess;
     if (tiled) {
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tridiag_tiled, TR_THREADS,
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tridiag_tiled, TT_THREADS,
                                                     tt_smem);
       tiled = per_sm >= 1;
     }
@@ -2420,8 +2660,10 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     double *A = A_in, *pd2 = parts;
     int nn = n;
     /* the first steps run in tiles or in L2, those of the last m_smem rows in shared memory */
-    int c_end = std::max(tiled ? tt_cs : 0, n - m_smem);
+    int c_end = tiled ? tt_cs : std::max(0, n - m_smem);
     tr_state *state = (tr_state *)((char *)bar + 80);
+    /* x (of k_tridiag, or v of the tiled steps) and y of step c_end - 1 */
+    double *xlast = (c_end & 1) ? vbuf : wbuf, *ylast = ybuf + (int64_t)((c_end + 1) & 1) * n;
     unsigned long long *phase = NULL;
     GP_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
     GP_CUDA(ctx, cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), ctx->stream));
@@ -2434,26 +2676,28 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       const int64_t ntiles = (int64_t)nt * (nt + 1) / 2;
       const size_t tile_d = (size_t)ntiles * TT * TT;
       const size_t part_d = (size_t)(tt_pr + tt_pc) * nt * TT; /* prow + pcol */
-      const size_t tri_bytes = sizeof(double) * (tile_d + part_d + 2 * (size_t)nt) +
+      const size_t yb_d = 2 * (size_t)nt * TT, zero_d = yb_d + 2 * (size_t)nt;
+      const size_t tri_bytes = sizeof(double) * (tile_d + part_d + zero_d) +
                                sizeof(unsigned) * (size_t)nt;
       int rc2 = gp_realloc(ctx, (void **)&ctx->d_tri, tri_bytes);
       if (rc2) return rc2;
       double *Tm = ctx->d_tri, *prow = Tm + tile_d, *pcol = prow + (size_t)nt * tt_pc * TT;
-      double *dotp = pcol + (size_t)nt * tt_pr * TT;
+      double *yb = pcol + (size_t)nt * tt_pr * TT, *dotp = yb + yb_d;
       unsigned *kcnt = (unsigned *)(dotp + 2 * (size_t)nt);
-      GP_CUDA(ctx, cudaMemsetAsync(kcnt, 0, sizeof(unsigned) * (size_t)nt, ctx->stream));
+      GP_CUDA(ctx, cudaMemsetAsync(yb, 0, sizeof(double) * zero_d + sizeof(unsigned) * (size_t)nt,
+                                   ctx->stream));
       int blocks = (int)std::min<int64_t>(ntiles, (int64_t)ctx->num_sms * 8);
       k_tri_to_tiles<<<blocks, 256, 0, ctx->stream>>>(A_in, n, nt, Tm);
       GP_LAUNCH_CHECK(ctx, "k_tri_to_tiles");
       int nt_ = nt, cs = tt_cs;
       const unsigned char *rgt = ctx->d_tt, *cgt = ctx->d_tt + (size_t)nt * nt;
-      void *args[] = {&A,    &Tm,   &nn,   &nt_,  &tt_pr, &tt_pc, &tt_maxr, &tt_maxc,
-                      &tt_maxi, &tt_R, &cs, &rgt, &cgt,  &d,     &e,       &tau,
-                      &vbuf, &wbuf, &ybuf, &prow, &pcol, &dotp,  &kcnt,    &pd2,
-                      &bar,  &d_err, &phase, &c_end, &state};
+      void *args[] = {&A,       &Tm,   &nn,    &nt_,   &tt_pr, &tt_pc, &tt_maxr, &tt_maxc,
+                      &tt_maxi, &cs,   &rgt,   &cgt,   &d,     &e,     &tau,
+                      &yb,      &xlast, &ylast, &prow, &pcol,  &dotp,  &kcnt,    &bar,
+                      &d_err,   &phase, &state};
       GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
       GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag_tiled, dim3((unsigned)G),
-                                               dim3(TR_THREADS), args, tt_smem, ctx->stream));
+                                               dim3(TT_THREADS), args, tt_smem, ctx->stream));
       ctx->launches++;
     } else {
       int64_t tot = (int64_t)n * n;
@@ -2475,8 +2719,7 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       const void *f = small ? (const void *)k_tridiag_smem<256, TR_SMALL_ORDER / 256>
                             : (const void *)k_tridiag_smem<TR_SMEM_NT, TR_SMEM_RPT>;
       const int Gm = tr_smem_blocks(m, (int)G);
-      const double *xp = (c_end & 1) ? vbuf : wbuf;
-      const double *yp = ybuf + (int64_t)((c_end + 1) & 1) * n;
+      const double *xp = xlast, *yp = ylast;
       uint4 *ctag = ytag + 2 * nd;
       unsigned *bar_s = bar + 1;
       void *args[] = {&A,  &nn,   &c_end, &d,     &e,     &tau,  &xp,
