@@ -33,15 +33,18 @@
  *   warp 1      one thread issues 2 x 4 tcgen05.mma (128 x N x 16, f16 -> f32) per k-block:
  *               the tile's two 128-row halves share the B tile;
  *   warps 2-9   decode the A tile, a thread per row: 16 bytes of codes (the next four
- *               k-blocks' loads in flight) become 64 fp16 values in the same swizzled layout,
- *               four codes at a time through byte permutes (every table value has a zero low
- *               byte, so one register holds the table); then fence.proxy.async and one arrival
- *               per warp;
+ *               k-blocks' loads in flight) become 64 fp16 values in the same swizzled layout;
+ *               then fence.proxy.async and one arrival per warp;
  *   warps 10-17 epilogue: per chunk tcgen05.ld the exact FP32 sums and add them to the tile's
  *               64-bit integer sums in global memory (atomics, 32 rows side by side).
- * The decode of the codes paces it: 128 x 128 tiles decoded each code again for every 128
- * columns and left the tensor pipe a quarter busy (the normal equations of 5,000 samples x
- * 200,000 SNPs, K = 20: 2.98 ms; with 256 x 256 tiles 1.41, 1.3 PFLOP/s).
+ * The decode is a mask per two values.  Missing codes are cleared in a word of 16 (or the word
+ * made observed bits), and its bit pairs f and f + 8 are, as the low bits of two fp16 numbers, the
+ * subnormals c 4^j 2^-24, j = f mod 5 or so (x_field): the factor 4^j is taken out of the other
+ * operand, whose slices are multiplied by 4^-j (exact) and lie in the fields' order.  Every product
+ * is an integer times 2^-24.  Byte permutes through a
+ * table, as before, took 200 instructions a row and k-block where this takes 75: with 256 x 256
+ * tiles the normal equations of 5,000 samples x 200,000 SNPs, K = 20, 1.41 -> 1.15 ms (128 x 128
+ * tiles, decoded again for every 128 columns: 2.98), the weights' two products 0.33 -> 0.26 each.
  */
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -71,10 +74,14 @@
 #define XERR_ACCF 13
 #define XERR_ACCE 14
 
-/* the 4-entry decode tables: the high byte of the fp16 value of codes 0, 1, 2, 3 (byte 0
- * first); the low bytes are zero */
-static const uint32_t LUT_MASK = 0x003C3C3Cu;  /* {1,1,1,0} */
-static const uint32_t LUT_COUNT = 0x00403C00u; /* {0,1,2,0} */
+/* where the code at position kk of a k-block goes among its 64 values, and its power j of four: the
+ * code is the bit pair f of its 32-bit word (the first code of a byte in the byte's high bits) */
+__device__ __forceinline__ void x_field(int kk, int *pos, int *j)
+{
+  const int f = (kk & 12) + 3 - (kk & 3);
+  *pos = (kk & ~15) + 2 * (f & 7) + (f >> 3);
+  *j = (f & 7) < 5 ? f & 7 : (f & 7) - 5;
+}
 /* k-blocks per exact FP32 chunk: 8,192 k with 10-bit slices, 4,096 with 12-bit ones */
 #define X_CHUNK_KB(digits) ((digits) == 5 ? 64 : 128)
 /* columns of a panel cut and multiplied at a time with 5 slices */
@@ -109,15 +116,15 @@ __host__ __device__ __forceinline__ int32_t x_split(int32_t tiles, int32_t nkb, 
 /*
  * codes: rows of ldc bytes (2-bit codes, MSB first, 3 = missing -> 0); output row r reads
  * code row row_map[r] (r itself when row_map is NULL); its k-block kb is the 16 bytes at
- * (kb % kb_period)*16, decoded with lut_lo for kb < kb_period and lut_hi otherwise (the
- * concatenated-k form [G | O]).  tn: slice columns per tile; nct column tiles.
+ * (kb % kb_period)*16, taken as allele counts or as the observed mask by count_lo for kb <
+ * kb_period and count_hi otherwise (the concatenated-k form [G | O]).  tn: slice columns per tile; nct column tiles.
  * sums: per row tile, slice column (nct * tn of them) and row of the tile the exact integer
  * sum, added atomically.
  */
 __global__ void __launch_bounds__(X_THREADS, 1)
 k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restrict__ codes,
                 int64_t ldc, const int32_t *__restrict__ row_map, int32_t nrows, int32_t tn,
-                int32_t nct, int32_t nkb, int32_t kb_period, uint32_t lut_lo, uint32_t lut_hi,
+                int32_t nct, int32_t nkb, int32_t kb_period, int count_lo, int count_hi,
                 int32_t ksplit, int32_t chunk_kb, unsigned long long *sums, int *err,
                 const gp_tc_batch *db)
 {
@@ -260,18 +267,18 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
             break;
           }
           if (half_on) {
-            const uint32_t tab = kb < kb_period ? lut_lo : lut_hi;
+            const bool count = kb < kb_period ? count_lo : count_hi;
             uint8_t *dst = rowp + s * XSTAGE_BYTES;
 #pragma unroll
-            for (int o = 0; o < 8; ++o) {
-              /* codes 8o..8o+7: bytes 2o, 2o+1 of the row's 16 */
-              uint32_t s01, s23, s45, s67;
-              const uint32_t hw = words[o >> 1] >> ((o & 1) * 16);
-              code_selectors(hw & 0xFFu, &s01, &s23);
-              code_selectors((hw >> 8) & 0xFFu, &s45, &s67);
-              *(uint4 *)(dst + (((uint32_t)o ^ sw) << 4)) =
-                  make_uint4(__byte_perm(tab, 0, s01), __byte_perm(tab, 0, s23),
-                             __byte_perm(tab, 0, s45), __byte_perm(tab, 0, s67));
+            for (int o = 0; o < 8; o += 2) {
+              uint32_t x = words[o >> 1];
+              const uint32_t gone = x & (x >> 1) & 0x55555555u; /* missing */
+              x = count ? x & ~(gone | gone << 1) : gone ^ 0x55555555u;
+              const uint32_t y = x >> 10;
+              *(uint4 *)(dst + (((uint32_t)o ^ sw) << 4)) = make_uint4(
+                  x & 0x00030003u, x & 0x000C000Cu, x & 0x00300030u, x & 0x00C000C0u);
+              *(uint4 *)(dst + (((uint32_t)(o + 1) ^ sw) << 4)) = make_uint4(
+                  x & 0x03000300u, y & 0x00030003u, y & 0x000C000Cu, y & 0x00300030u);
             }
             fence_proxy_async_smem();
           }
@@ -306,7 +313,7 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
             tmem_wait_ld();
 #pragma unroll
             for (int v = 0; v < 16; ++v) {
-              const long long z = __float2int_rn(__uint_as_float(f[v]));
+              const long long z = __float2int_rn(__uint_as_float(f[v]) * 0x1p24f);
               if (live) atomicAdd(out + (int64_t)(g + v) * XR, (unsigned long long)z);
             }
           }
@@ -646,11 +653,13 @@ k_panel_slices(const x_panels pan, int32_t nk, int32_t ncols,
   __syncthreads();
   for (int i = tid; i < SL_K * SL_C; i += blockDim.x) {
     const int cc = i / SL_K, kk = i - cc * SL_K;
-    int d[S];
+    int d[S], pos, j;
+    x_field(kk, &pos, &j);
+    const float scale = 1.f / (float)(1 << (2 * j));
     const bool bad = S == 5 && sexp[cc] == X_NONFINITE;
     slice<S>(bad ? 0.0 : sp[kk][cc], bad ? 0 : sexp[cc], neg, d);
 #pragma unroll
-    for (int t = 0; t < S; ++t) ss[S * cc + t][kk] = __int2half_rn(d[t]);
+    for (int t = 0; t < S; ++t) ss[S * cc + t][pos] = __float2half_rn((float)d[t] * scale);
   }
   __syncthreads();
   /* 32 S output rows x 64 halves: 8 threads write one row's 128 bytes */
@@ -862,8 +871,8 @@ int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols
   out->kb0 = kb0;
   out->k0 = k0;
   out->ldb = ldb;
-  out->lut_lo = pp[0].count ? LUT_COUNT : LUT_MASK;
-  out->lut_hi = npanels > 1 ? (pp[1].count ? LUT_COUNT : LUT_MASK) : out->lut_lo;
+  out->count_lo = pp[0].count != 0;
+  out->count_hi = npanels > 1 ? pp[1].count != 0 : out->count_lo;
   return GP_OK;
 }
 
@@ -913,7 +922,7 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   const int32_t nitems = tiles * ksplit;
   const int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
   k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->lut_lo, P->lut_hi,
+      P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->count_lo, P->count_hi,
       ksplit, X_CHUNK_KB(P->digits), sums, ctx->d_err, NULL);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
@@ -947,7 +956,7 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
                                     X_SMEM));
   /* every SM: the kernel takes the batch's row count, and with it its work items, from db */
   k_geno_panel_tc<<<ctx->num_sms, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, NULL, ldc, NULL, 0, P->tn, P->nct, P->kb0 * P->npanels, P->kb0, P->lut_lo, P->lut_hi,
+      P->tmb, NULL, ldc, NULL, 0, P->tn, P->nct, P->kb0 * P->npanels, P->kb0, P->count_lo, P->count_hi,
       1, X_CHUNK_KB(4), z, ctx->d_err, db);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   k_panel_combine<4><<<combine_grid(ctx, max_rows, P->ncols), 256, 0, ctx->stream>>>(

@@ -41,7 +41,7 @@ struct gp_tc_prepared {
   int32_t ncols, npanels, digits, kb0, k0;
   int32_t tn, nct; /* slice columns per tile, column tiles */
   int64_t ldb;
-  uint32_t lut_lo, lut_hi;
+  int count_lo, count_hi; /* the panels multiply counts (1) or observed masks (0) */
   CUtensorMap tmb;
 };
 size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits);
