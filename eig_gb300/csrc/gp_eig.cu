@@ -796,398 +796,6 @@ __device__ __forceinline__ ff2 ff_div_fast(ff2 a, ff2 b)
 }
 
 /*
- * A float-float value that carries its step: each half next to the step's tag in a 64-bit word
- * (64-bit accesses are not torn), so that a reader polls for the value itself and needs no
- * barrier, fence or second trip to L2 for it.  Tags are c + 1 for values of step c, never 0.
- */
-__device__ __forceinline__ void tag_store(uint4 *p, ff2 v, unsigned tag)
-{
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p),
-               "r"(__float_as_uint(v.h)), "r"(tag), "r"(__float_as_uint(v.l)), "r"(tag)
-               : "memory");
-}
-__device__ __forceinline__ uint4 tag_load(const uint4 *p)
-{
-  uint4 r;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(p)
-               : "memory");
-  return r;
-}
-
-/*
- * y and x of the rows q0 + u step (u < RPT, below n): all the loads of a round are in flight
- * together, and a round asks for what is missing only.  False when the wait ran out or another
- * block gave up.
- */
-template <int RPT>
-__device__ __forceinline__ bool tag_wait(const uint4 *yt, const uint4 *xt, int q0, int step, int n,
-                                         unsigned tag, ff2 *y, ff2 *x, int *err)
-{
-  unsigned need = 0;
-#pragma unroll
-  for (int u = 0; u < RPT; ++u)
-    if (q0 + u * step < n) need |= 3u << (2 * u);
-  uint64_t t0 = 0;
-  for (unsigned it = 0; need; ++it) {
-    uint4 ry[RPT], rx[RPT];
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      if (need & (1u << (2 * u))) ry[u] = tag_load(yt + q0 + u * step);
-      if (need & (2u << (2 * u))) rx[u] = tag_load(xt + q0 + u * step);
-    }
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      if ((need & (1u << (2 * u))) && ry[u].y == tag && ry[u].w == tag) {
-        y[u] = ff_make(__uint_as_float(ry[u].x), __uint_as_float(ry[u].z));
-        need &= ~(1u << (2 * u));
-      }
-      if ((need & (2u << (2 * u))) && rx[u].y == tag && rx[u].w == tag) {
-        x[u] = ff_make(__uint_as_float(rx[u].x), __uint_as_float(rx[u].z));
-        need &= ~(2u << (2 * u));
-      }
-    }
-    if (it == 0) t0 = globaltimer_ns();
-    if ((it & 63u) == 63u) {
-      if (*(volatile int *)err) return false;
-      if (globaltimer_ns() - t0 > GP_WAIT_NS) {
-        atomicExch(err, TR_ERR_BARRIER);
-        return false;
-      }
-    }
-  }
-  return true;
-}
-
-/* one level of ff_warp_sum */
-__device__ __forceinline__ ff2 ff_lazy_xor(ff2 v, int o)
-{
-  const float oh = __shfl_xor_sync(0xFFFFFFFFu, v.h, o), ol = __shfl_xor_sync(0xFFFFFFFFu, v.l, o);
-  const float s = __fadd_rn(v.h, oh);
-  const float bb = __fsub_rn(s, v.h);
-  const float er = __fadd_rn(__fsub_rn(v.h, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
-  return ff_make(s, __fadd_rn(__fadd_rn(v.l, ol), er));
-}
-
-/*
- * Steps c0 .. n-2 with the trailing matrix (order m = n - c0 <= NT RPT) in shared memory, and
- * the last diagonal entry: block b holds whole columns r = c0 + b, c0 + b + G, .. (both
- * triangles, as float-float pairs; at most 32 columns).  Per step:
- *   A   every block redundantly: y of step c-1 and column c are polled for in global memory
- *       (tagged values, double-buffered); x of step c-1 is still in svc, unscaled, with alpha - beta in the
- *       pivot's place: v = scale x; then y.v, w, the pending update of column c, its norm and
- *       the reflector
- *   B   each warp takes a segment of rows of two owned columns: pending update, written back,
- *       and the dots with x; the owner of column c + 1 publishes it; then the first warp adds
- *       the segments and publishes y = scale (A x)
- * No barrier over the blocks: a block cannot start step c before every block's y of step c-1
- * is there, and a block publishes y of step c only after it has read all of step c-1, so the
- * two buffers suffice; a block without a column after c leaves before step c, since nobody
- * would wait for its reading.  A step is a chain of latencies: four block barriers, one trip
- * through L2, three sums over the block.  Every warp takes part in those sums, so a block has
- * few: with 32 warps their instructions alone took half the step.  Reflectors, d, e and tau are stored as pairs and converted at the end (an
- * FP64 instruction occupies its quarter of the SM for 64 clocks).  n = 1,000: 6.3 ms of
- * 8.2 with the matrix in L2 and a grid barrier per step; n = 180 on 16 blocks: 0.51 of 1.34; the
- * last 1,740 columns of 5,000: 4 ms less.
- * Needs every block resident (a cooperative launch), ytag and ctag [2][n] zero.
- */
-template <int NT, int RPT>
-__device__ __forceinline__ bool tr_smem_steps(double *A, int n, int c0, double *d, double *e,
-                                              double *tau, const double *xprev,
-                                              const double *yprev0, uint4 *ytag, uint4 *ctag,
-                                              unsigned *count, unsigned &target, int *err,
-                                              double *smm, ff2 tau_p, ff2 scale_p, ff2 e_p,
-                                              bool have_p)
-{
-  constexpr int NW = NT / 32;
-  __shared__ ff2 red[NW], red1[NW];
-  __shared__ ff2 sdot[2 * NW];
-  __shared__ tr_step st;
-  __shared__ ff2 s_yc;
-  const int G = gridDim.x, b = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const ff2 ONE = ff_make(1.f, 0.f), ZERO = ff_make(0.f, 0.f);
-  const int m = n - c0;
-  double *svp = smm - c0, *swp = smm + m - c0, *svc = smm + 2 * m - c0; /* indexed by row */
-  double *cols = smm + 3 * (size_t)m - c0;                              /* column j at j m */
-  const int cfirst = have_p ? c0 - 1 : c0; /* first reflector stored as pairs */
-  const int nown = c0 + b < n ? (n - 1 - c0 - b) / G + 1 : 0;
-  for (int j = 0; j < nown; ++j)
-    for (int q = c0 + tid; q < n; q += blockDim.x)
-      cols[(size_t)j * m + q] = A[(int64_t)(c0 + b + j * G) * n + q];
-  for (int q = c0 + tid; q < n; q += blockDim.x)
-    ff_store(svc + q, have_p ? ff_load(xprev + q) : ZERO);
-  int j0 = 0; /* first owned column at or after c + 1 */
-  /* position from the owner of the last column: at step c < n-1 the blocks at positions below
-   * n-1-c own a column after c */
-  const int pos = ((n - 1 - c0) % G - b + G) % G;
-  __syncthreads();
-  bool fail = false;
-  for (int c = c0; pos < max(1, n - 1 - c); ++c) {
-    /* ---- A ---- */
-    const int nact = min(G, max(1, n - 1 - c)); /* blocks in this step */
-    ff2 x[RPT], y[RPT], v[RPT];
-    const uint4 *yt = ytag + (size_t)((c - 1) & 1) * n, *ct = ctag + (size_t)(c & 1) * n;
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const int q = c + tid + u * NT;
-      x[u] = y[u] = ZERO;
-      if (q >= n) continue;
-      if (c == c0) {
-        x[u] = ff_load(A + (int64_t)c * n + q);
-        if (have_p) y[u] = ff_load(yprev0 + q);
-      }
-    }
-    if (c > c0) fail = !tag_wait<RPT>(yt, ct, c + tid, NT, n, (unsigned)c, y, x, err);
-    ff2 dacc = ZERO;
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const int q = c + tid + u * NT;
-      v[u] = ZERO;
-      if (q < n && have_p) {
-        v[u] = q == c ? ONE : ff_mul(ff_load(svc + q), scale_p);
-        dacc = ff_acc_lazy(dacc, y[u], v[u]);
-      }
-    }
-    dacc = ff_warp_sum(dacc);
-    if (lane == 0) red1[warp] = dacc;
-    if (tid == 0) s_yc = y[0];
-    if (__syncthreads_or(fail)) {
-      fail = true;
-      break;
-    }
-    ff2 dsum = red1[lane & (NW - 1)];
-#pragma unroll
-    for (int o = NW / 2; o; o >>= 1) dsum = ff_lazy_xor(dsum, o);
-    dsum = ff_renorm(dsum);
-    const ff2 alpha_p = ff_scale(ff_mul(ff_mul(tau_p, tau_p), dsum), -0.5f);
-    const ff2 wpc = ff_fma(tau_p, s_yc, alpha_p); /* w(c) of step c-1, where v(c) = 1 */
-    ff2 nrm = ZERO;
-#pragma unroll
-    for (int u = 0; u < RPT; ++u) {
-      const int q = c + tid + u * NT;
-      if (q >= n) continue;
-      ff2 w = ZERO;
-      if (have_p) {
-        w = ff_fma(tau_p, y[u], ff_mul(alpha_p, v[u]));
-        x[u] = ff_fma(ff_neg(v[u]), wpc, x[u]);
-        x[u] = ff_add(x[u], ff_neg(w));
-      }
-      ff_store(svp + q, v[u]);
-      ff_store(swp + q, w);
-      ff_store(svc + q, x[u]);
-      if (q >= c + 2) nrm = ff_acc_lazy(nrm, x[u], x[u]);
-    }
-    nrm = ff_warp_sum(nrm);
-    if (lane == 0) red[warp] = nrm;
-    __syncthreads();
-    if (have_p && warp > 0) {
-      /* the reflector of step c-1, the blocks in turn by rows, while the first warp forms the
-       * next one */
-      for (int q = c + pos + (tid - 32) * nact; q < n; q += (NT - 32) * nact)
-        ff_store(A + (int64_t)(c - 1) * n + q, q == c ? e_p : ff_load(svp + q));
-    }
-    if (c == n - 1) {
-      if (tid == 0) ff_store(d + c, x[0]);
-      break;
-    }
-    if (warp == 0) {
-      ff2 xn2 = red[lane & (NW - 1)];
-#pragma unroll
-      for (int o = NW / 2; o; o >>= 1) xn2 = ff_lazy_xor(xn2, o);
-      xn2 = ff_renorm(xn2);
-      if (lane == 0) {
-        /* the reflector (dlarfg): beta = -sign(alpha) sqrt(alpha^2 + |x|^2), tau = (beta -
-         * alpha) / beta, scale = 1 / (alpha - beta) */
-        const ff2 alpha = ff_load(svc + c + 1);
-        ff2 beta = alpha, tau_c = ZERO, scale_c = ZERO;
-        if (xn2.h != 0.f) {
-          const ff2 sq = ff_fma(alpha, alpha, xn2);
-          /* the approximate instructions flush subnormals: far from them only */
-          const bool fast = sq.h > 1e-28f && sq.h < 1e28f;
-          const ff2 nrm2 = fast ? ff_sqrt_fast(sq) : ff_sqrt(sq);
-          beta = alpha.h >= 0.f ? ff_neg(nrm2) : nrm2;
-          const ff2 am = ff_add(alpha, ff_neg(beta));
-          tau_c = fast ? ff_div_fast(ff_neg(am), beta) : ff_div(ff_neg(am), beta);
-          scale_c = fast ? ff_div_fast(ONE, am) : ff_div(ONE, am);
-          ff_store(svc + c + 1, am);
-        }
-        st.beta = beta;
-        st.tau_c = tau_c;
-        st.scale_c = scale_c;
-        if (pos == 0) {
-          ff_store(d + c, ff_load(svc + c));
-          ff_store(e + c, beta);
-          ff_store(tau + c, tau_c);
-        }
-      }
-    } else if (tid == 32) {
-      /* the owned columns from c + 1 on and the segments of a pair of them: a power of two, as
-       * many as there are warps for, of at least 32 rows */
-      int j = j0;
-      if (c0 + b + j * G < c + 1) ++j;
-      const int npair = (nown - j + 1) >> 1, rows = n - 1 - c;
-      int sh = 0;
-      while ((npair << (sh + 1)) <= NW && (rows >> (sh + 1)) >= 32) ++sh;
-      st.b1_u0 = j;
-      st.b1_u1 = sh;
-    }
-    __syncthreads();
-    const ff2 scale_c = st.scale_c;
-    j0 = st.b1_u0;
-    const int sh = st.b1_u1, S = 1 << sh;
-    tau_p = st.tau_c;
-    scale_p = scale_c;
-    e_p = st.beta;
-    have_p = true;
-    /* ---- B: the owned columns r >= c + 1, two at a time ---- */
-    const int nc = nown - j0, nitem = ((nc + 1) >> 1) << sh;
-    const int seg = (((n - 1 - c + S - 1) >> sh) + 31) & ~31;
-    uint4 *cn = ctag + (size_t)((c + 1) & 1) * n;
-    /* an item per warp; with more pairs than warps (sh = 0) the dots of the later pairs wait
-     * in registers for the slots of the earlier ones: at most two rounds, 32 columns */
-    ff2 dab[2];
-#pragma unroll
-    for (int rd = 0; rd < 2; ++rd) {
-      const int it = warp + rd * NW;
-      ff2 da = ZERO, db = ZERO;
-      if (it < nitem) {
-        const int pi = it >> sh, sg = it & (S - 1);
-        const int ja = j0 + 2 * pi, ra = c0 + b + ja * G, rb = ra + G;
-        const bool two = rb < n;
-        double *ca = cols + (size_t)ja * m, *cb = two ? ca + m : ca;
-        const ff2 vra = ff_load(svp + ra), wra = ff_load(swp + ra);
-        const ff2 vrb = two ? ff_load(svp + rb) : ZERO, wrb = two ? ff_load(swp + rb) : ZERO;
-        const int qs = c + 1 + sg * seg, qe = min(n, qs + seg);
-        const bool next = ra == c + 1; /* the first of its block: never the second of a pair */
-#pragma unroll 2
-        for (int q = qs + lane; q < qe; q += 32) {
-          const ff2 vq = ff_load(svp + q), wq = ff_load(swp + q), xq = ff_load(svc + q);
-          const ff2 a = ff_sub2prod(ff_load(ca + q), vq, wra, wq, vra);
-          ff_store(ca + q, a);
-          if (next) tag_store(cn + q, a, (unsigned)(c + 1));
-          da = ff_acc_lazy(da, a, xq);
-          if (two) {
-            const ff2 a2 = ff_sub2prod(ff_load(cb + q), vq, wrb, wq, vrb);
-            ff_store(cb + q, a2);
-            db = ff_acc_lazy(db, a2, xq);
-          }
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          da = ff_lazy_xor(da, o);
-          db = ff_lazy_xor(db, o);
-        }
-      }
-      dab[rd] = lane ? db : da; /* lanes 0 and 1 carry a pair's two sums */
-      if (rd == 0) {
-        if (lane < 2) sdot[2 * warp + lane] = dab[0];
-        if (nitem <= NW) break;
-      }
-    }
-    if (nitem > NW) {
-      /* one segment per pair: a warp's own sums are complete */
-      if (lane < 2)
-#pragma unroll
-        for (int rd = 0; rd < 2; ++rd) {
-          const int col = 2 * (warp + rd * NW) + lane;
-          if (col < nc)
-            tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
-                      ff_mul(ff_renorm(dab[rd]), scale_c), (unsigned)(c + 1));
-        }
-      __syncthreads(); /* the vectors are rewritten by the next step */
-      continue;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      /* the segments of a column, slots 2 (pair S + segment) + column of the pair, by a tree */
-#pragma unroll
-      for (int h = 0; h < (2 * NW + 31) / 32; ++h) {
-        const int slot = lane + 32 * h;
-        ff2 t = slot < 2 * nitem ? sdot[slot] : ZERO;
-        for (int o = 1; o < S; o <<= 1) t = ff_lazy_xor(t, 2 * o);
-        const int col = 2 * (slot >> (sh + 1)) + (slot & 1);
-        if (((slot >> 1) & (S - 1)) == 0 && slot < 2 * nitem && col < nc)
-          tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
-                    ff_mul(ff_renorm(t), scale_c), (unsigned)(c + 1));
-      }
-    }
-  }
-  if (fail) return false;
-  /* when every block's pairs are stored: to FP64 */
-  target += G;
-  if (!tr_grid_sync(count, target, err)) return false;
-  for (int c = cfirst + b; c < n - 1; c += G)
-    for (int q = c + 1 + tid; q < n; q += blockDim.x) {
-      double *p = A + (int64_t)c * n + q;
-      *p = ff_to_double(ff_load(p));
-    }
-  if (b == 0)
-    for (int c = c0 + tid; c < n; c += blockDim.x) {
-      d[c] = ff_to_double(ff_load(d + c));
-      if (c < n - 1) {
-        e[c] = ff_to_double(ff_load(e + c));
-        tau[c] = ff_to_double(ff_load(tau + c));
-      }
-    }
-  return true;
-}
-
-/* what a launch's last step leaves for the next launch's first (float-float pairs) */
-struct tr_state {
-  ff2 tau, scale, e;
-};
-
-/* steps c0 .. n-2: from the start (c0 = 0), or after the steps of another kernel */
-template <int NT, int RPT>
-__global__ void __launch_bounds__(NT, 1)
-k_tridiag_smem(double *A, int n, int c0, double *d, double *e, double *tau, const double *xprev,
-               const double *yprev, uint4 *ytag, uint4 *ctag, const tr_state *state, unsigned *bar,
-               int *err)
-{
-  extern __shared__ double sh[];
-  const ff2 ZERO = ff_make(0.f, 0.f);
-  unsigned target = 0;
-  const bool have_p = c0 > 0;
-  tr_smem_steps<NT, RPT>(A, n, c0, d, e, tau, xprev, yprev, ytag, ctag, bar, target, err, sh,
-                         have_p ? state->tau : ZERO, have_p ? state->scale : ZERO,
-                         have_p ? state->e : ZERO, have_p);
-}
-
-#define TR_SMEM_NT 512 /* threads and rows per thread above TR_SMALL_ORDER rows */
-#define TR_SMEM_RPT 4
-#define TR_SMALL_ORDER 768 /* trailing orders up to this with 256 threads */
-
-/* steps 0 .. c_end - 1 by whole columns in L2: orders whose tiles' shared memory does not fit */
-__global__ void __launch_bounds__(TR_THREADS, 1)
-k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double *vbuf,
-          double *wbuf, double *ybuf, double *part_dot2, tr_state *state, unsigned *bar, int *err,
-          unsigned long long *phase_ns)
-{
-  extern __shared__ double sh[];
-  const ff2 ZERO = ff_make(0.f, 0.f);
-  unsigned target = 0;
-  ff2 tau_pf = ZERO, scale_pf = ZERO, e_pf = ZERO;
-  bool have_p = false;
-  /* phase_ns (optional, block 0): time in A, B (entry 1; entry 2 for the first 30% of the
-   * steps) and the barrier (entry 4) */
-  __shared__ unsigned long long s_ph[6];
-  const bool stamp = phase_ns != NULL && blockIdx.x == 0 && threadIdx.x == 0;
-  if (stamp) {
-    for (int i = 0; i < 5; ++i) s_ph[i] = 0ull;
-    s_ph[5] = globaltimer_ns();
-  }
-  if (!tr_full_steps(A, n, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
-                     sh + n, sh + 2 * n, tau_pf, scale_pf, e_pf, have_p, stamp ? s_ph : NULL))
-    return;
-  if (stamp)
-    for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *state = {tau_pf, scale_pf, e_pf};
-}
-
-/* ---------------------------------------------------------------------------------- */
-/*
  * Pairs of float-float numbers in the packed FP32 instructions (two operations in one issue
  * slot; each is rounded as its scalar form, so every formula below is the scalar one above it,
  * twice).
@@ -1357,6 +965,443 @@ __device__ __forceinline__ void pv_put(double *v, int q, ff2 a)
   f[2] = a.l;
 }
 
+/* a + b left unnormalised (ff_warp_sum's step) */
+__device__ __forceinline__ pf2 pf_add_lazy(pf2 a, pf2 b)
+{
+  const f2 s = f2_add(a.h, b.h);
+  const f2 bb = f2_sub(s, a.h);
+  const f2 er = f2_add(f2_sub(a.h, f2_sub(s, bb)), f2_sub(b.h, bb));
+  return pf_make(s, f2_add(f2_add(a.l, b.l), er));
+}
+__device__ __forceinline__ ff2 ff_add_lazy(ff2 a, ff2 b)
+{
+  const float s = __fadd_rn(a.h, b.h);
+  const float bb = __fsub_rn(s, a.h);
+  const float er = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
+  return ff_make(s, __fadd_rn(__fadd_rn(a.l, b.l), er));
+}
+/*
+ * A float-float value that carries its step: each half next to the step's tag in a 64-bit word
+ * (64-bit accesses are not torn), so that a reader polls for the value itself and needs no
+ * barrier, fence or second trip to L2 for it.  Tags are c + 1 for values of step c, never 0.
+ */
+__device__ __forceinline__ void tag_store(uint4 *p, ff2 v, unsigned tag)
+{
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p),
+               "r"(__float_as_uint(v.h)), "r"(tag), "r"(__float_as_uint(v.l)), "r"(tag)
+               : "memory");
+}
+__device__ __forceinline__ uint4 tag_load(const uint4 *p)
+{
+  uint4 r;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
+/*
+ * y and x of the rows q0 + (u / 2) step + u % 2 (u < RPT, at least c and below n): all the loads
+ * of a round are in flight together, and a round asks for what is missing only.  False when the wait ran out or another
+ * block gave up.
+ */
+template <int RPT>
+__device__ __forceinline__ bool tag_wait(const uint4 *yt, const uint4 *xt, int q0, int step, int c, int n,
+                                         unsigned tag, ff2 *y, ff2 *x, int *err)
+{
+  unsigned need = 0;
+#pragma unroll
+  for (int u = 0; u < RPT; ++u)
+    if (q0 + (u >> 1) * step + (u & 1) >= c && q0 + (u >> 1) * step + (u & 1) < n)
+      need |= 3u << (2 * u);
+  uint64_t t0 = 0;
+  for (unsigned it = 0; need; ++it) {
+    uint4 ry[RPT], rx[RPT];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      if (need & (1u << (2 * u))) ry[u] = tag_load(yt + q0 + (u >> 1) * step + (u & 1));
+      if (need & (2u << (2 * u))) rx[u] = tag_load(xt + q0 + (u >> 1) * step + (u & 1));
+    }
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      if ((need & (1u << (2 * u))) && ry[u].y == tag && ry[u].w == tag) {
+        y[u] = ff_make(__uint_as_float(ry[u].x), __uint_as_float(ry[u].z));
+        need &= ~(1u << (2 * u));
+      }
+      if ((need & (2u << (2 * u))) && rx[u].y == tag && rx[u].w == tag) {
+        x[u] = ff_make(__uint_as_float(rx[u].x), __uint_as_float(rx[u].z));
+        need &= ~(2u << (2 * u));
+      }
+    }
+    if (it == 0) t0 = globaltimer_ns();
+    if ((it & 63u) == 63u) {
+      if (*(volatile int *)err) return false;
+      if (globaltimer_ns() - t0 > GP_WAIT_NS) {
+        atomicExch(err, TR_ERR_BARRIER);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
+/* one level of ff_warp_sum */
+__device__ __forceinline__ ff2 ff_lazy_xor(ff2 v, int o)
+{
+  const float oh = __shfl_xor_sync(0xFFFFFFFFu, v.h, o), ol = __shfl_xor_sync(0xFFFFFFFFu, v.l, o);
+  const float s = __fadd_rn(v.h, oh);
+  const float bb = __fsub_rn(s, v.h);
+  const float er = __fadd_rn(__fsub_rn(v.h, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
+  return ff_make(s, __fadd_rn(__fadd_rn(v.l, ol), er));
+}
+
+/*
+ * Steps c0 .. n-2 with the trailing matrix (order m = n - c0 <= NT RPT) in shared memory, and
+ * the last diagonal entry: block b holds whole columns r = c0 + b, c0 + b + G, .. (both
+ * triangles, as float-float pairs; at most 32 columns).  Per step:
+ *   A   every block redundantly: y of step c-1 and column c are polled for in global memory
+ *       (tagged values, double-buffered); x of step c-1 is still in svc, unscaled, with alpha - beta in the
+ *       pivot's place: v = scale x; then y.v, w, the pending update of column c, its norm and
+ *       the reflector
+ *   B   each warp takes a segment of rows of two owned columns: pending update, written back,
+ *       and the dots with x; the owner of column c + 1 publishes it; then the first warp adds
+ *       the segments and publishes y = scale (A x)
+ * No barrier over the blocks: a block cannot start step c before every block's y of step c-1
+ * is there, and a block publishes y of step c only after it has read all of step c-1, so the
+ * two buffers suffice; a block without a column after c leaves before step c, since nobody
+ * would wait for its reading.  A step is a chain of latencies: four block barriers, one trip
+ * through L2, three sums over the block.  Every warp takes part in those sums, so a block has
+ * few: with 32 warps their instructions alone took half the step.  A thread's rows come in pairs for
+ * the packed FP32 instructions.  Reflectors, d, e and tau are stored as pairs and converted at the end (an
+ * FP64 instruction occupies its quarter of the SM for 64 clocks).  n = 1,000: 5.2 ms of
+ * 8.2 with the matrix in L2 and a grid barrier per step (5.9 before the packed pairs); n = 180 on 12
+ * blocks: 0.50 of 1.34; the last 1,706 columns of 5,000: 12.4 (13.1).
+ * Needs every block resident (a cooperative launch), ytag and ctag [2][n] zero.
+ */
+template <int NT, int RPT>
+__device__ __forceinline__ bool tr_smem_steps(double *A, int n, int c0, double *d, double *e,
+                                              double *tau, const double *xprev,
+                                              const double *yprev0, uint4 *ytag, uint4 *ctag,
+                                              unsigned *count, unsigned &target, int *err,
+                                              double *smm, ff2 tau_p, ff2 scale_p, ff2 e_p,
+                                              bool have_p)
+{
+  constexpr int NW = NT / 32;
+  __shared__ ff2 red[NW], red1[NW];
+  __shared__ ff2 sdot[2 * NW];
+  __shared__ tr_step st;
+  __shared__ ff2 s_yc;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const ff2 ONE = ff_make(1.f, 0.f), ZERO = ff_make(0.f, 0.f);
+  constexpr int RP = RPT / 2; /* pairs of rows per thread */
+  const int m = n - c0, mp = (m + 1) & ~1, np = mp / 2;
+  /* vectors of pairs over the rows from c0; column j at j mp */
+  double *svp = smm, *swp = smm + mp, *svc = smm + 2 * mp, *cols = smm + 3 * (size_t)mp;
+  const int cfirst = have_p ? c0 - 1 : c0; /* first reflector stored as pairs */
+  const int nown = c0 + b < n ? (n - 1 - c0 - b) / G + 1 : 0;
+  for (int j = 0; j < nown; ++j)
+    for (int q = tid; q < mp; q += NT)
+      pv_put(cols + (size_t)j * mp, q,
+             q < m ? ff_load(A + (int64_t)(c0 + b + j * G) * n + c0 + q) : ZERO);
+  for (int q = tid; q < mp; q += NT)
+    pv_put(svc, q, have_p && q < m ? ff_load(xprev + c0 + q) : ZERO);
+  int j0 = 0; /* first owned column at or after c + 1 */
+  /* position from the owner of the last column: at step c < n-1 the blocks at positions below
+   * n-1-c own a column after c */
+  const int pos = ((n - 1 - c0) % G - b + G) % G;
+  __syncthreads();
+  bool fail = false;
+  for (int c = c0; pos < max(1, n - 1 - c); ++c) {
+    /* ---- A ---- */
+    const int nact = min(G, max(1, n - 1 - c)); /* blocks in this step */
+    const int k = c - c0, P0 = k >> 1, odd = k & 1; /* the pair of c, whose first row may be done */
+    ff2 x[RPT], y[RPT];
+    const uint4 *yt = ytag + (size_t)((c - 1) & 1) * n, *ct = ctag + (size_t)(c & 1) * n;
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int q = c0 + 2 * (P0 + tid + (u >> 1) * NT) + (u & 1);
+      x[u] = y[u] = ZERO;
+      if (q < c || q >= n) continue;
+      if (c == c0) {
+        x[u] = ff_load(A + (int64_t)c * n + q);
+        if (have_p) y[u] = ff_load(yprev0 + q);
+      }
+    }
+    if (c > c0)
+      fail = !tag_wait<RPT>(yt, ct, c0 + 2 * (P0 + tid), 2 * NT, c, n, (unsigned)c, y, x, err);
+    pf2 x2[RP], y2[RP], v2[RP], dacc2 = pf_make(0, 0);
+    const pf2 scale2 = pf_dup(scale_p);
+#pragma unroll
+    for (int u = 0; u < RP; ++u) {
+      const int p = P0 + tid + u * NT;
+      x2[u] = pf_join(x[2 * u], x[2 * u + 1]);
+      y2[u] = pf_join(y[2 * u], y[2 * u + 1]);
+      v2[u] = pf_make(0, 0);
+      if (p < np && have_p) {
+        v2[u] = pf_mul(pv_load(svc, p), scale2);
+        if (p == P0) v2[u] = odd ? pf_join(ZERO, ONE) : pf_join(ONE, pf_odd(v2[u]));
+        dacc2 = pf_acc_lazy(dacc2, y2[u], v2[u], f2_neg(v2[u].h));
+      }
+    }
+    const ff2 dacc = ff_warp_sum(ff_add_lazy(pf_even(dacc2), pf_odd(dacc2)));
+    if (lane == 0) red1[warp] = dacc;
+    if (tid == 0) s_yc = odd ? y[1] : y[0];
+    if (__syncthreads_or(fail)) {
+      fail = true;
+      break;
+    }
+    ff2 dsum = red1[lane & (NW - 1)];
+#pragma unroll
+    for (int o = NW / 2; o; o >>= 1) dsum = ff_lazy_xor(dsum, o);
+    dsum = ff_renorm(dsum);
+    const ff2 alpha_p = ff_scale(ff_mul(ff_mul(tau_p, tau_p), dsum), -0.5f);
+    const ff2 wpc = ff_fma(tau_p, s_yc, alpha_p); /* w(c) of step c-1, where v(c) = 1 */
+    const pf2 tau2 = pf_dup(tau_p), alpha2 = pf_dup(alpha_p), nwpc2 = pf_dup(ff_neg(wpc));
+    pf2 nrm2 = pf_make(0, 0);
+#pragma unroll
+    for (int u = 0; u < RP; ++u) {
+      const int p = P0 + tid + u * NT;
+      if (p >= np) continue;
+      pf2 w = pf_make(0, 0), z = x2[u];
+      if (have_p) {
+        w = pf_fma(tau2, y2[u], pf_mul(alpha2, v2[u]));
+        z = pf_fma(v2[u], nwpc2, z);
+        z = pf_add(z, pf_make(f2_neg(w.h), f2_neg(w.l)));
+      }
+      pv_store(svp, p, v2[u]);
+      pv_store(swp, p, w);
+      pv_store(svc, p, z);
+      if (2 * p < k + 2) z = pf_join(ZERO, 2 * p + 1 < k + 2 ? ZERO : pf_odd(z));
+      nrm2 = pf_acc_lazy(nrm2, z, z, f2_neg(z.h));
+    }
+    const ff2 nrm = ff_warp_sum(ff_add_lazy(pf_even(nrm2), pf_odd(nrm2)));
+    if (lane == 0) red[warp] = nrm;
+    __syncthreads();
+    if (have_p && warp > 0) {
+      /* the reflector of step c-1, the blocks in turn by rows, while the first warp forms the
+       * next one */
+      for (int q = c + pos + (tid - 32) * nact; q < n; q += (NT - 32) * nact)
+        ff_store(A + (int64_t)(c - 1) * n + q, q == c ? e_p : pv_get(svp, q - c0));
+    }
+    if (c == n - 1) {
+      if (tid == 0) ff_store(d + c, pv_get(svc, k));
+      break;
+    }
+    if (warp == 0) {
+      ff2 xn2 = red[lane & (NW - 1)];
+#pragma unroll
+      for (int o = NW / 2; o; o >>= 1) xn2 = ff_lazy_xor(xn2, o);
+      xn2 = ff_renorm(xn2);
+      if (lane == 0) {
+        /* the reflector (dlarfg): beta = -sign(alpha) sqrt(alpha^2 + |x|^2), tau = (beta -
+         * alpha) / beta, scale = 1 / (alpha - beta) */
+        const ff2 alpha = pv_get(svc, k + 1);
+        ff2 beta = alpha, tau_c = ZERO, scale_c = ZERO;
+        if (xn2.h != 0.f) {
+          const ff2 sq = ff_fma(alpha, alpha, xn2);
+          /* the approximate instructions flush subnormals: far from them only */
+          const bool fast = sq.h > 1e-28f && sq.h < 1e28f;
+          const ff2 nrm2 = fast ? ff_sqrt_fast(sq) : ff_sqrt(sq);
+          beta = alpha.h >= 0.f ? ff_neg(nrm2) : nrm2;
+          const ff2 am = ff_add(alpha, ff_neg(beta));
+          tau_c = fast ? ff_div_fast(ff_neg(am), beta) : ff_div(ff_neg(am), beta);
+          scale_c = fast ? ff_div_fast(ONE, am) : ff_div(ONE, am);
+          pv_put(svc, k + 1, am);
+        }
+        st.beta = beta;
+        st.tau_c = tau_c;
+        st.scale_c = scale_c;
+        if (pos == 0) {
+          ff_store(d + c, pv_get(svc, k));
+          ff_store(e + c, beta);
+          ff_store(tau + c, tau_c);
+        }
+      }
+    } else if (tid == 32) {
+      /* the owned columns from c + 1 on and the segments of a pair of them: a power of two, as
+       * many as there are warps for, of at least 64 rows */
+      int j = j0;
+      if (c0 + b + j * G < c + 1) ++j;
+      const int npair = (nown - j + 1) >> 1, rows = n - 1 - c;
+      int sh = 0;
+      while ((npair << (sh + 1)) <= NW && (rows >> (sh + 1)) >= 64) ++sh;
+      st.b1_u0 = j;
+      st.b1_u1 = sh;
+    }
+    __syncthreads();
+    const ff2 scale_c = st.scale_c;
+    j0 = st.b1_u0;
+    const int sh = st.b1_u1, S = 1 << sh;
+    tau_p = st.tau_c;
+    scale_p = scale_c;
+    e_p = st.beta;
+    have_p = true;
+    /* ---- B: the owned columns r >= c + 1, two at a time ---- */
+    const int nc = nown - j0, nitem = ((nc + 1) >> 1) << sh;
+    const int pb = (k + 1) >> 1; /* the pair of c + 1, whose first row may be c */
+    const int seg = (((np - pb + S - 1) >> sh) + 31) & ~31;
+    uint4 *cn = ctag + (size_t)((c + 1) & 1) * n;
+    /* an item per warp; with more pairs than warps (sh = 0) the dots of the later pairs wait
+     * in registers for the slots of the earlier ones: at most two rounds, 32 columns */
+    ff2 dab[2];
+#pragma unroll
+    for (int rd = 0; rd < 2; ++rd) {
+      const int it = warp + rd * NW;
+      ff2 da = ZERO, db = ZERO;
+      if (it < nitem) {
+        const int pi = it >> sh, sg = it & (S - 1);
+        const int ja = j0 + 2 * pi, ra = c0 + b + ja * G, rb = ra + G;
+        const bool two = rb < n;
+        double *ca = cols + (size_t)ja * mp, *cb = two ? ca + mp : ca;
+        const pf2 vra = pf_dup(pv_get(svp, ra - c0)), wra = pf_dup(pv_get(swp, ra - c0));
+        const pf2 vrb = pf_dup(two ? pv_get(svp, rb - c0) : ZERO);
+        const pf2 wrb = pf_dup(two ? pv_get(swp, rb - c0) : ZERO);
+        const f2 vran = f2_neg(vra.h), wran = f2_neg(wra.h);
+        const f2 vrbn = f2_neg(vrb.h), wrbn = f2_neg(wrb.h);
+        const int ps = pb + sg * seg, pe = min(np, ps + seg);
+        const bool next = ra == c + 1; /* the first of its block: never the second of a pair */
+        pf2 da2 = pf_make(0, 0), db2 = da2;
+#pragma unroll 2
+        for (int p = ps + lane; p < pe; p += 32) {
+          const pf2 vq = pv_load(svp, p), wq = pv_load(swp, p);
+          pf2 xq = pv_load(svc, p);
+          if (p == pb && !odd) xq = pf_join(ZERO, pf_odd(xq)); /* k + 1 odd: the first row is c */
+          const f2 xn = f2_neg(xq.h);
+          const pf2 a = pf_sub2prod(pv_load(ca, p), vq, wra, wran, wq, vra, vran);
+          pv_store(ca, p, a);
+          if (next) {
+            const int q = c0 + 2 * p;
+            if (q > c) tag_store(cn + q, pf_even(a), (unsigned)(c + 1));
+            if (q + 1 < n) tag_store(cn + q + 1, pf_odd(a), (unsigned)(c + 1));
+          }
+          da2 = pf_acc_lazy(da2, a, xq, xn);
+          if (two) {
+            const pf2 a2 = pf_sub2prod(pv_load(cb, p), vq, wrb, wrbn, wq, vrb, vrbn);
+            pv_store(cb, p, a2);
+            db2 = pf_acc_lazy(db2, a2, xq, xn);
+          }
+        }
+        da = ff_add_lazy(pf_even(da2), pf_odd(da2));
+        db = ff_add_lazy(pf_even(db2), pf_odd(db2));
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          da = ff_lazy_xor(da, o);
+          db = ff_lazy_xor(db, o);
+        }
+      }
+      dab[rd] = lane ? db : da; /* lanes 0 and 1 carry a pair's two sums */
+      if (rd == 0) {
+        if (lane < 2) sdot[2 * warp + lane] = dab[0];
+        if (nitem <= NW) break;
+      }
+    }
+    if (nitem > NW) {
+      /* one segment per pair: a warp's own sums are complete */
+      if (lane < 2)
+#pragma unroll
+        for (int rd = 0; rd < 2; ++rd) {
+          const int col = 2 * (warp + rd * NW) + lane;
+          if (col < nc)
+            tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
+                      ff_mul(ff_renorm(dab[rd]), scale_c), (unsigned)(c + 1));
+        }
+      __syncthreads(); /* the vectors are rewritten by the next step */
+      continue;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      /* the segments of a column, slots 2 (pair S + segment) + column of the pair, by a tree */
+#pragma unroll
+      for (int h = 0; h < (2 * NW + 31) / 32; ++h) {
+        const int slot = lane + 32 * h;
+        ff2 t = slot < 2 * nitem ? sdot[slot] : ZERO;
+        for (int o = 1; o < S; o <<= 1) t = ff_lazy_xor(t, 2 * o);
+        const int col = 2 * (slot >> (sh + 1)) + (slot & 1);
+        if (((slot >> 1) & (S - 1)) == 0 && slot < 2 * nitem && col < nc)
+          tag_store(ytag + (size_t)(c & 1) * n + c0 + b + (j0 + col) * G,
+                    ff_mul(ff_renorm(t), scale_c), (unsigned)(c + 1));
+      }
+    }
+  }
+  if (fail) return false;
+  /* when every block's pairs are stored: to FP64 */
+  target += G;
+  if (!tr_grid_sync(count, target, err)) return false;
+  for (int c = cfirst + b; c < n - 1; c += G)
+    for (int q = c + 1 + tid; q < n; q += blockDim.x) {
+      double *p = A + (int64_t)c * n + q;
+      *p = ff_to_double(ff_load(p));
+    }
+  if (b == 0)
+    for (int c = c0 + tid; c < n; c += blockDim.x) {
+      d[c] = ff_to_double(ff_load(d + c));
+      if (c < n - 1) {
+        e[c] = ff_to_double(ff_load(e + c));
+        tau[c] = ff_to_double(ff_load(tau + c));
+      }
+    }
+  return true;
+}
+
+/* what a launch's last step leaves for the next launch's first (float-float pairs) */
+struct tr_state {
+  ff2 tau, scale, e;
+};
+
+/* steps c0 .. n-2: from the start (c0 = 0), or after the steps of another kernel */
+template <int NT, int RPT>
+__global__ void __launch_bounds__(NT, 1)
+k_tridiag_smem(double *A, int n, int c0, double *d, double *e, double *tau, const double *xprev,
+               const double *yprev, uint4 *ytag, uint4 *ctag, const tr_state *state, unsigned *bar,
+               int *err)
+{
+  extern __shared__ double sh[];
+  const ff2 ZERO = ff_make(0.f, 0.f);
+  unsigned target = 0;
+  const bool have_p = c0 > 0;
+  tr_smem_steps<NT, RPT>(A, n, c0, d, e, tau, xprev, yprev, ytag, ctag, bar, target, err, sh,
+                         have_p ? state->tau : ZERO, have_p ? state->scale : ZERO,
+                         have_p ? state->e : ZERO, have_p);
+}
+
+/* 256 threads at every order, of 2, 4 or 8 rows each (the loops over a thread's rows are
+ * unrolled): 512 threads of 4 rows took 13.7 ms where these take 12.4 at 1,706 rows, 6.8 against 5.2
+ * at 1,000; 128 threads 0.54 against 0.50 at 180.  Two rows a thread up to TR_SMALL_ORDER: 0.50 ms
+ * against 0.52 at 180, 1.53 against 1.44 at 400 */
+#define TR_SMEM_NT 256
+#define TR_SMEM_RPT 8
+#define TR_SMALL_ORDER 320
+
+/* steps 0 .. c_end - 1 by whole columns in L2: orders whose tiles' shared memory does not fit */
+__global__ void __launch_bounds__(TR_THREADS, 1)
+k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double *vbuf,
+          double *wbuf, double *ybuf, double *part_dot2, tr_state *state, unsigned *bar, int *err,
+          unsigned long long *phase_ns)
+{
+  extern __shared__ double sh[];
+  const ff2 ZERO = ff_make(0.f, 0.f);
+  unsigned target = 0;
+  ff2 tau_pf = ZERO, scale_pf = ZERO, e_pf = ZERO;
+  bool have_p = false;
+  /* phase_ns (optional, block 0): time in A, B (entry 1; entry 2 for the first 30% of the
+   * steps) and the barrier (entry 4) */
+  __shared__ unsigned long long s_ph[6];
+  const bool stamp = phase_ns != NULL && blockIdx.x == 0 && threadIdx.x == 0;
+  if (stamp) {
+    for (int i = 0; i < 5; ++i) s_ph[i] = 0ull;
+    s_ph[5] = globaltimer_ns();
+  }
+  if (!tr_full_steps(A, n, c_end, d, e, tau, vbuf, wbuf, ybuf, part_dot2, bar, target, err, sh,
+                     sh + n, sh + 2 * n, tau_pf, scale_pf, e_pf, have_p, stamp ? s_ph : NULL))
+    return;
+  if (stamp)
+    for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *state = {tau_pf, scale_pf, e_pf};
+}
+
+/* ---------------------------------------------------------------------------------- */
 /*
  * The same reduction (dsytd2, lower) with the trailing matrix held as its lower triangle only,
  * in TT x TT tiles: half the bytes per column step and two thirds of the float-float work of
@@ -1433,21 +1478,6 @@ __global__ void k_tri_to_tiles(const double *A, int n, int nt, double *Tm)
   }
 }
 
-/* a + b left unnormalised (ff_warp_sum's step) */
-__device__ __forceinline__ pf2 pf_add_lazy(pf2 a, pf2 b)
-{
-  const f2 s = f2_add(a.h, b.h);
-  const f2 bb = f2_sub(s, a.h);
-  const f2 er = f2_add(f2_sub(a.h, f2_sub(s, bb)), f2_sub(b.h, bb));
-  return pf_make(s, f2_add(f2_add(a.l, b.l), er));
-}
-__device__ __forceinline__ ff2 ff_add_lazy(ff2 a, ff2 b)
-{
-  const float s = __fadd_rn(a.h, b.h);
-  const float bb = __fsub_rn(s, a.h);
-  const float er = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
-  return ff_make(s, __fadd_rn(__fadd_rn(a.l, b.l), er));
-}
 /* sum over the lanes of 8 columns' dots (4 pairs), scattered: lanes 4k .. 4k+3 end with column k */
 __device__ __forceinline__ ff2 tt_scatter8(pf2 *cp, int lane)
 {
@@ -2500,15 +2530,16 @@ static void tt_tables(int nt, int pr, int pc, std::vector<unsigned char> &rgt,
 /* dynamic shared memory of tr_smem_steps for trailing order m on G blocks */
 static size_t tr_smem_bytes(int m, int G)
 {
-  return sizeof(double) * (3 * (size_t)m + (size_t)((m + G - 1) / G) * m);
+  return sizeof(double) * (size_t)(3 + (m + G - 1) / G) * (size_t)((m + 1) & ~1);
 }
 /* blocks for trailing order m: every block reads all of y and the column in each step, which
  * costs more the more blocks ask (about 1,900 clocks for 16 of them, 4,000 for 64, 6,700 for
- * 152 at m = 1,000), so no more than one for 12 columns, unless shared memory needs them
- * (m = 400: 1.71 ms on 32, 2.18 on 152; m = 1,000: 6.0 on 64, 6.4 on 152) */
+ * 152 at m = 1,000), so one for 15 columns, but up to ten for small orders, or what shared memory
+ * needs (m = 180: 0.515 ms on 12, 0.53 on 18, 0.61 on 6; m = 700: 3.10 on 50, 3.32 on 72; m = 1,000:
+ * 5.13 on 64, 5.28 on 100, 5.83 on 40) */
 static int tr_smem_blocks(int m, int G)
 {
-  int Gm = std::min(G, std::max(m / 12, (m + 31) / 32));
+  int Gm = std::min(G, std::max(std::max(m / 15, std::min(m / 8, 10)), (m + 31) / 32));
   while (Gm < G && tr_smem_bytes(m, Gm) > 200 * 1024) ++Gm;
   return Gm;
 }
@@ -2715,9 +2746,10 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       }
     }
     {
-      const int m = n - c_end, small = m <= TR_SMALL_ORDER;
-      const void *f = small ? (const void *)k_tridiag_smem<256, TR_SMALL_ORDER / 256>
-                            : (const void *)k_tridiag_smem<TR_SMEM_NT, TR_SMEM_RPT>;
+      const int m = n - c_end;
+      const void *f = m <= TR_SMALL_ORDER   ? (const void *)k_tridiag_smem<TR_SMEM_NT, 2>
+                      : m <= 4 * TR_SMEM_NT ? (const void *)k_tridiag_smem<TR_SMEM_NT, 4>
+                                            : (const void *)k_tridiag_smem<TR_SMEM_NT, TR_SMEM_RPT>;
       const int Gm = tr_smem_blocks(m, (int)G);
       const double *xp = xlast, *yp = ylast;
       uint4 *ctag = ytag + 2 * nd;
@@ -2725,8 +2757,7 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       void *args[] = {&A,  &nn,   &c_end, &d,     &e,     &tau,  &xp,
                       &yp, &ytag, &ctag,  &state, &bar_s, &d_err};
       GP_CUDA(ctx, gp_allow_smem(ctx, f));
-      GP_CUDA(ctx, cudaLaunchCooperativeKernel(f, dim3((unsigned)Gm),
-                                               dim3(small ? 256 : TR_SMEM_NT), args,
+      GP_CUDA(ctx, cudaLaunchCooperativeKernel(f, dim3((unsigned)Gm), dim3(TR_SMEM_NT), args,
                                                tr_smem_bytes(m, Gm), ctx->stream));
       ctx->launches++;
     }
