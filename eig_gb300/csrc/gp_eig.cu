@@ -2839,8 +2839,10 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     const int P = 32 / epw;
     const int nwarps = (n + epw - 1) / epw;
     const int blocks = (nwarps + 3) / 4;
-    /* FP64 brackets end at 1e-13 ||T||: the counts' own backward error is ~6e-14 ||T|| */
-    const double tol = 1e-13 * tnorm;
+    /* FP64 brackets end at 1e-13 ||T||: the counts' own backward error is ~6e-14 ||T||.  Half a
+     * bracket is the error, and with 32 points the check alone can end at 0.9e-13 (4e-14 measured
+     * for orders up to 608, 1e-14 with a step more): narrower where a step is cheap */
+    const double tol = (P >= 16 ? 3e-14 : 1e-13) * tnorm;
     if (use_smem)
       GP_CUDA(ctx, gp_allow_smem(ctx, (const void *)k_multisect));
     k_multisect<<<blocks, 128, use_smem ? smem : 0, ctx->stream>>>(d, e2, n, gl, gu, tnorm, pivmin,
