@@ -113,20 +113,51 @@ __host__ __device__ __forceinline__ int32_t x_split(int32_t tiles, int32_t nkb, 
   return best;
 }
 
+/* a column's power of two from the bits of its largest magnitude; X_NONFINITE (5 slices) for an
+ * infinity or NaN */
+#define X_NONFINITE (-(1 << 30))
+template <int S>
+__device__ __forceinline__ int x_exponent(unsigned long long mx)
+{
+  if (S == 5 && mx >= 0x7FF0000000000000ull) return X_NONFINITE;
+  int e = 0;
+  if (mx) frexp(__longlong_as_double((long long)mx), &e); /* v = f 2^e, f in [0.5, 1) */
+  return e;
+}
+
+/*
+ * The slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
+ * narrow): N = rint(x 2^F) from the double's mantissa and exponent (round half to even), F = 40
+ * with S = 4 slices of 10 bits, 59 with 5 of 12, then balanced digits from the bottom: all but
+ * the first in [-2^(b-1), 2^(b-1) - 1], d_0 = the rest (at most 1024 = 2^(40-30) or
+ * 2048 = 2^(59-48) since |N| <= 2^F), so that x = sum_t d_t 2^(b(S-1-t) - F) + O(2^-F-1).
+ */
+/* z 2^(e - 40), rounded once: what k_panel_combine<4> makes of the slices' sums */
+__device__ __forceinline__ double x_scaled(long long z, int e)
+{
+  const double v = __ll2double_rn(z);
+  if (e > -900 && e < 900) return v * __longlong_as_double((long long)(e - 40 + 1023) << 52);
+  return ldexp(v, e - 40);
+}
+
 /*
  * codes: rows of ldc bytes (2-bit codes, MSB first, 3 = missing -> 0); output row r reads
  * code row row_map[r] (r itself when row_map is NULL); its k-block kb is the 16 bytes at
  * (kb % kb_period)*16, taken as allele counts or as the observed mask by count_lo for kb <
  * kb_period and count_hi otherwise (the concatenated-k form [G | O]).  tn: slice columns per tile; nct column tiles.
  * sums: per row tile, slice column (nct * tn of them) and row of the tile the exact integer
- * sum, added atomically.
+ * sum, added atomically.  With Y (ksplit 1 and 4 slices) the item that has all of a row's sums
+ * writes the products themselves, Y[row][column] by mx, the columns' largest magnitudes: the
+ * slices' sums make one 64-bit integer, kept in Y's place between chunks.  No buffer of sums
+ * is cleared, added to and read again (200,000 x 20 products over 5,000 samples: 0.40 -> 0.30 ms).
  */
 __global__ void __launch_bounds__(X_THREADS, 1)
 k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restrict__ codes,
                 int64_t ldc, const int32_t *__restrict__ row_map, int32_t nrows, int32_t tn,
                 int32_t nct, int32_t nkb, int32_t kb_period, int count_lo, int count_hi,
-                int32_t ksplit, int32_t chunk_kb, unsigned long long *sums, int *err,
-                const gp_tc_batch *db)
+                int32_t ksplit, int32_t chunk_kb, unsigned long long *sums,
+                const unsigned long long *__restrict__ mx, double *Y, int64_t ldy, int32_t ncols,
+                int *err, const gp_tc_batch *db)
 {
   if (db) {
     /* a device-resident loop's batch: rows and their count are read at run time */
@@ -306,7 +337,26 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
           break;
         }
         tc_fence_after();
-        if (any)
+        if (any && Y) {
+          const bool first = c0 == kb0, last = c0 + chunk_kb >= kb1;
+          double *yr = Y + (int64_t)(rt * XR + row) * ldy;
+          for (int g = 0; g < tn; g += 16) {
+            uint32_t f[16];
+            tmem_ld16(t_acc + g, f);
+            tmem_wait_ld();
+#pragma unroll
+            for (int v = 0; v < 16; v += 4) {
+              const int32_t c = (ct * tn + g + v) >> 2;
+              if (!live || c >= ncols) continue;
+              long long z = 0;
+#pragma unroll
+              for (int t = 0; t < 4; ++t)
+                z = (z << 10) + __float2int_rn(__uint_as_float(f[v + t]) * 0x1p24f);
+              if (!first) z += __double_as_longlong(yr[c]);
+              yr[c] = last ? x_scaled(z, x_exponent<4>(__ldg(mx + c))) : __longlong_as_double(z);
+            }
+          }
+        } else if (any)
           for (int g = 0; g < tn; g += 16) {
             uint32_t f[16];
             tmem_ld16(t_acc + g, f);
@@ -571,23 +621,6 @@ __global__ void k_panel_absmax(const x_panels pan, int32_t nk, int32_t ncols,
 /* exponent e_c with max|P| < 2^e_c (frexp) of a column's mx, 0 for an all-zero column; with 5
  * slices X_NONFINITE for one with an infinity or NaN (its products are NaN, as FP64 products of
  * 0 and it are) */
-#define X_NONFINITE (-(1 << 30))
-template <int S>
-__device__ __forceinline__ int x_exponent(unsigned long long mx)
-{
-  if (S == 5 && mx >= 0x7FF0000000000000ull) return X_NONFINITE;
-  int e = 0;
-  if (mx) frexp(__longlong_as_double((long long)mx), &e); /* v = f 2^e, f in [0.5, 1) */
-  return e;
-}
-
-/*
- * The slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
- * narrow): N = rint(x 2^F) from the double's mantissa and exponent (round half to even), F = 40
- * with S = 4 slices of 10 bits, 59 with 5 of 12, then balanced digits from the bottom: all but
- * the first in [-2^(b-1), 2^(b-1) - 1], d_0 = the rest (at most 1024 = 2^(40-30) or
- * 2048 = 2^(59-48) since |N| <= 2^F), so that x = sum_t d_t 2^(b(S-1-t) - F) + O(2^-F-1).
- */
 template <int S>
 __device__ __forceinline__ void slice(double v, int e, bool neg, int d[S])
 {
@@ -909,22 +942,27 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   if (nrows < 1) return GP_OK;
   if (A->k0 != P->k0 || A->ldc < (int64_t)P->kb0 * XK / 4)
     return gp_fail(ctx, GP_ERR_ARG, "gp_tc_apply: code operand and panel disagree");
-  const size_t sum_bytes = gp_tc_sum_bytes(P->digits * P->ncols, nrows);
-  unsigned long long *sums;
-  int rc = gp_scratch5(ctx, sum_bytes + 256, (void **)&sums);
-  if (rc) return rc;
-  GP_CUDA(ctx, cudaMemsetAsync(sums, 0, sum_bytes, ctx->stream));
-  GP_CUDA(ctx, cudaFuncSetAttribute(k_geno_panel_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    X_SMEM));
   const int32_t nkb = P->kb0 * P->npanels;
   const int32_t tiles = (nrows + XR - 1) / XR * P->nct;
   const int32_t ksplit = x_split(tiles, nkb, ctx->num_sms);
+  const bool whole = ksplit == 1 && P->digits == 4;
+  unsigned long long *sums = NULL;
+  if (!whole) {
+    const size_t sum_bytes = gp_tc_sum_bytes(P->digits * P->ncols, nrows);
+    int rc = gp_scratch5(ctx, sum_bytes + 256, (void **)&sums);
+    if (rc) return rc;
+    GP_CUDA(ctx, cudaMemsetAsync(sums, 0, sum_bytes, ctx->stream));
+  }
+  GP_CUDA(ctx, cudaFuncSetAttribute(k_geno_panel_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    X_SMEM));
   const int32_t nitems = tiles * ksplit;
   const int grid = nitems < ctx->num_sms ? nitems : ctx->num_sms;
   k_geno_panel_tc<<<grid, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->count_lo, P->count_hi,
-      ksplit, X_CHUNK_KB(P->digits), sums, ctx->d_err, NULL);
+      P->tmb, A->codes, A->ldc, A->row_map, nrows, P->tn, P->nct, nkb, P->kb0, P->count_lo,
+      P->count_hi, ksplit, X_CHUNK_KB(P->digits), sums, P->mx, whole ? d_Y : NULL, ldy, P->ncols,
+      ctx->d_err, NULL);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
+  if (whole) return GP_OK;
   (P->digits == 5 ? k_panel_combine<5> : k_panel_combine<4>)
       <<<combine_grid(ctx, nrows, P->ncols), 256, 0, ctx->stream>>>(
           sums, P->nct * P->tn, nrows, P->ncols, P->mx, d_Y, ldy, NULL);
@@ -956,8 +994,8 @@ int gp_tc_apply_dev(gp_ctx *ctx, const gp_tc_batch *db, int32_t max_rows, int64_
                                     X_SMEM));
   /* every SM: the kernel takes the batch's row count, and with it its work items, from db */
   k_geno_panel_tc<<<ctx->num_sms, X_THREADS, X_SMEM, ctx->stream>>>(
-      P->tmb, NULL, ldc, NULL, 0, P->tn, P->nct, P->kb0 * P->npanels, P->kb0, P->count_lo, P->count_hi,
-      1, X_CHUNK_KB(4), z, ctx->d_err, db);
+      P->tmb, NULL, ldc, NULL, 0, P->tn, P->nct, P->kb0 * P->npanels, P->kb0, P->count_lo,
+      P->count_hi, 1, X_CHUNK_KB(4), z, NULL, NULL, 0, 0, ctx->d_err, db);
   GP_LAUNCH_CHECK(ctx, "k_geno_panel_tc");
   k_panel_combine<4><<<combine_grid(ctx, max_rows, P->ncols), 256, 0, ctx->stream>>>(
       z, wcols, 0, P->ncols, P->mx, d_Y, ldy, db);
