@@ -16,8 +16,7 @@ read-back are inside the timed region.
 smartpca, restated in oracle/smartpca_oracle.c) on the host cores with all threads over a
 bounded SNP sample of the same workload, in the same unit.
 
-One GPU only: the path does not shard (one PCA per panel) and the split Gram's cluster
-schedule multicasts its TMA loads within this GPU's own memory, so the GPU arm refuses
+One GPU only: the path does not shard (one PCA per panel), so the GPU arm refuses
 --gpus N > 1 and a torchrun launch with WORLD_SIZE > 1: rank 0 prints one JSON line with an
 "unavailable" reason and every rank exits 0 without touching a GPU.  The reference arm (CPU)
 runs on rank 0 alone; the other ranks exit 0 without work.
@@ -872,13 +871,13 @@ def tridiag_roofline(res, peaks, peak_kind):
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": tridiag_traffic(n),
             "kernel": "k_tridiag_tiled (float-float Householder tridiagonalisation, order %d, "
-                      "one cooperative launch: lower-triangle tiles while the trailing order "
-                      "exceeds 2,500, then whole columns; %.1f ms by CUDA events)" % (n, ms),
+                      "lower-triangle tiles until the rest fits the shared memories, then "
+                      "k_tridiag_smem; %.1f ms by CUDA events for both)" % (n, ms),
             "algorithmic_bytes": alg,
             "note": "DRAM traffic is below the algorithmic bytes: the tiled lower triangle "
                     "(103 MB at N=5,000) mostly stays in L2; the tiled steps are bound by "
-                    "the per-step chain of phase A, part sums and the grid barrier, and FP32-pipe "
-                    "issue (~62 instructions per lower-triangle element and step)",
+                    "the FP32 pipe (53 operations per lower-triangle element and step) and "
+                    "a step's chain of phase A, part sums and the grid barrier",
             "peak_kind": "HBM copy, %s" % peak_kind}
 
 
@@ -935,8 +934,7 @@ def main():
               "l2": "inputs larger than L2 (packed panel %.0f MB)" % (
                   cfg["nsnp"] * max((nind + 3) // 4, 48) / 1e6)}
     if args.impl == "gpu" and world > 1:
-        # one GPU only: no multi-GPU path exists (and the split Gram's cluster schedule must not
-        # run in a multi-GPU process group); nothing touches a GPU here
+        # one GPU only: no multi-GPU path exists; nothing touches a GPU here
         if rank == 0:
             print(json.dumps({"metric": METRIC, "n_gpus": world, "impl": "gpu",
                               "unavailable": "one GPU only: smartpca's path runs one PCA per "
