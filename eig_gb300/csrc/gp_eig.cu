@@ -1418,17 +1418,22 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
  * block has about the same number of parts).  So the product's index block K (TT indices)
  * has pc row-part contributors (blocks (rg(K), *)) and, for each of its units, pr column-part
  * contributors (blocks (*, cg(u))).  Per step:
- *   A   every block: the pending w of step c-1 from its y, the pending update of column c read
- *       from the tiles, its norm, the reflector; y.v from the index blocks' partial dots.  v of
- *       step c-1 is still in shared memory
+ *   A   every block: y of step c-1, the index blocks' partial dots y.v and column c are polled for
+ *       as tagged values (tag_store); the pending w of step c-1, the pending update of column c,
+ *       its norm, the reflector.  v of step c-1 is still in shared memory
  *   B   each warp takes parts of the block: the pending rank-2 update of step c-1 (written
  *       back), the row dots (two rows per lane) and, off the diagonal, the column dots (a
- *       reduce-scatter over the warp per 8 columns); the block sums its parts per tile row and
+ *       reduce-scatter over the warp per 8 columns), and column c + 1 published as it is then; the
+ *       block sums its parts per tile row and
  *       per column unit in a fixed order and publishes them, one arrival (release) on the
  *       index block's counter per published sum; block K mod G waits (acquire, bounded) for
  *       index block K's pc + (TT/TT_U)*pr arrivals and sums them in a fixed order into y and
- *       the index block's partial y.v
- *   --- grid barrier
+ *       the index block's partial y.v, published
+ * No barrier over the blocks in a step: every index block's sums have a contribution of every
+ * block of its row group and of its units' column groups, so a block starts step c only when
+ * every block has published its sums of step c-1 and with that has read all of step c-2: two
+ * buffers suffice, and the arrival counters never mix steps.  A grid barrier stands where the tiles
+ * change hands (every TT steps) and where a block could have no tile row (see there).
  * Rows and columns up to c keep their values (the pending-update vectors and v are zero there),
  * so that phase A of a block still reading column c never sees it change.  Every sum has a
  * fixed order.
@@ -1437,11 +1442,12 @@ k_tridiag(double *A, int n, int c_end, double *d, double *e, double *tau, double
  * Packed over two columns the operations take half the slots, and with 16 warps instead of 32 the
  * registers hold the next columns while these are worked on (parts of an early step of order
  * 5,000: 69,000 -> 52,000 clocks; 20 and 24 warps spill and are slower).  The chain around them,
- * some 30,000 clocks a step, is A (14,000: y and the column of every block from L2, then the
- * vectors, packed too), the sums, the arrivals and their wait (10,000), the terms of y, all read
- * before any is added (3,000), and the grid barrier (4,000).  Order 5,000: 114 -> 100 ms; 3,600:
- * 57 -> 52.  Down to the order that fits shared memory these steps beat whole columns (2,500:
- * 28.4 -> 26.5 ms), which remain for orders whose vectors leave no room for the slots.
+ * some 25,000 clocks a step, is A (14,000: y and the column of every block from L2, then the
+ * vectors, packed too), the sums, the arrivals and their wait (10,000) and the terms of y, all read
+ * before any is added (3,000).  With a grid barrier in every step and the column read from the tiles
+ * order 5,000 took 98.8 ms, now 92.5 (3,600: 50.2 -> 46.9, 2,500: 25.5 -> 24.2), 114 before the packed
+ * pairs.  Down to the order that fits shared memory these steps beat whole columns (2,500: 28.4 ms),
+ * which remain for orders whose vectors leave no room for the slots.
  */
 #define TT 64
 #define TT_U 16                /* columns per column unit */
@@ -1498,6 +1504,47 @@ __device__ __forceinline__ ff2 tt_scatter8(pf2 *cp, int lane)
   return ff_renorm(ff_add_lazy(r, ff_shfl_xor(r, 1)));
 }
 
+/*
+ * y and the column at the indices q + u TT_THREADS (u < TT_POLL, below npad) into sy and sx: tagged
+ * values, all the loads of a round in flight together, a round asking for what is missing only.
+ * False when the wait ran out or another block gave up.
+ */
+#define TT_POLL 2 /* indices a thread polls for at a time: 1 took 96 ms, 3 106 (spills), 2 92.5 */
+__device__ __forceinline__ bool tt_wait(const uint4 *yt, const uint4 *ct, int q, int npad,
+                                        unsigned ytag, unsigned ctag, double *sy, double *sx,
+                                        int *err)
+{
+  unsigned need = 0;
+#pragma unroll
+  for (int u = 0; u < TT_POLL; ++u)
+    if (q + u * TT_THREADS < npad) need |= 3u << (2 * u);
+  uint64_t t0 = 0;
+  for (unsigned it = 0; need; ++it) {
+    uint4 r[2 * TT_POLL];
+#pragma unroll
+    for (int k = 0; k < 2 * TT_POLL; ++k)
+      if (need & (1u << k)) r[k] = tag_load((k & 1 ? ct : yt) + q + (k >> 1) * TT_THREADS);
+#pragma unroll
+    for (int k = 0; k < 2 * TT_POLL; ++k) {
+      const unsigned tag = k & 1 ? ctag : ytag;
+      if ((need & (1u << k)) && r[k].y == tag && r[k].w == tag) {
+        pv_put(k & 1 ? sx : sy, q + (k >> 1) * TT_THREADS,
+               ff_make(__uint_as_float(r[k].x), __uint_as_float(r[k].z)));
+        need &= ~(1u << k);
+      }
+    }
+    if (it == 0) t0 = globaltimer_ns();
+    if ((it & 63u) == 63u) {
+      if (*(volatile int *)err) return false;
+      if (globaltimer_ns() - t0 > GP_WAIT_NS) {
+        atomicExch(err, TR_ERR_WAIT);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
 /* two pairs of columns of the lane's rows (lane, lane + 32), from the first pair's address */
 __device__ __forceinline__ void tt_load(pf2 a[2][2], const double *p0)
 {
@@ -1515,7 +1562,7 @@ __device__ __forceinline__ void tt_load(pf2 a[2][2], const double *p0)
  * read while these are worked on. */
 #define TT_H 8
 __device__ __forceinline__ void tt_halves(double *Tm, const int4 *items, int h0, int h1, int seg,
-                                          int dead, const double *svp, const double *swp,
+                                          int dead, uint4 *cnext, const double *svp, const double *swp,
                                           const double *svc, double *rseg, double *cslot, int lane)
 {
   if (h0 >= h1) return;
@@ -1563,6 +1610,11 @@ __device__ __forceinline__ void tt_halves(double *Tm, const int4 *items, int h0,
           const pf2 a1 = pf_sub2prod(a[k][1], pr1, wpc, wpn, qr1, vpc, vpn);
           pv_store(p0 + (size_t)(cb + k) * (2 * TT), 0, a0);
           pv_store(p0 + (size_t)(cb + k) * (2 * TT), 32, a1);
+          if (p == dead >> 1) { /* the next step's column */
+            const int r = I * TT + lane;
+            tag_store(cnext + r, dead & 1 ? pf_odd(a0) : pf_even(a0), (unsigned)dead + 1u);
+            tag_store(cnext + r + 32, dead & 1 ? pf_odd(a1) : pf_even(a1), (unsigned)dead + 1u);
+          }
           ra0 = pf_acc_lazy(ra0, a0, vc, vn);
           ra1 = pf_acc_lazy(ra1, a1, vc, vn);
           cp[cb + k] = pf_dot2(a0, vr0, a1, vr1);
@@ -1611,8 +1663,8 @@ __host__ __device__ inline size_t tt_smem_bytes(int nt, int maxr, int maxc, int 
 __global__ void __launch_bounds__(TT_THREADS, 1)
 k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, int maxc,
                 int maxi, int cs, const unsigned char *rgt, const unsigned char *cgt,
-                double *d, double *e, double *tau, double *yb, double *xlast, double *ylast,
-                double *prow, double *pcol, double *dotp, unsigned *kcnt, unsigned *bar, int *err,
+                double *d, double *e, double *tau, uint4 *yt, uint4 *ct, uint4 *dott,
+                double *xlast, double *ylast, double *prow, double *pcol, unsigned *kcnt, unsigned *bar, int *err,
                 unsigned long long *phase_ns, tr_state *state)
 {
   extern __shared__ double sh[];
@@ -1637,7 +1689,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
   __shared__ int s_seg[TT_WARPS]; /* each warp's first row slot */
   const int G = gridDim.x, b = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool active = b < pr * pc;
+  const bool active = b < pr * pc, all = G == pr * pc;
   const int ga = active ? b / pc : 0, gb = active ? b - (b / pc) * pc : 0;
   const ff2 ONE = ff_make(1.f, 0.f), ZERO = ff_make(0.f, 0.f);
   unsigned *count = bar;
@@ -1725,35 +1777,45 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
       svc = t;
     }
     const ff2 tau_pf = s_tau_p, e_pf = s_e_p;
-    double *ycur = yb + (size_t)(c & 1) * npad;
-    const double *yprev = yb + (size_t)((c + 1) & 1) * npad;
+    uint4 *ycur = yt + (size_t)(c & 1) * npad;
+    const uint4 *yprev = yt + (size_t)((c + 1) & 1) * npad, *ccur = ct + (size_t)(c & 1) * npad;
     const int p0 = c / 2, odd = c & 1, np = npad / 2;
-    ff2 pacc = ZERO;
-    if (warp == TT_WARPS - 1) {
-      /* y.v of step c-1: its index blocks' partial dots (from (c-1+1)/TT on), in order */
-      const double *pprev = dotp + (size_t)((c + 1) & 1) * nt;
-      for (int k = c / TT + lane; k < nt; k += 32) pacc = ff_add(pacc, ff_load(pprev + k));
-    }
-    {
-      const int Jc = c / TT, kc = (c - Jc * TT) / 2;
-#pragma unroll 4
-      for (int p = p0 + threadIdx.x; p < np; p += TT_THREADS) {
+    bool fail = false;
+    if (c == 0) {
+      for (int p = threadIdx.x; p < np; p += TT_THREADS) {
         const int q = 2 * p, I = q / TT;
-        const float4 *a = reinterpret_cast<const float4 *>(Tm + tt_tile(I, Jc) * (TT * TT)) +
-                          kc * TT + (q - I * TT);
-        const float4 a0 = a[0], a1 = a[1];
-        const pf2 y = pv_load(yprev, p);
-        pv_store(svc, p, pf_make(f2_make(odd ? a0.y : a0.x, odd ? a1.y : a1.x),
-                                 f2_make(odd ? a0.w : a0.z, odd ? a1.w : a1.z)));
-        pv_store(swp, p, y);
-        if (p == p0) s_yc = odd ? pf_odd(y) : pf_even(y);
+        const double *a = Tm + tt_tile(I, 0) * (TT * TT) + 2 * (q - I * TT);
+        pv_store(svc, p, pf_join(pf_even(pv_load(a, 0)), pf_even(pv_load(a, 1))));
+        pv_store(swp, p, pf_make(0, 0));
+      }
+      if (threadIdx.x == 0) s_yc = s_slotf = ZERO;
+    } else {
+      for (int q = 2 * p0 + threadIdx.x; q < npad && !fail; q += TT_POLL * TT_THREADS)
+        fail = !tt_wait(yprev, ccur, q, npad, (unsigned)c, (unsigned)c + 1u, swp, svc, err);
+      if (threadIdx.x == (unsigned)odd) s_yc = pv_get(swp, c); /* its own store */
+      if (warp == TT_WARPS - 1) {
+        /* y.v of step c-1: its index blocks' partial dots (from (c-1+1)/TT on), in order */
+        const uint4 *dprev = dott + (size_t)((c + 1) & 1) * nt;
+        ff2 pacc = ZERO;
+        for (int k = c / TT + lane; k < nt && !fail; k += 32) {
+          uint4 r = tag_load(dprev + k);
+          const uint64_t t0 = globaltimer_ns();
+          for (unsigned it = 1; r.y != (unsigned)c || r.w != (unsigned)c; ++it) {
+            if ((it & 63u) == 0 &&
+                (*(volatile int *)err || globaltimer_ns() - t0 > GP_WAIT_NS)) {
+              atomicCAS(err, 0, TR_ERR_WAIT);
+              fail = true;
+              break;
+            }
+            r = tag_load(dprev + k);
+          }
+          pacc = ff_add(pacc, ff_make(__uint_as_float(r.x), __uint_as_float(r.z)));
+        }
+        for (int o = 16; o; o >>= 1) pacc = ff_add(pacc, ff_shfl_xor(pacc, o));
+        if (lane == 0) s_slotf = pacc;
       }
     }
-    if (warp == TT_WARPS - 1) {
-      for (int o = 16; o; o >>= 1) pacc = ff_add(pacc, ff_shfl_xor(pacc, o));
-      if (lane == 0) s_slotf = pacc;
-    }
-    __syncthreads();
+    if (__syncthreads_or(fail)) return;
     {
       const ff2 alpha_pf = ff_scale(ff_mul(ff_mul(tau_pf, tau_pf), s_slotf), -0.5f);
       const ff2 wpc = ff_fma(tau_pf, s_yc, alpha_pf);
@@ -1836,7 +1898,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
     const int nr = s_nr, nc = s_nc, ni = s_ni;
     __syncthreads();
     tt_halves(Tm, items, 2 * ni * warp / TT_WARPS, 2 * ni * (warp + 1) / TT_WARPS, s_seg[warp],
-              c + 1, svp, swp, svc, rseg, cslot, lane);
+              c + 1, ct + (size_t)((c + 1) & 1) * npad, svp, swp, svc, rseg, cslot, lane);
     __syncthreads();
     /* the block's sums, in part order: row parts of its tile rows, column parts of its units
      * (tile row kr's k-th unit is part rowb[kr] + k); then one arrival per published sum on its
@@ -1912,7 +1974,7 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
         const int q = K * TT + i;
         ff2 dv = ZERO;
         if (g == 0) {
-          pv_put(ycur, q, y);
+          tag_store(ycur + q, y, (unsigned)c + 1u);
           dv = ff_mul(y, pv_get(svc, q));
         }
         /* the warp's four indices, lanes 0, 8, 16 and 24 */
@@ -1923,18 +1985,24 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
         if (threadIdx.x < 32) {
           ff2 t = lane < TT_WARPS ? s_dot[lane] : ZERO;
           for (int o = 16; o; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
-          if (threadIdx.x == 0) ff_store(dotp + (size_t)(c & 1) * nt + K, t);
+          if (threadIdx.x == 0) tag_store(dott + (size_t)(c & 1) * nt + K, t, (unsigned)c + 1u);
         }
         __syncthreads();
       }
     }
     TT_STAMP(c < early ? 2 : 1)
-    if (threadIdx.x == 0) { /* read again only after the grid barrier's block barriers */
+    if (threadIdx.x == 0) { /* read again only after the barrier below */
       s_tau_p = tau_c;
       s_e_p = beta;
     }
-    target += G;
-    if (!tr_grid_sync(count, target, err)) return;
+    /* a grid barrier only where the tiles change hands, at the end, and where a block might have
+     * no sum to publish in the next two steps (it could then fall behind by more than a buffer) */
+    if ((c + 2) / TT != J0 || c == cs - 1 || !all || nt - (c + 3) / TT < pr) {
+      target += G;
+      if (!tr_grid_sync(count, target, err)) return;
+    } else {
+      __syncthreads(); /* the scalars; the vectors are rewritten from here on */
+    }
     TT_STAMP(4)
   }
   /* the trailing block (indices >= cs) of the block's parts into A as float-float pairs, both
@@ -1956,7 +2024,8 @@ k_tridiag_tiled(double *A, double *Tm, int n, int nt, int pr, int pc, int maxr, 
   }
   for (int q = cs + b * TT_THREADS + threadIdx.x; q < n; q += G * TT_THREADS) {
     ff_store(xlast + q, pv_get(svc, q));
-    ff_store(ylast + q, pv_get(yb + (size_t)((cs + 1) & 1) * npad, q));
+    const uint4 y = tag_load(yt + (size_t)((cs + 1) & 1) * npad + q);
+    ff_store(ylast + q, ff_make(__uint_as_float(y.x), __uint_as_float(y.z)));
   }
   if (stamp)
     for (int i = 0; i < 5; ++i) phase_ns[i] = s_ph[i];
@@ -2707,15 +2776,16 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       const int64_t ntiles = (int64_t)nt * (nt + 1) / 2;
       const size_t tile_d = (size_t)ntiles * TT * TT;
       const size_t part_d = (size_t)(tt_pr + tt_pc) * nt * TT; /* prow + pcol */
-      const size_t yb_d = 2 * (size_t)nt * TT, zero_d = yb_d + 2 * (size_t)nt;
-      const size_t tri_bytes = sizeof(double) * (tile_d + part_d + zero_d) +
+      const size_t tags = 4 * (size_t)nt * TT + 2 * (size_t)nt; /* y, columns, dots, twice */
+      const size_t tri_bytes = sizeof(double) * (tile_d + part_d) + sizeof(uint4) * tags +
                                sizeof(unsigned) * (size_t)nt;
       int rc2 = gp_realloc(ctx, (void **)&ctx->d_tri, tri_bytes);
       if (rc2) return rc2;
       double *Tm = ctx->d_tri, *prow = Tm + tile_d, *pcol = prow + (size_t)nt * tt_pc * TT;
-      double *yb = pcol + (size_t)nt * tt_pr * TT, *dotp = yb + yb_d;
-      unsigned *kcnt = (unsigned *)(dotp + 2 * (size_t)nt);
-      GP_CUDA(ctx, cudaMemsetAsync(yb, 0, sizeof(double) * zero_d + sizeof(unsigned) * (size_t)nt,
+      uint4 *yt = (uint4 *)(pcol + (size_t)nt * tt_pr * TT), *ct = yt + 2 * (size_t)nt * TT;
+      uint4 *dott = ct + 2 * (size_t)nt * TT;
+      unsigned *kcnt = (unsigned *)(dott + 2 * (size_t)nt);
+      GP_CUDA(ctx, cudaMemsetAsync(yt, 0, sizeof(uint4) * tags + sizeof(unsigned) * (size_t)nt,
                                    ctx->stream));
       int blocks = (int)std::min<int64_t>(ntiles, (int64_t)ctx->num_sms * 8);
       k_tri_to_tiles<<<blocks, 256, 0, ctx->stream>>>(A_in, n, nt, Tm);
@@ -2724,8 +2794,8 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
       const unsigned char *rgt = ctx->d_tt, *cgt = ctx->d_tt + (size_t)nt * nt;
       void *args[] = {&A,       &Tm,   &nn,    &nt_,   &tt_pr, &tt_pc, &tt_maxr, &tt_maxc,
                       &tt_maxi, &cs,   &rgt,   &cgt,   &d,     &e,     &tau,
-                      &yb,      &xlast, &ylast, &prow, &pcol,  &dotp,  &kcnt,    &bar,
-                      &d_err,   &phase, &state};
+                      &yt,      &ct,   &dott,  &xlast, &ylast, &prow,  &pcol,    &kcnt,
+                      &bar,     &d_err, &phase, &state};
       GP_CUDA(ctx, cudaEventRecord(ctx->ev_tr0, ctx->stream));
       GP_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_tridiag_tiled, dim3((unsigned)G),
                                                dim3(TT_THREADS), args, tt_smem, ctx->stream));
