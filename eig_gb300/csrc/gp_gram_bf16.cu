@@ -35,7 +35,7 @@
  *
  * What bounds it is the shared memory's 128 bytes a clock: a 128x128x16 MMA reads 8 KB, so the 12
  * MMAs of a k-block read 96 KB and its boxes' 64 KB come in: 1,250 clocks, against 768 of tensor
- * work; measured 1,285 (5,000 x 600,000 in split fp16: 35.7 ms with the transpose, 43.4 before the
+ * work; measured 1,285 (5,000 x 600,000 in split fp16: 34.6 ms with the transpose, 43.4 before the
  * warp-wide issue, the k-block layout and the parts).  The pieces of the running sums fill the
  * TMEM, so a CTA's tile cannot be larger.  Tried and not kept: pairs of CTAs (cta_group::2,
  * 256x128, 120 KB a k-block) wait for one another's barriers, 1,430 clocks (1,000 with the loads
@@ -460,15 +460,19 @@ __global__ void k_split_tables(const int32_t *kept, int32_t nkept, const double 
 #define MT_SNP 64
 #define MT_ROWS 256
 #define MT_SPAN 256
-#define MT_PITCH_W (MT_SPAN / 4 + 1) /* 65 words: rows one bank apart */
+/* shared-memory words of SNP u: a warp's lanes ask for the SNPs 8 g + k, g = 0 .. 7, and four rows;
+ * with 65 words and 4 table entries a SNP two of them shared a bank in the records and all eight
+ * in the table (5,000 x 150,000: 0.89 ms, now 0.62, 5 TB/s) */
+#define MT_REC(u) ((u) * (MT_SPAN / 4 + 1) + ((u) >> 5) * 4)
+#define MT_TAB(u) ((u) * 4 + ((u) >> 3) * 4)
 __global__ void __launch_bounds__(256)
 k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t *__restrict__ rows,
                   int32_t nrows, const int32_t *__restrict__ cols, const int32_t *__restrict__ kept,
                   int32_t nkept, const uint32_t *__restrict__ split, int32_t k0, int32_t npad,
                   __nv_bfloat16 *xhi, __nv_bfloat16 *xlo)
 {
-  __shared__ uint32_t srec[MT_SNP][MT_PITCH_W];
-  __shared__ uint32_t stab[MT_SNP][4];
+  __shared__ uint32_t srec[MT_REC(MT_SNP)];
+  __shared__ uint32_t stab[MT_TAB(MT_SNP)];
   __shared__ int64_t srecoff[MT_SNP];
   const int tid = threadIdx.x;
   const int32_t kt = blockIdx.x, r0 = blockIdx.y * MT_ROWS;
@@ -487,7 +491,7 @@ k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
   {
     const int u = tid >> 2, g = tid & 3;
     const int32_t k = kbase + u;
-    stab[u][g] = k < nkept ? __ldg(split + 4 * k + g) : 0u;
+    stab[MT_TAB(u) + g] = k < nkept ? __ldg(split + 4 * k + g) : 0u;
   }
   __syncthreads();
   if (fast && span > 0) {
@@ -496,10 +500,11 @@ k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
       const int u = i / nvec, v = i - u * nvec;
       uint4 val = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
       if (srecoff[u] >= 0) val = __ldg((const uint4 *)(geno + srecoff[u] + base + 16 * v));
-      srec[u][4 * v] = val.x;
-      srec[u][4 * v + 1] = val.y;
-      srec[u][4 * v + 2] = val.z;
-      srec[u][4 * v + 3] = val.w;
+      uint32_t *dst = srec + MT_REC(u) + 4 * v;
+      dst[0] = val.x;
+      dst[1] = val.y;
+      dst[2] = val.z;
+      dst[3] = val.w;
     }
   }
   __syncthreads();
@@ -517,10 +522,10 @@ k_split_transpose(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
         const int uu = g8 * 8 + u;
         uint32_t byte;
         if (fast)
-          byte = (srec[uu][b >> 2] >> ((b & 3) * 8)) & 0xFFu;
+          byte = (srec[MT_REC(uu) + (b >> 2)] >> ((b & 3) * 8)) & 0xFFu;
         else
           byte = srecoff[uu] >= 0 ? __ldg(geno + srecoff[uu] + (sidx >> 2)) : 0xFFu;
-        const uint32_t pair = stab[uu][(byte >> sh) & 3u];
+        const uint32_t pair = stab[MT_TAB(uu) + ((byte >> sh) & 3u)];
         hv[u >> 1] |= (pair & 0xFFFFu) << ((u & 1) * 16);
         lv[u >> 1] |= (pair >> 16) << ((u & 1) * 16);
       }
