@@ -35,7 +35,7 @@
  *
  * What bounds it is the shared memory's 128 bytes a clock: a 128x128x16 MMA reads 8 KB, so the 12
  * MMAs of a k-block read 96 KB and its boxes' 64 KB come in: 1,250 clocks, against 768 of tensor
- * work; measured 1,285 (5,000 x 600,000 in split fp16: 34.6 ms with the transpose, 43.4 before the
+ * work; measured 1,285 (5,000 x 600,000 in split fp16: 35.0 ms with the transpose, 43.4 before the
  * warp-wide issue, the k-block layout and the parts).  The pieces of the running sums fill the
  * TMEM, so a CTA's tile cannot be larger.  Tried and not kept: pairs of CTAs (cta_group::2,
  * 256x128, 120 KB a k-block) wait for one another's barriers, 1,430 clocks (1,000 with the loads
