@@ -50,6 +50,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
+#include <limits.h>
 #include <math.h>
 
 #include "gp_geno_tc.h"
@@ -396,7 +397,8 @@ k_geno_panel_tc(const __grid_constant__ CUtensorMap tm_b, const uint8_t *__restr
  * row stride ldc bytes; pad k (>= nk) and pad rows are 3.  A transpose through shared
  * memory: CTA (kt, rt) covers 128 kept SNPs x 128 rows; when the rows' samples span at most
  * CB_SPAN record bytes, the 128 records' byte ranges are read once (coalesced), and two
- * threads build each row's 32 output bytes; wider spans read per thread.
+ * threads build each row's 32 output bytes; wider spans read per thread.  The samples may come
+ * in any order and repeat, so the span is that of the least and the greatest of them.
  */
 #define CB_SNP 128
 #define CB_ROWS 128
@@ -409,18 +411,26 @@ k_codes_by_sample(const uint8_t *__restrict__ geno, int64_t rlen, const int32_t 
 {
   __shared__ uint32_t srec[CB_SNP][CB_PITCH_W];
   __shared__ int64_t soff[CB_SNP];
+  __shared__ int32_t win[2]; /* the rows' first and last record byte */
   const int tid = threadIdx.x;
   const int32_t r0 = blockIdx.y * CB_ROWS;
-  int32_t base = 0, span = 0;
-  if (r0 < nsamp) {
-    const int32_t rl = (r0 + CB_ROWS < nsamp ? r0 + CB_ROWS : nsamp) - 1;
-    base = (samp[r0] >> 2) & ~15;
-    span = (samp[rl] >> 2) - base + 1;
-  }
-  const bool fast = span <= CB_SPAN;
   const int rl = tid >> 1, half = tid & 1;
   const int32_t r = r0 + rl;
   const int32_t sidx = r < nsamp ? samp[r] : 0;
+  if (tid == 0) {
+    win[0] = INT_MAX;
+    win[1] = -1;
+  }
+  __syncthreads();
+  const int32_t first = __reduce_min_sync(0xffffffffu, r < nsamp ? sidx >> 2 : INT_MAX);
+  const int32_t last = __reduce_max_sync(0xffffffffu, r < nsamp ? sidx >> 2 : -1);
+  if ((tid & 31) == 0) {
+    atomicMin(&win[0], first);
+    atomicMax(&win[1], last);
+  }
+  __syncthreads();
+  const int32_t base = win[1] < 0 ? 0 : win[0] & ~15, span = win[1] < 0 ? 0 : win[1] - base + 1;
+  const bool fast = span <= CB_SPAN;
   /* the CTA walks the SNP tiles of its row block (grid-stride over x) */
   const int32_t nkt = (int32_t)((ldc * 4 + CB_SNP - 1) / CB_SNP);
   for (int32_t kt = blockIdx.x; kt < nkt; kt += gridDim.x) {

@@ -167,7 +167,8 @@ int gp_snp_weights(gp_ctx *ctx, int32_t numeigs, double *ffvecs, double *fxvecs,
  * kept columns where it has a genotype, solve the masked normal equations
  * (E^T E) a = E^T r with E_sj = fxscal_j ffvecs_js and r_s = g fancy_s - xmean_s by
  * Cholesky; b_j = fxscal_j (xrow . ffvecs_j) is the orthogonal projection.
- * samples [nproj] indices into the loaded samples; acoeffs/bcoeffs [numeigs*nproj]
+ * samples [nproj] indices into the loaded samples, in any order, repeats allowed;
+ * acoeffs/bcoeffs [numeigs*nproj]
  * (coefficient j of sample q at [j*nproj+q]); nobs [nproj] observed kept SNPs;
  * status [nproj]: 0 ok, 1 = nobs <= numeigs (sample dropped, "insufficient data"),
  * 2 = not positive definite (acoeffs left untouched, as the reference keeps the previous
