@@ -407,10 +407,18 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
   }
   if (rc) return rc;
 
+  /* FP64 without population fill: exact integer sums on the tensor cores, whose scale comes back
+   * with the kill flags, in one copy */
+  const bool exact = opts->precision == GP_PREC_FP64 && ctx->npop == 0;
+  const size_t part_at = gp_killed_bytes(nc) - sizeof(double) * GP_EXACT_PARTS;
+  if (exact) {
+    rc = gp_gram_exact_max(ctx, (double *)(ctx->d_killed + part_at));
+    if (rc) return rc;
+  }
   /* kept-column list (ascending) built from the kill flags */
-  std::vector<uint8_t> hk((size_t)nc);
-  GP_CUDA(ctx, gp_memcpy(ctx, hk.data(), ctx->d_killed, (size_t)nc, cudaMemcpyDeviceToHost,
-                               ctx->stream));
+  std::vector<uint8_t> hk(exact ? gp_killed_bytes(nc) : (size_t)nc);
+  GP_CUDA(ctx, gp_memcpy(ctx, hk.data(), ctx->d_killed, hk.size(), cudaMemcpyDeviceToHost,
+                         ctx->stream));
   GP_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   std::vector<int32_t> kept;
   kept.reserve((size_t)nc);
@@ -424,16 +432,18 @@ extern "C" int gp_xtx(gp_ctx *ctx, const gp_xtx_opts *opts, int32_t *n0, int32_t
 
   GP_CUDA(ctx, cudaEventRecord(ctx->ev_g0, ctx->stream));
   ctx->gram_launches = 0;
-  /* FP64: exact integer sums on the tensor cores.  usepopsformissing's filled values are no
-   * linear function of the genotype and keep the FP64-pipe kernel, which also takes over when
-   * the device has no room for the digits of one block of SNPs. */
+  /* usepopsformissing's filled values are no linear function of the genotype and keep the
+   * FP64-pipe kernel, which also takes over when the device has no room for the digits of one
+   * block of SNPs */
   bool symmetric = false;
   if (opts->precision != GP_PREC_FP64) {
     rc = gp_gram_split(ctx, opts->precision);
   } else {
     rc = GP_ERR_NOMEM;
-    if (ctx->npop == 0 && ctx->nkept > 0) {
-      rc = gp_gram_exact(ctx);
+    if (exact && ctx->nkept > 0) {
+      double part[GP_EXACT_PARTS];
+      memcpy(part, hk.data() + part_at, sizeof part);
+      rc = gp_gram_exact(ctx, part);
       symmetric = rc == GP_OK;
     }
     if (rc == GP_ERR_NOMEM) {

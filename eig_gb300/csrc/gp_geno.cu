@@ -317,7 +317,7 @@ extern "C" int gp_set_snps(gp_ctx *ctx, const int32_t *snp_index, int32_t ncols)
       return gp_fail(ctx, GP_ERR_ARG, "gp_set_snps: snp index %d out of range", snp_index[i]);
   int rc = gp_realloc(ctx, (void **)&ctx->d_cols, sizeof(int32_t) * (size_t)ncols);
   if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_cnt, sizeof(int32_t) * 3 * (size_t)ncols);
-  if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_killed, (size_t)ncols);
+  if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_killed, gp_killed_bytes(ncols));
   if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_vtab, sizeof(double) * 4 * (size_t)ncols);
   if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_xmean, sizeof(double) * (size_t)ncols);
   if (!rc) rc = gp_realloc(ctx, (void **)&ctx->d_xfancy, sizeof(double) * (size_t)ncols);

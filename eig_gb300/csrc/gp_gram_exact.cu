@@ -14,26 +14,35 @@
  * into five balanced digits of 12 bits, integers of at most 2048 that fp16 holds exactly.  A
  * tensor-core sum of {-1, 0, 1} times such digits over at most 4,096 SNPs (both terms: at most
  * 4,096 per SNP) is an integer of at most 2^24, which the FP32 accumulator holds exactly.  The
- * digit sums of a chunk are combined into two 64-bit integers (the three upper digits, the two
+ * digit sums of a chunk are combined into two 64-bit integers (the three upper digits, the
  * lower ones) and added to the tile's sums in global memory with 64-bit integer atomics, whose
  * order does not matter: the Gram is the same whatever the tile shape, split or schedule, and
  * its error is the rounding of R (2^-53 of each value, 2^-60 of the largest) and one rounding
- * of the result, less than a sequence of FP64 additions leaves.
+ * of the result.
  *
- * What bounds it: ten fp16 products per genotype pair, i.e. the tensor pipe (GB300's FP64 pipe
- * runs at about 1/2,000 of its fp16 rate).  2,003 samples x 120,011 SNPs: 4.7 ms in all, of
+ * The scale is set by the rarest SNP (|R| up to 4 n where one allele is seen once, about 4 for
+ * common ones), so 2^(E-60) can be more than what a sequence of FP64 additions leaves, about
+ * 2^-53 sqrt(m) of a sum of m SNPs.  Then (ex_digits) six digits are cut, 71 bits below the scale,
+ * and T1 is the entry of the more frequent homozygote plus or minus f, unrounded like the
+ * products R, so that the value of most samples enters exactly.  Relative error of the Gram of
+ * 5,000 samples x 2,000 SNPs with frequencies down to 1/(2n): 8e-15 with five digits, 1.4e-15 on
+ * the FP64 pipe, 6e-17 with six.
+ *
+ * What bounds it: ten (twelve) fp16 products per genotype pair, i.e. the tensor pipe (GB300's FP64
+ * pipe runs at about 1/2,000 of its fp16 rate).  2,003 samples x 120,011 SNPs: 4.4 ms in all, of
  * 485 ms on the FP64 pipe; relative error against 64 bits 1.0e-15, of 9.3e-15.
  *
  *   k_exact_max     the largest |R| of the kept SNPs
- *   k_exact_slices  the right operand: per block of 48 samples and 64 SNPs and per term the
- *                   240 x 64 tile (digit t of sample jj in row 48 t + jj) in the 128-byte
- *                   swizzle of shared memory, stored as one contiguous piece so that a stage
- *                   of the Gram kernel is a single bulk copy
- *   k_gram_exact    256 x 48 tiles of the lower triangle, per 64 SNPs and term two
+ *   k_exact_begin   the kept SNPs' records; the sums cleared
+ *   k_exact_slices  the right operand: per block of 48 samples (40 with six digits) and 64 SNPs
+ *                   and per term the 240 x 64 tile (digit t of sample jj in row 48 t + jj) in the
+ *                   128-byte swizzle of shared memory, stored as one contiguous piece so that a
+ *                   stage of the Gram kernel is a single bulk copy
+ *   k_gram_exact    256 x 48 (40) tiles of the lower triangle, per 64 SNPs and term two
  *                   128 x 240 x 16 MMAs per k step sharing the right tile (so that it streams
  *                   at half the rate a 128-row tile would need):
  *                     warp 0       bulk copies of right tiles into a 3-stage ring
- *                     warp 1       one thread issues the MMAs
+ *                     warp 1       issues the MMAs
  *                     warps 2-9    decode h and o from the rows' 2-bit codes into the stages,
  *                                  a thread per row
  *                     warps 10-17  after a chunk: tcgen05.ld, combine, atomics
@@ -42,15 +51,16 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <math.h>
 
 #include "gp_geno_tc.h"
 #include "gp_internal.h"
 #include "gp_tc.cuh"
 
 #define EX_ROWS 256                    /* tile rows: two 128-row accumulators */
-#define EX_J 48                        /* tile columns (samples) */
-#define EX_S 5                         /* digits */
-#define EX_N (EX_J * EX_S)             /* MMA columns */
+#define EX_N 240                       /* MMA columns: digits x samples */
+#define EX_J(S) (EX_N / (S))           /* tile columns (samples) with S digits: 48 or 40 */
+#define EX_BITS(S) (12 * (S) - 1)      /* bits below the scale */
 #define EX_K 64                        /* SNPs per k-block */
 #define EX_A_BYTES (128 * EX_K * 2)
 #define EX_B_BYTES (EX_N * EX_K * 2)   /* 30,720: a multiple of the swizzle's 1,024 */
@@ -62,7 +72,7 @@
 #define EX_THREADS (64 + 32 * (EX_DEC_WARPS + EX_EPI_WARPS))
 #define EX_SMEM (EX_STAGES * EX_STAGE_BYTES + 1024 + 256)
 #define EX_PF 4                        /* k-blocks of codes a decoder loads ahead */
-#define EX_TILE (EX_ROWS * EX_J)       /* elements of a tile's sums */
+#define EX_TILE(S) (EX_ROWS * EX_J(S)) /* elements of a tile's sums */
 #define EX_D1 256                      /* TMEM column of the second accumulator */
 /* right operand per pass over it: bounds the scratch memory, and a pass of a 5,000-sample
  * panel still has 21,000 SNPs */
@@ -75,18 +85,19 @@
 
 /* ---- tiles of the lower triangle ------------------------------------------------------ */
 
-/* 48-column tiles of tile row bi: those that start at or before its last row */
-__host__ __device__ __forceinline__ int32_t ex_row_tiles(int32_t bi, int32_t n)
+/* J-column tiles of tile row bi: those that start at or before its last row */
+__host__ __device__ __forceinline__ int32_t ex_row_tiles(int32_t bi, int32_t n, int32_t J)
 {
   int32_t last = (bi + 1) * EX_ROWS < n ? (bi + 1) * EX_ROWS : n;
-  return (last + EX_J - 1) / EX_J;
+  return (last + J - 1) / J;
 }
 
+template <int S>
 __device__ __forceinline__ void ex_tile(int32_t t, int32_t n, int32_t *bi, int32_t *jt)
 {
   int32_t b = 0;
   for (;;) {
-    const int32_t c = ex_row_tiles(b, n);
+    const int32_t c = ex_row_tiles(b, n, EX_J(S));
     if (t < c) break;
     t -= c;
     ++b;
@@ -96,96 +107,127 @@ __device__ __forceinline__ void ex_tile(int32_t t, int32_t n, int32_t *bi, int32
 }
 
 /* which 128-row halves of a tile hold an entry of the lower triangle */
+template <int S>
 __device__ __forceinline__ void ex_halves(int32_t bi, int32_t jt, int32_t n, bool *h0, bool *h1)
 {
-  *h0 = bi * EX_ROWS + 127 >= jt * EX_J;
+  *h0 = bi * EX_ROWS + 127 >= jt * EX_J(S);
   *h1 = bi * EX_ROWS + 128 < n;
 }
 
 /* ---- digits ---------------------------------------------------------------------------- */
 
-__device__ __forceinline__ int ex_exponent(const unsigned long long *mx)
+/* per block of the grid the largest |R| of its SNPs (a killed SNP's table is zero) */
+__global__ void __launch_bounds__(256)
+k_exact_max(int32_t ncols, const double *__restrict__ vtab, const double *__restrict__ xfancy,
+            double *part)
 {
-  const double v = __longlong_as_double((long long)*mx);
-  int e = 0;
-  if (v > 0.0) frexp(v, &e); /* v < 2^e */
-  return e;
-}
-
-__global__ void k_exact_max(const int32_t *__restrict__ kept, int32_t nkept,
-                            const int32_t *__restrict__ cols, const double *__restrict__ vtab,
-                            const double *__restrict__ xfancy, int32_t *snprec,
-                            unsigned long long *mx)
-{
+  __shared__ double sm[8];
   double m = 0.0;
-  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nkept; k += gridDim.x * blockDim.x) {
-    const int32_t c = kept[k];
-    snprec[k] = cols[c];
+  for (int32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncols; c += gridDim.x * blockDim.x) {
     const double f = fmax(fabs(xfancy[c]), fabs(vtab[4 * (int64_t)c + 1]));
     for (int g = 0; g < 3; ++g) m = fmax(m, f * fabs(vtab[4 * (int64_t)c + g]));
   }
   for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.0)
-    atomicMax(mx, (unsigned long long)__double_as_longlong(m));
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) m = fmax(m, sm[w]);
+    part[blockIdx.x] = m;
+  }
+}
+
+/* the record index of each kept SNP; the sums cleared (nsums: an even count) */
+__global__ void k_exact_begin(const int32_t *__restrict__ kept, int32_t nkept,
+                              const int32_t *__restrict__ cols, int32_t *snprec,
+                              unsigned long long *sums, int64_t nsums)
+{
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t k = t; k < nkept; k += step) snprec[k] = cols[kept[k]];
+  for (int64_t i = t; i < nsums / 2; i += step) ((ulonglong2 *)sums)[i] = make_ulonglong2(0, 0);
+}
+
+/* the lower S - 1 of S balanced digits of 12 bits into h[first + 1 ..], the rest of N into h[first] */
+template <int S>
+__device__ __forceinline__ void ex_cut(long long N, __half *h)
+{
+#pragma unroll
+  for (int t = S - 1; t >= 1; --t) {
+    const int d = (int)((N + 2048) & 4095) - 2048;
+    h[t] = __int2half_rn(d);
+    N = (N - d) >> 12; /* exact */
+  }
+  h[0] = __int2half_rn((int)N); /* at most 2048: |R| < 2^E */
 }
 
 /*
  * One CTA per k-block (blockIdx.x, kept SNPs kb0*64 + 64 x ..) and group of EX_SJT right tiles.
  * The digits of the block's SNPs for every code are cut once into shared memory (per SNP and
- * code five words: term 1's digits 0-4 and term 2's); a thread then takes 8 SNPs of one sample
- * and writes the ten 16-byte pieces of its rows; 8 neighbouring threads complete a 128-byte
- * line.  The octets of SNPs are 164 words apart, 4 banks, so that the 8 threads of a line read
- * different banks.  Writing 20 bytes per genotype to HBM bounds it.
+ * code S words: term 1's digits and term 2's); a thread then takes 8 SNPs of one sample
+ * and writes the 2 S 16-byte pieces of its rows; 8 neighbouring threads complete a 128-byte
+ * line.  The octets of SNPs are 164 (196) words apart, 4 banks, so that the 8 threads of a line
+ * read different banks.  Writing 4 S bytes per genotype to HBM bounds it.
  */
 #define EX_SJT 8
-#define EX_OCT 164
-__global__ void __launch_bounds__(384)
+#define EX_OCT(S) (32 * (S) + 4)
+template <int S>
+__global__ void __launch_bounds__(8 * EX_J(S))
 k_exact_slices(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t ntj,
                const int32_t *__restrict__ kept, int32_t nkept, const double *__restrict__ vtab,
-               const double *__restrict__ xfancy, const unsigned long long *__restrict__ mx,
-               int32_t kb0, uint8_t *__restrict__ B)
+               const double *__restrict__ xfancy, int e, int32_t kb0, uint8_t *__restrict__ B)
 {
-  __shared__ uint32_t tab[8 * EX_OCT];
+  __shared__ uint32_t tab[8 * EX_OCT(S)];
   const int tid = threadIdx.x;
   const int32_t kb = kb0 + (int32_t)blockIdx.x;
   {
-    /* entry (SNP u, term st, code g): 384 entries, one per thread; code 3 stays zero */
-    for (int i = tid; i < 8 * EX_OCT; i += blockDim.x) tab[i] = 0;
+    for (int i = tid; i < 8 * EX_OCT(S); i += blockDim.x) tab[i] = 0;
     __syncthreads();
-    const int u = tid / 6, st = (tid / 3) & 1, g = tid % 3;
-    const int32_t k = kb * EX_K + u;
-    if (k < nkept) {
+    /* entry (SNP u, term st, code g); code 3 stays zero */
+    for (int i = tid; i < 6 * EX_K; i += blockDim.x) {
+      const int u = i / 6, st = (i / 3) & 1, g = i % 3;
+      const int32_t k = kb * EX_K + u;
+      if (k >= nkept) continue;
       const int64_t c = kept[k];
-      const double v = vtab[4 * c + g], r = (st ? vtab[4 * c + 1] : xfancy[c]) * v;
-      /* r 2^(59 - E): a power of two within range for any table of this path */
-      long long N = __double2ll_rn(scalbn(r, 59 - ex_exponent(mx)));
-      __half *h = (__half *)(tab + (u >> 3) * EX_OCT + (u & 7) * 20 + g * 5) + 5 * st;
-#pragma unroll
-      for (int t = 4; t >= 1; --t) {
-        const int d = (int)((N + 2048) & 4095) - 2048;
-        h[t] = __int2half_rn(d);
-        N = (N - d) >> 12; /* exact */
+      const double v = vtab[4 * c + g];
+      __half *h = (__half *)(tab + (u >> 3) * EX_OCT(S) + (u & 7) * (4 * S) + g * S) + S * st;
+      if (S == 5) {
+        /* R 2^(59 - E): a power of two within range for any table of this path */
+        const double r = (st ? vtab[4 * c + 1] : xfancy[c]) * v;
+        ex_cut<5>(__double2ll_rn(scalbn(r, EX_BITS(5) - e)), h);
+      } else {
+        /* f, or T1 = T0 + f or T2 - f by TwoSum (Knuth), and R by the FMA's exact product, each as
+         * a sum a + al; R 2^(35 - E) = N + (the part of R 2^(71 - E) below it), three digits each */
+        double a = xfancy[c], al = 0.0;
+        if (st) {
+          const double t0 = vtab[4 * c], t2 = vtab[4 * c + 2];
+          const double x = fabs(t0) <= fabs(t2) ? t0 : t2, y = fabs(t0) <= fabs(t2) ? a : -a;
+          a = x + y;
+          const double z = a - x;
+          al = (x - (a - z)) + (y - z);
+        }
+        const double r = __dmul_rn(a, v), rl = fma(al, v, fma(a, v, -r));
+        const double w = scalbn(r, 35 - e), N = rint(w);
+        ex_cut<3>((long long)N, h);
+        ex_cut<3>(__double2ll_rn(fma(w - N, 0x1p36, scalbn(rl, 71 - e))), h + 3);
       }
-      h[0] = __int2half_rn((int)N); /* at most 2048: |r| < 2^E */
     }
   }
   __syncthreads();
   const int o = tid & 7, jj = tid >> 3;
-  const uint32_t *to = tab + o * EX_OCT;
+  const uint32_t *to = tab + o * EX_OCT(S);
   const int32_t jt1 = min(ntj, ((int32_t)blockIdx.y + 1) * EX_SJT);
   for (int32_t jt = (int32_t)blockIdx.y * EX_SJT; jt < jt1; ++jt) {
-    const int32_t j = jt * EX_J + jj;
+    const int32_t j = jt * EX_J(S) + jj;
     /* codes 8o..8o+7 of the block: bytes 2o, 2o+1 of the row's 16, MSB first */
     uint32_t cw = 0xFFFFu;
     if (j < n) cw = *(const uint16_t *)(codes + (int64_t)j * ldc + (int64_t)kb * 16 + 2 * o);
-    uint32_t out[10][4];
+    uint32_t out[2 * S][4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const int b0 = (p >> 1) * 8 + 6 - 4 * (p & 1);
-      const uint32_t *e0 = to + (2 * p) * 20 + ((cw >> b0) & 3u) * 5;
-      const uint32_t *e1 = to + (2 * p + 1) * 20 + ((cw >> (b0 - 2)) & 3u) * 5;
+      const uint32_t *e0 = to + (2 * p) * (4 * S) + ((cw >> b0) & 3u) * S;
+      const uint32_t *e1 = to + (2 * p + 1) * (4 * S) + ((cw >> (b0 - 2)) & 3u) * S;
 #pragma unroll
-      for (int w = 0; w < 5; ++w) {
+      for (int w = 0; w < S; ++w) {
         const uint32_t x = e0[w], y = e1[w];
         out[2 * w][p] = __byte_perm(x, y, 0x5410);
         out[2 * w + 1][p] = __byte_perm(x, y, 0x7632);
@@ -193,9 +235,9 @@ k_exact_slices(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_
     }
     uint8_t *dst = B + ((int64_t)blockIdx.x * ntj + jt) * (2 * EX_B_BYTES);
 #pragma unroll
-    for (int d = 0; d < 10; ++d) {
-      const int r = (d % EX_S) * EX_J + jj;
-      *(uint4 *)(dst + (d / EX_S) * EX_B_BYTES + r * 128 + ((o ^ (r & 7)) << 4)) =
+    for (int d = 0; d < 2 * S; ++d) {
+      const int r = (d % S) * EX_J(S) + jj;
+      *(uint4 *)(dst + (d / S) * EX_B_BYTES + r * 128 + ((o ^ (r & 7)) << 4)) =
           make_uint4(out[d][0], out[d][1], out[d][2], out[d][3]);
     }
   }
@@ -223,6 +265,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r)
       : "r"(taddr));
 }
 
+template <int S>
 __global__ void __launch_bounds__(EX_THREADS, 1)
 k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t ntiles, int32_t ntj,
              int32_t kb0, int32_t nkb, int32_t ksplit, const uint8_t *__restrict__ B,
@@ -262,7 +305,7 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
     bool ok = true;
     for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
       int32_t bi, jt;
-      ex_tile(w % ntiles, n, &bi, &jt);
+      ex_tile<S>(w % ntiles, n, &bi, &jt);
       const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
       for (int32_t kb = a; kb < b && ok; ++kb) {
         const uint8_t *src = B + ((int64_t)kb * ntj + jt) * (2 * EX_B_BYTES);
@@ -296,8 +339,8 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
     for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
       int32_t bi, jt;
       bool h0, h1;
-      ex_tile(w % ntiles, n, &bi, &jt);
-      ex_halves(bi, jt, n, &h0, &h1);
+      ex_tile<S>(w % ntiles, n, &bi, &jt);
+      ex_halves<S>(bi, jt, n, &h0, &h1);
       const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
       for (int32_t c0 = a; c0 < b && ok; c0 += EX_CHUNK_KB, ++chunk) {
         const int32_t c1 = min(b, c0 + EX_CHUNK_KB);
@@ -339,8 +382,8 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
     for (int32_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
       int32_t bi, jt;
       bool h0, h1;
-      ex_tile(w % ntiles, n, &bi, &jt);
-      ex_halves(bi, jt, n, &h0, &h1);
+      ex_tile<S>(w % ntiles, n, &bi, &jt);
+      ex_halves<S>(bi, jt, n, &h0, &h1);
       const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
       const int32_t grow = bi * EX_ROWS + r;
       const bool half_on = r < 128 ? h0 : h1, live = half_on && grow < n;
@@ -398,12 +441,12 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
       int32_t bi, jt;
       bool h0, h1;
       const int32_t tile = w % ntiles;
-      ex_tile(tile, n, &bi, &jt);
-      ex_halves(bi, jt, n, &h0, &h1);
+      ex_tile<S>(tile, n, &bi, &jt);
+      ex_halves<S>(bi, jt, n, &h0, &h1);
       const int32_t a = w / ntiles * kb_per, b = min(nkb, a + kb_per);
       /* column u of this warp's 32 rows, all lanes together; upper sums, then lower */
       unsigned long long *out =
-          sums + (int64_t)tile * (2 * EX_TILE) + (half * 4 + q) * (EX_J * 32) + lane;
+          sums + (int64_t)tile * (2 * EX_TILE(S)) + (half * 4 + q) * (EX_J(S) * 32) + lane;
       for (int32_t c0 = a; c0 < b; c0 += EX_CHUNK_KB, ++chunk) {
         const bool got = mbar_wait(accf, chunk & 1u, abort_flag, err, EXERR_ACCF);
         if (!__all_sync(0xffffffffu, got)) {
@@ -413,19 +456,21 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
         tc_fence_after();
         if (half ? h1 : h0) {
 #pragma unroll
-          for (int g = 0; g < EX_J / 8; ++g) {
-            uint32_t d[EX_S][8];
+          for (int g = 0; g < EX_J(S) / 8; ++g) {
+            uint32_t d[S][8];
 #pragma unroll
-            for (int t = 0; t < EX_S; ++t) tmem_ld8(t_acc + t * EX_J + 8 * g, d[t]);
+            for (int t = 0; t < S; ++t) tmem_ld8(t_acc + t * EX_J(S) + 8 * g, d[t]);
             tmem_wait_ld();
 #pragma unroll
             for (int v = 0; v < 8; ++v) {
-              long long S[EX_S];
+              long long hi = 0, lo = 0;
 #pragma unroll
-              for (int t = 0; t < EX_S; ++t) S[t] = __float2int_rn(__uint_as_float(d[t][v]));
+              for (int t = 0; t < 3; ++t) hi = (hi << 12) + __float2int_rn(__uint_as_float(d[t][v]));
+#pragma unroll
+              for (int t = 3; t < S; ++t) lo = (lo << 12) + __float2int_rn(__uint_as_float(d[t][v]));
               const int at = (8 * g + v) * 32;
-              atomicAdd(out + at, (unsigned long long)((S[0] << 24) + (S[1] << 12) + S[2]));
-              atomicAdd(out + EX_TILE + at, (unsigned long long)((S[3] << 12) + S[4]));
+              atomicAdd(out + at, (unsigned long long)hi);
+              atomicAdd(out + EX_TILE(S) + at, (unsigned long long)lo);
             }
           }
         }
@@ -451,30 +496,29 @@ k_gram_exact(const uint8_t *__restrict__ codes, int64_t ldc, int32_t n, int32_t 
 }
 
 /*
- * XTX[i][j] = XTX[j][i] = 2^(E-59) (2^24 hi + lo) for the tile's entries of the lower triangle;
- * a CTA per 128 rows x 24 columns, transposed through shared memory so that both the row
- * pieces (24 doubles) and the column pieces (128 doubles) are written contiguously.
+ * XTX[i][j] = XTX[j][i] = 2^(E-59) (2^24 hi + lo), or 2^(E-71) (2^36 hi + lo) with six digits,
+ * for the tile's entries of the lower triangle; a CTA per 128 rows x half of the columns, transposed through shared memory so that both the row
+ * pieces (24 or 20 doubles) and the column pieces (128 doubles) are written contiguously.
  */
-#define EX_FC (EX_J / 2)
+template <int S>
 __global__ void __launch_bounds__(256)
-k_exact_finish(const unsigned long long *__restrict__ sums, const unsigned long long *__restrict__ mx,
-               int32_t n, double *x)
+k_exact_finish(const unsigned long long *__restrict__ sums, int e, int32_t n, double *x)
 {
+  constexpr int EX_FC = EX_J(S) / 2;
   __shared__ double sm[128][EX_FC + 1];
   int32_t bi, jt;
-  ex_tile((int32_t)blockIdx.x, n, &bi, &jt);
+  ex_tile<S>((int32_t)blockIdx.x, n, &bi, &jt);
   const int half = (int)blockIdx.y, jh = (int)blockIdx.z;
-  const int32_t i0 = bi * EX_ROWS + 128 * half, j0 = jt * EX_J + jh * EX_FC;
+  const int32_t i0 = bi * EX_ROWS + 128 * half, j0 = jt * EX_J(S) + jh * EX_FC;
   bool h0, h1;
-  ex_halves(bi, jt, n, &h0, &h1);
+  ex_halves<S>(bi, jt, n, &h0, &h1);
   if (!(half ? h1 : h0)) return;
-  const int e = ex_exponent(mx) - 59;
   for (int p = threadIdx.x; p < 128 * EX_FC; p += blockDim.x) {
     const int lane = p & 31, c = (p >> 5) % EX_FC, q = (p >> 5) / EX_FC;
-    const unsigned long long *src = sums + (int64_t)blockIdx.x * (2 * EX_TILE) +
-                                    (half * 4 + q) * (EX_J * 32) + (jh * EX_FC + c) * 32 + lane;
-    const double hi = (double)(long long)src[0], lo = (double)(long long)src[EX_TILE];
-    sm[q * 32 + lane][c] = scalbn(fma(hi, 0x1p24, lo), e);
+    const unsigned long long *src = sums + (int64_t)blockIdx.x * (2 * EX_TILE(S)) +
+                                    (half * 4 + q) * (EX_J(S) * 32) + (jh * EX_FC + c) * 32 + lane;
+    const double hi = (double)(long long)src[0], lo = (double)(long long)src[EX_TILE(S)];
+    sm[q * 32 + lane][c] = scalbn(fma(hi, S == 5 ? 0x1p24 : 0x1p36, lo), e - EX_BITS(S));
   }
   __syncthreads();
   for (int p = threadIdx.x; p < 128 * EX_FC; p += blockDim.x) {
@@ -509,28 +553,44 @@ static int32_t ex_split(int32_t ntiles, int32_t nkb, int32_t sms)
   return best;
 }
 
-int gp_gram_exact(gp_ctx *ctx)
+/*
+ * Digits for a largest |R| below 2^e over nk SNPs.  The rounding of R leaves an entry an error of
+ * about 2^(e-61) sqrt(nk), a sequence of FP64 additions 2^-55 nk (their partial sums are about
+ * sqrt(nk) with the SNPs' signs mixed): five digits where the first is at most half of the second.
+ * Panels of common SNPs (e = 6 or 7) take five from 16 SNPs on.  Six cost 1.2 times the MMAs: 5,003
+ * samples x 20,000 SNPs with frequencies from 2e-4 on 4.66 ms, of 3.97, and 2,003 x 20,011 0.91, of
+ * 0.78.
+ */
+static int ex_digits(int e, int32_t nk) { return 2 * (e - 5) <= ilogb((double)nk) ? 5 : 6; }
+
+int gp_gram_exact_max(gp_ctx *ctx, double *d_part)
+{
+  k_exact_max<<<GP_EXACT_PARTS, 256, 0, ctx->stream>>>(ctx->ncols, ctx->d_vtab, ctx->d_xfancy, d_part);
+  GP_LAUNCH_CHECK(ctx, "k_exact_max");
+  return GP_OK;
+}
+
+template <int S>
+static int gram_exact(gp_ctx *ctx, int e)
 {
   const int32_t n = ctx->nrows, nk = ctx->nkept;
-  const int32_t ntj = (n + EX_J - 1) / EX_J, nkb = (nk + EX_K - 1) / EX_K;
+  const int32_t ntj = (n + EX_J(S) - 1) / EX_J(S), nkb = (nk + EX_K - 1) / EX_K;
   int32_t ntiles = 0;
-  for (int32_t b = 0; b * EX_ROWS < n; ++b) ntiles += ex_row_tiles(b, n);
-  uint8_t *base, *B;
+  for (int32_t b = 0; b * EX_ROWS < n; ++b) ntiles += ex_row_tiles(b, n, EX_J(S));
+  uint8_t *B;
   unsigned long long *sums;
   int32_t *snprec;
   int rc = gp_scratch(ctx, sizeof(int32_t) * (size_t)nk, (void **)&snprec);
   if (rc) return rc;
-  const size_t sum_bytes = sizeof(*sums) * 2 * EX_TILE * (size_t)ntiles;
-  rc = gp_scratch5(ctx, 256 + sum_bytes, (void **)&base);
+  const size_t sum_bytes = sizeof(*sums) * 2 * EX_TILE(S) * (size_t)ntiles;
+  rc = gp_scratch5(ctx, sum_bytes, (void **)&sums);
   if (rc) return rc;
-  unsigned long long *mx = (unsigned long long *)base; /* ahead of the sums: one memset */
-  sums = mx + 32;
   /* the right operand of as many k-blocks as fit the budget, fewer where memory is short */
   const size_t per_kb = 2 * EX_B_BYTES * (size_t)ntj;
   int32_t kbp = (int32_t)(EX_BUDGET / (int64_t)per_kb);
   {
-    const char *e = getenv("GP_EXACT_BUDGET_BYTES"); /* tests: several passes on a small panel */
-    if (e && atoll(e) > 0) kbp = (int32_t)(atoll(e) / (int64_t)per_kb);
+    const char *env = getenv("GP_EXACT_BUDGET_BYTES"); /* tests: several passes on a small panel */
+    if (env && atoll(env) > 0) kbp = (int32_t)(atoll(env) / (int64_t)per_kb);
   }
   if (kbp < 1) kbp = 1;
   if (kbp > nkb) kbp = nkb;
@@ -542,33 +602,43 @@ int gp_gram_exact(gp_ctx *ctx)
   }
   if (rc) return rc;
 
-  GP_CUDA(ctx, cudaMemsetAsync(mx, 0, 256 + sum_bytes, ctx->stream));
   rc = gp_tc_begin(ctx);
   if (rc) return rc;
-  int blocks = (nk + 255) / 256;
-  if (blocks > ctx->num_sms * 4) blocks = ctx->num_sms * 4;
-  k_exact_max<<<blocks, 256, 0, ctx->stream>>>(ctx->d_kept, nk, ctx->d_cols, ctx->d_vtab,
-                                               ctx->d_xfancy, snprec, mx);
-  GP_LAUNCH_CHECK(ctx, "k_exact_max");
+  const int64_t nsums = (int64_t)(sum_bytes / sizeof(*sums));
+  const int64_t work = nsums / 2 > nk ? nsums / 2 : nk;
+  const int64_t blocks = (work + 255) / 256 < ctx->num_sms * 16 ? (work + 255) / 256 : ctx->num_sms * 16;
+  k_exact_begin<<<(unsigned)blocks, 256, 0, ctx->stream>>>(ctx->d_kept, nk, ctx->d_cols, snprec, sums,
+                                                          nsums);
+  GP_LAUNCH_CHECK(ctx, "k_exact_begin");
   gp_tc_codes A;
   rc = gp_tc_codes_for(ctx, 1, ctx->d_rows, n, snprec, nk, 1, &A);
   if (rc) return rc;
-  GP_CUDA(ctx, cudaFuncSetAttribute(k_gram_exact, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  GP_CUDA(ctx, cudaFuncSetAttribute(k_gram_exact<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     EX_SMEM));
   for (int32_t kb0 = 0; kb0 < nkb; kb0 += kbp) {
     const int32_t cur = nkb - kb0 < kbp ? nkb - kb0 : kbp;
     dim3 sg((unsigned)cur, (unsigned)((ntj + EX_SJT - 1) / EX_SJT));
-    k_exact_slices<<<sg, 384, 0, ctx->stream>>>(A.codes, A.ldc, n, ntj, ctx->d_kept, nk,
-                                                ctx->d_vtab, ctx->d_xfancy, mx, kb0, B);
+    k_exact_slices<S><<<sg, 8 * EX_J(S), 0, ctx->stream>>>(A.codes, A.ldc, n, ntj, ctx->d_kept, nk,
+                                                          ctx->d_vtab, ctx->d_xfancy, e, kb0, B);
     GP_LAUNCH_CHECK(ctx, "k_exact_slices");
     const int32_t ks = ex_split(ntiles, cur, ctx->num_sms);
     const int32_t items = ntiles * ks;
-    k_gram_exact<<<items < ctx->num_sms ? items : ctx->num_sms, EX_THREADS, EX_SMEM, ctx->stream>>>(
+    k_gram_exact<S><<<items < ctx->num_sms ? items : ctx->num_sms, EX_THREADS, EX_SMEM,
+                      ctx->stream>>>(
         A.codes, A.ldc, n, ntiles, ntj, kb0, cur, ks, B, sums, ctx->d_err);
     GP_LAUNCH_CHECK(ctx, "k_gram_exact");
     ctx->gram_launches++;
   }
-  k_exact_finish<<<dim3((unsigned)ntiles, 2, 2), 256, 0, ctx->stream>>>(sums, mx, n, ctx->d_xtx);
+  k_exact_finish<S><<<dim3((unsigned)ntiles, 2, 2), 256, 0, ctx->stream>>>(sums, e, n, ctx->d_xtx);
   GP_LAUNCH_CHECK(ctx, "k_exact_finish");
   return GP_OK;
+}
+
+int gp_gram_exact(gp_ctx *ctx, const double *part)
+{
+  double big = 0.0;
+  for (int i = 0; i < GP_EXACT_PARTS; ++i) big = part[i] > big ? part[i] : big;
+  int e = 0;
+  if (big > 0.0) frexp(big, &e); /* big < 2^e */
+  return ex_digits(e, ctx->nkept) == 5 ? gram_exact<5>(ctx, e) : gram_exact<6>(ctx, e);
 }

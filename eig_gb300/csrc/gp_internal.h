@@ -38,7 +38,7 @@ struct gp_ctx {
 
   /* per-column state of the last gp_xtx */
   int32_t *d_cnt;        /* [3*ncols]: n0, n1, nmiss */
-  uint8_t *d_killed;     /* [ncols] */
+  uint8_t *d_killed;     /* [ncols], then the exact Gram's partial maxima */
   double *d_vtab;        /* [4*ncols]: value of code 0,1,2,3(missing)=0 */
   double *d_xmean;       /* [ncols] */
   double *d_xfancy;      /* [ncols] */
@@ -180,8 +180,16 @@ int gp_lsq_fill_tables(gp_ctx *ctx, const int32_t *d_samp, const int32_t *d_spop
 int gp_gram_fp64(gp_ctx *ctx);
 /* the FP64 Gram as exact integer sums on the tensor cores (both triangles written), queued on
  * ctx->stream: gp_tc_check reports its bounded waits; needs at least one kept SNP and no
- * population fill; GP_ERR_NOMEM leaves the Gram untouched */
-int gp_gram_exact(gp_ctx *ctx);
+ * population fill; GP_ERR_NOMEM leaves the Gram untouched.  part [GP_EXACT_PARTS] (host): the
+ * partial maxima that gp_gram_exact_max queues on the stream, which set its scale */
+#define GP_EXACT_PARTS 128
+/* bytes of d_killed: a flag per column, then the partial maxima */
+static inline size_t gp_killed_bytes(int32_t ncols)
+{
+  return ((size_t)ncols + 7) / 8 * 8 + sizeof(double) * GP_EXACT_PARTS;
+}
+int gp_gram_exact_max(gp_ctx *ctx, double *d_part);
+int gp_gram_exact(gp_ctx *ctx, const double *part);
 int gp_gram_split(gp_ctx *ctx, int precision);
 /* the trace of the Gram; its upper triangle is filled first unless `symmetric` */
 int gp_launch_symmetrize_trace(gp_ctx *ctx, double *d_trace, bool symmetric);

@@ -773,9 +773,9 @@ extern "C" int64_t gp_smartpca_footprint(int32_t nind, int64_t nsnp, int32_t pre
   int64_t work;
   if (precision == GP_PREC_FP64) {
     /* lsqproject's panel of pair products and its slices (256 columns at a time), the SNP-major
-     * sums of the weights, or the exact Gram: its right operand (20 bytes per genotype, at most
+     * sums of the weights, or the exact Gram: its right operand (20 or 24 bytes per genotype, at most
      * 2 GiB at a time), integer sums and sample-major codes */
-    int64_t slices = 20 * (n + 48) * (m + 64);
+    int64_t slices = 24 * (n + 48) * (m + 64);
     if (slices > (int64_t)2 << 30) slices = (int64_t)2 << 30;
     const int64_t cols5 = 5 * (k * (k + 1) / 2 + 1) < 1280 ? 5 * (k * (k + 1) / 2 + 1) + 127 : 1280;
     if (slices < 2 * m * cols5) slices = 2 * m * cols5;

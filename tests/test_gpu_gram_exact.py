@@ -73,3 +73,54 @@ def test_passes_give_the_same_bits(gpu, monkeypatch):
     one = check(gpu, rec, rows, cols, n)
     monkeypatch.setenv("GP_EXACT_BUDGET_BYTES", str(5 * 7 * 61440))
     assert np.array_equal(check(gpu, rec, rows, cols, n), one)
+
+
+def values(rec, n, alt=1):
+    """(tables [m][4], codes [m][n], kept) by the oracle"""
+    m = len(rec)
+    s = O.pass_columns(rec, np.arange(m, dtype=np.int32), np.arange(n, dtype=np.int32),
+                       altnormstyle=alt)
+    code = O.unpack(rec, n)
+    return s.tab.reshape(-1, 4), np.where(code < 0, 3, code), s.killed == 0, s.xfancy
+
+
+# panels whose rarest allele is seen once and that take six digits: edges of the 40-column tiles, of
+# the 64-SNP blocks and of a chunk of 4,096 SNPs; a cohort of several thousand samples
+@pytest.mark.parametrize("n,m", [(39, 60), (40, 63), (41, 50), (81, 65), (255, 64), (257, 130),
+                                 (601, 4160), (5003, 600)])
+def test_rare_variants(gpu, n, m, monkeypatch):
+    r = np.random.default_rng(n + m)
+    p = 0.5 * (1.0 / n) ** r.random(m)
+    p = np.where(r.random(m) < 0.5, p, 1 - p)
+    g = (r.random((m, n)) < p[:, None]).astype(np.int8) + (r.random((m, n)) < p[:, None])
+    g[r.random((m, n)) < 0.03] = -1
+    g[0], g[0, n // 2], g[1], g[1, n // 3] = 0, 1, 2, 1
+    g[2, ::2], g[2, 1::2] = 0, 1
+    rec = O.pack(g)
+    gpu.load_genotypes(rec, n)
+    gpu.set_samples(np.arange(n, dtype=np.int32))
+    gpu.set_snps(np.arange(m, dtype=np.int32))
+    got = gpu.xtx(altnormstyle=1)["XTX"]
+    tab, code, keep, fancy = values(rec, n)
+    v = np.take_along_axis(tab, code, axis=1)
+    # some rows against all samples, in long double
+    q = np.unique(np.r_[0, n // 3, n // 2, n - 1, r.choice(n, min(n, 36), replace=False)])
+    X = np.zeros((len(q), n), np.longdouble)
+    for a in range(0, m, 64):
+        X += v[a:a + 64, q].T.astype(np.longdouble) @ v[a:a + 64].astype(np.longdouble)
+    X = X.astype(float)
+    # the value of the more frequent homozygote (T0 or T2) enters as it is, the others as it plus or
+    # minus f: two roundings of their own and one of its; 72 bits below the scale for each term; the
+    # combination and the rounding of the result
+    base = np.where(np.abs(tab[:, 0]) <= np.abs(tab[:, 2]), 0, 2)
+    other = (code != base[:, None]) & (code != 3) & keep[:, None]
+    a = np.where(other, 2 * np.abs(v) + np.abs(tab[np.arange(m), base])[:, None], 0.0)
+    u = 2.0 ** -53
+    f = np.maximum(np.abs(fancy), np.abs(tab[:, 1])) * keep
+    scale = 2.0 * np.max(f[:, None] * np.abs(tab))
+    tol = (u * (a[:, q].T @ np.abs(v) + np.abs(v[:, q]).T @ a) + 4 * u * np.abs(X)
+           + 2 * m * 2.0 ** -72 * scale)
+    assert np.all(np.abs(got[q] - X) <= tol)
+    assert np.array_equal(got, got.T)
+    monkeypatch.setenv("GP_EXACT_BUDGET_BYTES", str(((n + 39) // 40) * 61440))
+    assert np.array_equal(gpu.xtx(altnormstyle=1)["XTX"], got)
