@@ -147,9 +147,9 @@ __device__ __forceinline__ double x_scaled(long long z, int e)
  * (kb % kb_period)*16, taken as allele counts or as the observed mask by count_lo for kb <
  * kb_period and count_hi otherwise (the concatenated-k form [G | O]).  tn: slice columns per tile; nct column tiles.
  * sums: per row tile, slice column (nct * tn of them) and row of the tile the exact integer
- * sum, added atomically.  With Y (ksplit 1 and 4 slices) the item that has all of a row's sums
- * writes the products themselves, Y[row][column] by mx, the columns' largest magnitudes: the
- * slices' sums make one 64-bit integer, kept in Y's place between chunks.  No buffer of sums
+ * sum, added atomically.  With Y (ksplit 1, 4 slices, gp_tc_sums_fit) the item that has all of a
+ * row's sums writes the products themselves, Y[row][column] by mx, the columns' largest magnitudes:
+ * the slices' sums make one 64-bit integer, kept in Y's place between chunks.  No buffer of sums
  * is cleared, added to and read again (200,000 x 20 products over 5,000 samples: 0.40 -> 0.30 ms).
  */
 __global__ void __launch_bounds__(X_THREADS, 1)
@@ -955,7 +955,7 @@ int gp_tc_apply(gp_ctx *ctx, const gp_tc_codes *A, const gp_tc_prepared *P, doub
   const int32_t nkb = P->kb0 * P->npanels;
   const int32_t tiles = (nrows + XR - 1) / XR * P->nct;
   const int32_t ksplit = x_split(tiles, nkb, ctx->num_sms);
-  const bool whole = ksplit == 1 && P->digits == 4;
+  const bool whole = ksplit == 1 && P->digits == 4 && gp_tc_sums_fit((int64_t)nkb * XK);
   unsigned long long *sums = NULL;
   if (!whole) {
     const size_t sum_bytes = gp_tc_sum_bytes(P->digits * P->ncols, nrows);

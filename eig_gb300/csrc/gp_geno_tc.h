@@ -48,6 +48,9 @@ size_t gp_tc_prepared_bytes(int npanels, int32_t ncols, int32_t k0, int digits);
 /* slice the panels into caller storage of gp_tc_prepared_bytes bytes (device) */
 int gp_tc_prepare(gp_ctx *ctx, int npanels, const gp_tc_panel *pp, int32_t ncols, int32_t k0,
                   int digits, void *storage, gp_tc_prepared *out);
+/* whether a row's four slice sums over k values (of all panels) fit one 64-bit integer: a term is at
+ * most a count of 2 times 2^40 */
+static inline bool gp_tc_sums_fit(int64_t k) { return k <= (int64_t)1 << 21; }
 /* Y[r][c] = products of the code operand with a prepared panel, queued on ctx->stream.  Its
  * bounded waits report through ctx->d_err: gp_tc_begin clears it ahead of any number of
  * products, gp_tc_check waits for them and returns the error */
