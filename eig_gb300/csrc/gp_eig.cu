@@ -981,24 +981,24 @@ __device__ __forceinline__ ff2 ff_add_lazy(ff2 a, ff2 b)
   return ff_make(s, __fadd_rn(__fadd_rn(a.l, b.l), er));
 }
 /*
- * A float-float value that carries its step: each half next to the step's tag in a 64-bit word
- * (64-bit accesses are not torn), so that a reader polls for the value itself and needs no
- * barrier, fence or second trip to L2 for it.  Tags are c + 1 for values of step c, never 0.
+ * A float-float value that carries its step: each half next to the step's tag in a 64-bit word, so
+ * that a reader polls for the value itself and needs no barrier, fence or second trip to L2 for it.
+ * The two words are the elements of one vector access: each is read and written whole, in no
+ * order between them, so the reader looks at both tags.  Tags are c + 1 for values of step c,
+ * never 0.
  */
 __device__ __forceinline__ void tag_store(uint4 *p, ff2 v, unsigned tag)
 {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p),
-               "r"(__float_as_uint(v.h)), "r"(tag), "r"(__float_as_uint(v.l)), "r"(tag)
+  const unsigned long long t = (unsigned long long)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p),
+               "l"(t | __float_as_uint(v.h)), "l"(t | __float_as_uint(v.l))
                : "memory");
 }
 __device__ __forceinline__ uint4 tag_load(const uint4 *p)
 {
-  uint4 r;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(p)
-               : "memory");
-  return r;
+  unsigned long long h, l;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(h), "=l"(l) : "l"(p) : "memory");
+  return make_uint4((unsigned)h, (unsigned)(h >> 32), (unsigned)l, (unsigned)(l >> 32));
 }
 
 /*
