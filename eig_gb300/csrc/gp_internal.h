@@ -132,8 +132,8 @@ int gp_realloc(gp_ctx *ctx, void **ptr, size_t bytes);
  * inside the copy (72 MB of 64 KB pages: 4 ms, of which the copy itself is 0.5; 3,001-sample Gram
  * 6.0 -> 4.8 ms, 125 MB of converted records 6.4 -> 3.4).  gp_out_pages has a few
  * threads bring the pages in while the device computes; gp_copy_out copies a piece as soon as
- * its pages are there.  The contents are not touched; pinned or small destinations are left
- * alone.  The threads end with the object.
+ * its pages are there.  The contents are not touched; destinations that are pinned, small or there
+ * already are left alone.  The threads end with the object.
  */
 struct gp_out_pages {
   gp_out_pages(void *dst, size_t bytes);
