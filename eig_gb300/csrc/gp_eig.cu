@@ -989,16 +989,22 @@ __device__ __forceinline__ ff2 ff_add_lazy(ff2 a, ff2 b)
  */
 __device__ __forceinline__ void tag_store(uint4 *p, ff2 v, unsigned tag)
 {
-  const unsigned long long t = (unsigned long long)tag << 32;
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p),
-               "l"(t | __float_as_uint(v.h)), "l"(t | __float_as_uint(v.l))
-               : "memory");
+  asm volatile(
+      "{\n\t.reg .b64 h, l;\n\tmov.b64 h, {%1, %3};\n\tmov.b64 l, {%2, %3};\n\t"
+      "st.relaxed.gpu.global.v2.b64 [%0], {h, l};\n\t}\n" ::"l"(p),
+      "r"(__float_as_uint(v.h)), "r"(__float_as_uint(v.l)), "r"(tag)
+      : "memory");
 }
 __device__ __forceinline__ uint4 tag_load(const uint4 *p)
 {
-  unsigned long long h, l;
-  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(h), "=l"(l) : "l"(p) : "memory");
-  return make_uint4((unsigned)h, (unsigned)(h >> 32), (unsigned)l, (unsigned)(l >> 32));
+  uint4 r;
+  asm volatile(
+      "{\n\t.reg .b64 h, l;\n\tld.relaxed.gpu.global.v2.b64 {h, l}, [%4];\n\t"
+      "mov.b64 {%0, %1}, h;\n\tmov.b64 {%2, %3}, l;\n\t}\n"
+      : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+      : "l"(p)
+      : "memory");
+  return r;
 }
 
 /*
