@@ -9,7 +9,7 @@
  *   2. all eigenvalues of T by multisection on Sturm counts (the published bisection method:
  *      the count of negative pivots of the LDL^T factorisation of T - x I equals the number
  *      of eigenvalues below x), several lanes per eigenvalue index: FP32 brackets first,
- *      then float-float, checked and finished in FP64 to 1e-13 ||T||;
+ *      then float-float, checked and finished in FP64 to 3e-14 ||T|| (1e-13 above 6,080);
  *   3. the top nvec eigenvectors of T by inverse iteration, one block per vector: LU with
  *      partial pivoting of the tridiagonal T - lambda I (Gaussian elimination with row
  *      interchanges) and three solves from a fixed pseudo-random start, then modified
@@ -227,7 +227,7 @@ __device__ __forceinline__ int sturm_count_ff(const float *dh, const float *dl, 
  * narrow the bracket to ~4e-7 ||T|| (widened by 64 eps_32 ||T||), float-float counts on the
  * FP32 pipe narrow it to ~1e-12 ||T|| (widened by 16 2^-44 ||T||).  The first FP64 count takes
  * the bracket's ends among its points, which checks it (back to the Gershgorin bracket if that
- * fails), and FP64 counts narrow it to tol: n = 5,000 8.2 ms, of 10.1, and 1,000 0.95, of
+ * fails), and FP64 counts narrow it to tol: n = 5,000 9.2 ms, of 10.1, and 1,000 0.95, of
  * 1.13, with a check of its own and a bracket four times as wide.  (Three points per lane in
  * the FP32 and float-float phases took longer, 12.0 and 1.5 ms: they are bound by issue.)
  * Grid: one CTA of 4 warps per SM; d, e2 and their FP32 hi/lo copies in shared memory
@@ -2915,10 +2915,13 @@ int gp_eig_sym(gp_ctx *ctx, double *A_in, int32_t n, int32_t nvec, double *d_eva
     const int P = 32 / epw;
     const int nwarps = (n + epw - 1) / epw;
     const int blocks = (nwarps + 3) / 4;
-    /* FP64 brackets end at 1e-13 ||T||: the counts' own backward error is ~6e-14 ||T||.  Half a
-     * bracket is the error, and with 32 points the check alone can end at 0.9e-13 (4e-14 measured
-     * for orders up to 608, 1e-14 with a step more): narrower where a step is cheap */
-    const double tol = (P >= 16 ? 3e-14 : 1e-13) * tnorm;
+    /* Half of the last FP64 bracket is the error, and how wide it gets depends on the points a step
+     * has: with a limit of 1e-13 ||T|| the largest error over all eigenvalues was 3.5e-14 of the norm
+     * at 2,500 and 5.1e-14 at 3,600 and 5,000, with 3e-14 it is 0.8e-14, 0.9e-14 and 1.3e-14 for
+     * 3.5 ms of 2.9, 5.3 of 4.6 and 9.2 of 8.2 (orders to 1,800 are the same).  With fewer than three
+     * points (orders above 6,080) a step costs more, 14.7 ms of 13.4 at 6,200, for less: 1e-13 there,
+     * 4.9e-14 */
+    const double tol = (P >= 3 ? 3e-14 : 1e-13) * tnorm;
     if (use_smem)
       GP_CUDA(ctx, gp_allow_smem(ctx, (const void *)k_multisect));
     k_multisect<<<blocks, 128, use_smem ? smem : 0, ctx->stream>>>(d, e2, n, gl, gu, tnorm, pivmin,
