@@ -877,7 +877,9 @@ def tridiag_roofline(res, peaks, peak_kind):
             "note": "DRAM traffic is below the algorithmic bytes: the tiled lower triangle "
                     "(103 MB at N=5,000) mostly stays in L2; the tiled steps are bound by "
                     "the FP32 pipe (53 operations per lower-triangle element and step) and "
-                    "a step's chain of phase A, part sums and the grid barrier",
+                    "a step's chain: y and the column from L2, the vectors, the part sums and "
+                    "their arrivals.  traffic: captured with a grid barrier in every step "
+                    "(profiles/tridiag_tiled_5000_dram.md), the same tiles and parts",
             "peak_kind": "HBM copy, %s" % peak_kind}
 
 

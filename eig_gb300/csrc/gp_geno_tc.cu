@@ -3,8 +3,8 @@
  *
  *   Y[r][c] = sum_k A_r(k) P[k][c]
  *
- * A_r(k) is a small integer decoded from a 2-bit genotype code through a 4-entry table
- * (observed mask {1,1,1,0} or allele count {0,1,2,0}); P is an FP64 panel.  Each column of
+ * A_r(k) is a small integer decoded from a 2-bit genotype code (observed mask {1,1,1,0} or
+ * allele count {0,1,2,0}); P is an FP64 panel.  Each column of
  * P is scaled by a power of two 2^e_c >= max|P[.][c]| and cut into 4 fixed-point slices,
  * x = P/2^e_c = sum_t q_t 1024^-(t+1) with |q_0| <= 1024 and |q_t| <= 512 (t > 0): integers
  * that fp16 holds exactly.  A tensor-core MMA of {0,1,2} by such integers over at most 8,192
@@ -16,7 +16,7 @@
  * The FP64 precision's products take 5 slices of 12 bits (x = sum_t q_t 2^-(11 + 12 t),
  * |q_t| <= 2048, at most 4,096 k values per chunk): an error of 2^-60 of the column maximum,
  * below what FP64 additions in sequence leave, for 5/4 of the MMAs.  They replace the FP64
- * pipe's products (1,501 x 80,003, K = 10, weights and lsqproject: 59.4 ms there, 2.5 here).
+ * pipe's products (1,501 x 80,003, K = 10, weights and lsqproject: 59.4 ms there, 1.56 here).
  *
  * This is how the masked per-sample normal equations of lsqproject (regressit
  * src/regsubs.c:19-26, lsqproj src/eigensrc/smartpca.c:4690-4712), the sample scores fxvecs
@@ -30,8 +30,8 @@
  * B tile and k range they stream and B is read from DRAM about once per wave instead of once
  * per row tile):
  *   warp 0      TMA of the B tile (slice columns x 64 k, fp16, 128-byte swizzle), 3 stages;
- *   warp 1      one thread issues 2 x 4 tcgen05.mma (128 x N x 16, f16 -> f32) per k-block:
- *               the tile's two 128-row halves share the B tile;
+ *   warp 1      issues 2 x 4 tcgen05.mma (128 x N x 16, f16 -> f32) per k-block, converged, one
+ *               elected lane each: the tile's two 128-row halves share the B tile;
  *   warps 2-9   decode the A tile, a thread per row: 16 bytes of codes (the next four
  *               k-blocks' loads in flight) become 64 fp16 values in the same swizzled layout;
  *               then fence.proxy.async and one arrival per warp;
@@ -114,8 +114,9 @@ __host__ __device__ __forceinline__ int32_t x_split(int32_t tiles, int32_t nkb, 
   return best;
 }
 
-/* a column's power of two from the bits of its largest magnitude; X_NONFINITE (5 slices) for an
- * infinity or NaN */
+/* exponent e_c with max|P| < 2^e_c (frexp) from the bits of a column's largest magnitude, 0 for an
+ * all-zero column; with 5 slices X_NONFINITE for one with an infinity or NaN (its products are NaN,
+ * as FP64 products of 0 and it are) */
 #define X_NONFINITE (-(1 << 30))
 template <int S>
 __device__ __forceinline__ int x_exponent(unsigned long long mx)
@@ -126,13 +127,6 @@ __device__ __forceinline__ int x_exponent(unsigned long long mx)
   return e;
 }
 
-/*
- * The slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
- * narrow): N = rint(x 2^F) from the double's mantissa and exponent (round half to even), F = 40
- * with S = 4 slices of 10 bits, 59 with 5 of 12, then balanced digits from the bottom: all but
- * the first in [-2^(b-1), 2^(b-1) - 1], d_0 = the rest (at most 1024 = 2^(40-30) or
- * 2048 = 2^(59-48) since |N| <= 2^F), so that x = sum_t d_t 2^(b(S-1-t) - F) + O(2^-F-1).
- */
 /* z 2^(e - 40), rounded once: what k_panel_combine<4> makes of the slices' sums */
 __device__ __forceinline__ double x_scaled(long long z, int e)
 {
@@ -628,9 +622,13 @@ __global__ void k_panel_absmax(const x_panels pan, int32_t nk, int32_t ncols,
     if (smx[i]) atomicMax(mx + i, smx[i]);
 }
 
-/* exponent e_c with max|P| < 2^e_c (frexp) of a column's mx, 0 for an all-zero column; with 5
- * slices X_NONFINITE for one with an infinity or NaN (its products are NaN, as FP64 products of
- * 0 and it are) */
+/*
+ * The slices of x = sign P / 2^e_c (|x| < 1) in integer arithmetic (GB300's FP64 pipe is
+ * narrow): N = rint(x 2^F) from the double's mantissa and exponent (round half to even), F = 40
+ * with S = 4 slices of 10 bits, 59 with 5 of 12, then balanced digits from the bottom: all but
+ * the first in [-2^(b-1), 2^(b-1) - 1], d_0 = the rest (at most 1024 = 2^(40-30) or
+ * 2048 = 2^(59-48) since |N| <= 2^F), so that x = sum_t d_t 2^(b(S-1-t) - F) + O(2^-F-1).
+ */
 template <int S>
 __device__ __forceinline__ void slice(double v, int e, bool neg, int d[S])
 {

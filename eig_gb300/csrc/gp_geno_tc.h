@@ -26,10 +26,10 @@ struct gp_tc_codes {
   int32_t k0;
 };
 
-/* inv: room for nind_all integers when the samples of a sum over SNPs are distinct (the faster
- * transpose then applies), or NULL */
 /* bytes of the code operand built by gp_tc_build_codes: rows_pad * ldc */
 int gp_tc_code_bytes(int sum_over_snps, int32_t nsamp, int32_t nk, int64_t *ldc, int32_t *rows_pad);
+/* the code operand of the samples d_samp, in any order, into codes.  inv: room for nind_all integers
+ * when the samples of a sum over SNPs are distinct (the faster transpose then applies), or NULL */
 int gp_tc_build_codes(gp_ctx *ctx, int sum_over_snps, const int32_t *d_samp, int32_t nsamp,
                       const int32_t *d_snprec, int32_t nk, int32_t *inv, uint8_t *codes,
                       gp_tc_codes *out);

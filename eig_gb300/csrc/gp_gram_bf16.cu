@@ -21,9 +21,9 @@
  * Kernel structure (persistent, one CTA per SM, 18 warps):
  *   warp 0      TMA producer: per k-block of 64 SNPs four 16 KB boxes (A hi/lo, B hi/lo)
  *               into a 3-stage shared-memory ring;
- *   warp 1      allocates 512 TMEM columns; one thread issues 12 (or 16) tcgen05.mma
- *               (128x128x16) per k-block into FP32 accumulator buffer (chunk & 1),
- *               columns 0-255;
+ *   warp 1      allocates 512 TMEM columns; issues 12 (or 16) tcgen05.mma (128x128x16) per
+ *               k-block, converged, one elected lane each, into FP32 accumulator buffer
+ *               (chunk & 1), columns 0-255;
  *   warps 2-17  epilogue: at the end of each chunk read the FP32 buffer (tcgen05.ld),
  *               release it and add it into registers; every GP_FOLD chunks fold those into
  *               the (hi, lo) running sums in TMEM columns 256-511; after the last chunk of a

@@ -61,7 +61,14 @@ const char *gp_last_error(const gp_ctx *ctx);
 int gp_open(int device, gp_ctx **out);
 void gp_close(gp_ctx *ctx);
 
-/* Device memory the handle currently holds, in bytes. */
+/*
+ * Device memory the handle currently holds, in bytes.  A handle keeps its panel, results and the
+ * workspaces of its calls, each as large as its largest call needed, until gp_release or gp_close:
+ * gp_xtx at FP64 up to 2 GiB of digits, about 8 N^2 bytes of integer sums and N M / 4 of codes, in
+ * the split precisions up to 24 GiB of operands, gp_fastpca 8 (I + 1) L (M + N) bytes and some panels of
+ * 8 L M (55,000 x 500,000, L 20, I 10: about 9 GB).  A caller that shares the device with others
+ * gives them back with gp_release.
+ */
 int gp_device_bytes(const gp_ctx *ctx, int64_t *bytes);
 
 /*
