@@ -503,10 +503,10 @@ __device__ __forceinline__ ff2 ff_dot2(ff2 a, ff2 x, ff2 b, ff2 y)
 }
 
 /* acc += a x with the accumulator left unnormalised (acc.h the running TwoSum of the high
- * products, acc.l every lower-order term): 12 FP32 operations against 15 for ff_fma.  acc.l takes
- * an FP32 rounding of the lower-order terms per step, so over the dots here (a lane's share of a
- * tile row, 40 terms at order 5,000 and 90 at 7,600; of a column in shared memory at most 27) its
- * error stays of the order of the normalised accumulation's, which rounds the whole pair each time.
+ * products, acc.l every lower-order term): 12 FP32 operations against 15 for ff_fma.  The dots here
+ * take some 40 terms (a lane's share of a tile row at order 5,000; at most 27 of a column in shared
+ * memory); normalising the tiled ones every 4, 8 or 16 terms changed neither the eigenvalues' error
+ * nor the vectors' residuals in the third digit (orders 2,500 to 5,000) and took 0.5 ms of 93.
  * ff_renorm makes the pair normalised again. */
 __device__ __forceinline__ ff2 ff_acc_lazy(ff2 acc, ff2 a, ff2 x)
 {
